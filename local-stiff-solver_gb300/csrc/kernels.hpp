@@ -170,6 +170,10 @@ struct MasDev {
     const int32_t *cbase[MAS_MAXL] = {};
     const uint8_t *ccnt[MAS_MAXL] = {};
     int32_t ncoarse = 0;                // total coarse banks
+    const int32_t *cmap = nullptr;      // (L-1) x nb: item of every node at level l = 1 .. L-1
+    const unsigned *need = nullptr;     // per coarse bank: banks of the level below that hold its items' parts
+    const uint8_t *uncoupled = nullptr; // per coarse bank: no couplings between its items
+    unsigned *arrive = nullptr;         // per coarse bank: arrivals of the running apply (zero between applies)
     int64_t tile_elems = 0;             // inverse elements per bank
     int64_t bank_bytes0 = 0;            // > 0: level-0 banks hold FP32 diagonal and BF16 off-diagonal tiles, this stride
     int64_t level_elems = 0;            // elements of the level-vector buffers
@@ -192,9 +196,10 @@ struct CoarseMembers {
 // partial: nchunk * bd * bd * 32 doubles of scratch
 void launch_mas_assemble_coarse(const BsrDev &A, const MasDev &m, const int32_t *cmap /* nb*(L-1) */,
                                 const CoarseMembers &mb, double *partial, double *stage, cudaStream_t s);
-// pad zero diagonals, invert (symmetric sweep), write bank tiles (FP32 or FP64)
+// pad zero diagonals, invert (symmetric sweep), write bank tiles (FP32 or FP64);
+// uncoupled (optional): per bank, 1 if no entry couples two of its items
 void launch_mas_invert(int bd, int64_t nbanks, const double *stage, void *out, bool fp32, int *bad,
-                       cudaStream_t s, bool bf16_offdiag = false);
+                       cudaStream_t s, uint8_t *uncoupled = nullptr, bool bf16_offdiag = false);
 // bytes of one bank with FP32 diagonal and BF16 off-diagonal tiles
 int64_t mas_bank_bytes_bf16(int bd);
 // z = MAS^-1 xin (acc: z += MAS^-1 xin).  dot_mode 1: st->gamma = rdot.z;

@@ -11,11 +11,11 @@
 // 32 x 32 tiles (c, c2), c <= c2; tile element [d][r] holds
 // Inv[c*32 + r][c2*32 + (r+d) % 32], d = 0..16 for diagonal tiles (d = 16 kept
 // twice, so 17*32 entries = the packed-triangle size plus 16) and d = 0..31 for
-// off-diagonal tiles.  A warp owns a bank, lane r owns row r of every tile:
-// every tile load is one 128-byte (FP32) / 256-byte (FP64) coalesced line,
-// and the symmetric partner term travels by warp shuffle instead of being
-// stored twice.  The inverse streams from HBM once per apply with evict-first
-// loads; residual and coarse vectors stay in L2.
+// off-diagonal tiles.  Row r of a tile is at lane r of every 32-entry line,
+// so a warp's access to a tile, direct or transposed, is 32 consecutive or
+// rotated words (128 bytes in FP32, 256 in FP64): one half of the symmetric
+// matrix is stored and read from HBM, both halves of the product run from
+// shared memory.  Residual and coarse vectors stay in L2.
 #include <cuda_bf16.h>
 
 #include <type_traits>
@@ -30,103 +30,72 @@ int64_t mas_bank_bytes_bf16(int bd) { return (int64_t)bd * 17 * 32 * 4 + (int64_
 
 namespace {
 
-constexpr unsigned FULL = 0xffffffffu;
-
 template <int BD>
 __host__ __device__ constexpr int64_t tile_elems() { return (int64_t)BD * 17 * 32 + (int64_t)BD * (BD - 1) / 2 * 1024; }
 
-template <typename T>
-__device__ __forceinline__ T ld_stream(const T *p) { return __ldcs(p); }
-
-// y = Inv x for one bank; lane r holds x[c] = x_{c*32+r}.
-template <int BD, typename T>
-__device__ __forceinline__ void tile_symv(const T *__restrict__ tile, const T (&x)[BD], T (&y)[BD], int lane)
+// The bank product y = Inv x, split over warps.  With x in shared memory,
+// output row r (= lane) of component c1 takes, for every component c and
+// rotation e = 0..31, Inv[c1*32 + r][c*32 + (r+e) % 32] * x[c*32 + (r+e) % 32].
+// That entry is tile (c1, c)[e][r] for c1 <= c (e <= 16 on the diagonal) and,
+// by symmetry, tile (c, c1)[32 - e][(r+e) % 32] otherwise: both a conflict-free
+// (coalesced) access of 32 consecutive or rotated words, so neither operand nor
+// product moves by shuffle and every multiply-add is one FMA.  (The shuffled
+// form, one warp per bank, spent 429 FP64 instructions and two shuffles per
+// entry on a 96 x 96 bank against 288 FMAs here, in one dependent chain: 42 us
+// for a handful of FP64 banks.)
+//
+// ROTS rotations starting at e0; BF: off-diagonal tiles in BF16 words.
+template <int BD, int ROTS, bool BF, typename T, typename Ld>
+__device__ __forceinline__ void bank_rows(const Ld &ld, const T *__restrict__ xs, int e0, int lane, T (&y)[BD])
 {
 #pragma unroll
     for (int c = 0; c < BD; ++c) y[c] = T(0);
-    const T *__restrict__ t = tile;
+#pragma unroll 4
+    for (int q = 0; q < ROTS; ++q) {
+        const int e = e0 + q, idx = (lane + e) & 31, t = (32 - e) & 31;
 #pragma unroll
-    for (int c = 0; c < BD; ++c) {
-        {
-            T a = ld_stream(t + lane);
-            y[c] += a * x[c];
+        for (int c = 0; c < BD; ++c) {
+            const T x = xs[c * 32 + idx];
 #pragma unroll
-            for (int d = 1; d < 16; ++d) {
-                a = ld_stream(t + d * 32 + lane);
-                const T xs = __shfl_sync(FULL, x[c], (lane + d) & 31);
-                y[c] += a * xs;
-                const T tr = a * x[c];
-                y[c] += __shfl_sync(FULL, tr, (lane - d) & 31);
+            for (int c1 = 0; c1 < BD; ++c1) {
+                // element offset of tile (lo, hi), row-major over c <= c2
+                const int lo = c1 < c ? c1 : c, hi = c1 < c ? c : c1;
+                const int ndiag = hi == lo ? lo : lo + 1;  // diagonal tiles before this one
+                const int noff = lo * (BD - 1) - lo * (lo - 1) / 2 + (hi > lo ? hi - lo - 1 : 0);
+                const int off = hi == lo ? (e <= 16 ? e * 32 + lane : t * 32 + idx)
+                                         : (c1 < c ? e * 32 + lane : t * 32 + idx);
+                y[c1] += ld(ndiag, noff, hi == lo, off) * x;
             }
-            a = ld_stream(t + 16 * 32 + lane);
-            y[c] += a * __shfl_xor_sync(FULL, x[c], 16);
-            t += 17 * 32;
-        }
-#pragma unroll
-        for (int c2 = c + 1; c2 < BD; ++c2) {
-#pragma unroll 8
-            for (int d = 0; d < 32; ++d) {
-                const T a = ld_stream(t + d * 32 + lane);
-                const T xs = __shfl_sync(FULL, x[c2], (lane + d) & 31);
-                y[c] += a * xs;
-                const T tr = a * x[c];
-                y[c2] += __shfl_sync(FULL, tr, (lane - d) & 31);
-            }
-            t += 32 * 32;
         }
     }
 }
 
-// tile_symv for a bank whose diagonal tiles are FP32 and whose off-diagonal
-// tiles (c < c2) are BF16 (the same order: for each c, tile (c, c) then the
-// tiles (c, c2 > c)).  In a BF16 tile, 32-bit word k * 32 + r holds the
-// entries [2k][r] (low half) and [2k + 1][r] (high half), so every warp load
-// is still one 128-byte line; a BF16 value widens to FP32 exactly by a shift.
-template <int BD>
-__device__ __forceinline__ void tile_symv_bf(const unsigned char *__restrict__ bank, const float (&x)[BD],
-                                             float (&y)[BD], int lane)
-{
-#pragma unroll
-    for (int c = 0; c < BD; ++c) y[c] = 0.f;
-    const unsigned char *t = bank;
-#pragma unroll
-    for (int c = 0; c < BD; ++c) {
-        {
-            const float *__restrict__ dt = reinterpret_cast<const float *>(t);
-            float a = ld_stream(dt + lane);
-            y[c] += a * x[c];
-#pragma unroll
-            for (int d = 1; d < 16; ++d) {
-                a = ld_stream(dt + d * 32 + lane);
-                const float xs = __shfl_sync(FULL, x[c], (lane + d) & 31);
-                y[c] += a * xs;
-                const float tr = a * x[c];
-                y[c] += __shfl_sync(FULL, tr, (lane - d) & 31);
-            }
-            a = ld_stream(dt + 16 * 32 + lane);
-            y[c] += a * __shfl_xor_sync(FULL, x[c], 16);
-            t += 17 * 32 * sizeof(float);
+// entry loaders: tile (ndiag diagonal and noff off-diagonal tiles before it)
+template <typename T, bool BF>
+struct TileLd {
+    const unsigned char *base;
+    __device__ __forceinline__ T operator()(int ndiag, int noff, bool diag, int off) const
+    {
+        if (BF) {
+            const unsigned char *t = base + ndiag * (17 * 32 * 4) + noff * 2048;
+            if (diag) return (T) reinterpret_cast<const float *>(t)[off];
+            // word (d / 2) * 32 + r holds entries d (low half) and d + 1 (high half)
+            const int d = off >> 5, r = off & 31;
+            const unsigned h = reinterpret_cast<const unsigned short *>(t)[(d >> 1) * 64 + 2 * r + (d & 1)];
+            return (T)__uint_as_float(h << 16);
         }
-#pragma unroll
-        for (int c2 = c + 1; c2 < BD; ++c2) {
-            const unsigned int *__restrict__ ot = reinterpret_cast<const unsigned int *>(t);
-#pragma unroll 4
-            for (int k = 0; k < 16; ++k) {
-                const unsigned int w = __ldcs(ot + k * 32 + lane);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int d = 2 * k + h;
-                    const float a = __uint_as_float(h ? (w & 0xffff0000u) : (w << 16));
-                    const float xs = __shfl_sync(FULL, x[c2], (lane + d) & 31);
-                    y[c] += a * xs;
-                    const float tr = a * x[c];
-                    y[c2] += __shfl_sync(FULL, tr, (lane - d) & 31);
-                }
-            }
-            t += 32 * 32 * sizeof(unsigned short);
-        }
+        return (reinterpret_cast<const T *>(base) + ndiag * (17 * 32) + noff * 1024)[off];
     }
+};
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // ------------------------------------------------------------------ setup
 
@@ -340,21 +309,24 @@ __device__ void sweep_invert(double *S, int ld, double *col, double *scol, int *
 
 template <int BD, typename T, bool BF>
 __global__ void __launch_bounds__(256, 2) mas_invert_kernel(const double *__restrict__ stage, T *__restrict__ out,
-                                                         int *bad)
+                                                         int *bad, uint8_t *__restrict__ uncoupled)
 {
     constexpr int N = 32 * BD, LD = N + 1;
     extern __shared__ double sm[];
     double *S = sm, *col = sm + N * LD, *scol = col + N;
     const int64_t bank = blockIdx.x;
     const double *src = stage + bank * N * N;
+    bool coupled = false;  // an entry between two different items of the bank
     for (int idx = threadIdx.x; idx < N * N; idx += blockDim.x) {
         const int r = idx / N, c = idx % N;
         if (r > c) continue;  // the upper triangle is all the sweep uses
         double v = src[(int64_t)r * N + c];
+        coupled |= ((r ^ c) & 31) != 0 && v != 0.0;
         if (r == c && v == 0.0) v = 1.0;  // padding (MASPreconditioner.cu:779-796)
         S[r * LD + c] = v;
     }
-    __syncthreads();
+    coupled = __syncthreads_or(coupled);
+    if (uncoupled && threadIdx.x == 0) uncoupled[bank] = coupled ? 0 : 1;
     sweep_invert<N>(S, LD, col, scol, bad);
     // the swept entry (i, j), i <= j
     auto entry = [&](int i, int j) -> double { return S[i * LD + j]; };
@@ -397,174 +369,300 @@ __global__ void __launch_bounds__(256, 2) mas_invert_kernel(const double *__rest
 
 // Segmented sums of one bank: 32 items (values staged item-major in xs, the
 // target aggregate of each item in ks) into ncc aggregates.  Output slot
-// s = k * BD + c (aggregate k, component c) belongs to lane s % 32, which adds
-// the items of aggregate k in item order: no FP64 shuffles (each costs 16
-// cycles of the SM's FP64 pipe on this part), a fixed summation order, and in
-// FP32 mode no FP64 instruction at all.
+// s = k * BD + c (aggregate k, component c) belongs to a group of P lanes, P
+// the largest power of two with ncc * BD * P <= 32 (1 beyond): lane q of the
+// group adds the items j = q, q + P, ... of aggregate k and the group's sums
+// meet by shuffles, in one fixed order.  An FP64 add costs the pipe a whole
+// warp however few lanes take part: with one aggregate (a connected
+// partition) this is 4 + 3 adds instead of 32.
 template <int BD, typename T>
 __device__ __forceinline__ void bank_segment_sums(const T *xs, const uint8_t *ks, int ncc, T *__restrict__ out,
                                                   int lane)
 {
-    for (int sl = lane; sl < ncc * BD; sl += 32) {
-        const int k = sl / BD, c = sl - k * BD;
+    const int slots = ncc * BD;
+    int lg = 0;
+    while (lg < 5 && (slots << (lg + 1)) <= 32) ++lg;
+    const int P = 1 << lg, sub = lane & (P - 1);
+    for (int s0 = 0; s0 < slots; s0 += 32 >> lg) {
+        const int sl = s0 + (lane >> lg), k = sl / BD, c = sl - k * BD;
         T acc = T(0);
+        if (sl < slots) {
 #pragma unroll 8
-        for (int j = 0; j < 32; ++j)
-            if (ks[j] == k) acc += xs[j * BD + c];
-        out[(int64_t)k * BD + c] = acc;
+            for (int j = sub; j < 32; j += P)
+                if (ks[j] == k) acc += xs[j * BD + c];
+        }
+        for (int o = P >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (sl < slots && sub == 0) out[sl] = acc;
     }
 }
 
-// level 0 -> level 1: per-part component sums of r
+// The restriction of r to every coarse level in one launch.
+//
+// A warp sums one partition's rows into its level-1 items and then reports to
+// the level-1 banks that hold them (arrive[g], at most two banks).  The warp
+// whose report is a bank's last queues it in its CTA, whose warps restrict the
+// queued banks to the next level the same way.  Nothing waits: whoever
+// completes a bank continues with it, and each sum has one fixed order whoever
+// runs it.  Level by level this took L - 1 launches of 5 to 11 us each, nearly
+// all latency.  (The products of the ready banks stay in a launch of their
+// own: run here, by the CTA that completes a bank, they pile up on the few
+// CTAs that hold a clamped face -- 235 us instead of 100 on 648k DOFs.)
 template <int BD, typename T, typename XT>
-__global__ void __launch_bounds__(256) restrict0_kernel(MasDev m, const XT *__restrict__ r, T *__restrict__ v,
-                                                        const int *done)
+__global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__restrict__ r, T *__restrict__ v,
+                                                       const int *done)
 {
     if (done && *done) return;
-    __shared__ T xs_all[8][32 * BD];
-    __shared__ uint8_t ks_all[8][32];
+    constexpr int N = 32 * BD, W = 8;
+    __shared__ T xs_all[W][N];
+    __shared__ uint8_t ks_all[W][32];
+    // ready banks, level << 28 | bank: at most 16 level-1 banks per round and
+    // twice the previous level's at each of up to five further levels
+    __shared__ unsigned queue[1024];
+    __shared__ int qn;
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     T *xs = xs_all[wl];
     uint8_t *ks = ks_all[wl];
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    T *v1 = v + m.voff[1];
-    for (int64_t p = w0; p < m.nparts; p += nw) {
-        const int32_t lo = m.part_off[p], cnt = m.part_off[p + 1] - lo;
-        // the part's values are one contiguous run: coalesced loads
-#pragma unroll
-        for (int q = 0; q < BD; ++q) {
-            const int e = q * 32 + lane;
-            xs[e] = e < cnt * BD ? (T)r[(int64_t)lo * BD + e] : T(0);
+    if (threadIdx.x == 0) qn = 0;
+    __syncthreads();
+    // reports items [i0, i0 + cnt) of level l as written; queues completed banks
+    auto report = [&](int l, int32_t i0, int cnt) {
+        __threadfence();
+        __syncwarp();
+        if (lane < 2 && cnt > 0) {
+            const int32_t b0 = i0 >> 5, b1 = (i0 + cnt - 1) >> 5, b = b0 + lane;
+            if (b <= b1) {
+                const int32_t g = m.boff[l] + b;
+                if (atomicAdd(m.arrive + g, 1u) + 1u == m.need[g]) {
+                    m.arrive[g] = 0u;
+                    __threadfence();
+                    queue[atomicAdd(&qn, 1)] = (unsigned)l << 28 | (unsigned)b;
+                }
+            }
         }
-        ks[lane] = lane < cnt ? m.key0[lo + lane] : (uint8_t)0xff;
         __syncwarp();
-        bank_segment_sums<BD, T>(xs, ks, m.ccnt0[p], v1 + (int64_t)m.cbase0[p] * BD, lane);
-        __syncwarp();
+    };
+    for (int64_t p0 = (int64_t)blockIdx.x * W; p0 < m.nparts; p0 += (int64_t)gridDim.x * W) {
+        const int64_t p = p0 + wl;
+        if (p < m.nparts) {
+            const int32_t lo = m.part_off[p], cnt = m.part_off[p + 1] - lo;
+            // the part's values are one contiguous run: coalesced loads
+#pragma unroll
+            for (int q = 0; q < BD; ++q) {
+                const int e = q * 32 + lane;
+                xs[e] = e < cnt * BD ? (T)r[(int64_t)lo * BD + e] : T(0);
+            }
+            ks[lane] = lane < cnt ? m.key0[lo + lane] : (uint8_t)0xff;
+            const int32_t i0 = m.cbase0[p];
+            const int nc = m.ccnt0[p];
+            __syncwarp();
+            bank_segment_sums<BD, T>(xs, ks, nc, v + m.voff[1] + (int64_t)i0 * BD, lane);
+            report(1, i0, nc);
+        }
+        __syncthreads();
+        int head = 0, n = qn;
+        while (head < n) {
+            for (int k = head + wl; k < n; k += W) {
+                const int l = (int)(queue[k] >> 28);
+                if (l + 1 >= m.L) continue;
+                const int32_t b = (int32_t)(queue[k] & 0x0fffffffu), i0 = b * 32;
+                const int cnt = min(32, m.nitems[l] - i0);
+                const T *vl = v + m.voff[l] + (int64_t)i0 * BD;
+#pragma unroll
+                for (int q = 0; q < BD; ++q) {
+                    const int e = q * 32 + lane;
+                    xs[e] = e < cnt * BD ? __ldcg(vl + e) : T(0);
+                }
+                ks[lane] = lane < cnt ? m.key[l][i0 + lane] : (uint8_t)0xff;
+                const int32_t j0 = m.cbase[l][b];
+                const int nc = m.ccnt[l][b];
+                __syncwarp();
+                bank_segment_sums<BD, T>(xs, ks, nc, v + m.voff[l + 1] + (int64_t)j0 * BD, lane);
+                report(l + 1, j0, nc);
+            }
+            __syncthreads();
+            head = n;
+            n = qn;
+        }
+        if (threadIdx.x == 0) qn = 0;
+        __syncthreads();
     }
 }
 
-// level l -> level l+1 (l >= 1)
-template <int BD, typename T>
-__global__ void __launch_bounds__(256) restrict_kernel(MasDev m, int l, T *__restrict__ v, const int *done)
-{
-    if (done && *done) return;
-    __shared__ T xs_all[8][32 * BD];
-    __shared__ uint8_t ks_all[8][32];
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    T *xs = xs_all[wl];
-    uint8_t *ks = ks_all[wl];
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const T *vl = v + m.voff[l];
-    T *vn = v + m.voff[l + 1];
-    const uint8_t *key_l = m.key[l];
-    const uint8_t *ccnt_l = m.ccnt[l];
-    const int32_t *cbase_l = m.cbase[l];
-    const int32_t nitems = m.nitems[l];
-    for (int64_t b = w0; b < m.nbanks[l]; b += nw) {
-        const int64_t i0 = b * 32;
-        const int cnt = nitems - i0 < 32 ? (int)(nitems - i0) : 32;
-#pragma unroll
-        for (int q = 0; q < BD; ++q) {
-            const int e = q * 32 + lane;
-            xs[e] = e < cnt * BD ? vl[i0 * BD + e] : T(0);
-        }
-        ks[lane] = lane < cnt ? key_l[i0 + lane] : (uint8_t)0xff;
-        __syncwarp();
-        bank_segment_sums<BD, T>(xs, ks, ccnt_l[b], vn + (int64_t)cbase_l[b] * BD, lane);
-        __syncwarp();
-    }
-}
-
-// all coarse banks: u_l = Inv_l v_l
+// u_g = Inv_g v_g for every coarse bank, one CTA of eight warps per bank: each
+// warp takes four rotations, whose loads are all in flight together (the
+// banks are few and L2-resident, so this is one latency, not a stream).  In a
+// bank without couplings between its items (uncoupled: Dirichlet rows, which
+// never merge and fill a third of the coarse banks of a clamped cube) every
+// entry off rotation 0 is an exact zero, and only that rotation is taken.
+// Level vectors are whole banks back to back: bank g starts at element g * N.
 template <int BD, typename T>
 __global__ void __launch_bounds__(256) symv_coarse_kernel(MasDev m, const T *__restrict__ invc,
                                                           const T *__restrict__ v, T *__restrict__ u,
                                                           const int *done)
 {
     if (done && *done) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t g = w0; g < m.ncoarse; g += nw) {
-        int l = 1;
-        while (l + 1 < m.L && g >= m.boff[l + 1]) ++l;
-        const int64_t b = g - m.boff[l];
-        const int64_t e0 = m.voff[l] + (b * 32 + lane) * BD;
-        T x[BD], y[BD];
+    constexpr int N = 32 * BD, W = 8;
+    __shared__ T xs[N];
+    __shared__ T red[W][N];
+    const int tid = threadIdx.x, lane = tid & 31, wl = tid >> 5;
+    const int64_t g = blockIdx.x;
+    const int o = (tid % BD) * 32 + tid / BD;  // component-major place of element tid
+    if (tid < N) xs[o] = v[g * N + tid];
+    const bool uncoupled = m.uncoupled[g];
+    __syncthreads();
+    T y[BD];
+    const TileLd<T, false> ld{reinterpret_cast<const unsigned char *>(invc + g * m.tile_elems)};
+    if (uncoupled) {
+        if (wl > 0) return;
+        bank_rows<BD, 1, false, T>(ld, xs, 0, lane, y);
 #pragma unroll
-        for (int c = 0; c < BD; ++c) x[c] = v[e0 + c];
-        tile_symv<BD, T>(invc + g * m.tile_elems, x, y, lane);
+        for (int c = 0; c < BD; ++c) u[g * N + lane * BD + c] = y[c];
+        return;
+    }
+    bank_rows<BD, 32 / W, false, T>(ld, xs, wl * (32 / W), lane, y);
 #pragma unroll
-        for (int c = 0; c < BD; ++c) u[e0 + c] = y[c];
+    for (int c = 0; c < BD; ++c) red[wl][c * 32 + lane] = y[c];
+    __syncthreads();
+    if (tid < N) {
+        T sum = red[0][o];
+#pragma unroll
+        for (int w = 1; w < W; ++w) sum += red[w][o];
+        u[g * N + tid] = sum;
     }
 }
 
-// u_1 += P (u_2 + P (u_3 + ...)): every level-1 item gathers its ancestors'
-// corrections and sums them from the top level down, as level-by-level
-// prolongation would, in one launch.
-template <int BD, typename T>
-__global__ void __launch_bounds__(256) prolong_all_kernel(MasDev m, T *__restrict__ u, const int *done)
+// level 0: z = Inv_0 x (+ the coarse corrections), optional accumulate and r.z;
+// x in FP64, or in FP32 (XT = float) when it comes from the FP32 residual.
+//
+// A CTA of four warps works on GB consecutive banks at a time (one 96-row,
+// two 64-row or four 32-row banks: the banks of one group are one contiguous
+// run of HBM).  The next groups' inverses stream into shared-memory stages by
+// 16-byte asynchronous copies while this group's product runs from its stage,
+// and the vector operands are loaded a group ahead; WB warps share a bank, each taking 32 / WB rotations, and their
+// partial sums meet in shared memory in warp order.  A node adds its
+// ancestors' coarse corrections here (cmap: its item at every level), so no
+// separate prolongation runs.
+template <int BD, bool BF>
+constexpr int bank_bytes(size_t elem)
 {
-    if (done && *done) return;
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m.nitems[1]) return;
-    int64_t item[MAS_MAXL];
-    item[1] = k;
-    for (int l = 1; l + 1 < m.L; ++l) item[l + 1] = m.cbase[l][item[l] >> 5] + m.key[l][item[l]];
-#pragma unroll
-    for (int c = 0; c < BD; ++c) {
-        T acc = u[m.voff[m.L - 1] + item[m.L - 1] * BD + c];
-        for (int l = m.L - 2; l >= 1; --l) acc = u[m.voff[l] + item[l] * BD + c] + acc;
-        u[m.voff[1] + k * BD + c] = acc;
-    }
+    return BF ? BD * 17 * 32 * 4 + BD * (BD - 1) / 2 * 2048 : (int)(tile_elems<BD>() * elem);
+}
+template <int BD>
+struct BankGroup {
+    static constexpr int WB = BD == 3 ? 4 : BD, GB = 4 / WB;
+};
+// Stages of shared memory per CTA: with four of up to 20 KB, three CTAs per SM
+// keep nine groups in flight (two stages on six CTAs kept six: 147 us against
+// 122 us at 33k FP32 banks); the larger FP64 stages are bound by the FP64
+// pipe, where five one-stage CTAs cover each other's loads.
+template <int BD, typename T, bool BF>
+constexpr int bank_stages()
+{
+    return (BF ? 4 : (int)sizeof(T)) * tile_elems<BD>() * BankGroup<BD>::GB <= 20480 ? 2 : 1;
 }
 
-// level 0: z = Inv_0 x (+ coarse correction u_1), optional accumulate and r.z;
-// x in FP64, or in FP32 (XT = float) when it comes from the FP32 residual
 template <int BD, typename T, bool ACC, int DOT, typename XT, bool BF = false>
-__global__ void __launch_bounds__(256) symv0_kernel(MasDev m, const T *__restrict__ inv0, const T *__restrict__ u,
+__global__ void __launch_bounds__(128) symv0_kernel(MasDev m, const T *__restrict__ inv0, const T *__restrict__ u,
                                                     const XT *__restrict__ xin, double *__restrict__ z,
                                                     double scale, const double *__restrict__ rdot, PcgState *st,
                                                     GridReduce gr, const int *done, float *__restrict__ z32,
                                                     float *__restrict__ z_lo)
 {
     if (done && *done) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    constexpr int N = 32 * BD, WB = BankGroup<BD>::WB, GB = BankGroup<BD>::GB;
+    constexpr int BANK_B = bank_bytes<BD, BF>(sizeof(T)), STAGE_B = BANK_B * GB, NST = bank_stages<BD, T, BF>();
+    extern __shared__ __align__(16) unsigned char stage[];
+    __shared__ T xs[GB][N];
+    __shared__ T red[4][N];
+    const int tid = threadIdx.x, lane = tid & 31, wl = tid >> 5;
+    const int64_t ngroups = (m.nparts + GB - 1) / GB;
+    const unsigned char *src = reinterpret_cast<const unsigned char *>(inv0);
+    auto fill = [&](int st_, int64_t g) {
+        const int64_t b0 = g * GB, left = m.nparts - b0;
+        const int bytes = left < GB ? (int)left * BANK_B : STAGE_B;
+        for (int k = tid * 16; k < bytes; k += 128 * 16) cp_async16(stage + st_ * STAGE_B + k, src + b0 * BANK_B + k);
+    };
+    // thread t owns vector element t % N of bank t / N of the group
+    const int bk = tid / N, el = tid % N, node = el / BD, comp = el % BD;
+    // The chain partition -> node -> items -> corrections is loaded over three
+    // groups (partition bounds two groups ahead, a node's operands and items one
+    // group ahead), so that no step waits for the one before it.
+    struct Bounds {
+        int32_t lo, hi;
+    };
+    auto bounds = [&](int64_t g) {
+        Bounds b{0, 0};
+        const int64_t p = g * GB + bk;
+        if (bk < GB && g < ngroups && p < m.nparts) b = {m.part_off[p], m.part_off[p + 1]};
+        return b;
+    };
+    struct Operand {
+        XT x;
+        double z, rd;
+        int32_t item[MAS_MAXL - 1];
+        int64_t e;  // -1: no element
+    };
+    auto operand = [&](Bounds b) {
+        Operand o;
+        const int32_t i = b.lo + node;
+        const bool ok = i < b.hi;
+        o.e = ok ? (int64_t)i * BD + comp : -1;
+        o.x = ok ? xin[o.e] : XT(0);
+        o.z = ACC && ok ? z[o.e] : 0.0;
+        o.rd = DOT && ok ? rdot[o.e] : 0.0;
+#pragma unroll
+        for (int l = 1; l < MAS_MAXL; ++l) o.item[l - 1] = ok && l < m.L ? m.cmap[(int64_t)(l - 1) * m.nb + i] : 0;
+        return o;
+    };
     double dot[1] = {0.0};
-    const T *u1 = u + m.voff[1];
-    for (int64_t p = w0; p < m.nparts; p += nw) {
-        const int32_t lo = m.part_off[p], node = lo + lane;
-        const bool valid = node < m.part_off[p + 1];
-        T x[BD], y[BD];
+    int64_t g = blockIdx.x;
+    const int64_t step = gridDim.x;
+    int cur = 0;
 #pragma unroll
-        for (int c = 0; c < BD; ++c) x[c] = valid ? (T)xin[(int64_t)node * BD + c] : T(0);
-        if constexpr (BF && std::is_same<T, float>::value)
-            tile_symv_bf<BD>(reinterpret_cast<const unsigned char *>(inv0) + p * m.bank_bytes0, x, y, lane);
-        else
-            tile_symv<BD, T>(inv0 + p * m.tile_elems, x, y, lane);
-        if (valid) {
-            int64_t cidx = -1;
-            if (m.L > 1) cidx = (int64_t)(m.cbase0[p] + m.key0[node]) * BD;
+    for (int q = 0; q < NST - 1; ++q) {
+        if (g + q * step < ngroups) fill(q, g + q * step);
+        cp_async_commit();
+    }
+    Operand o = operand(bounds(g));
+    Bounds nb = bounds(g + step);
+    for (; g < ngroups; g += step) {
+        const int64_t gf = g + (NST - 1) * step;
+        if (gf < ngroups) fill(cur + NST - 1 < NST ? cur + NST - 1 : cur - 1, gf);
+        cp_async_commit();
+        if (bk < GB) xs[bk][comp * 32 + node] = (T)o.x;
+        T cu[MAS_MAXL - 1];
 #pragma unroll
-            for (int c = 0; c < BD; ++c) {
-                double val = (double)y[c];
-                if (cidx >= 0) val += (double)u1[cidx + c];
-                val *= scale;
-                const int64_t e = (int64_t)node * BD + c;
-                if (ACC) val += z[e];
-                z[e] = val;
-                if (z32) {
-                    const float h = (float)val;
-                    z32[e] = h;
-                    if (z_lo) z_lo[e] = (float)(val - (double)h);
-                }
-                if (DOT) dot[0] += rdot[e] * val;
+        for (int l = 1; l < MAS_MAXL; ++l)
+            cu[l - 1] = o.e >= 0 && l < m.L ? u[m.voff[l] + (int64_t)o.item[l - 1] * BD + comp] : T(0);
+        const Operand nx = operand(nb);
+        nb = bounds(g + 2 * step);
+        cp_async_wait<NST - 1>();
+        __syncthreads();
+        T y[BD];
+        const TileLd<T, BF> ld{stage + cur * STAGE_B + (wl / WB) * BANK_B};
+        bank_rows<BD, 32 / WB, BF, T>(ld, xs[wl / WB], (wl % WB) * (32 / WB), lane, y);
+#pragma unroll
+        for (int c = 0; c < BD; ++c) red[wl][c * 32 + lane] = y[c];
+        __syncthreads();
+        if (o.e >= 0) {
+            T sum = red[bk * WB][comp * 32 + node];
+#pragma unroll
+            for (int w = 1; w < WB; ++w) sum += red[bk * WB + w][comp * 32 + node];
+            T corr = cu[MAS_MAXL - 2];  // top level down, as level-by-level prolongation adds them
+#pragma unroll
+            for (int l = MAS_MAXL - 2; l >= 1; --l) corr = cu[l - 1] + corr;
+            double val = ((double)sum + (double)corr) * scale;
+            if (ACC) val += o.z;
+            z[o.e] = val;
+            if (z32) {
+                const float h = (float)val;
+                z32[o.e] = h;
+                if (z_lo) z_lo[o.e] = (float)(val - (double)h);
             }
+            if (DOT) dot[0] += o.rd * val;
         }
+        o = nx;
+        cur = cur + 1 < NST ? cur + 1 : 0;
     }
     if (DOT) {
         double tot[1];
@@ -580,29 +678,44 @@ __global__ void __launch_bounds__(256) symv0_kernel(MasDev m, const T *__restric
     }
 }
 
+// Grid of a level-0 launch: every resident CTA, at most one per bank group.
+template <int BD, typename T, bool BF>
+int symv0_grid(int64_t nparts)
+{
+    constexpr int GB = BankGroup<BD>::GB;
+    constexpr int cta = bank_stages<BD, T, BF>() * bank_bytes<BD, BF>(sizeof(T)) * GB + (BD == 3 ? 4096 : 2048) + 5 * 32 * BD * (int)sizeof(T);
+    constexpr int per_sm = 227 * 1024 / cta < 12 ? 227 * 1024 / cta : 12;
+    return grid_for(nparts, GB, sm_grid(per_sm));
+}
+
+template <int BD, typename T, bool ACC, int DOT, typename XT, bool BF>
+void symv0_launch(const MasDev &m, const T *inv0, const T *u, const XT *xin, double *z, double scale,
+                  const double *rdot, PcgState *st, GridReduce gr, const int *done, cudaStream_t s, float *z32,
+                  float *z_lo)
+{
+    const size_t smem = (size_t)bank_stages<BD, T, BF>() * bank_bytes<BD, BF>(sizeof(T)) * BankGroup<BD>::GB;
+    raise_smem_limit((const void *)symv0_kernel<BD, T, ACC, DOT, XT, BF>, smem);
+    symv0_kernel<BD, T, ACC, DOT, XT, BF><<<symv0_grid<BD, T, BF>(m.nparts), 128, smem, s>>>(
+        m, inv0, u, xin, z, scale, rdot, st, gr, done, z32, z_lo);
+}
+
 template <int BD, typename T, typename XT>
 void mas_apply_dot_t(const MasDev &m, const T *inv0, const T *invc, T *v, T *u, const XT *xin, double *z,
                      bool acc, double scale, const double *rdot, PcgState *st, int dot_mode, GridReduce gr,
                      const int *done, cudaStream_t s, float *z32, float *z_lo)
 {
-    if (m.L > 1) {
-        restrict0_kernel<BD, T, XT><<<grid_for((int64_t)m.nparts * 32, 256, sm_grid(16)), 256, 0, s>>>(m, xin, v, done);
-        for (int l = 1; l + 1 < m.L; ++l)
-            restrict_kernel<BD, T><<<grid_for((int64_t)m.nbanks[l] * 32, 256, sm_grid(16)), 256, 0, s>>>(m, l, v, done);
-        symv_coarse_kernel<BD, T><<<grid_for((int64_t)m.ncoarse * 32, 256, sm_grid(16)), 256, 0, s>>>(m, invc, v, u,
-                                                                                                   done);
-        if (m.L > 2)
-            prolong_all_kernel<BD, T><<<grid_for(m.nitems[1], 256, 1 << 30), 256, 0, s>>>(m, u, done);
+    if (m.L > 1)
+    {
+        restrict_kernel<BD, T, XT><<<grid_for(m.nparts, 8, sm_grid(8)), 256, 0, s>>>(m, xin, v, done);
+        symv_coarse_kernel<BD, T><<<(unsigned)m.ncoarse, 256, 0, s>>>(m, invc, v, u, done);
     }
-    const int grid = grid_for((int64_t)m.nparts * 32, 256, sm_grid(16));
 #define LSS_S0(A_, D_)                                                                                          \
     do {                                                                                                        \
         if (std::is_same<T, float>::value && m.bank_bytes0 > 0)                                                 \
-            symv0_kernel<BD, T, A_, D_, XT, true><<<grid, 256, 0, s>>>(m, inv0, u, xin, z, scale, rdot, st, gr,   \
-                                                                       done, z32, z_lo);                        \
+            symv0_launch<BD, T, A_, D_, XT, std::is_same<T, float>::value>(m, inv0, u, xin, z, scale, rdot, st, \
+                                                                           gr, done, s, z32, z_lo);             \
         else                                                                                                    \
-            symv0_kernel<BD, T, A_, D_, XT, false><<<grid, 256, 0, s>>>(m, inv0, u, xin, z, scale, rdot, st, gr,  \
-                                                                        done, z32, z_lo);                       \
+            symv0_launch<BD, T, A_, D_, XT, false>(m, inv0, u, xin, z, scale, rdot, st, gr, done, s, z32, z_lo); \
     } while (0)
     if (dot_mode == 0) {
         if (acc) LSS_S0(true, 0);
@@ -656,7 +769,7 @@ void launch_mas_assemble_coarse(const BsrDev &A, const MasDev &m, const int32_t 
 }
 
 template <int BD, typename T, bool BF = false>
-static void invert_t(int64_t nbanks, const double *stage, T *out, int *bad, cudaStream_t s)
+static void invert_t(int64_t nbanks, const double *stage, T *out, int *bad, uint8_t *uncoupled, cudaStream_t s)
 {
     constexpr int N = 32 * BD;
     const size_t smem = (size_t)(N * (N + 1) + 2 * N) * sizeof(double);
@@ -666,44 +779,44 @@ static void invert_t(int64_t nbanks, const double *stage, T *out, int *bad, cuda
         const int64_t cnt = std::min<int64_t>(nbanks - b0, 1 << 30);
         T *o = BF ? reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(out) + b0 * mas_bank_bytes_bf16(BD))
                   : out + b0 * mas_tile_elems(BD);
-        mas_invert_kernel<BD, T, BF><<<(unsigned)cnt, 256, smem, s>>>(stage + b0 * N * N, o, bad);
+        mas_invert_kernel<BD, T, BF><<<(unsigned)cnt, 256, smem, s>>>(stage + b0 * N * N, o, bad,
+                                                                      uncoupled ? uncoupled + b0 : nullptr);
     }
     LSS_LAUNCH_CHECK();
 }
 
 void launch_mas_invert(int bd, int64_t nbanks, const double *stage, void *out, bool fp32, int *bad, cudaStream_t s,
-                       bool bf16_offdiag)
+                       uint8_t *uncoupled, bool bf16_offdiag)
 {
     if (nbanks == 0) return;
     if (bf16_offdiag) {
         if (!fp32) fail(LSS_ERR_INTERNAL, "BF16 off-diagonal tiles need the FP32 MAS");
-        if (bd == 1) invert_t<1, float, true>(nbanks, stage, (float *)out, bad, s);
-        else if (bd == 2) invert_t<2, float, true>(nbanks, stage, (float *)out, bad, s);
-        else invert_t<3, float, true>(nbanks, stage, (float *)out, bad, s);
+        if (bd == 1) invert_t<1, float, true>(nbanks, stage, (float *)out, bad, uncoupled, s);
+        else if (bd == 2) invert_t<2, float, true>(nbanks, stage, (float *)out, bad, uncoupled, s);
+        else invert_t<3, float, true>(nbanks, stage, (float *)out, bad, uncoupled, s);
         return;
     }
     if (fp32) {
-        if (bd == 1) invert_t<1, float>(nbanks, stage, (float *)out, bad, s);
-        else if (bd == 2) invert_t<2, float>(nbanks, stage, (float *)out, bad, s);
-        else invert_t<3, float>(nbanks, stage, (float *)out, bad, s);
+        if (bd == 1) invert_t<1, float>(nbanks, stage, (float *)out, bad, uncoupled, s);
+        else if (bd == 2) invert_t<2, float>(nbanks, stage, (float *)out, bad, uncoupled, s);
+        else invert_t<3, float>(nbanks, stage, (float *)out, bad, uncoupled, s);
     } else {
-        if (bd == 1) invert_t<1, double>(nbanks, stage, (double *)out, bad, s);
-        else if (bd == 2) invert_t<2, double>(nbanks, stage, (double *)out, bad, s);
-        else invert_t<3, double>(nbanks, stage, (double *)out, bad, s);
+        if (bd == 1) invert_t<1, double>(nbanks, stage, (double *)out, bad, uncoupled, s);
+        else if (bd == 2) invert_t<2, double>(nbanks, stage, (double *)out, bad, uncoupled, s);
+        else invert_t<3, double>(nbanks, stage, (double *)out, bad, uncoupled, s);
     }
 }
 
 void launch_mas_level0(const MasDev &m, const void *inv0, const void *u, bool fp32, const double *xin, double *z,
                        cudaStream_t s)
 {
-    const int grid = grid_for((int64_t)m.nparts * 32, 256, sm_grid(16));
     GridReduce gr{};
-#define LSS_L0(BD_, T_)                                                                                        \
-    symv0_kernel<BD_, T_, false, 0, double><<<grid, 256, 0, s>>>(m, (const T_ *)inv0, (const T_ *)u, xin, z, 1.0,   \
-                                                                 nullptr, nullptr, gr, nullptr, nullptr, nullptr)
-#define LSS_L0BF(BD_)                                                                                          \
-    symv0_kernel<BD_, float, false, 0, double, true><<<grid, 256, 0, s>>>(                                     \
-        m, (const float *)inv0, (const float *)u, xin, z, 1.0, nullptr, nullptr, gr, nullptr, nullptr, nullptr)
+#define LSS_L0(BD_, T_)                                                                                          \
+    symv0_launch<BD_, T_, false, 0, double, false>(m, (const T_ *)inv0, (const T_ *)u, xin, z, 1.0, nullptr, nullptr, \
+                                                   gr, nullptr, s, nullptr, nullptr)
+#define LSS_L0BF(BD_)                                                                                            \
+    symv0_launch<BD_, float, false, 0, double, true>(m, (const float *)inv0, (const float *)u, xin, z, 1.0, nullptr, \
+                                                     nullptr, gr, nullptr, s, nullptr, nullptr)
     if (fp32 && m.bank_bytes0 > 0) {
         if (m.bd == 2) LSS_L0BF(2);
         else LSS_L0BF(3);

@@ -251,6 +251,25 @@ void HybridSolver::analyze(int32_t n, int64_t nnz, const int32_t *outer, const i
     }
     mas_.ncoarse = boff;
     mas_.level_elems = voff;
+    mas_.cmap = d_cmap_.data();
+    // how many banks of the level below report to every coarse bank (a bank's
+    // items are consecutive at the next level, so they lie in at most two banks)
+    std::vector<unsigned> need(std::max(boff, 1), 0u);
+    for (int l = 1; l < cs_.L; ++l) {
+        const std::vector<int32_t> &base = l == 1 ? cs_.cbase0 : cs_.cbase[l - 1];
+        const std::vector<uint8_t> &cnt = l == 1 ? cs_.ccnt0 : cs_.ccnt[l - 1];
+        for (size_t b = 0; b < base.size(); ++b)
+            if (cnt[b])
+                for (int32_t q = base[b] >> 5; q <= (base[b] + cnt[b] - 1) >> 5; ++q) ++need[mas_.boff[l] + q];
+    }
+    d_need_.upload(need, stream_);
+    d_arrive_.resize(need.size());
+    d_arrive_.zero(stream_);
+    mas_.need = d_need_.data();
+    mas_.arrive = d_arrive_.data();
+    d_uncoupled_.resize(need.size());
+    d_uncoupled_.zero(stream_);
+    mas_.uncoupled = d_uncoupled_.data();
     LSS_CUDA(cudaStreamSynchronize(stream_));
     have_pattern_ = true;
     stats_["time_analyze"] = secs(t0);
@@ -686,14 +705,15 @@ void HybridSolver::setup_mas()
         d_stage0_.resize((size_t)nparts * N * N);
         d_stage0_.zero(stream_);
         launch_mas_assemble0(A_, d_part_of_.data(), d_part_off_.data(), d_stage0_.data(), stream_);
-        launch_mas_invert(bd, nparts, d_stage0_.data(), d_inv0_.data(), mas_fp32_, d_bad_.data(), stream_, bf);
+        launch_mas_invert(bd, nparts, d_stage0_.data(), d_inv0_.data(), mas_fp32_, d_bad_.data(), stream_, nullptr, bf);
     }
     if (ncoarse > 0) {
         d_stagec_.resize((size_t)ncoarse * N * N);
         d_stagec_.zero(stream_);
         d_cpartial_.resize((size_t)std::max<int64_t>(memb_.nchunk, 1) * bd * bd * 32);
         launch_mas_assemble_coarse(A_, mas_, d_cmap_.data(), memb_, d_cpartial_.data(), d_stagec_.data(), stream_);
-        launch_mas_invert(bd, ncoarse, d_stagec_.data(), d_invc_.data(), mas_fp32_, d_bad_.data(), stream_);
+        launch_mas_invert(bd, ncoarse, d_stagec_.data(), d_invc_.data(), mas_fp32_, d_bad_.data(), stream_,
+                          d_uncoupled_.data());
     }
     int bad = 0;
     LSS_CUDA(cudaMemcpyAsync(&bad, d_bad_.data(), sizeof(int), cudaMemcpyDeviceToHost, stream_));

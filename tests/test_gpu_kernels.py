@@ -1,0 +1,60 @@
+"""Edge sizes of the solver's kernels (GPU): one block row up to several CTAs'
+worth, every block size, isolated nodes (banks without couplings)."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+pytestmark = pytest.mark.gpu
+
+
+def block_system(nb, bs, seed, isolated=0, reach=40, degree=6):
+    """Symmetric, strictly diagonally dominant block system on nb nodes of a
+    random graph with couplings up to `reach` nodes apart; the last `isolated`
+    nodes couple to nothing (their rows have off-diagonals inside the node)."""
+    rng = np.random.default_rng(seed)
+    m = max(nb - isolated, 1)
+    i = rng.integers(0, m, size=degree * m // 2)
+    j = np.clip(i + rng.integers(1, reach + 1, size=len(i)), 0, m - 1)
+    keep = i != j
+    G = sp.csr_matrix((np.ones(int(keep.sum())), (i[keep], j[keep])), shape=(nb, nb))
+    G = ((G + G.T) != 0).astype(np.float64) + sp.identity(nb)
+    B = sp.kron(G, np.ones((bs, bs)), format="csr")
+    B.data = rng.uniform(-1.0, 1.0, size=B.nnz)
+    A = (B + B.T) * 0.5
+    A = A - sp.diags(A.diagonal())
+    d = np.asarray(abs(A).sum(axis=1)).ravel() + rng.uniform(0.5, 1.5, size=nb * bs)
+    A = (A + sp.diags(d)).tocsc()
+    A.sum_duplicates()
+    A.sort_indices()
+    return A
+
+
+def make_solver(bs, precision="fp64", extra=None, **params):
+    import lss
+    gb = {"precision": precision}
+    gb.update(extra or {})
+    return lss.Solver.create({"solver": "GPUHybrid", "GPUHybrid": {"block_size": bs, **params}, "gb300": gb})
+
+
+@pytest.mark.parametrize("bs", [1, 2, 3])
+@pytest.mark.parametrize("nb,isolated", [(1, 0), (2, 1), (31, 0), (33, 0), (70, 64), (129, 0), (1100, 200), (5000, 1500)])
+def test_mas_apply_edge_sizes(bs, nb, isolated, built):
+    """MAS against the CPU restatement on the same partition.  The blocks are
+    diagonally dominant with a condition number of at most a few hundred, so the two
+    FP64 inverses differ by less than 1e-12 relative and the FP32 ones by
+    less than 1e-4; coarse vectors and uncoupled banks add exact copies."""
+    from oracle import oracle as O
+    A = block_system(nb, bs, seed=nb + bs, isolated=isolated)
+    params = {"block_size": bs, "do_hybrid_precond": False}
+    r = np.random.default_rng(nb).standard_normal(A.shape[0])
+    zo = None
+    for precision, tol in (("fp64", 1e-12), ("mixed", 1e-4)):
+        s = make_solver(bs, precision, do_hybrid_precond=False)
+        s.factorize(A)
+        if zo is None:
+            perm, offs = s.partition()
+            zo = O.CpuSolver(A, params, perm=perm, part_offsets=offs).precond(r)
+        z = s.mas_apply(r)
+        assert np.linalg.norm(z - zo) <= tol * np.linalg.norm(zo), (precision, nb)
+        np.testing.assert_array_equal(s.mas_apply(r), z)  # fixed order of every sum
+        s.close()
