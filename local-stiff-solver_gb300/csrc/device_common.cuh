@@ -7,10 +7,40 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <utility>
 
 #include "kernels.hpp"
 
 namespace lss {
+
+// Programmatic dependent launch: a kernel launched by launch_pdl may be
+// dispatched while its predecessor in the stream still runs; pdl_enter lets
+// the next launch be dispatched at once and waits for the predecessor's
+// completion (and memory) -- the launch latency overlaps the predecessor's tail
+// instead of adding to it.  Before pdl_enter a kernel may only read what no
+// kernel of the running sequence writes.
+__device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... KArgs, typename... Args>
+void launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                Args &&...args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    LSS_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
+}
 
 constexpr int WARP = 32;
 constexpr int BANK = 32;  // MAS bank width (MASPreconditioner.cu:33)

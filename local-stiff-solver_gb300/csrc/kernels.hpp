@@ -218,6 +218,12 @@ void launch_mas_level0(const MasDev &m, const void *inv0, const void *u, bool fp
                        cudaStream_t s);
 
 // ---------------------------------------------------------------- stiff blocks
+// One warp of the dense apply: rows [row0, row0 + 32) of a subdomain of m DOFs
+// (first stiff DOF off), columns [slice * width, (slice + 1) * width).
+struct StiffWarp {
+    int64_t inv_off;
+    int32_t off, m, row0, slice, nsl, width;
+};
 struct StiffDev {
     int32_t nsub = 0, ndof = 0;
     int32_t ndof_dense = 0;            // DOFs j < ndof_dense belong to subdomains with a dense inverse
@@ -229,7 +235,12 @@ struct StiffDev {
     const double *inv = nullptr;       // row-major m x m per subdomain
     const float *inv32 = nullptr;
     double *t = nullptr;               // ndof scratch
+    const StiffWarp *warps = nullptr;  // single right-hand-side apply of the dense inverses
+    int32_t nwarps = 0;
 };
+// the warps of the dense apply for the subdomains 0 .. ndense-1
+std::vector<StiffWarp> stiff_warps(const std::vector<int32_t> &off, const std::vector<int64_t> &inv_off,
+                                   int32_t ndense);
 
 void launch_stiff_extract(const BsrDev &A, const StiffDev &S, double *stage, cudaStream_t s);
 // dense inverses of the subdomains 0 .. nsub-1 (each at most STIFF_DENSE_MAX DOFs)

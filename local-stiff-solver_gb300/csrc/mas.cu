@@ -367,31 +367,34 @@ __global__ void __launch_bounds__(256, 2) mas_invert_kernel(const double *__rest
 
 // ------------------------------------------------------------------ apply
 
-// Segmented sums of one bank: 32 items (values staged item-major in xs, the
-// target aggregate of each item in ks) into ncc aggregates.  Output slot
-// s = k * BD + c (aggregate k, component c) belongs to a group of P lanes, P
-// the largest power of two with ncc * BD * P <= 32 (1 beyond): lane q of the
-// group adds the items j = q, q + P, ... of aggregate k and the group's sums
-// meet by shuffles, in one fixed order.  An FP64 add costs the pipe a whole
-// warp however few lanes take part: with one aggregate (a connected
-// partition) this is 4 + 3 adds instead of 32.
+// Segmented sums of one bank: 32 items (values staged item-major in xs; lane j
+// passes the target aggregate of item j, 0xff for none) into ncc aggregates.
+// Output slot s = k * BD + c (aggregate k, component c) belongs to a group of P
+// lanes, P the largest power of two with ncc * BD * P <= 32 (1 beyond): lane q
+// of the group adds the items j = q, q + P, ... of aggregate k in order, found
+// by its mask, and the group's sums meet by shuffles.  An FP64 add costs the
+// pipe a whole warp however few lanes take part: one aggregate (a connected
+// partition) takes 4 + 3 adds and 32 aggregates (uncoupled items) one add per
+// pass, where testing every item against every slot took 32 per pass.
 template <int BD, typename T>
-__device__ __forceinline__ void bank_segment_sums(const T *xs, const uint8_t *ks, int ncc, T *__restrict__ out,
-                                                  int lane)
+__device__ __forceinline__ void bank_segment_sums(const T *xs, uint8_t key, unsigned *mask, int ncc,
+                                                  T *__restrict__ out, int lane)
 {
+    const unsigned same = __match_any_sync(0xffffffffu, (unsigned)key);
+    if (key < 32 && __ffs(same) - 1 == lane) mask[key] = same;
+    __syncwarp();
     const int slots = ncc * BD;
     int lg = 0;
     while (lg < 5 && (slots << (lg + 1)) <= 32) ++lg;
-    const int P = 1 << lg, sub = lane & (P - 1);
+    const int sub = lane & ((1 << lg) - 1);
+    // every 2^lg-th item, starting at sub
+    const unsigned every = (lg == 0 ? ~0u : lg == 1 ? 0x55555555u : lg == 2 ? 0x11111111u : lg == 3 ? 0x01010101u
+                            : lg == 4 ? 0x00010001u : 1u) << sub;
     for (int s0 = 0; s0 < slots; s0 += 32 >> lg) {
         const int sl = s0 + (lane >> lg), k = sl / BD, c = sl - k * BD;
         T acc = T(0);
-        if (sl < slots) {
-#pragma unroll 8
-            for (int j = sub; j < 32; j += P)
-                if (ks[j] == k) acc += xs[j * BD + c];
-        }
-        for (int o = P >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        for (unsigned m = sl < slots ? mask[k] & every : 0u; m; m &= m - 1) acc += xs[(__ffs(m) - 1) * BD + c];
+        for (int o = (1 << lg) >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (sl < slots && sub == 0) out[sl] = acc;
     }
 }
@@ -414,14 +417,14 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
     if (done && *done) return;
     constexpr int N = 32 * BD, W = 8;
     __shared__ T xs_all[W][N];
-    __shared__ uint8_t ks_all[W][32];
+    __shared__ unsigned mask_all[W][32];
     // ready banks, level << 28 | bank: at most 16 level-1 banks per round and
     // twice the previous level's at each of up to five further levels
     __shared__ unsigned queue[1024];
     __shared__ int qn;
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     T *xs = xs_all[wl];
-    uint8_t *ks = ks_all[wl];
+    unsigned *mask = mask_all[wl];
     if (threadIdx.x == 0) qn = 0;
     __syncthreads();
     // reports items [i0, i0 + cnt) of level l as written; queues completed banks
@@ -451,11 +454,11 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
                 const int e = q * 32 + lane;
                 xs[e] = e < cnt * BD ? (T)r[(int64_t)lo * BD + e] : T(0);
             }
-            ks[lane] = lane < cnt ? m.key0[lo + lane] : (uint8_t)0xff;
+            const uint8_t key = lane < cnt ? m.key0[lo + lane] : (uint8_t)0xff;
             const int32_t i0 = m.cbase0[p];
             const int nc = m.ccnt0[p];
             __syncwarp();
-            bank_segment_sums<BD, T>(xs, ks, nc, v + m.voff[1] + (int64_t)i0 * BD, lane);
+            bank_segment_sums<BD, T>(xs, key, mask, nc, v + m.voff[1] + (int64_t)i0 * BD, lane);
             report(1, i0, nc);
         }
         __syncthreads();
@@ -472,11 +475,11 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
                     const int e = q * 32 + lane;
                     xs[e] = e < cnt * BD ? __ldcg(vl + e) : T(0);
                 }
-                ks[lane] = lane < cnt ? m.key[l][i0 + lane] : (uint8_t)0xff;
+                const uint8_t key = lane < cnt ? m.key[l][i0 + lane] : (uint8_t)0xff;
                 const int32_t j0 = m.cbase[l][b];
                 const int nc = m.ccnt[l][b];
                 __syncwarp();
-                bank_segment_sums<BD, T>(xs, ks, nc, v + m.voff[l + 1] + (int64_t)j0 * BD, lane);
+                bank_segment_sums<BD, T>(xs, key, mask, nc, v + m.voff[l + 1] + (int64_t)j0 * BD, lane);
                 report(l + 1, j0, nc);
             }
             __syncthreads();

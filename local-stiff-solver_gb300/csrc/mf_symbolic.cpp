@@ -19,7 +19,13 @@
 namespace lss {
 namespace {
 
-constexpr int32_t LEAF_DOFS = 48;
+// Node sets up to this many DOFs are eliminated as one front.  Every level of
+// the tree is two dependent launches of each solve and a chain of panel steps
+// of the factorization, while a front of this size is still a few microseconds
+// of FP64 work on the whole GPU: a 1,263-DOF ball in mixed precision took 145
+// us per iteration with leaves of 48 DOFs (six levels), 128 with 160 and 116
+// with 384 (three); 512 gains no more there and costs a fifth of the factorization.
+constexpr int32_t LEAF_DOFS = 384;
 
 struct Nd {
     const std::vector<int32_t> &aoff, &adj;  // local node graph (no self loops)

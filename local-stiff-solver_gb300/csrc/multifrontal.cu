@@ -9,11 +9,12 @@
 //                   rank-32 update of the upper-triangle tiles, panel write-back;
 //                   then the swept rows are mirrored into the lower triangle
 // (the original entries are assembled into every front once, before level 0).
-// Solve, per level: a gather extend-add of every front's vector and a forward
-// GEMV launch (leaves first), then one backward GEMV launch per level (root
-// first) and one scatter.  GEMV CTAs take 32 output columns and at most 256
-// of a front's rows; larger fronts split their rows over several CTAs whose
-// partial sums the last CTA of the group adds in a fixed order.  The
+// Solve: one forward GEMV launch per level (leaves first; the extend-add of the
+// front's vector is gathered by the GEMV CTAs, in the batched solve by a
+// launch before), then one backward GEMV launch per level (root first; in the
+// batched solve a scatter ends it).  GEMV CTAs take 32 output columns and at
+// most 256 of a front's rows; larger fronts split their rows over several CTAs
+// whose partial sums the last CTA of the group adds in a fixed order.  The
 // per-level launches use programmatic dependent launch.  The solve with one
 // right-hand side is FP64; the batched solve with 16 reads the fronts as
 // double-float pairs (below).
@@ -97,23 +98,33 @@ __global__ void __launch_bounds__(256) mf_assemble_kernel(BsrDev A, StiffDev S, 
     }
 }
 
-// children's Schur complements into the parent (upper triangle), in child order
+// Children's Schur complements into the parent (upper triangle), in child
+// order: a warp owns a row of the parent front, so every entry has one writer
+// and its children add in order.  (One CTA per front, which this was, took 300
+// us for the 500-row fronts of a 3k-DOF subdomain.)
 __global__ void __launch_bounds__(256) mf_extend_add_kernel(MfView v, MfWork w, double *__restrict__ F)
 {
-    const int32_t N = w.front[blockIdx.x];
+    const int i = find_front(w, blockIdx.x);
+    const int32_t N = w.front[i];
     const int32_t fN = v.s[N] + v.u[N];
-    double *Fn = F + v.foff[N];
+    const int32_t r = (int32_t)(blockIdx.x - w.prefix[i]) * 8 + (int32_t)(threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (r >= fN) return;
+    double *Fr = F + v.foff[N] + (int64_t)r * fN;
     for (int32_t ci = v.child_off[N]; ci < v.child_off[N + 1]; ++ci) {
         const int32_t c = v.child[ci], sc = v.s[c], uc = v.u[c], fc = sc + uc;
-        const double *Fc = F + v.foff[c];
-        const int32_t *map = v.ea_map + v.bnd_off[c];
-        const int64_t total = (int64_t)uc * uc;
-        for (int64_t e = threadIdx.x; e < total; e += blockDim.x) {
-            const int32_t a = (int32_t)(e / uc), bb = (int32_t)(e % uc);
-            if (a > bb) continue;
-            Fn[(int64_t)map[a] * fN + map[bb]] += Fc[(int64_t)(sc + a) * fc + sc + bb];
+        const int32_t *map = v.ea_map + v.bnd_off[c];  // ascending
+        int32_t a = 0, e = uc;
+        while (a < e) {
+            const int32_t mid = (a + e) >> 1;
+            if (map[mid] < r) a = mid + 1;
+            else e = mid;
         }
-        __syncthreads();
+        if (a < uc && map[a] == r) {
+            const double *Fc = F + v.foff[c] + (int64_t)(sc + a) * fc + sc;
+            for (int32_t bb = a + lane; bb < uc; bb += 32) Fr[map[bb]] += Fc[bb];
+        }
+        __syncwarp();  // the next child's lanes take other columns of the row
     }
 }
 
@@ -180,55 +191,87 @@ __device__ __forceinline__ double up(const double *Fn, int f, int r, int c)
     return r <= c ? Fn[(int64_t)r * f + c] : Fn[(int64_t)c * f + r];
 }
 
-// Dinv = (S[K][K])^-1 for the panel K = [k0, k0 + t)
+// Dinv = (S[K][K])^-1 for the panel K = [k0, k0 + t).  Eight warps hold the
+// block in registers (lane = column, warp w the rows w, w + 8, ...); the warp
+// of the pivot row publishes it with its scaled copy, so a pivot costs one
+// barrier and four multiply-adds a thread (the sweep in shared memory: three
+// barriers a pivot, 45 us a block against 12).
 __global__ void __launch_bounds__(256) mf_blk_diag_kernel(MfView v, MfWork w, const double *__restrict__ F, int k0,
                                                           double *__restrict__ Dinv, int *bad)
 {
-    __shared__ double D[PW * (PW + 1)], col[PW], scol[PW];
+    __shared__ double row[2][PW], srow[2][PW];
     const int i = blockIdx.x;
     const int32_t N = w.front[i];
     const int s = v.s[N], f = s + v.u[N];
     if (s <= k0) return;
-    const int t = min(PW, s - k0), ld = PW + 1;
+    const int t = min(PW, s - k0), c = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const double *Fn = F + v.foff[N];
-    for (int e = threadIdx.x; e < t * t; e += blockDim.x) {
-        const int r = e / t, c = e % t;
-        D[r * ld + c] = up(Fn, f, k0 + r, k0 + c);
+    double d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = wl + 8 * q;
+        d[q] = r < t && c < t ? up(Fn, f, k0 + r, k0 + c) : 0.0;
     }
-    __syncthreads();
-    sweep_leading(D, ld, t, t, col, scol, bad);
-    for (int e = threadIdx.x; e < PW * PW; e += blockDim.x) {
-        const int r = e / PW, c = e % PW;
-        Dinv[(int64_t)i * PW * PW + e] = (r < t && c < t) ? -D[r * ld + c] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll 1
+        for (int pw = 0; pw < 8; ++pw) {  // pivot p = pw + 8 q, row p in register q of warp pw
+            const int p = pw + 8 * q, b = p & 1;
+            if (p >= t) break;
+            if (wl == pw) {
+                const double piv = __shfl_sync(0xffffffffu, d[q], p), rpiv = 1.0 / piv;
+                if (c == 0 && (!isfinite(piv) || piv == 0.0)) atomicOr(bad, 16);
+                row[b][c] = d[q];
+                srow[b][c] = c == p ? -rpiv : d[q] * rpiv;
+            }
+            __syncthreads();
+            const double rc = row[b][c], sc = srow[b][c];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = wl + 8 * k;
+                if (r == p) d[k] = sc;
+                else if (c == p) d[k] = srow[b][r];
+                else d[k] -= srow[b][r] * rc;
+            }
+        }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = wl + 8 * q;
+        Dinv[(int64_t)i * PW * PW + r * PW + c] = r < t && c < t ? -d[q] : 0.0;
     }
 }
 
-// P[r][:] = S[r][K] Dinv for every row r outside K (one thread per row)
-__global__ void __launch_bounds__(128) mf_blk_panel_kernel(MfView v, MfWork w, const double *__restrict__ F, int k0,
+// P[r][:] = S[r][K] Dinv for the rows r outside K, eight rows per CTA (one per
+// warp, lane = column): a thread per row left most SMs idle (58 us a panel)
+__global__ void __launch_bounds__(256) mf_blk_panel_kernel(MfView v, MfWork w, const double *__restrict__ F, int k0,
                                                            const double *__restrict__ Dinv, double *__restrict__ P)
 {
-    __shared__ double Ds[PW * PW];
+    __shared__ double Ds[PW * PW], Sr[8][PW];
     const int i = find_front(w, blockIdx.x);
     const int32_t N = w.front[i];
     const int s = v.s[N], f = s + v.u[N];
     if (s <= k0) return;
     const int t = min(PW, s - k0);
-    for (int e = threadIdx.x; e < PW * PW; e += blockDim.x) Ds[e] = Dinv[(int64_t)i * PW * PW + e];
-    __syncthreads();
-    const int r = (int)(blockIdx.x - w.prefix[i]) * blockDim.x + threadIdx.x;
-    if (r >= f || (r >= k0 && r < k0 + t)) return;
+    const int c = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const int r0 = (int)(blockIdx.x - w.prefix[i]) * 8;
     const double *Fn = F + v.foff[N];
-    double acc[PW];
-#pragma unroll
-    for (int c = 0; c < PW; ++c) acc[c] = 0.0;
-    for (int q = 0; q < t; ++q) {
-        const double a = up(Fn, f, r, k0 + q);
-#pragma unroll
-        for (int c = 0; c < PW; ++c) acc[c] += a * Ds[q * PW + c];
+    for (int e = threadIdx.x; e < PW * PW; e += blockDim.x) Ds[e] = Dinv[(int64_t)i * PW * PW + e];
+    {
+        // rows before the panel lie along the storage rows, rows after it along the columns
+        const bool before = r0 + 8 <= k0;
+        const int rl = before ? wl : (int)(threadIdx.x & 7), q = before ? c : (int)(threadIdx.x >> 3);
+        const int r = r0 + rl;
+        Sr[rl][q] = r < f && q < t ? up(Fn, f, r, k0 + q) : 0.0;
     }
-    double *Pr = P + v.poff[N] + (int64_t)r * PW;
+    __syncthreads();
+    const int r = r0 + wl;
+    if (r >= f || (r >= k0 && r < k0 + t)) return;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int c = 0; c < PW; ++c) Pr[c] = c < t ? acc[c] : 0.0;
+    for (int q = 0; q < PW; q += 4)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[k] += Sr[wl][q + k] * Ds[(q + k) * PW + c];
+    P[v.poff[N] + (int64_t)r * PW + c] = c < t ? (acc[0] + acc[1]) + (acc[2] + acc[3]) : 0.0;
 }
 
 // S[a][b] -= sum_q P[a][q] S[k0+q][b] on the upper-triangle 32 x 32 tiles,
@@ -333,44 +376,19 @@ __global__ void __launch_bounds__(256) mf_mirror_kernel(MfView v, MfWork w, doub
 
 // ---- solve
 
-// Programmatic dependent launch across the solve's per-level kernels: each
-// lets the next launch be dispatched at once and waits for the previous
-// grid's completion (and memory) before it reads anything -- the launches'
-// latency overlaps the previous level's tail instead of adding to it.
-__device__ __forceinline__ void pdl_enter()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename... KArgs, typename... Args>
-void launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                Args &&...args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    LSS_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
-}
-
 constexpr int NR_COLS = 32;    // output columns per GEMV CTA of the solves
 constexpr int NR_KROWS = 256;  // front rows per GEMV CTA of the solves
 
 __host__ __device__ __forceinline__ int nr_kchunks(int rows) { return (rows + NR_KROWS - 1) / NR_KROWS; }
 
-// ---- solve with one right-hand side (FP64).  The same decomposition as the
-// batched solve below: per level, CTAs of 256 entries gather each front's
-// vector (right-hand side + the children's contributions, children in
-// order), then GEMV CTAs of 32 columns x at most 256 front rows (8 warps =
-// 8 row slices, lane = column), fronts with more rows split over several
-// CTAs whose partial sums the last CTA of the group adds in row-chunk order.
+// ---- solve with one right-hand side (FP64): one launch per level and
+// direction.  GEMV CTAs of 32 columns x at most 256 front rows (8 warps = 8
+// row slices, lane = column) gather their part of the front's vector
+// themselves (right-hand side + the children's contributions, children in
+// order); fronts with more rows are split over several CTAs whose partial
+// sums the last CTA of the group adds in row-chunk order.  All of a CTA's
+// sizes and offsets are one descriptor (the work-list search and the symbolic
+// arrays behind it were six dependent loads), and the backward pass updates z.
 
 constexpr int NR_COLS1 = 32;
 
@@ -424,85 +442,75 @@ __device__ __forceinline__ bool combine1(NrScratch1 sc, int kc, int nkc, double 
     return true;
 }
 
-// forward, step 1: W_N = [t_own ; 0] + the children's contributions (gathered)
-__global__ void __launch_bounds__(256) mf_fassemble1_kernel(MfView v, MfWork w, const int32_t *__restrict__ gptr,
-                                                            const int32_t *__restrict__ gsrc, const StiffDev S,
-                                                            double *__restrict__ W, const int *done)
+// entry e of a front's vector: [t_own ; 0] + the children's contributions
+__device__ __forceinline__ double mf_gather1(const MfCta &c, int q, const MfView &v, const StiffDev &S,
+                                             const int32_t *__restrict__ gptr, const int32_t *__restrict__ gsrc,
+                                             const double *__restrict__ W)
 {
-    pdl_enter();
-    if (done && *done) return;
-    const int i = find_front(w, blockIdx.x);
-    const int32_t N = w.front[i];
-    const int s = v.s[N], f = s + v.u[N];
-    const int q = (int)(blockIdx.x - w.prefix[i]) * 256 + (int)threadIdx.x;
-    if (q >= f) return;
-    const int64_t e = (int64_t)v.woff[N] + q;
-    double acc = q < s ? S.t[v.pos2j[v.p0[N] + q]] : 0.0;
-    for (int32_t g = gptr[e]; g < gptr[e + 1]; ++g) acc += W[gsrc[g]];
-    W[e] = acc;
+    const int64_t e = (int64_t)c.woff + q;
+    const int32_t g0 = gptr[e], g1 = gptr[e + 1];
+    double acc = q < c.s ? S.t[v.pos2j[c.p0 + q]] : 0.0;
+    for (int32_t g = g0; g < g1; ++g) acc += W[gsrc[g]];
+    return acc;
 }
 
-// forward, step 2: W_N[bnd] -= P W_N[own] over the CTA's boundary columns
-__global__ void __launch_bounds__(256) mf_forward_kernel(MfView v, MfWork w, const double *__restrict__ F,
-                                                         double *__restrict__ W, NrScratch1 sc, const int *done)
+// forward: W_N[bnd] = gathered - P W_N[own] over the CTA's boundary columns;
+// the CTAs of the first columns also keep W_N[own] for the backward pass
+__global__ void __launch_bounds__(256) mf_forward_kernel(MfView v, const MfCta *__restrict__ ctas,
+                                                         const int32_t *__restrict__ gptr,
+                                                         const int32_t *__restrict__ gsrc, const StiffDev S,
+                                                         const double *__restrict__ F, double *__restrict__ W,
+                                                         NrScratch1 sc, const int *done)
 {
-    pdl_enter();
-    if (done && *done) return;
     __shared__ double xs[NR_KROWS], red[256], res[NR_COLS1];
-    const int i = find_front(w, blockIdx.x);
-    const int32_t N = w.front[i];
-    const int s = v.s[N], u = v.u[N], f = s + u;
-    const int nkc = nr_kchunks(s), local = (int)(blockIdx.x - w.prefix[i]);
-    const int kc = local % nkc, col0 = s + (local / nkc) * NR_COLS1, ncol = min(NR_COLS1, f - col0);
-    const int q0 = kc * NR_KROWS, nrow = min(NR_KROWS, s - q0);
-    double *Wn = W + v.woff[N];
-    for (int r = threadIdx.x; r < nrow; r += blockDim.x) xs[r] = Wn[q0 + r];
-    __syncthreads();
-    gemv1(F + v.foff[N], f, col0, ncol, q0, nrow, xs, red, res);
-    if (!combine1(sc, kc, nkc, res, ncol)) return;
-    if (threadIdx.x < ncol) Wn[col0 + threadIdx.x] -= res[threadIdx.x];
-}
-
-// backward: x_own = F11^-1 (w_own - F12 x_bnd) = -(columns of the swept front) . [w_own; x_bnd]
-__global__ void __launch_bounds__(256) mf_backward_kernel(MfView v, MfWork w, const double *__restrict__ F,
-                                                          const double *__restrict__ W, double *__restrict__ X,
-                                                          NrScratch1 sc, const int *done)
-{
+    const MfCta c = ctas[blockIdx.x];
     pdl_enter();
     if (done && *done) return;
-    __shared__ double vec[NR_KROWS], red[256], res[NR_COLS1];
-    const int i = find_front(w, blockIdx.x);
-    const int32_t N = w.front[i];
-    const int s = v.s[N], u = v.u[N], f = s + u;
-    const int nkc = nr_kchunks(f), local = (int)(blockIdx.x - w.prefix[i]);
-    const int kc = local % nkc, c0 = (local / nkc) * NR_COLS1, ncol = min(NR_COLS1, s - c0);
-    const int q0 = kc * NR_KROWS, nrow = min(NR_KROWS, f - q0);
-    const double *Wn = W + v.woff[N];
-    const int32_t *bp = v.bnd_pos + v.bnd_off[N];
-    for (int r = threadIdx.x; r < nrow; r += blockDim.x) {
-        const int q = q0 + r;
-        vec[r] = q < s ? Wn[q] : X[bp[q - s]];
+    const int t = threadIdx.x;
+    if (t < c.nrow) {
+        const double a = mf_gather1(c, c.q0 + t, v, S, gptr, gsrc, W);
+        xs[t] = a;
+        if (c.col0 == c.s) W[(int64_t)c.woff + c.q0 + t] = a;
     }
+    const double base = t < c.ncol ? mf_gather1(c, c.col0 + t, v, S, gptr, gsrc, W) : 0.0;
     __syncthreads();
-    gemv1(F + v.foff[N], f, c0, ncol, q0, nrow, vec, red, res);
-    if (!combine1(sc, kc, nkc, res, ncol)) return;
-    if (threadIdx.x < ncol) X[v.p0[N] + c0 + threadIdx.x] = -res[threadIdx.x];
+    gemv1(F + c.foff, c.f, c.col0, c.ncol, c.q0, c.nrow, xs, red, res);
+    if (!combine1(sc, c.kc, c.nkc, res, c.ncol)) return;
+    if (t < c.ncol) W[(int64_t)c.woff + c.col0 + t] = base - res[t];
 }
 
-__global__ void mf_scatter_kernel(MfView v, const StiffDev S, const double *__restrict__ X, double *__restrict__ z,
-                                  float *__restrict__ z32, float *__restrict__ z_lo, const int *done)
+// backward: x_own = F11^-1 (w_own - F12 x_bnd) = -(columns of the swept front) . [w_own; x_bnd],
+// added to z (a root has no forward launch and gathers w_own here)
+__global__ void __launch_bounds__(256) mf_backward_kernel(MfView v, const MfCta *__restrict__ ctas,
+                                                          const int32_t *__restrict__ gptr,
+                                                          const int32_t *__restrict__ gsrc, const StiffDev S,
+                                                          const double *__restrict__ F, const double *__restrict__ W,
+                                                          double *__restrict__ X, NrScratch1 sc,
+                                                          double *__restrict__ z, float *__restrict__ z32,
+                                                          float *__restrict__ z_lo, const int *done)
 {
+    __shared__ double vec[NR_KROWS], red[256], res[NR_COLS1];
+    const MfCta c = ctas[blockIdx.x];
+    const int t = threadIdx.x, q = c.q0 + t;
+    const int32_t bp = t < c.nrow && q >= c.s ? v.bnd_pos[c.bnd_off + q - c.s] : 0;
+    const int32_t d = t < c.ncol ? S.dofs[v.pos2j[c.p0 + c.col0 + t]] : 0;
     pdl_enter();
     if (done && *done) return;
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= v.npos) return;
-    const int32_t d = S.dofs[v.pos2j[p]];
-    const double nz = z[d] + X[p];
-    z[d] = nz;
-    if (z32) {
-        const float h = (float)nz;
-        z32[d] = h;
-        if (z_lo) z_lo[d] = (float)(nz - (double)h);
+    if (t < c.nrow)
+        vec[t] = q >= c.s ? X[bp] : (c.s == c.f ? mf_gather1(c, q, v, S, gptr, gsrc, W) : W[(int64_t)c.woff + q]);
+    const double zd = t < c.ncol ? z[d] : 0.0;
+    __syncthreads();
+    gemv1(F + c.foff, c.f, c.col0, c.ncol, c.q0, c.nrow, vec, red, res);
+    if (!combine1(sc, c.kc, c.nkc, res, c.ncol)) return;
+    if (t < c.ncol) {
+        X[c.p0 + c.col0 + t] = -res[t];
+        const double nz = zd - res[t];
+        z[d] = nz;
+        if (z32) {
+            const float h = (float)nz;
+            z32[d] = h;
+            if (z_lo) z_lo[d] = (float)(nz - (double)h);
+        }
     }
 }
 
@@ -818,10 +826,10 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
     auto F_of = [&](int32_t id) { return (int64_t)M.s[id] + M.u[id]; };
     for (int h = 0; h < M.levels; ++h) {
         Level &L = levels_[h];
-        make(L.ea, lv_ea[h], [](int32_t) { return (int64_t)1; });
+        make(L.ea, lv_ea[h], [&](int32_t id) { return (F_of(id) + 7) / 8; });
         make(L.small, lv_small[h], [](int32_t) { return (int64_t)1; });
         make(L.diag, lv_large[h], [](int32_t) { return (int64_t)1; });
-        make(L.panel, lv_large[h], [&](int32_t id) { return (F_of(id) + 127) / 128; });
+        make(L.panel, lv_large[h], [&](int32_t id) { return (F_of(id) + 7) / 8; });
         make(L.update, lv_large[h], [&](int32_t id) {
             const int64_t T = (F_of(id) + 31) / 32;
             return T * (T + 1) / 2;
@@ -829,7 +837,6 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
         make(L.write, lv_large[h], [&](int32_t id) { return (F_of(id) * PW + 255) / 256; });
         make(L.mirror, lv_large[h], [&](int32_t id) { return (F_of(id) * M.s[id] + 255) / 256; });
         make(L.fasm_nr, lv_all[h], [&](int32_t id) { return (F_of(id) + 15) / 16; }, true);
-        make(L.fasm1, lv_all[h], [&](int32_t id) { return (F_of(id) + 255) / 256; }, true);
         make(L.fwd_nr, lv_all[h], [&](int32_t id) {
             return (int64_t)((M.u[id] + NR_COLS - 1) / NR_COLS) * nr_kchunks(M.s[id]);
         }, true);
@@ -838,6 +845,41 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
         }, true);
         for (int32_t id : lv_large[h]) L.max_s_large = std::max(L.max_s_large, M.s[id]);
     }
+    // GEMV CTAs of the single right-hand-side solve
+    std::vector<MfCta> ctas;
+    auto add_ctas = [&](int32_t id, int32_t first, int32_t cols, int32_t rows) {
+        const int32_t nkc = nr_kchunks(rows);
+        for (int32_t c0 = 0; c0 < cols; c0 += NR_COLS1)
+            for (int32_t kc = 0; kc < nkc; ++kc) {
+                MfCta c;
+                c.foff = M.foff[id];
+                c.s = M.s[id];
+                c.f = M.s[id] + M.u[id];
+                c.col0 = first + c0;
+                c.ncol = std::min(NR_COLS1, cols - c0);
+                c.q0 = kc * NR_KROWS;
+                c.nrow = std::min(NR_KROWS, rows - c.q0);
+                c.kc = kc;
+                c.nkc = nkc;
+                c.woff = M.woff[id];
+                c.p0 = M.p0[id];
+                c.bnd_off = M.bnd_off[id];
+                c.pad = 0;
+                ctas.push_back(c);
+            }
+    };
+    int64_t max1 = 1;
+    for (int h = 0; h < M.levels; ++h) {
+        Level &L = levels_[h];
+        L.fwd1 = (int64_t)ctas.size();
+        for (int32_t id : lv_all[h]) add_ctas(id, M.s[id], M.u[id], M.s[id]);
+        L.nfwd1 = (int32_t)((int64_t)ctas.size() - L.fwd1);
+        L.bwd1 = (int64_t)ctas.size();
+        for (int32_t id : lv_all[h]) add_ctas(id, 0, M.s[id], M.s[id] + M.u[id]);
+        L.nbwd1 = (int32_t)((int64_t)ctas.size() - L.bwd1);
+        max1 = std::max<int64_t>({max1, L.nfwd1, L.nbwd1});
+    }
+    d_ctas_.upload(ctas, st);
     // extend-add as a gather: per entry of W, the child entries that add into it
     std::vector<int32_t> gptr((size_t)M.welems + 1, 0), gsrc;
     {
@@ -886,7 +928,7 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
     d_F_.resize(M.elems);
     d_w_.resize(std::max<int64_t>(M.welems, 1));
     // scratch of the split fronts' partial sums (both solves), zeroed counters
-    int64_t maxctas = 1;
+    int64_t maxctas = max1;
     for (const Level &L : levels_) maxctas = std::max({maxctas, L.fwd_nr.ctas, L.bwd_nr.ctas});
     d_part1_.resize((size_t)maxctas * NR_COLS1);
     d_nrcnt_.resize((size_t)maxctas);
@@ -928,7 +970,7 @@ void MfFactor::factorize(const BsrDev &A, const StiffDev &S, int *bad, cudaStrea
     raise_smem_limit((const void *)mf_sweep_small_kernel, small_smem);
     for (const Level &L : levels_) {
         if (L.ea.count) {
-            mf_extend_add_kernel<<<L.ea.count, 256, 0, st>>>(v, L.ea, F);
+            mf_extend_add_kernel<<<(unsigned)L.ea.ctas, 256, 0, st>>>(v, L.ea, F);
             LSS_LAUNCH_CHECK();
         }
         if (L.small.count) {
@@ -938,7 +980,7 @@ void MfFactor::factorize(const BsrDev &A, const StiffDev &S, int *bad, cudaStrea
         if (L.diag.count) {
             for (int k0 = 0; k0 < L.max_s_large; k0 += PW) {
                 mf_blk_diag_kernel<<<L.diag.count, 256, 0, st>>>(v, L.diag, F, k0, d_D_.data(), bad);
-                mf_blk_panel_kernel<<<(unsigned)L.panel.ctas, 128, 0, st>>>(v, L.panel, F, k0, d_D_.data(),
+                mf_blk_panel_kernel<<<(unsigned)L.panel.ctas, 256, 0, st>>>(v, L.panel, F, k0, d_D_.data(),
                                                                             d_P_.data());
                 mf_blk_update_kernel<<<(unsigned)L.update.ctas, 256, 0, st>>>(v, L.update, F, k0, d_P_.data());
                 mf_blk_write_kernel<<<(unsigned)L.write.ctas, 256, 0, st>>>(v, L.write, F, k0, d_P_.data(),
@@ -957,23 +999,20 @@ void MfFactor::solve(const StiffDev &S, double *z, float *z32, float *z_lo, cons
     const MfView v = make_view(p0_, s_, u_, woff_, bnd_off_, bnd_pos_, child_off_, child_, ea_map_, front_of_pos_,
                                pos2j_, j2pos_, poff_, foff_, sym_.j_base, sym_.npos);
     const NrScratch1 sc{d_part1_.data(), d_nrcnt_.data()};
-    for (const Level &L : levels_) {
-        launch_pdl(mf_fassemble1_kernel, (unsigned)L.fasm1.ctas, 256, 0, st, v, L.fasm1, gptr_, gsrc_, S,
-                   d_w_.data(), done);
-        if (L.fwd_nr.ctas > 0)
-            launch_pdl(mf_forward_kernel, (unsigned)L.fwd_nr.ctas, 256, 0, st, v, L.fwd_nr,
-                       (const double *)d_F_.data(), d_w_.data(), sc, done);
-        LSS_LAUNCH_CHECK();
-    }
+    const double *F = d_F_.data();
+    for (const Level &L : levels_)
+        if (L.nfwd1 > 0) {
+            launch_pdl(mf_forward_kernel, (unsigned)L.nfwd1, 256, 0, st, v, d_ctas_.data() + L.fwd1, gptr_, gsrc_, S, F,
+                       d_w_.data(), sc, done);
+            LSS_LAUNCH_CHECK();
+        }
     for (int h = (int)levels_.size() - 1; h >= 0; --h) {
         const Level &L = levels_[h];
-        launch_pdl(mf_backward_kernel, (unsigned)L.bwd_nr.ctas, 256, 0, st, v, L.bwd_nr, (const double *)d_F_.data(),
-                   (const double *)d_w_.data(), d_x_.data(), sc, done);
+        if (L.nbwd1 == 0) continue;
+        launch_pdl(mf_backward_kernel, (unsigned)L.nbwd1, 256, 0, st, v, d_ctas_.data() + L.bwd1, gptr_, gsrc_, S, F,
+                   (const double *)d_w_.data(), d_x_.data(), sc, z, z32, z_lo, done);
         LSS_LAUNCH_CHECK();
     }
-    launch_pdl(mf_scatter_kernel, (unsigned)((sym_.npos + 255) / 256), 256, 0, st, v, S, (const double *)d_x_.data(),
-               z, z32, z_lo, done);
-    LSS_LAUNCH_CHECK();
 }
 
 void MfFactor::make_pairs(cudaStream_t st)

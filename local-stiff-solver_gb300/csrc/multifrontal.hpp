@@ -72,6 +72,13 @@ struct MfWork {
     const int32_t *cta_item = nullptr;  // optional: per CTA its index i (saves the search)
 };
 
+// One GEMV CTA of the single right-hand-side solve: columns [col0, col0 + ncol)
+// x rows [q0, q0 + nrow) of a front, row chunk kc of nkc.
+struct MfCta {
+    int64_t foff;
+    int32_t s, f, col0, ncol, q0, nrow, kc, nkc, woff, p0, bnd_off, pad;
+};
+
 // The device side: symbolic arrays, front storage, solve vectors, and the
 // per-level work lists of every kernel.
 class MfFactor {
@@ -97,13 +104,16 @@ public:
 
 private:
     struct Level {
-        MfWork ea, small, diag, panel, update, write, mirror, fasm_nr, fwd_nr, bwd_nr, fasm1;
+        MfWork ea, small, diag, panel, update, write, mirror, fasm_nr, fwd_nr, bwd_nr;
         int32_t max_s_large = 0;
+        int64_t fwd1 = 0, bwd1 = 0;  // descriptors of the single right-hand-side solve (into d_ctas_)
+        int32_t nfwd1 = 0, nbwd1 = 0;
     };
     MfSymbolic sym_;
     std::vector<Level> levels_;
     DBuf<int32_t> d_i32_;  // symbolic arrays and work-list fronts
     DBuf<int64_t> d_i64_;  // front offsets and work-list prefixes
+    DBuf<MfCta> d_ctas_;
     DBuf<double> d_F_, d_w_, d_x_, d_P_, d_D_;
     DBuf<float2> d_wb_, d_xb_;  // solve vectors of the batched solve (double-float pairs)
     DBuf<float2> d_Fp_;         // fronts as (hi, lo) FP32 pairs, for the batched solve
@@ -114,7 +124,7 @@ private:
                   *bnd_pos_ = nullptr, *child_off_ = nullptr, *child_ = nullptr, *ea_map_ = nullptr,
                   *front_of_pos_ = nullptr, *pos2j_ = nullptr, *j2pos_ = nullptr, *poff_ = nullptr;
     const int64_t *foff_ = nullptr;
-    const int32_t *gptr_ = nullptr, *gsrc_ = nullptr;  // extend-add gather lists (batched solve)
+    const int32_t *gptr_ = nullptr, *gsrc_ = nullptr;  // extend-add gather lists
 };
 
 }  // namespace lss

@@ -574,6 +574,7 @@ void HybridSolver::setup_stiff()
         d_sinvoff_.release();
         d_sinv_.release();
         d_sinv32_.release();
+        d_swarps_.release();
         d_st_.release();
         mf_ = std::make_unique<MfFactor>();
         h_sdofs_.clear();
@@ -597,6 +598,10 @@ void HybridSolver::setup_stiff()
         stiff_.inv_off = d_sinvoff_.data();
         stiff_.inv = d_sinv_.data();
         stiff_.t = d_st_.data();
+        const std::vector<StiffWarp> warps = stiff_warps(off, inv_off, ndense);
+        d_swarps_.upload(warps, stream_);
+        stiff_.warps = d_swarps_.data();
+        stiff_.nwarps = (int32_t)warps.size();
     }
     stats_["stiff_layout_reused"] = same ? 1.0 : 0.0;
     d_sinv_.zero(stream_);

@@ -134,6 +134,7 @@ private:
     DBuf<int64_t> d_sinvoff_;
     DBuf<double> d_sinv_, d_st_;
     DBuf<float> d_sinv32_;
+    DBuf<StiffWarp> d_swarps_;
     std::unique_ptr<MfFactor> mf_;  // subdomains above STIFF_DENSE_MAX DOFs
     // host copies of the stiff layout (batched solves merge them)
     std::vector<int32_t> h_sdofs_, h_soff_;

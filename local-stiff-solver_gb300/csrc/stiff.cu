@@ -5,8 +5,8 @@
 // (GPUHybrid.cu:993-1411), and applies next_z = z + S^T A_SS^-1 S (r - A z)
 // (dss_precond_iter, GPUHybrid.cu:544-675).  Here a subdomain of up to
 // STIFF_DENSE_MAX DOFs is gathered into a dense FP64 block, inverted in FP64
-// by the symmetric sweep (one CTA in shared memory) and applied as a
-// warp-per-row GEMV fused with the scatter; larger subdomains get the FP64
+// by the symmetric sweep (one CTA in shared memory) and applied as a GEMV
+// fused with the scatter; larger subdomains get the FP64
 // multifrontal factor (multifrontal.cu).  The residual rows r - A z are only
 // computed on the stiff rows (the reference forms the full product and
 // gathers it).
@@ -103,50 +103,67 @@ __global__ void __launch_bounds__(256) invert_small_kernel(const int32_t *__rest
     }
 }
 
-// t_j = r_d (- (A z)_d) for the stiff DOFs d = dofs[j]: one thread per DOF
-// walking its row (a few to a few dozen terms), so no warp reduction -- an FP64
-// shuffle sum would cost the FP64 pipe five full warps per DOF
-template <int BD>
+// t_j = r_d (- (A z)_d) for the stiff DOFs d = dofs[j], LANES threads per DOF
+// (blocks l = lane, lane + LANES, ... of its row; the sums meet by shuffles).
+// The stiff DOFs are few, so this is bound by the latency of the row's chain
+// bounds -> columns -> z: one thread walking a row of 15 blocks took 14 us,
+// eight of them 6; the two or three shuffled FP64 adds cost the pipe less than
+// the row's products.
+template <int BD, int LANES>
 __global__ void __launch_bounds__(256) gather_kernel(BsrDev A, StiffDev S, const double *__restrict__ r,
                                                      const double *__restrict__ z, bool residual, const int *done)
 {
+    const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const int lane = threadIdx.x % LANES;
+    const bool valid = j < S.ndof;
+    const int32_t d = valid ? S.dofs[j] : 0, i = d / BD, comp = d % BD;
+    const int32_t b = valid ? A.rows[i] : 0, len = valid ? A.rows[i + 1] - b : 0;
+    pdl_enter();
     if (done && *done) return;
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= S.ndof) return;
-    const int32_t d = S.dofs[j];
-    double t = r[d];
+    double acc = 0.0;
     if (residual) {
-        const int32_t i = d / BD, comp = d % BD;
-        const int32_t b = A.rows[i], len = A.rows[i + 1] - b;
         const double *v = A.vals + (int64_t)b * BD * BD;
-        double acc = 0.0;
-        for (int32_t l = 0; l < len; ++l) {
+#pragma unroll 2
+        for (int32_t l = lane; l < len; l += LANES) {
             const int32_t c = A.cols[b + l];
 #pragma unroll
             for (int k = 0; k < BD; ++k) acc += v[(int64_t)(comp * BD + k) * len + l] * z[(int64_t)c * BD + k];
         }
-        t -= acc;
+        acc = group_sum<LANES>(acc);
     }
-    S.t[j] = t;
+    if (valid && lane == 0) S.t[j] = r[d] - acc;
 }
 
-// z_S += Inv t over the dense subdomains: one thread per stiff DOF row j,
-// the row read as column j of the transposed storage (consecutive threads,
-// consecutive addresses), the sum in column order -- no FP64 shuffles
+// z_S += Inv t over the dense subdomains, by the warps of StiffDev::warps: a
+// warp takes 32 rows of one subdomain (lane = row, read as a column of the
+// transposed storage, so a load is one line) and one of nsl slices of the
+// columns; the slices' sums meet in shared memory in slice order.  Slices hold
+// at most 24 columns: one thread summing a whole row of up to 160 took 30 to
+// 45 us of dependent loads.
 template <typename VT>
 __global__ void __launch_bounds__(256) apply_kernel(StiffDev S, const VT *__restrict__ inv, double *__restrict__ z,
                                                     float *__restrict__ z32, float *__restrict__ z_lo, const int *done)
 {
+    __shared__ double red[8][32];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const int32_t wi = blockIdx.x * 8 + wl;
+    const StiffWarp w = wi < S.nwarps ? S.warps[wi] : StiffWarp{};
+    const bool row = lane < w.m - w.row0;
+    const int32_t d = row ? S.dofs[w.off + w.row0 + lane] : 0;
+    pdl_enter();
     if (done && *done) return;
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= S.ndof_dense) return;
-    const int32_t s = S.sub_of[j], o = S.off[s], m = S.off[s + 1] - o;
-    const VT *__restrict__ col = inv + S.inv_off[s] + (j - o);
-    const double *__restrict__ t = S.t + o;
     double acc = 0.0;
-#pragma unroll 4
-    for (int32_t q = 0; q < m; ++q) acc += (double)col[(int64_t)q * m] * t[q];
-    const int32_t d = S.dofs[j];
+    if (row) {
+        const VT *__restrict__ col = inv + w.inv_off + w.row0 + lane;
+        const double *__restrict__ t = S.t + w.off;
+        const int32_t q1 = min(w.m, (w.slice + 1) * w.width);
+#pragma unroll 8
+        for (int32_t q = w.slice * w.width; q < q1; ++q) acc += (double)col[(int64_t)q * w.m] * t[q];
+    }
+    red[wl][lane] = acc;
+    __syncthreads();
+    if (!row || w.slice > 0) return;
+    for (int k = 1; k < w.nsl; ++k) acc += red[wl + k][lane];
     const double nz = z[d] + acc;
     z[d] = nz;
     if (z32) {
@@ -205,11 +222,13 @@ void launch_stiff_gather(const BsrDev &A, const StiffDev &S, const double *r, co
                          const int *done, cudaStream_t s)
 {
     if (S.ndof == 0) return;
-    const int grid = (int)(((int64_t)S.ndof + 255) / 256);
+    auto go = [&](auto kernel, int lanes) {
+        launch_pdl(kernel, (unsigned)(((int64_t)S.ndof * lanes + 255) / 256), 256, 0, s, A, S, r, z, residual, done);
+    };
     switch (A.bd) {
-    case 1: gather_kernel<1><<<grid, 256, 0, s>>>(A, S, r, z, residual, done); break;
-    case 2: gather_kernel<2><<<grid, 256, 0, s>>>(A, S, r, z, residual, done); break;
-    default: gather_kernel<3><<<grid, 256, 0, s>>>(A, S, r, z, residual, done); break;
+    case 1: go(gather_kernel<1, 4>, 4); break;
+    case 2: go(gather_kernel<2, 8>, 8); break;
+    default: go(gather_kernel<3, 8>, 8); break;
     }
     LSS_LAUNCH_CHECK();
 }
@@ -217,11 +236,28 @@ void launch_stiff_gather(const BsrDev &A, const StiffDev &S, const double *r, co
 void launch_stiff_apply(const StiffDev &S, bool fp32, double *z, const int *done, cudaStream_t s, float *z32,
                         float *z_lo)
 {
-    if (S.ndof_dense == 0) return;
-    const int grid = (int)(((int64_t)S.ndof_dense + 255) / 256);
-    if (fp32) apply_kernel<float><<<grid, 256, 0, s>>>(S, S.inv32, z, z32, z_lo, done);
-    else apply_kernel<double><<<grid, 256, 0, s>>>(S, S.inv, z, z32, z_lo, done);
+    if (S.nwarps == 0) return;
+    const unsigned grid = (unsigned)((S.nwarps + 7) / 8);
+    if (fp32) launch_pdl(apply_kernel<float>, grid, 256, 0, s, S, S.inv32, z, z32, z_lo, done);
+    else launch_pdl(apply_kernel<double>, grid, 256, 0, s, S, S.inv, z, z32, z_lo, done);
     LSS_LAUNCH_CHECK();
+}
+
+std::vector<StiffWarp> stiff_warps(const std::vector<int32_t> &off, const std::vector<int64_t> &inv_off,
+                                   int32_t ndense)
+{
+    std::vector<StiffWarp> out;
+    // groups of 8, 4, 2, 1 warps in this order: no group straddles a CTA
+    for (int nsl = 8; nsl >= 1; nsl /= 2)
+        for (int32_t s = 0; s < ndense; ++s) {
+            const int32_t m = off[s + 1] - off[s];
+            const int need = m <= 24 ? 1 : (m <= 48 ? 2 : (m <= 96 ? 4 : 8));
+            if (need != nsl) continue;
+            for (int32_t r = 0; r < m; r += 32)
+                for (int k = 0; k < nsl; ++k)
+                    out.push_back({inv_off[s], off[s], m, r, k, nsl, (m + nsl - 1) / nsl});
+        }
+    return out;
 }
 
 }  // namespace lss

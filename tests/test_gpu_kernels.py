@@ -58,3 +58,29 @@ def test_mas_apply_edge_sizes(bs, nb, isolated, built):
         assert np.linalg.norm(z - zo) <= tol * np.linalg.norm(zo), (precision, nb)
         np.testing.assert_array_equal(s.mas_apply(r), z)  # fixed order of every sum
         s.close()
+
+
+@pytest.mark.parametrize("bs", [1, 2, 3])
+@pytest.mark.parametrize("m", [1, 24, 25, 49, 97, 160, 161, 384, 390, 900, 1700])
+def test_stiff_apply_edge_sizes(bs, m, built):
+    """A_SS^-1 r on m given DOFs: every warp split of the dense apply, its
+    limit (160), one multifrontal front, a tree, fronts of several row chunks.
+    Diagonally dominant blocks (condition at most a few hundred): 1e-12 of a
+    dense solve."""
+    nb = 2400 // bs
+    A = block_system(nb, bs, seed=7 * m + bs)
+    dofs = np.arange(5, 5 + m)
+    s = make_solver(bs, extra={"composition": "additive"}, select_bad_dofs_from_l1_norm=False,
+                    decompose_subdomains=False, expand_subdomains=False)
+    s.set_problematic_dofs(dofs)
+    s.factorize(A)
+    np.testing.assert_array_equal(s.selected_dofs(), dofs)
+    r = np.random.default_rng(m).standard_normal(A.shape[0])
+    d = s.precond(r) - s.mas_apply(r)
+    x = np.linalg.solve(A.T[dofs][:, dofs].toarray(), r[dofs])
+    scale = np.linalg.norm(s.mas_apply(r)[dofs])  # the difference cancels the MAS part
+    assert np.linalg.norm(d[dofs] - x) <= 1e-12 * (np.linalg.norm(x) + scale)
+    rest = np.ones(A.shape[0], bool)
+    rest[dofs] = False
+    assert np.all(d[rest] == 0.0)
+    s.close()
