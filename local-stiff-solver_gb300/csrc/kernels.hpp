@@ -47,12 +47,15 @@ struct GmmState {
 
 void launch_row_l1_norms(int32_t n, int64_t nnz, const int32_t *outer, const double *vals, double *rn,
                          cudaStream_t s);
+// resp (optional, n): the responsibilities between the two passes of an EM
+// iteration (recomputed without it, to the same bits); bits (optional,
+// (n + 31) / 32): the selection flags from mark to scatter
 void launch_gmm(int32_t n, const double *rn, GmmState *st, int max_iterations, double tol, GridReduce gr,
-                cudaStream_t s);
+                cudaStream_t s, double2 *resp = nullptr);
 void launch_gmm_mark(int32_t n, const double *rn, const GmmState *st, double threshold, int32_t *block_count,
-                     double *block_margin, cudaStream_t s);
+                     double *block_margin, cudaStream_t s, uint32_t *bits = nullptr);
 void launch_gmm_scatter(int32_t n, const double *rn, const GmmState *st, double threshold,
-                        const int32_t *block_offset, int32_t *out, cudaStream_t s);
+                        const int32_t *block_offset, int32_t *out, cudaStream_t s, const uint32_t *bits = nullptr);
 
 // Gershgorin data of the selected rows (filter_subdomains, GPUHybrid.cu:936-958):
 // for every selected original row k, diag = A_kk and off = sum of |A_kj| over
@@ -181,25 +184,26 @@ struct MasDev {
 
 int64_t mas_tile_elems(int bd);
 
-// Galerkin assembly into per-bank dense N x N FP64 staging (N = 32 bd)
-void launch_mas_assemble0(const BsrDev &A, const int32_t *part_of, const int32_t *part_off, double *stage,
-                          cudaStream_t s);
-// members of the coarse items in chunks (CoarseSpace::memb_rows,
-// item_chunk, chunk_r0), device copies; items are numbered flat over levels
-// 1..L-1
+// Galerkin assembly of the coarse banks into dense N x N FP64 staging (N = 32 bd)
+// members of the coarse items in chunks and the chunks in segments
+// (CoarseSpace), device copies; items are numbered flat over levels 1..L-1
 struct CoarseMembers {
     const int32_t *rows = nullptr;
-    const int32_t *item_chunk = nullptr;  // nitem + 1
+    const int32_t *chunk_item = nullptr;  // nchunk
     const int32_t *chunk_r0 = nullptr;    // nchunk + 1
-    int64_t nitem = 0, nchunk = 0;
+    const int32_t *seg_c0 = nullptr;      // nseg + 1
+    const int32_t *item_seg = nullptr;    // nitem + 1
+    int64_t nitem = 0, nchunk = 0, nseg = 0;
 };
-// partial: nchunk * bd * bd * 32 doubles of scratch
-void launch_mas_assemble_coarse(const BsrDev &A, const MasDev &m, const int32_t *cmap /* nb*(L-1) */,
-                                const CoarseMembers &mb, double *partial, double *stage, cudaStream_t s);
-// pad zero diagonals, invert (symmetric sweep), write bank tiles (FP32 or FP64);
-// uncoupled (optional): per bank, 1 if no entry couples two of its items
-void launch_mas_invert(int bd, int64_t nbanks, const double *stage, void *out, bool fp32, int *bad,
-                       cudaStream_t s, uint8_t *uncoupled = nullptr, bool bf16_offdiag = false);
+// partial: (nchunk + nseg) * bd * bd * 32 doubles of scratch
+void launch_mas_assemble_coarse(const BsrDev &A, const MasDev &m, const CoarseMembers &mb, double *partial,
+                                double *stage, cudaStream_t s);
+// every bank: level 0 gathered from the operator, coarse levels from their
+// staging; pad zero diagonals, invert (symmetric sweep), write bank tiles (FP32
+// or FP64, level 0 optionally with BF16 off-diagonal tiles); uncoupled: per
+// coarse bank, 1 if no entry couples two of its items
+void launch_mas_invert(const BsrDev &A, const MasDev &m, const double *stagec, void *out0, void *outc, bool fp32,
+                       bool bf16_offdiag, int *bad, uint8_t *uncoupled, cudaStream_t s);
 // bytes of one bank with FP32 diagonal and BF16 off-diagonal tiles
 int64_t mas_bank_bytes_bf16(int bd);
 // z = MAS^-1 xin (acc: z += MAS^-1 xin).  dot_mode 1: st->gamma = rdot.z;

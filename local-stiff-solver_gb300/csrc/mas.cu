@@ -99,156 +99,137 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 // ------------------------------------------------------------------ setup
 
+// Galerkin blocks of every coarse level, deterministically, in three passes.
+// Pass 1: one warp per chunk of at most MEMB_CHUNK = 32 member rows of a coarse
+// item ci (its row strip of the bank matrix).  The lanes first look up, for all
+// rows of the chunk together, the bank slot of every block's column item; then
+// 32 / BD^2 groups of BD^2 lanes (one per block entry) add the blocks of a row
+// into the group's own strip in shared memory, and the strips are added in
+// group order.  Pass 2 adds up to SEG_CHUNKS consecutive chunks of an item,
+// pass 3 an item's segments and writes the upper triangle (each entry belongs
+// to exactly one item, so the stores never collide).  Every sum runs in one
+// fixed order (no atomics): two factorizations of the same matrix give
+// bit-identical coarse inverses.
+//
+// An FP64 add costs the pipe a whole warp however few lanes need it: matching
+// lanes by column item and adding them group by group ran 9 adds per block of
+// a row (27 ms on four levels of 1M rows); entry-parallel groups run one per
+// three blocks.
 template <int BD>
-__global__ void __launch_bounds__(256) assemble0_kernel(BsrDev A, const int32_t *__restrict__ part_of,
-                                                        const int32_t *__restrict__ part_off,
-                                                        double *__restrict__ stage)
+__global__ void __launch_bounds__(128) assemble_coarse_chunk_kernel(BsrDev A, MasDev m, CoarseMembers mb,
+                                                                    double *__restrict__ partial)
 {
-    constexpr int N = 32 * BD;
-    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.nb) return;
-    const int32_t p = part_of[i], lo = part_off[p], hi = part_off[p + 1], li = i - lo;
-    double *base = stage + (int64_t)p * N * N;
-    const int32_t b = A.rows[i], len = A.rows[i + 1] - b;
-    const double *v = A.vals + (int64_t)b * BD * BD;
-    for (int32_t l = 0; l < len; ++l) {
-        const int32_t j = A.cols[b + l];
-        if (j < lo || j >= hi) continue;
-        const int32_t lj = j - lo;
-#pragma unroll
-        for (int bi = 0; bi < BD; ++bi)
-#pragma unroll
-            for (int bj = 0; bj < BD; ++bj)
-                base[(int64_t)(bi * 32 + li) * N + bj * 32 + lj] = v[(int64_t)(bi * BD + bj) * len + l];
-    }
-}
-
-// Galerkin blocks of every coarse level, deterministically, in two passes.
-// Pass 1: one warp per chunk of at most MEMB_CHUNK member rows of a coarse
-// item ci (its row strip of the bank matrix), lane c accumulating the BD x BD
-// block of the column items cj with cj % 32 == c.  The chunk's rows come in
-// ascending order and each row's blocks in column order; the blocks of a
-// 32-wide piece whose column item falls into the same bank are handed to
-// their owner lanes one at a time by shuffles.  Pass 2: one warp per item sums
-// its chunks' partial strips in chunk order and writes the upper triangle
-// (each entry belongs to exactly one item, so the stores never collide).
-// Every sum runs in one fixed order (no atomics): two factorizations of the
-// same matrix give bit-identical coarse inverses.
-__device__ __forceinline__ void flat_item(const MasDev &m, int64_t w, int &l, int32_t &ci)
-{
-    l = 1;
-    while (l < m.L && w >= m.nitems[l]) w -= m.nitems[l++];
-    ci = (int32_t)w;
-}
-
-template <int BD>
-__global__ void __launch_bounds__(256) assemble_coarse_chunk_kernel(BsrDev A, MasDev m, const int32_t *__restrict__ cmap,
-                                                                    CoarseMembers mb, double *__restrict__ partial)
-{
-    __shared__ int8_t slot_all[8][32];  // per warp: column slot -> lane holding its group sum
-    const int lane = threadIdx.x & 31;
-    int8_t *slot = slot_all[threadIdx.x >> 5];
-    slot[lane] = -1;
-    __syncwarp();
-    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    constexpr int NE = BD * BD, G = 32 / NE, W = 4;
+    __shared__ double acc_all[W][G * 32 * NE];
+    __shared__ uint8_t slot_all[W][32][32];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * W + wl;
     if (c >= mb.nchunk) return;
-    // the chunk's item: last i with item_chunk[i] <= c
-    int32_t lo = 0, hi = mb.nitem - 1;
-    while (lo < hi) {
-        const int32_t mid = (lo + hi + 1) >> 1;
-        if (mb.item_chunk[mid] <= c) lo = mid;
-        else hi = mid - 1;
+    double *acc = acc_all[wl];
+    uint8_t(*slot)[32] = slot_all[wl];
+    int64_t ci = mb.chunk_item[c];
+    int l = 1;
+    while (l < m.L && ci >= m.nitems[l]) ci -= m.nitems[l++];
+    const int32_t *map = m.cmap + (int64_t)(l - 1) * A.nb;
+    const int32_t bank = (int32_t)(ci >> 5), r0 = mb.chunk_r0[c], nr = mb.chunk_r0[c + 1] - r0;
+    const int32_t row = lane < nr ? mb.rows[r0 + lane] : 0;
+    const int32_t rb = lane < nr ? A.rows[row] : 0, rlen = lane < nr ? A.rows[row + 1] - rb : 0;
+    for (int k = lane; k < G * 32 * NE; k += 32) acc[k] = 0.0;
+    auto lookup = [&](int32_t at) -> uint8_t {  // bank slot of block `at`'s column item, 255 outside the bank
+        const int32_t cj = map[A.cols[at]];
+        return (cj >> 5) == bank ? (uint8_t)(cj & 31) : (uint8_t)255;
+    };
+#pragma unroll 8
+    for (int j = 0; j < nr; ++j) {
+        const int32_t b = __shfl_sync(0xffffffffu, rb, j), len = __shfl_sync(0xffffffffu, rlen, j);
+        if (lane < len) slot[j][lane] = lookup(b + lane);
     }
-    int l;
-    int32_t ci;
-    flat_item(m, lo, l, ci);
-    const int32_t *map = cmap + (int64_t)(l - 1) * A.nb;
-    double acc[BD * BD];
+    __syncwarp();
+    const int grp = lane / NE, k = lane - grp * NE;
+    double *mine = acc + (grp * 32) * NE + k;
+    for (int j = 0; j < nr; ++j) {
+        const int32_t b = __shfl_sync(0xffffffffu, rb, j), len = __shfl_sync(0xffffffffu, rlen, j);
+        if (grp >= G) continue;
+        const double *v = A.vals + (int64_t)b * NE + (int64_t)k * len;
+        int q = grp;
+        for (; q < len && q < 32; q += 4 * G) {  // four values in flight
+            double x[4];
+            uint8_t s[4];
 #pragma unroll
-    for (int k = 0; k < BD * BD; ++k) acc[k] = 0.0;
-    for (int32_t r = mb.chunk_r0[c]; r < mb.chunk_r0[c + 1]; ++r) {
-        const int32_t i = mb.rows[r];
-        const int32_t b = A.rows[i], len = A.rows[i + 1] - b;
-        const double *v = A.vals + (int64_t)b * BD * BD;
-        for (int32_t q0 = 0; q0 < len; q0 += 32) {
-            const int32_t q = q0 + lane;
-            int32_t cj = -1;
-            double val[BD * BD];
-            if (q < len) {
-                cj = map[A.cols[b + q]];
-#pragma unroll
-                for (int k = 0; k < BD * BD; ++k) val[k] = v[(int64_t)k * len + q];
-            } else {
-#pragma unroll
-                for (int k = 0; k < BD * BD; ++k) val[k] = 0.0;
+            for (int t = 0; t < 4; ++t) {
+                const int at = q + t * G;
+                s[t] = at < len && at < 32 ? slot[j][at] : (uint8_t)255;
+                x[t] = s[t] != 255 ? v[at] : 0.0;
             }
-            const bool mine = cj >= 0 && (cj >> 5) == (ci >> 5);
-            if (!__any_sync(0xffffffffu, mine)) continue;
-            // lanes holding the same column item form a group; its leader (lowest
-            // lane) sums the group in lane order, then hands the sum to the lane
-            // that owns the item's slot -- groups proceed in parallel
-            const unsigned grp = __match_any_sync(0xffffffffu, mine ? cj : (int32_t)(0x80000000u | (unsigned)lane));
-            const bool leader = mine && __ffs(grp) - 1 == lane;
-            unsigned rest = mine ? grp & (grp - 1) : 0u;
-            const int rounds = __reduce_max_sync(0xffffffffu, __popc(rest));
-            double gs[BD * BD];
 #pragma unroll
-            for (int k = 0; k < BD * BD; ++k) gs[k] = val[k];
-            for (int it = 0; it < rounds; ++it) {
-                const bool have = rest != 0u;
-                const int src = have ? __ffs(rest) - 1 : lane;
-                rest &= rest - 1u;
-#pragma unroll
-                for (int k = 0; k < BD * BD; ++k) {
-                    const double x = __shfl_sync(0xffffffffu, val[k], src);
-                    if (have) gs[k] += x;
-                }
-            }
-            if (leader) slot[cj & 31] = (int8_t)lane;
-            __syncwarp();
-            const int from = slot[lane];
-            __syncwarp();
-            if (leader) slot[cj & 31] = -1;
-#pragma unroll
-            for (int k = 0; k < BD * BD; ++k) {
-                const double x = __shfl_sync(0xffffffffu, gs[k], from >= 0 ? from : lane);
-                if (from >= 0) acc[k] += x;
-            }
-            __syncwarp();
+            for (int t = 0; t < 4; ++t)
+                if (s[t] != 255) mine[s[t] * NE] += x[t];
+        }
+        for (q = grp + (32 - grp + G - 1) / G * G; q < len; q += G) {  // rows of more than 32 blocks
+            const uint8_t s = lookup(b + q);
+            if (s != 255) mine[s * NE] += v[q];
         }
     }
-    double *out = partial + c * (BD * BD * 32);
+    __syncwarp();
+    // strip entry (slot, k) at [k][slot]
+    double *out = partial + c * (NE * 32);
+    for (int e = lane; e < NE * 32; e += 32) {
+        double sum = 0.0;
 #pragma unroll
-    for (int k = 0; k < BD * BD; ++k) out[k * 32 + lane] = acc[k];
+        for (int g = 0; g < G; ++g) sum += acc[g * 32 * NE + e];
+        out[(e % NE) * 32 + e / NE] = sum;
+    }
+}
+
+// Adds partial strips [ptr[w], ptr[w + 1]) in order; eight strips in flight.
+template <int BD>
+__device__ __forceinline__ void sum_strips(const double *__restrict__ partial, int32_t c0, int32_t c1, int lane,
+                                           double (&acc)[BD * BD])
+{
+#pragma unroll
+    for (int k = 0; k < BD * BD; ++k) acc[k] = 0.0;
+#pragma unroll 4
+    for (int32_t c = c0; c < c1; ++c) {
+        const double *p = partial + (int64_t)c * (BD * BD * 32);
+#pragma unroll
+        for (int k = 0; k < BD * BD; ++k) acc[k] += p[k * 32 + lane];
+    }
+}
+
+template <int BD>
+__global__ void __launch_bounds__(256) assemble_coarse_seg_kernel(CoarseMembers mb, const double *__restrict__ partial,
+                                                                  double *__restrict__ seg)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= mb.nseg) return;
+    double acc[BD * BD];
+    sum_strips<BD>(partial, mb.seg_c0[w], mb.seg_c0[w + 1], lane, acc);
+#pragma unroll
+    for (int k = 0; k < BD * BD; ++k) seg[w * (BD * BD * 32) + k * 32 + lane] = acc[k];
 }
 
 template <int BD>
 __global__ void __launch_bounds__(256) assemble_coarse_sum_kernel(MasDev m, CoarseMembers mb,
-                                                                  const double *__restrict__ partial,
+                                                                  const double *__restrict__ seg,
                                                                   double *__restrict__ stage)
 {
     constexpr int N = 32 * BD;
     const int lane = threadIdx.x & 31;
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= mb.nitem) return;
-    int l;
-    int32_t ci;
-    flat_item(m, w, l, ci);
-    const int32_t g = m.boff[l] + (ci >> 5);
+    int64_t ci = w;
+    int l = 1;
+    while (l < m.L && ci >= m.nitems[l]) ci -= m.nitems[l++];
+    const int64_t g = m.boff[l] + (ci >> 5);
     double acc[BD * BD];
-#pragma unroll
-    for (int k = 0; k < BD * BD; ++k) acc[k] = 0.0;
-    for (int32_t c = mb.item_chunk[w]; c < mb.item_chunk[w + 1]; ++c) {
-        const double *p = partial + (int64_t)c * (BD * BD * 32);
-#pragma unroll
-        for (int k = 0; k < BD * BD; ++k) acc[k] += p[k * 32 + lane];
-    }
-    double *base = stage + (int64_t)g * N * N;
+    sum_strips<BD>(seg, mb.item_seg[w], mb.item_seg[w + 1], lane, acc);
+    double *base = stage + g * N * N;
 #pragma unroll
     for (int bi = 0; bi < BD; ++bi)
 #pragma unroll
         for (int bj = 0; bj < BD; ++bj) {
-            const int row = bi * 32 + (ci & 31), col = bj * 32 + lane;
+            const int row = bi * 32 + (int)(ci & 31), col = bj * 32 + lane;
             if (row <= col) base[(int64_t)row * N + col] = acc[bi * BD + bj];
         }
 }
@@ -307,32 +288,66 @@ __device__ void sweep_invert(double *S, int ld, double *col, double *scol, int *
     }
 }
 
-template <int BD, typename T, bool BF>
-__global__ void __launch_bounds__(256, 2) mas_invert_kernel(const double *__restrict__ stage, T *__restrict__ out,
-                                                         int *bad, uint8_t *__restrict__ uncoupled)
+// One CTA per bank, the level-0 banks (CTAs [0, nparts)) first and the coarse
+// ones after them in the same launch: a few banks are one sweep's latency (215
+// us of dependent pivots), which a launch per level paid twice.  A level-0 bank
+// is gathered straight from the operator's rows; a coarse bank from its dense
+// Galerkin staging (upper triangle).
+template <int BD, typename T, bool BF0>
+__global__ void __launch_bounds__(256, 2) mas_invert_kernel(BsrDev A, const int32_t *__restrict__ part_off,
+                                                            int64_t nparts, void *__restrict__ out0,
+                                                            const double *__restrict__ stagec, T *__restrict__ outc,
+                                                            int *bad, uint8_t *__restrict__ uncoupled)
 {
     constexpr int N = 32 * BD, LD = N + 1;
     extern __shared__ double sm[];
     double *S = sm, *col = sm + N * LD, *scol = col + N;
-    const int64_t bank = blockIdx.x;
-    const double *src = stage + bank * N * N;
-    bool coupled = false;  // an entry between two different items of the bank
-    for (int idx = threadIdx.x; idx < N * N; idx += blockDim.x) {
-        const int r = idx / N, c = idx % N;
-        if (r > c) continue;  // the upper triangle is all the sweep uses
-        double v = src[(int64_t)r * N + c];
-        coupled |= ((r ^ c) & 31) != 0 && v != 0.0;
-        if (r == c && v == 0.0) v = 1.0;  // padding (MASPreconditioner.cu:779-796)
-        S[r * LD + c] = v;
+    const bool fine = (int64_t)blockIdx.x < nparts;
+    const int64_t bank = fine ? blockIdx.x : (int64_t)blockIdx.x - nparts;
+    if (fine) {
+        for (int idx = threadIdx.x; idx < N * LD; idx += blockDim.x) S[idx] = 0.0;
+        __syncthreads();
+        const int32_t lo = part_off[bank], hi = part_off[bank + 1];
+        const int g = threadIdx.x & 7;  // eight threads per block row
+        for (int32_t i = lo + (int32_t)(threadIdx.x >> 3); i < hi; i += (int32_t)(blockDim.x >> 3)) {
+            const int32_t b = A.rows[i], len = A.rows[i + 1] - b;
+            const double *v = A.vals + (int64_t)b * BD * BD;
+            for (int32_t l = g; l < len; l += 8) {
+                const int32_t j = A.cols[b + l];
+                if (j < lo || j >= hi) continue;
+#pragma unroll
+                for (int bi = 0; bi < BD; ++bi)
+#pragma unroll
+                    for (int bj = 0; bj < BD; ++bj) {
+                        const int r = bi * 32 + (i - lo), c = bj * 32 + (j - lo);
+                        if (r <= c) S[r * LD + c] = v[(int64_t)(bi * BD + bj) * len + l];
+                    }
+            }
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < N; t += blockDim.x)
+            if (S[t * LD + t] == 0.0) S[t * LD + t] = 1.0;  // padding (MASPreconditioner.cu:779-796)
+    } else {
+        const double *src = stagec + bank * N * N;
+        bool coupled = false;  // an entry between two different items of the bank
+        for (int idx = threadIdx.x; idx < N * N; idx += blockDim.x) {
+            const int r = idx / N, c = idx % N;
+            if (r > c) continue;  // the upper triangle is all the sweep uses
+            double v = src[(int64_t)r * N + c];
+            coupled |= ((r ^ c) & 31) != 0 && v != 0.0;
+            if (r == c && v == 0.0) v = 1.0;
+            S[r * LD + c] = v;
+        }
+        coupled = __syncthreads_or(coupled);
+        if (threadIdx.x == 0) uncoupled[bank] = coupled ? 0 : 1;
     }
-    coupled = __syncthreads_or(coupled);
-    if (uncoupled && threadIdx.x == 0) uncoupled[bank] = coupled ? 0 : 1;
+    __syncthreads();
     sweep_invert<N>(S, LD, col, scol, bad);
     // the swept entry (i, j), i <= j
     auto entry = [&](int i, int j) -> double { return S[i * LD + j]; };
     // tiles
-    if (BF) {  // FP32 diagonal tiles, BF16 off-diagonal tiles (round to nearest even)
-        unsigned char *dst = reinterpret_cast<unsigned char *>(out) + bank * (int64_t)(BD * 17 * 32 * 4 + BD * (BD - 1) / 2 * 2048);
+    if (BF0 && fine) {  // FP32 diagonal tiles, BF16 off-diagonal tiles (round to nearest even)
+        unsigned char *dst = reinterpret_cast<unsigned char *>(out0) + bank * (int64_t)(BD * 17 * 32 * 4 + BD * (BD - 1) / 2 * 2048);
         for (int c = 0; c < BD; ++c)
             for (int c2 = c; c2 < BD; ++c2) {
                 const int nd = (c == c2) ? 17 : 32;
@@ -349,7 +364,7 @@ __global__ void __launch_bounds__(256, 2) mas_invert_kernel(const double *__rest
             }
         return;
     }
-    T *dst = out + bank * tile_elems<BD>();
+    T *dst = (fine ? reinterpret_cast<T *>(out0) : outc) + bank * tile_elems<BD>();
     int64_t off = 0;
     for (int c = 0; c < BD; ++c)
         for (int c2 = c; c2 < BD; ++c2) {
@@ -736,78 +751,61 @@ void mas_apply_dot_t(const MasDev &m, const T *inv0, const T *invc, T *v, T *u, 
 
 }  // namespace
 
-void launch_mas_assemble0(const BsrDev &A, const int32_t *part_of, const int32_t *part_off, double *stage,
-                          cudaStream_t s)
+template <int BD>
+static void assemble_coarse_t(const BsrDev &A, const MasDev &m, const CoarseMembers &mb, double *partial, double *stage,
+                              cudaStream_t s)
 {
-    const int grid = (int)((A.nb + 255) / 256);
-    if (grid == 0) return;
-    switch (A.bd) {
-    case 1: assemble0_kernel<1><<<grid, 256, 0, s>>>(A, part_of, part_off, stage); break;
-    case 2: assemble0_kernel<2><<<grid, 256, 0, s>>>(A, part_of, part_off, stage); break;
-    default: assemble0_kernel<3><<<grid, 256, 0, s>>>(A, part_of, part_off, stage); break;
-    }
+    double *seg = partial + mb.nchunk * (BD * BD * 32);
+    assemble_coarse_chunk_kernel<BD><<<(unsigned)((mb.nchunk + 3) / 4), 128, 0, s>>>(A, m, mb, partial);
+    assemble_coarse_seg_kernel<BD><<<(unsigned)((mb.nseg + 7) / 8), 256, 0, s>>>(mb, partial, seg);
+    assemble_coarse_sum_kernel<BD><<<(unsigned)((mb.nitem + 7) / 8), 256, 0, s>>>(m, mb, seg, stage);
     LSS_LAUNCH_CHECK();
 }
 
-void launch_mas_assemble_coarse(const BsrDev &A, const MasDev &m, const int32_t *cmap, const CoarseMembers &mb,
-                                double *partial, double *stage, cudaStream_t s)
+void launch_mas_assemble_coarse(const BsrDev &A, const MasDev &m, const CoarseMembers &mb, double *partial,
+                                double *stage, cudaStream_t s)
 {
     if (mb.nitem == 0 || m.L < 2) return;
-    const int g1 = (int)((mb.nchunk * 32 + 255) / 256), g2 = (int)((mb.nitem * 32 + 255) / 256);
-    switch (A.bd) {
-    case 1:
-        assemble_coarse_chunk_kernel<1><<<g1, 256, 0, s>>>(A, m, cmap, mb, partial);
-        assemble_coarse_sum_kernel<1><<<g2, 256, 0, s>>>(m, mb, partial, stage);
-        break;
-    case 2:
-        assemble_coarse_chunk_kernel<2><<<g1, 256, 0, s>>>(A, m, cmap, mb, partial);
-        assemble_coarse_sum_kernel<2><<<g2, 256, 0, s>>>(m, mb, partial, stage);
-        break;
-    default:
-        assemble_coarse_chunk_kernel<3><<<g1, 256, 0, s>>>(A, m, cmap, mb, partial);
-        assemble_coarse_sum_kernel<3><<<g2, 256, 0, s>>>(m, mb, partial, stage);
-        break;
-    }
-    LSS_LAUNCH_CHECK();
+    if (A.bd == 1) assemble_coarse_t<1>(A, m, mb, partial, stage, s);
+    else if (A.bd == 2) assemble_coarse_t<2>(A, m, mb, partial, stage, s);
+    else assemble_coarse_t<3>(A, m, mb, partial, stage, s);
 }
 
-template <int BD, typename T, bool BF = false>
-static void invert_t(int64_t nbanks, const double *stage, T *out, int *bad, uint8_t *uncoupled, cudaStream_t s)
+template <int BD, typename T, bool BF0 = false>
+static void invert_t(const BsrDev &A, const MasDev &m, const double *stagec, void *out0, void *outc, int *bad,
+                     uint8_t *uncoupled, cudaStream_t s)
 {
     constexpr int N = 32 * BD;
     const size_t smem = (size_t)(N * (N + 1) + 2 * N) * sizeof(double);
-    LSS_CUDA(cudaFuncSetAttribute(mas_invert_kernel<BD, T, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    for (int64_t b0 = 0; b0 < nbanks; b0 += 1 << 30) {
-        const int64_t cnt = std::min<int64_t>(nbanks - b0, 1 << 30);
-        T *o = BF ? reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(out) + b0 * mas_bank_bytes_bf16(BD))
-                  : out + b0 * mas_tile_elems(BD);
-        mas_invert_kernel<BD, T, BF><<<(unsigned)cnt, 256, smem, s>>>(stage + b0 * N * N, o, bad,
-                                                                      uncoupled ? uncoupled + b0 : nullptr);
-    }
+    raise_smem_limit((const void *)mas_invert_kernel<BD, T, BF0>, smem);
+    mas_invert_kernel<BD, T, BF0><<<(unsigned)((int64_t)m.nparts + m.ncoarse), 256, smem, s>>>(
+        A, m.part_off, m.nparts, out0, stagec, (T *)outc, bad, uncoupled);
     LSS_LAUNCH_CHECK();
 }
 
-void launch_mas_invert(int bd, int64_t nbanks, const double *stage, void *out, bool fp32, int *bad, cudaStream_t s,
-                       uint8_t *uncoupled, bool bf16_offdiag)
+void launch_mas_invert(const BsrDev &A, const MasDev &m, const double *stagec, void *out0, void *outc, bool fp32,
+                       bool bf16_offdiag, int *bad, uint8_t *uncoupled, cudaStream_t s)
 {
-    if (nbanks == 0) return;
-    if (bf16_offdiag) {
-        if (!fp32) fail(LSS_ERR_INTERNAL, "BF16 off-diagonal tiles need the FP32 MAS");
-        if (bd == 1) invert_t<1, float, true>(nbanks, stage, (float *)out, bad, uncoupled, s);
-        else if (bd == 2) invert_t<2, float, true>(nbanks, stage, (float *)out, bad, uncoupled, s);
-        else invert_t<3, float, true>(nbanks, stage, (float *)out, bad, uncoupled, s);
-        return;
+    if ((int64_t)m.nparts + m.ncoarse == 0) return;
+    if (bf16_offdiag && !fp32) fail(LSS_ERR_INTERNAL, "BF16 off-diagonal tiles need the FP32 MAS");
+#define LSS_INV(...) invert_t<__VA_ARGS__>(A, m, stagec, out0, outc, bad, uncoupled, s)
+    switch (A.bd) {
+    case 1:
+        if (fp32) LSS_INV(1, float);  // one tile: no off-diagonal tiles to store in BF16
+        else LSS_INV(1, double);
+        break;
+    case 2:
+        if (bf16_offdiag) LSS_INV(2, float, true);
+        else if (fp32) LSS_INV(2, float);
+        else LSS_INV(2, double);
+        break;
+    default:
+        if (bf16_offdiag) LSS_INV(3, float, true);
+        else if (fp32) LSS_INV(3, float);
+        else LSS_INV(3, double);
+        break;
     }
-    if (fp32) {
-        if (bd == 1) invert_t<1, float>(nbanks, stage, (float *)out, bad, uncoupled, s);
-        else if (bd == 2) invert_t<2, float>(nbanks, stage, (float *)out, bad, uncoupled, s);
-        else invert_t<3, float>(nbanks, stage, (float *)out, bad, uncoupled, s);
-    } else {
-        if (bd == 1) invert_t<1, double>(nbanks, stage, (double *)out, bad, uncoupled, s);
-        else if (bd == 2) invert_t<2, double>(nbanks, stage, (double *)out, bad, uncoupled, s);
-        else invert_t<3, double>(nbanks, stage, (double *)out, bad, uncoupled, s);
-    }
+#undef LSS_INV
 }
 
 void launch_mas_level0(const MasDev &m, const void *inv0, const void *u, bool fp32, const double *xin, double *z,

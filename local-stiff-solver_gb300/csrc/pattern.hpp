@@ -46,13 +46,14 @@ struct CoarseSpace {
     // deterministic Galerkin assembly
     std::vector<int32_t> memb_ptr, memb_rows;
     std::vector<int64_t> memb_base;               // L entries (level 0 unused)
-    // the members split into chunks of at most MEMB_CHUNK rows (one warp
-    // each); item i (flat over levels 1..L-1) owns chunks
-    // [item_chunk[i], item_chunk[i+1]); chunk c covers memb_rows[chunk_r0[c] ..
-    // chunk_r0[c+1]) -- consecutive chunks of an item are contiguous
-    std::vector<int32_t> item_chunk, chunk_r0;
+    // the members split into chunks of at most MEMB_CHUNK rows (one warp each)
+    // and an item's chunks into segments of at most SEG_CHUNKS; chunk c belongs
+    // to item chunk_item[c] (flat over levels 1..L-1) and covers
+    // memb_rows[chunk_r0[c] .. chunk_r0[c+1]), segment s the chunks
+    // [seg_c0[s], seg_c0[s+1]), item i the segments [item_seg[i], item_seg[i+1])
+    std::vector<int32_t> chunk_item, chunk_r0, seg_c0, item_seg;
 };
-constexpr int32_t MEMB_CHUNK = 128;
+constexpr int32_t MEMB_CHUNK = 32, SEG_CHUNKS = 32;
 
 CoarseSpace build_coarse_space(const Pattern &P, int max_coarse_levels);
 

@@ -8,9 +8,9 @@
 //     changes are below gmm_tol (:795-857);
 //   * jump test |mean1| / |mean0| > threshold, selection {i : g0_i < g1_i}
 //     in ascending order (:859-879).
-// Differences in form, not in result: the responsibilities are recomputed
-// instead of stored (the E-step is a pure function of the row norm and the
-// previous parameters), every reduction is a deterministic fixed-order grid
+// Differences in form, not in result: the responsibilities live from one pass
+// to the next only (or are recomputed: the E-step is a pure function of the row
+// norm and the previous parameters), every reduction is a deterministic fixed-order grid
 // reduction, and the parameters stay on the device between passes (the
 // reference reads every reduction back to the host).
 #include "device_common.cuh"
@@ -46,10 +46,19 @@ __global__ void __launch_bounds__(256) l1_norm_kernel(int32_t n, const int32_t *
 __global__ void __launch_bounds__(256) stats_kernel(int32_t n, const double *__restrict__ rn,
                                                     GmmState *st, GridReduce gr)
 {
-    __shared__ double smin[8], smax[8];
+    __shared__ double smem[32], smin[8], smax[8];
     __shared__ bool last;
     double s[1] = {0.0};
     double mn = INFINITY, mx = -INFINITY;
+    auto cta_minmax = [&]() {  // valid in thread 0
+        mn = warp_min(mn);
+        mx = warp_max(mx);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) { smin[threadIdx.x >> 5] = mn; smax[threadIdx.x >> 5] = mx; }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) { mn = fmin(mn, smin[w]); mx = fmax(mx, smax[w]); }
+    };
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const double x = rn[i];
@@ -57,29 +66,37 @@ __global__ void __launch_bounds__(256) stats_kernel(int32_t n, const double *__r
         mn = fmin(mn, x);
         mx = fmax(mx, x);
     }
-    mn = warp_min(mn);
-    mx = warp_max(mx);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) { smin[wid] = mn; smax[wid] = mx; }
-    __syncthreads();
+    block_sum<1>(s, smem);
+    cta_minmax();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) { mn = fmin(mn, smin[w]); mx = fmax(mx, smax[w]); }
+        gr.partials[blockIdx.x] = s[0];
         gr.partials[GRID_MAX * 2 + blockIdx.x] = mn;
         gr.partials[GRID_MAX * 3 + blockIdx.x] = mx;
+        __threadfence();
+        last = atomicAdd(gr.counter, 1u) == gridDim.x - 1;
     }
-    double tot[1];
-    if (grid_sum<1>(s, gr, tot)) {
-        double gmn = INFINITY, gmx = -INFINITY;
-        for (int b = 0; b < (int)gridDim.x; ++b) {
-            gmn = fmin(gmn, __ldcg(gr.partials + GRID_MAX * 2 + b));
-            gmx = fmax(gmx, __ldcg(gr.partials + GRID_MAX * 3 + b));
-        }
-        st->sum = tot[0];
-        st->mean = tot[0] / n;
-        st->mn = gmn;
-        st->mx = gmx;
+    __syncthreads();
+    if (!last) return;
+    // the last CTA to arrive: all of its threads share the partials (one thread
+    // alone took 100 to 185 us over the minima and maxima of a full grid)
+    __threadfence();
+    s[0] = 0.0;
+    mn = INFINITY;
+    mx = -INFINITY;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+        s[0] += __ldcg(gr.partials + b);
+        mn = fmin(mn, __ldcg(gr.partials + GRID_MAX * 2 + b));
+        mx = fmax(mx, __ldcg(gr.partials + GRID_MAX * 3 + b));
     }
-    (void)last;
+    block_sum<1>(s, smem);
+    cta_minmax();
+    if (threadIdx.x == 0) {
+        st->sum = s[0];
+        st->mean = s[0] / n;
+        st->mn = mn;
+        st->mx = mx;
+        *gr.counter = 0u;
+    }
 }
 
 __global__ void __launch_bounds__(256) var_kernel(int32_t n, const double *__restrict__ rn, GmmState *st,
@@ -112,16 +129,26 @@ __global__ void __launch_bounds__(256) var_kernel(int32_t n, const double *__res
 struct Resp {
     double g0, g1, lg0, lg1;
 };
-__device__ __noinline__ Resp estep(double x, double w0, double w1, double m0, double m1, double v0, double v1)
+// the parameters and the logarithms that every row shares (five of a row's
+// nine transcendentals, and FP64 arithmetic is what the E-step costs)
+struct Mixture {
+    double m0, m1, v0, v1, log_w0, log_w1, half_log0, half_log1;
+    __device__ __forceinline__ Mixture(double w0, double w1, double m0_, double m1_, double v0_, double v1_)
+        : m0(m0_), m1(m1_), v0(v0_), v1(v1_)
+    {
+        const double two_pi = 2.0 * 3.14159265358979323846;
+        log_w0 = log(w0);
+        log_w1 = log(w1);
+        half_log0 = __dmul_rn(-0.5, log(__dmul_rn(two_pi, v0)));
+        half_log1 = __dmul_rn(-0.5, log(__dmul_rn(two_pi, v1)));
+    }
+};
+__device__ __forceinline__ Resp estep(double x, const Mixture &q)
 {
-    const double two_pi = 2.0 * 3.14159265358979323846;
-    const double log_w0 = log(w0), log_w1 = log(w1);
-    const double d0 = __dsub_rn(x, m0), d1 = __dsub_rn(x, m1);
-    const double logN0 = __dsub_rn(__dmul_rn(-0.5, log(__dmul_rn(two_pi, v0))),
-                                   __ddiv_rn(__dmul_rn(__dmul_rn(0.5, d0), d0), v0));
-    const double logN1 = __dsub_rn(__dmul_rn(-0.5, log(__dmul_rn(two_pi, v1))),
-                                   __ddiv_rn(__dmul_rn(__dmul_rn(0.5, d1), d1), v1));
-    const double lg0 = __dadd_rn(log_w0, logN0), lg1 = __dadd_rn(log_w1, logN1);
+    const double d0 = __dsub_rn(x, q.m0), d1 = __dsub_rn(x, q.m1);
+    const double logN0 = __dsub_rn(q.half_log0, __ddiv_rn(__dmul_rn(__dmul_rn(0.5, d0), d0), q.v0));
+    const double logN1 = __dsub_rn(q.half_log1, __ddiv_rn(__dmul_rn(__dmul_rn(0.5, d1), d1), q.v1));
+    const double lg0 = __dadd_rn(q.log_w0, logN0), lg1 = __dadd_rn(q.log_w1, logN1);
     const double mx = fmax(lg0, lg1);
     const double lt = __dadd_rn(mx, log(__dadd_rn(exp(__dsub_rn(lg0, mx)), exp(__dsub_rn(lg1, mx)))));
     Resp r;
@@ -135,15 +162,17 @@ __device__ __noinline__ Resp estep(double x, double w0, double w1, double m0, do
 // pass A: responsibilities with the current parameters; sums of g and g*x;
 // the last CTA performs the weight and mean updates (GPUHybrid.cu:823-833).
 __global__ void __launch_bounds__(256) em_pass_a(int32_t n, const double *__restrict__ rn, GmmState *st,
-                                                 GridReduce gr)
+                                                 GridReduce gr, double2 *__restrict__ resp)
 {
     if (st->converged) return;
     const double w0 = st->w0, w1 = st->w1, m0 = st->m0, m1 = st->m1, v0 = st->v0, v1 = st->v1;
+    const Mixture mix(w0, w1, m0, m1, v0, v1);
     double s[4] = {0.0, 0.0, 0.0, 0.0};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const double x = rn[i];
-        const Resp r = estep(x, w0, w1, m0, m1, v0, v1);
+        const Resp r = estep(x, mix);
+        if (resp) resp[i] = make_double2(r.g0, r.g1);
         s[0] += r.g0;
         s[1] += r.g1;
         s[2] += __dmul_rn(r.g0, x);
@@ -166,19 +195,26 @@ __global__ void __launch_bounds__(256) em_pass_a(int32_t n, const double *__rest
 // responsibilities; the last CTA applies var_reg and the stopping test
 // (GPUHybrid.cu:835-856).
 __global__ void __launch_bounds__(256) em_pass_b(int32_t n, const double *__restrict__ rn, GmmState *st,
-                                                 GridReduce gr, double tol)
+                                                 GridReduce gr, double tol, const double2 *__restrict__ resp)
 {
     if (st->converged) return;
     const double w0 = st->ew0, w1 = st->ew1, m0 = st->em0, m1 = st->em1, v0 = st->ev0, v1 = st->ev1;
     const double nm0 = st->m0, nm1 = st->m1;
+    const Mixture mix(w0, w1, m0, m1, v0, v1);
     double s[2] = {0.0, 0.0};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const double x = rn[i];
-        const Resp r = estep(x, w0, w1, m0, m1, v0, v1);
+        double2 g;
+        if (resp) {
+            g = resp[i];
+        } else {
+            const Resp r = estep(x, mix);
+            g = make_double2(r.g0, r.g1);
+        }
         const double d0 = __dsub_rn(x, nm0), d1 = __dsub_rn(x, nm1);
-        s[0] += __dmul_rn(__dmul_rn(r.g0, d0), d0);
-        s[1] += __dmul_rn(__dmul_rn(r.g1, d1), d1);
+        s[0] += __dmul_rn(__dmul_rn(g.x, d0), d0);
+        s[1] += __dmul_rn(__dmul_rn(g.y, d1), d1);
     }
     double t[2];
     if (grid_sum<2>(s, gr, t)) {
@@ -197,7 +233,7 @@ __global__ void __launch_bounds__(256) em_pass_b(int32_t n, const double *__rest
 __global__ void __launch_bounds__(256) mark_kernel(int32_t n, const double *__restrict__ rn,
                                                    const GmmState *st, double threshold,
                                                    int32_t *__restrict__ block_count,
-                                                   double *__restrict__ block_margin)
+                                                   double *__restrict__ block_margin, uint32_t *__restrict__ bits)
 {
     __shared__ int wcount[8];
     __shared__ double wmargin[8];
@@ -206,14 +242,18 @@ __global__ void __launch_bounds__(256) mark_kernel(int32_t n, const double *__re
     bool flag = false;
     double margin = INFINITY;
     if (i < n && st->esteps > 0) {
-        const Resp r = estep(rn[i], st->ew0, st->ew1, st->em0, st->em1, st->ev0, st->ev1);
+        const Resp r = estep(rn[i], Mixture(st->ew0, st->ew1, st->em0, st->em1, st->ev0, st->ev1));
         flag = jump && (r.g0 < r.g1);
         margin = fabs(r.lg0 - r.lg1);
     }
     const unsigned b = __ballot_sync(0xffffffffu, flag);
     margin = warp_min(margin);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) { wcount[wid] = __popc(b); wmargin[wid] = margin; }
+    if (lane == 0) {
+        wcount[wid] = __popc(b);
+        wmargin[wid] = margin;
+        if (bits && i < n) bits[i >> 5] = b;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         int c = 0;
@@ -227,14 +267,16 @@ __global__ void __launch_bounds__(256) mark_kernel(int32_t n, const double *__re
 __global__ void __launch_bounds__(256) scatter_kernel(int32_t n, const double *__restrict__ rn,
                                                       const GmmState *st, double threshold,
                                                       const int32_t *__restrict__ block_offset,
-                                                      int32_t *__restrict__ out)
+                                                      int32_t *__restrict__ out, const uint32_t *__restrict__ bits)
 {
     __shared__ int wbase[8];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool jump = st->esteps > 0 && fabs(st->m1) / fabs(st->m0) > threshold;
     bool flag = false;
-    if (i < n && jump) {
-        const Resp r = estep(rn[i], st->ew0, st->ew1, st->em0, st->em1, st->ev0, st->ev1);
+    if (bits) {
+        flag = i < n && (bits[i >> 5] >> (i & 31) & 1u);
+    } else if (i < n && jump) {
+        const Resp r = estep(rn[i], Mixture(st->ew0, st->ew1, st->em0, st->em1, st->ev0, st->ev1));
         flag = r.g0 < r.g1;
     }
     const unsigned b = __ballot_sync(0xffffffffu, flag);
@@ -351,33 +393,37 @@ void launch_row_l1_norms(int32_t n, int64_t nnz, const int32_t *outer, const dou
 }
 
 void launch_gmm(int32_t n, const double *rn, GmmState *st, int max_iterations, double tol, GridReduce gr,
-                cudaStream_t s)
+                cudaStream_t s, double2 *resp)
 {
     const int grid = grid_for(n, 256, sm_grid(8));
     stats_kernel<<<grid, 256, 0, s>>>(n, rn, st, gr);
     LSS_LAUNCH_CHECK();
     var_kernel<<<grid, 256, 0, s>>>(n, rn, st, gr);
     LSS_LAUNCH_CHECK();
+    // up to four 64-thread CTAs per SM while they hold every row: the E-step is
+    // bound by the FP64 pipe of the SMs it runs on, and 3000 rows in 256-thread
+    // CTAs used 12 of them (28 us a pass)
+    const int threads = n <= sm_grid(4) * 64 ? 64 : 256, egrid = grid_for(n, threads, sm_grid(8));
     for (int it = 0; it < max_iterations; ++it) {
-        em_pass_a<<<grid, 256, 0, s>>>(n, rn, st, gr);
-        em_pass_b<<<grid, 256, 0, s>>>(n, rn, st, gr, tol);
+        em_pass_a<<<egrid, threads, 0, s>>>(n, rn, st, gr, resp);
+        em_pass_b<<<egrid, threads, 0, s>>>(n, rn, st, gr, tol, resp);
     }
     LSS_LAUNCH_CHECK();
 }
 
 void launch_gmm_mark(int32_t n, const double *rn, const GmmState *st, double threshold, int32_t *block_count,
-                     double *block_margin, cudaStream_t s)
+                     double *block_margin, cudaStream_t s, uint32_t *bits)
 {
     const int grid = (int)((n + 255) / 256);
-    if (grid > 0) mark_kernel<<<grid, 256, 0, s>>>(n, rn, st, threshold, block_count, block_margin);
+    if (grid > 0) mark_kernel<<<grid, 256, 0, s>>>(n, rn, st, threshold, block_count, block_margin, bits);
     LSS_LAUNCH_CHECK();
 }
 
 void launch_gmm_scatter(int32_t n, const double *rn, const GmmState *st, double threshold,
-                        const int32_t *block_offset, int32_t *out, cudaStream_t s)
+                        const int32_t *block_offset, int32_t *out, cudaStream_t s, const uint32_t *bits)
 {
     const int grid = (int)((n + 255) / 256);
-    if (grid > 0) scatter_kernel<<<grid, 256, 0, s>>>(n, rn, st, threshold, block_offset, out);
+    if (grid > 0) scatter_kernel<<<grid, 256, 0, s>>>(n, rn, st, threshold, block_offset, out, bits);
     LSS_LAUNCH_CHECK();
 }
 

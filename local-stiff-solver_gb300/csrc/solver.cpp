@@ -200,20 +200,24 @@ void HybridSolver::analyze(int32_t n, int64_t nnz, const int32_t *outer, const i
     // MAS device maps
     const int32_t nparts = (int32_t)pat_.part.part_offsets.size() - 1;
     d_part_off_.upload(pat_.part.part_offsets, stream_);
-    d_part_of_.upload(cs_.part_of, stream_);
     d_key0_.upload(cs_.key0, stream_);
     d_ccnt0_.upload(cs_.ccnt0, stream_);
     d_cbase0_.upload(cs_.cbase0, stream_);
     d_cmap_.upload(cs_.cmap, stream_);
-    d_memb_ptr_.upload(cs_.item_chunk, stream_);
+    d_chunk_item_.upload(cs_.chunk_item, stream_);
+    d_seg_c0_.upload(cs_.seg_c0, stream_);
+    d_item_seg_.upload(cs_.item_seg, stream_);
     d_memb_rows_.upload(cs_.memb_rows, stream_);
     d_chunk_r0_.upload(cs_.chunk_r0, stream_);
     memb_ = CoarseMembers();
     memb_.rows = d_memb_rows_.data();
-    memb_.item_chunk = d_memb_ptr_.data();
+    memb_.chunk_item = d_chunk_item_.data();
     memb_.chunk_r0 = d_chunk_r0_.data();
-    memb_.nitem = (int64_t)cs_.item_chunk.size() - 1;
-    memb_.nchunk = (int64_t)cs_.chunk_r0.size() - 1;
+    memb_.seg_c0 = d_seg_c0_.data();
+    memb_.item_seg = d_item_seg_.data();
+    memb_.nitem = (int64_t)cs_.item_seg.size() - 1;
+    memb_.nchunk = (int64_t)cs_.chunk_item.size();
+    memb_.nseg = (int64_t)cs_.seg_c0.size() - 1;
     d_key_.clear();
     d_ccnt_.clear();
     d_cbase_.clear();
@@ -390,11 +394,14 @@ void HybridSolver::select_stiff(const CscView &A)
         st.zero(stream_);
         if (d_outer_.size() != (size_t)n + 1) d_outer_.upload(h_outer_, stream_);
         launch_row_l1_norms(n, A.nnz, d_outer_.data(), d_csc_.data(), rn.data(), stream_);
-        launch_gmm(n, rn.data(), st.data(), p_.max_gmm_iterations, p_.gmm_tol, gr_, stream_);
+        DBuf<double2> resp(n);
+        DBuf<uint32_t> bits(((size_t)n + 31) / 32);
+        launch_gmm(n, rn.data(), st.data(), p_.max_gmm_iterations, p_.gmm_tol, gr_, stream_, resp.data());
         const int nblk = (n + 255) / 256;
         DBuf<int32_t> bcount(nblk), boffs(nblk);
         DBuf<double> bmargin(nblk);
-        launch_gmm_mark(n, rn.data(), st.data(), p_.jump_threshold, bcount.data(), bmargin.data(), stream_);
+        launch_gmm_mark(n, rn.data(), st.data(), p_.jump_threshold, bcount.data(), bmargin.data(), stream_,
+                        bits.data());
         std::vector<int32_t> hc = bcount.download(stream_);
         std::vector<double> hm = bmargin.download(stream_);
         std::vector<GmmState> hs = st.download(stream_);
@@ -410,7 +417,8 @@ void HybridSolver::select_stiff(const CscView &A)
         if (total > 0) {
             boffs.upload(ho, stream_);
             DBuf<int32_t> out(total);
-            launch_gmm_scatter(n, rn.data(), st.data(), p_.jump_threshold, boffs.data(), out.data(), stream_);
+            launch_gmm_scatter(n, rn.data(), st.data(), p_.jump_threshold, boffs.data(), out.data(), stream_,
+                               bits.data());
             sel = out.download(stream_);
         }
         const GmmState &g = hs[0];
@@ -703,23 +711,16 @@ void HybridSolver::setup_mas()
     d_inv0_.resize(bf ? (size_t)(nparts * mas_.bank_bytes0) : (size_t)(nparts * te * esz));
     d_invc_.resize(std::max<int64_t>(ncoarse, 1) * te * esz);
     d_bad_.zero(stream_);
-    // the dense staging of the Galerkin blocks stays allocated across the
-    // factorizations of a pattern (no cudaMalloc / cudaFree of GBs per step)
-    {
-        // level 0 (no atomics: every entry comes from its own row)
-        d_stage0_.resize((size_t)nparts * N * N);
-        d_stage0_.zero(stream_);
-        launch_mas_assemble0(A_, d_part_of_.data(), d_part_off_.data(), d_stage0_.data(), stream_);
-        launch_mas_invert(bd, nparts, d_stage0_.data(), d_inv0_.data(), mas_fp32_, d_bad_.data(), stream_, nullptr, bf);
-    }
+    // the dense staging of the coarse Galerkin blocks stays allocated across the
+    // factorizations of a pattern (no cudaMalloc / cudaFree per step)
     if (ncoarse > 0) {
         d_stagec_.resize((size_t)ncoarse * N * N);
         d_stagec_.zero(stream_);
-        d_cpartial_.resize((size_t)std::max<int64_t>(memb_.nchunk, 1) * bd * bd * 32);
-        launch_mas_assemble_coarse(A_, mas_, d_cmap_.data(), memb_, d_cpartial_.data(), d_stagec_.data(), stream_);
-        launch_mas_invert(bd, ncoarse, d_stagec_.data(), d_invc_.data(), mas_fp32_, d_bad_.data(), stream_,
-                          d_uncoupled_.data());
+        d_cpartial_.resize((size_t)std::max<int64_t>(memb_.nchunk + memb_.nseg, 1) * bd * bd * 32);
+        launch_mas_assemble_coarse(A_, mas_, memb_, d_cpartial_.data(), d_stagec_.data(), stream_);
     }
+    launch_mas_invert(A_, mas_, d_stagec_.data(), d_inv0_.data(), d_invc_.data(), mas_fp32_, bf, d_bad_.data(),
+                      d_uncoupled_.data(), stream_);
     int bad = 0;
     LSS_CUDA(cudaMemcpyAsync(&bad, d_bad_.data(), sizeof(int), cudaMemcpyDeviceToHost, stream_));
     LSS_CUDA(cudaStreamSynchronize(stream_));

@@ -119,14 +119,15 @@ private:
     DBuf<int64_t> d_src_;
     // MAS
     MasDev mas_;
-    DBuf<int32_t> d_part_off_, d_cbase0_, d_part_of_, d_cmap_, d_memb_ptr_, d_memb_rows_, d_chunk_r0_;
+    DBuf<int32_t> d_part_off_, d_cbase0_, d_cmap_, d_chunk_item_, d_seg_c0_, d_item_seg_, d_memb_rows_,
+        d_chunk_r0_;
     CoarseMembers memb_;
     DBuf<uint8_t> d_key0_, d_ccnt0_, d_uncoupled_;
     DBuf<unsigned> d_need_, d_arrive_;  // coarse banks: contributing banks below, arrivals of an apply
     std::vector<DBuf<uint8_t>> d_key_, d_ccnt_;
     std::vector<DBuf<int32_t>> d_cbase_;
     DBuf<char> d_inv0_, d_invc_, d_v_, d_u_;
-    DBuf<double> d_stage0_, d_stagec_, d_cpartial_;  // MAS Galerkin staging, kept per pattern
+    DBuf<double> d_stagec_, d_cpartial_;  // coarse Galerkin staging, kept per pattern
     bool mas_fp32_ = false;
     // stiff blocks
     StiffDev stiff_;
