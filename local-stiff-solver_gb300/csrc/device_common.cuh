@@ -14,16 +14,15 @@
 namespace lss {
 
 // Programmatic dependent launch: a kernel launched by launch_pdl may be
-// dispatched while its predecessor in the stream still runs; pdl_enter lets
-// the next launch be dispatched at once and waits for the predecessor's
-// completion (and memory) -- the launch latency overlaps the predecessor's tail
-// instead of adding to it.  Before pdl_enter a kernel may only read what no
-// kernel of the running sequence writes.
-__device__ __forceinline__ void pdl_enter()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// dispatched once every CTA of its predecessor in the stream has ended, ahead
+// of the flush and launch latency between two dependent grids (2 to 6% of a
+// solve of up to 100k DOFs).  pdl_enter waits for the predecessor's completion
+// and memory; before it a kernel may only read what no kernel of the running
+// sequence writes.  No kernel lets its successor in earlier
+// (griddepcontrol.launch_dependents): waiting CTAs then fill the SMs that
+// drain first and pile up there, which took a 648k-DOF FP64 solve from 214 to
+// 311 ms.
+__device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
 void launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
@@ -112,6 +111,40 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], GridReduce gr, double 
         return true;
     }
     return false;
+}
+
+// The PCG's scalar sums.  The kernel that forms the addends leaves the sum's
+// parts with put_sum; the next kernel that needs the scalar adds them in every
+// CTA with get_sum.  PcgSum::direct: one part per CTA, nothing else -- the
+// fence, counter and last-CTA tail of grid_sum cost 3 to 4 us at the end of a
+// kernel, the consumer's sum 0.6 us at its start.  Otherwise grid_sum leaves
+// one part: with many CTAs per SM summing, the parts' FP64 adds would cost the
+// pipe more than the tail (PCG_DIRECT_ROWS).
+__device__ __forceinline__ void put_sum(double v, GridReduce gr, PcgSum out)
+{
+    double a[1] = {v};
+    if (out.direct) {
+        __shared__ double smem[32];
+        block_sum<1>(a, smem);
+        if (threadIdx.x == 0) out.part[blockIdx.x] = a[0];
+        return;
+    }
+    double tot[1];
+    if (grid_sum<1>(a, gr, tot)) out.part[0] = tot[0];
+}
+
+// the sum, in every thread of the CTA (all of them must call it)
+__device__ __forceinline__ double get_sum(PcgSum in)
+{
+    if (in.count == 1) return __ldcg(in.part);
+    __shared__ double smem[32];
+    double a[1] = {0.0};
+    for (int i = threadIdx.x; i < in.count; i += blockDim.x) a[0] += __ldcg(in.part + i);
+    block_sum<1>(a, smem);
+    __syncthreads();
+    if (threadIdx.x == 0) smem[0] = a[0];
+    __syncthreads();
+    return smem[0];
 }
 
 // Grid-wide min/max (deterministic, order independent).

@@ -28,6 +28,16 @@ struct GridReduce {
     unsigned *counter = nullptr; // one arrival counter
 };
 
+// A scalar sum of the PCG between the kernel that forms it and those that use
+// it (device_common.cuh): `count` parts.
+struct PcgSum {
+    double *part = nullptr;  // GRID_MAX
+    int count = 1;
+    int direct = 0;          // one part per CTA of the producing kernel
+};
+// consumers of at most two CTAs per SM add the parts themselves
+constexpr int64_t PCG_DIRECT_ROWS = 2 * 152 * 1024;
+
 inline int grid_for(long long work_items, int items_per_cta, int max_ctas)
 {
     long long g = (work_items + items_per_cta - 1) / items_per_cta;
@@ -110,38 +120,41 @@ constexpr int PCG_HIST = 64;  // alpha / beta history kept for the Lanczos estim
 
 struct PcgState {
     double bb, gamma, alpha, beta, pAp, rr, rel_eps, abs_eps;
+    double rz;  // r.z of the current residual; gamma is the one that alpha was formed from
     int iter, done, max_iter, pad;
     double hist_alpha[PCG_HIST], hist_beta[PCG_HIST];
 };
 
 void launch_dot(int64_t n, const double *a, const double *b, double *out, GridReduce gr, cudaStream_t s);
-// Ap = A p; pAp = p.Ap; alpha = gamma / pAp with the reference's breakdown tests
-void launch_pcg_spmv_alpha(const BsrDev &A, const double *p, double *Ap, PcgState *st, GridReduce gr,
-                           cudaStream_t s);
-// x += alpha p; r -= alpha Ap; rr = r.r; convergence tests
-// r32 (optional): also r rounded to FP32
+// Ap = A p and the parts of p.Ap
+void launch_pcg_spmv_alpha(const BsrDev &A, const double *p, double *Ap, const PcgState *st, GridReduce gr,
+                           PcgSum &pap, cudaStream_t s);
+// alpha = r.z / p.Ap with the reference's breakdown tests; x += alpha p;
+// r -= alpha Ap; the parts of r.r.  r32 (optional): also r rounded to FP32
 void launch_pcg_update_xr(int64_t n, double *x, double *r, const double *p, const double *Ap, PcgState *st,
-                          GridReduce gr, cudaStream_t s, float *r32 = nullptr);
+                          GridReduce gr, PcgSum pap, PcgSum &rr, cudaStream_t s, float *r32 = nullptr);
 // the same with A p as df32 (hi, lo) pairs
 void launch_pcg_update_xr_df(int64_t n, double *x, double *r, const double *p, const float2 *Ap_df, PcgState *st,
-                             GridReduce gr, cudaStream_t s, float *r32 = nullptr);
+                             GridReduce gr, PcgSum pap, PcgSum &rr, cudaStream_t s, float *r32 = nullptr);
 void launch_df_to_double(int64_t n, const float2 *src, double *dst, cudaStream_t s);
 // the damping estimate's probe, v_i = ((i * 2654435761) mod 2^32) / 2^32 - 0.5 over
 // original indices i, written in the permuted order
 void launch_probe(int64_t nb, int bd, const int32_t *perm, double *dst, cudaStream_t s);
-// p = z + beta p
+// beta = r.z / gamma; p = z + beta p (first: p = z)
 // p_df (optional): the df32 split of the new p, the x operand of the df32 SpMV
-void launch_pcg_update_p(int64_t n, double *p, const double *z, const PcgState *st, cudaStream_t s,
+void launch_pcg_update_p(int64_t n, double *p, const double *z, PcgState *st, PcgSum rz, bool first, cudaStream_t s,
                          float2 *p_df = nullptr);
 // dst = (fl32(src), fl32(src - fl32(src)))
 void launch_split(int64_t n, const double *src, float2 *dst, cudaStream_t s);
-// Ap = A p, p.Ap and alpha like launch_pcg_spmv_alpha, with the products and
+// Ap = A p and p.Ap like launch_pcg_spmv_alpha, with the products and
 // row sums in double-float arithmetic on the FP32 pipe: A and p as (hi, lo)
 // FP32 pairs (both to 2^-48 relative), error-free products and sums
 // (TwoProd / TwoSum), the result rounded to FP64 once per row component.
-void launch_pcg_spmv_alpha_df(const BsrDev &A, const float2 *p_df, float2 *Ap_df, PcgState *st, GridReduce gr,
-                              cudaStream_t s);
-void launch_copy(int64_t n, const double *src, double *dst, const int *done, cudaStream_t s);
+void launch_pcg_spmv_alpha_df(const BsrDev &A, const float2 *p_df, float2 *Ap_df, const PcgState *st, GridReduce gr,
+                              PcgSum &pap, cudaStream_t s);
+// the parts of r.z
+void launch_pcg_rz(int64_t n, const double *r, const double *z, const PcgState *st, GridReduce gr, PcgSum &rz,
+                   cudaStream_t s);
 void launch_permute(int64_t nb, int bd, const int32_t *perm, const double *src, double *dst, bool to_new,
                     cudaStream_t s);
 void launch_grad_pattern(int32_t n, const int32_t *outer, const int32_t *inner, const double *lambda,
@@ -206,15 +219,15 @@ void launch_mas_invert(const BsrDev &A, const MasDev &m, const double *stagec, v
                        bool bf16_offdiag, int *bad, uint8_t *uncoupled, cudaStream_t s);
 // bytes of one bank with FP32 diagonal and BF16 off-diagonal tiles
 int64_t mas_bank_bytes_bf16(int bd);
-// z = MAS^-1 xin (acc: z += MAS^-1 xin).  dot_mode 1: st->gamma = rdot.z;
-// dot_mode 2: st->beta = rdot.z / st->gamma, st->gamma = rdot.z.
-// z = scale * MAS^-1 xin, or z += scale * MAS^-1 xin with acc.
+// z = scale * MAS^-1 xin, or z += scale * MAS^-1 xin with acc; rz (optional):
+// the parts of rdot.z.  rr (optional): the sum of the residual just updated,
+// against which the first launch tests for convergence (GPUHybrid.cu:1488-1496).
 // z32 (optional): also store z rounded to FP32 (the input of the FP32 residual)
 // and, with z_lo, the remainder z - z32 rounded to FP32.
 // xin32 (optional, FP32 MAS only): an FP32 input used in place of xin.
 void launch_mas_apply(const MasDev &m, const void *inv0, const void *invc, void *v, void *u, bool fp32,
                       const double *xin, double *z, bool acc, double scale, const double *rdot, PcgState *st,
-                      int dot_mode, GridReduce gr, const int *done, cudaStream_t s, float *z32 = nullptr,
+                      const PcgSum *rr, PcgSum *rz, GridReduce gr, cudaStream_t s, float *z32 = nullptr,
                       const float *xin32 = nullptr, float *z_lo = nullptr);
 
 // level-0 bank SYMV alone (z = Inv_0 xin + coarse correction already in u), for timing

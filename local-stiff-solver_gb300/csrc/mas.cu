@@ -427,9 +427,23 @@ __device__ __forceinline__ void bank_segment_sums(const T *xs, uint8_t key, unsi
 // CTAs that hold a clamped face -- 235 us instead of 100 on 648k DOFs.)
 template <int BD, typename T, typename XT>
 __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__restrict__ r, T *__restrict__ v,
-                                                       const int *done)
+                                                       PcgState *st, PcgSum rr)
 {
-    if (done && *done) return;
+    pdl_enter();
+    if (st && st->done) return;
+    if (rr.part) {  // the updated residual's convergence tests (GPUHybrid.cu:1488-1496)
+        const double t = get_sum(rr);
+        int stop = STOP_RUNNING;
+        if (!(t == t) || isinf(t)) stop = STOP_NONFINITE;
+        else if (st->rel_eps > 0 && t / st->bb < st->rel_eps) stop = STOP_CONVERGED_REL;
+        else if (st->abs_eps > 0 && t < st->abs_eps) stop = STOP_CONVERGED_ABS;
+        else if (st->iter >= st->max_iter) stop = STOP_MAX_ITER;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            st->rr = t;
+            if (stop) st->done = stop;
+        }
+        if (stop) return;
+    }
     constexpr int N = 32 * BD, W = 8;
     __shared__ T xs_all[W][N];
     __shared__ unsigned mask_all[W][32];
@@ -518,15 +532,16 @@ __global__ void __launch_bounds__(256) symv_coarse_kernel(MasDev m, const T *__r
                                                           const T *__restrict__ v, T *__restrict__ u,
                                                           const int *done)
 {
-    if (done && *done) return;
     constexpr int N = 32 * BD, W = 8;
     __shared__ T xs[N];
     __shared__ T red[W][N];
     const int tid = threadIdx.x, lane = tid & 31, wl = tid >> 5;
     const int64_t g = blockIdx.x;
     const int o = (tid % BD) * 32 + tid / BD;  // component-major place of element tid
-    if (tid < N) xs[o] = v[g * N + tid];
     const bool uncoupled = m.uncoupled[g];
+    pdl_enter();
+    if (done && *done) return;
+    if (tid < N) xs[o] = v[g * N + tid];
     __syncthreads();
     T y[BD];
     const TileLd<T, false> ld{reinterpret_cast<const unsigned char *>(invc + g * m.tile_elems)};
@@ -579,14 +594,13 @@ constexpr int bank_stages()
     return (BF ? 4 : (int)sizeof(T)) * tile_elems<BD>() * BankGroup<BD>::GB <= 20480 ? 2 : 1;
 }
 
-template <int BD, typename T, bool ACC, int DOT, typename XT, bool BF = false>
+template <int BD, typename T, bool ACC, bool DOT, typename XT, bool BF = false>
 __global__ void __launch_bounds__(128) symv0_kernel(MasDev m, const T *__restrict__ inv0, const T *__restrict__ u,
                                                     const XT *__restrict__ xin, double *__restrict__ z,
-                                                    double scale, const double *__restrict__ rdot, PcgState *st,
+                                                    double scale, const double *__restrict__ rdot, PcgSum rz,
                                                     GridReduce gr, const int *done, float *__restrict__ z32,
                                                     float *__restrict__ z_lo)
 {
-    if (done && *done) return;
     constexpr int N = 32 * BD, WB = BankGroup<BD>::WB, GB = BankGroup<BD>::GB;
     constexpr int BANK_B = bank_bytes<BD, BF>(sizeof(T)), STAGE_B = BANK_B * GB, NST = bank_stages<BD, T, BF>();
     extern __shared__ __align__(16) unsigned char stage[];
@@ -632,20 +646,30 @@ __global__ void __launch_bounds__(128) symv0_kernel(MasDev m, const T *__restric
         for (int l = 1; l < MAS_MAXL; ++l) o.item[l - 1] = ok && l < m.L ? m.cmap[(int64_t)(l - 1) * m.nb + i] : 0;
         return o;
     };
-    double dot[1] = {0.0};
+    double dot = 0.0;
     int64_t g = blockIdx.x;
     const int64_t step = gridDim.x;
     int cur = 0;
+    // the inverses and maps do not change within a solve: their first loads need
+    // not wait for the preceding kernel
+    constexpr int AHEAD = NST > 1 ? NST - 1 : 1;
 #pragma unroll
-    for (int q = 0; q < NST - 1; ++q) {
+    for (int q = 0; q < AHEAD; ++q) {
         if (g + q * step < ngroups) fill(q, g + q * step);
         cp_async_commit();
     }
-    Operand o = operand(bounds(g));
+    const Bounds b0 = bounds(g);
     Bounds nb = bounds(g + step);
+    pdl_enter();
+    if (done && *done) {
+        cp_async_wait<0>();
+        return;
+    }
+    Operand o = operand(b0);
     for (; g < ngroups; g += step) {
         const int64_t gf = g + (NST - 1) * step;
-        if (gf < ngroups) fill(cur + NST - 1 < NST ? cur + NST - 1 : cur - 1, gf);
+        if (gf < ngroups && (NST > 1 || g != (int64_t)blockIdx.x))
+            fill(cur + NST - 1 < NST ? cur + NST - 1 : cur - 1, gf);
         cp_async_commit();
         if (bk < GB) xs[bk][comp * 32 + node] = (T)o.x;
         T cu[MAS_MAXL - 1];
@@ -677,23 +701,12 @@ __global__ void __launch_bounds__(128) symv0_kernel(MasDev m, const T *__restric
                 z32[o.e] = h;
                 if (z_lo) z_lo[o.e] = (float)(val - (double)h);
             }
-            if (DOT) dot[0] += o.rd * val;
+            if (DOT) dot += o.rd * val;
         }
         o = nx;
         cur = cur + 1 < NST ? cur + 1 : 0;
     }
-    if (DOT) {
-        double tot[1];
-        if (grid_sum<1>(dot, gr, tot)) {
-            // DOT == 1: initial gamma (GPUHybrid.cu:1450-1451); DOT == 2: new gamma and
-            // beta = gamma_new / gamma_old (GPUHybrid.cu:1501-1504)
-            if (DOT == 2) {
-                st->beta = tot[0] / st->gamma;
-                if (st->iter >= 1 && st->iter <= PCG_HIST) st->hist_beta[st->iter - 1] = st->beta;
-            }
-            st->gamma = tot[0];
-        }
-    }
+    if (DOT) put_sum(dot, gr, rz);
 }
 
 // Grid of a level-0 launch: every resident CTA, at most one per bank group.
@@ -706,44 +719,46 @@ int symv0_grid(int64_t nparts)
     return grid_for(nparts, GB, sm_grid(per_sm));
 }
 
-template <int BD, typename T, bool ACC, int DOT, typename XT, bool BF>
+template <int BD, typename T, bool ACC, bool DOT, typename XT, bool BF>
 void symv0_launch(const MasDev &m, const T *inv0, const T *u, const XT *xin, double *z, double scale,
-                  const double *rdot, PcgState *st, GridReduce gr, const int *done, cudaStream_t s, float *z32,
+                  const double *rdot, PcgSum *rz, GridReduce gr, const int *done, cudaStream_t s, float *z32,
                   float *z_lo)
 {
     const size_t smem = (size_t)bank_stages<BD, T, BF>() * bank_bytes<BD, BF>(sizeof(T)) * BankGroup<BD>::GB;
+    const int grid = symv0_grid<BD, T, BF>(m.nparts);
+    if (rz) {
+        rz->direct = (int64_t)m.nb * BD <= PCG_DIRECT_ROWS;
+        rz->count = rz->direct ? grid : 1;
+    }
     raise_smem_limit((const void *)symv0_kernel<BD, T, ACC, DOT, XT, BF>, smem);
-    symv0_kernel<BD, T, ACC, DOT, XT, BF><<<symv0_grid<BD, T, BF>(m.nparts), 128, smem, s>>>(
-        m, inv0, u, xin, z, scale, rdot, st, gr, done, z32, z_lo);
+    launch_pdl(symv0_kernel<BD, T, ACC, DOT, XT, BF>, grid, 128, smem, s, m, inv0, u, xin, z, scale, rdot,
+               rz ? *rz : PcgSum{}, gr, done, z32, z_lo);
 }
 
 template <int BD, typename T, typename XT>
 void mas_apply_dot_t(const MasDev &m, const T *inv0, const T *invc, T *v, T *u, const XT *xin, double *z,
-                     bool acc, double scale, const double *rdot, PcgState *st, int dot_mode, GridReduce gr,
-                     const int *done, cudaStream_t s, float *z32, float *z_lo)
+                     bool acc, double scale, const double *rdot, PcgState *st, const PcgSum *rr, PcgSum *rz,
+                     GridReduce gr, cudaStream_t s, float *z32, float *z_lo)
 {
-    if (m.L > 1)
-    {
-        restrict_kernel<BD, T, XT><<<grid_for(m.nparts, 8, sm_grid(8)), 256, 0, s>>>(m, xin, v, done);
-        symv_coarse_kernel<BD, T><<<(unsigned)m.ncoarse, 256, 0, s>>>(m, invc, v, u, done);
-    }
+    if (m.L < 2) fail(LSS_ERR_INTERNAL, "a MAS hierarchy has at least one coarse level");
+    const int *done = &st->done;
+    launch_pdl(restrict_kernel<BD, T, XT>, grid_for(m.nparts, 8, sm_grid(8)), 256, 0, s, m, xin, v, st,
+               rr ? *rr : PcgSum{});
+    launch_pdl(symv_coarse_kernel<BD, T>, (unsigned)m.ncoarse, 256, 0, s, m, invc, (const T *)v, u, done);
 #define LSS_S0(A_, D_)                                                                                          \
     do {                                                                                                        \
         if (std::is_same<T, float>::value && m.bank_bytes0 > 0)                                                 \
-            symv0_launch<BD, T, A_, D_, XT, std::is_same<T, float>::value>(m, inv0, u, xin, z, scale, rdot, st, \
+            symv0_launch<BD, T, A_, D_, XT, std::is_same<T, float>::value>(m, inv0, u, xin, z, scale, rdot, rz, \
                                                                            gr, done, s, z32, z_lo);             \
         else                                                                                                    \
-            symv0_launch<BD, T, A_, D_, XT, false>(m, inv0, u, xin, z, scale, rdot, st, gr, done, s, z32, z_lo); \
+            symv0_launch<BD, T, A_, D_, XT, false>(m, inv0, u, xin, z, scale, rdot, rz, gr, done, s, z32, z_lo); \
     } while (0)
-    if (dot_mode == 0) {
-        if (acc) LSS_S0(true, 0);
-        else LSS_S0(false, 0);
-    } else if (dot_mode == 1) {
-        if (acc) LSS_S0(true, 1);
-        else LSS_S0(false, 1);
+    if (rz) {
+        if (acc) LSS_S0(true, true);
+        else LSS_S0(false, true);
     } else {
-        if (acc) LSS_S0(true, 2);
-        else LSS_S0(false, 2);
+        if (acc) LSS_S0(true, false);
+        else LSS_S0(false, false);
     }
 #undef LSS_S0
     LSS_LAUNCH_CHECK();
@@ -813,10 +828,10 @@ void launch_mas_level0(const MasDev &m, const void *inv0, const void *u, bool fp
 {
     GridReduce gr{};
 #define LSS_L0(BD_, T_)                                                                                          \
-    symv0_launch<BD_, T_, false, 0, double, false>(m, (const T_ *)inv0, (const T_ *)u, xin, z, 1.0, nullptr, nullptr, \
+    symv0_launch<BD_, T_, false, false, double, false>(m, (const T_ *)inv0, (const T_ *)u, xin, z, 1.0, nullptr, nullptr, \
                                                    gr, nullptr, s, nullptr, nullptr)
 #define LSS_L0BF(BD_)                                                                                            \
-    symv0_launch<BD_, float, false, 0, double, true>(m, (const float *)inv0, (const float *)u, xin, z, 1.0, nullptr, \
+    symv0_launch<BD_, float, false, false, double, true>(m, (const float *)inv0, (const float *)u, xin, z, 1.0, nullptr, \
                                                      nullptr, gr, nullptr, s, nullptr, nullptr)
     if (fp32 && m.bank_bytes0 > 0) {
         if (m.bd == 2) LSS_L0BF(2);
@@ -837,15 +852,15 @@ void launch_mas_level0(const MasDev &m, const void *inv0, const void *u, bool fp
 
 void launch_mas_apply(const MasDev &m, const void *inv0, const void *invc, void *v, void *u, bool fp32,
                       const double *xin, double *z, bool acc, double scale, const double *rdot, PcgState *st,
-                      int dot_mode, GridReduce gr, const int *done, cudaStream_t s, float *z32, const float *xin32,
+                      const PcgSum *rr, PcgSum *rz, GridReduce gr, cudaStream_t s, float *z32, const float *xin32,
                       float *z_lo)
 {
 #define LSS_MAS(BD_, T_)                                                                                          \
     mas_apply_dot_t<BD_, T_, double>(m, (const T_ *)inv0, (const T_ *)invc, (T_ *)v, (T_ *)u, xin, z, acc, scale, \
-                                     rdot, st, dot_mode, gr, done, s, z32, z_lo)
+                                     rdot, st, rr, rz, gr, s, z32, z_lo)
 #define LSS_MAS32(BD_)                                                                                            \
     mas_apply_dot_t<BD_, float, float>(m, (const float *)inv0, (const float *)invc, (float *)v, (float *)u, xin32, \
-                                       z, acc, scale, rdot, st, dot_mode, gr, done, s, z32, z_lo)
+                                       z, acc, scale, rdot, st, rr, rz, gr, s, z32, z_lo)
     if (xin32) {
         if (!fp32) fail(LSS_ERR_INTERNAL, "an FP32 input needs the FP32 MAS");
         if (m.bd == 1) LSS_MAS32(1);

@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(256) residual_kernel(BsrDev A, const VT *__res
                                                        const double *__restrict__ r, const XT *__restrict__ x,
                                                        double *__restrict__ y, const int *done)
 {
+    pdl_enter();
     if (done && *done) return;
     const int lane = threadIdx.x % LANES;
     constexpr int RPW = 32 / LANES;  // block rows per warp and sweep
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(256) residual32_kernel(BsrDev A, const float *
                                                          const double *__restrict__ r64,
                                                          const float *__restrict__ x_lo, const int *done)
 {
+    pdl_enter();
     if (done && *done) return;
     const int lane = threadIdx.x % LANES;
     constexpr int RPW = 32 / LANES;
@@ -131,17 +133,19 @@ __global__ void __launch_bounds__(256) residual32_kernel(BsrDev A, const float *
     }
 }
 
-// Ap = A p, p.Ap, then alpha with the breakdown tests (GPUHybrid.cu:1458-1480)
+// Ap = A p and p.Ap (GPUHybrid.cu:1458-1462)
 template <int BD, int LANES>
 __global__ void __launch_bounds__(256) spmv_alpha_kernel(BsrDev A, const double *__restrict__ p,
-                                                         double *__restrict__ Ap, PcgState *st, GridReduce gr)
+                                                         double *__restrict__ Ap, const PcgState *st, GridReduce gr,
+                                                         PcgSum pap)
 {
+    pdl_enter();
     if (st->done) return;
     const int lane = threadIdx.x % LANES;
     constexpr int RPW = 32 / LANES;  // block rows per warp and sweep
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    double dot[1] = {0.0};
+    double dot = 0.0;
     // warp-uniform trip count: every lane reaches the group shuffles together
     for (int64_t wr = w0 * RPW; wr < A.nb; wr += nw * RPW) {
         const int64_t i = wr + (threadIdx.x & 31) / LANES;
@@ -153,67 +157,77 @@ __global__ void __launch_bounds__(256) spmv_alpha_kernel(BsrDev A, const double 
             for (int k = 0; k < BD; ++k)
                 if (k % LANES == lane) {
                     Ap[i * BD + k] = acc[k];
-                    dot[0] += p[i * BD + k] * acc[k];
+                    dot += p[i * BD + k] * acc[k];
                 }
         }
     }
-    double tot[1];
-    if (grid_sum<1>(dot, gr, tot)) {
-        st->iter += 1;
-        const double pAp = tot[0];
-        st->pAp = pAp;
-        if (pAp == 0.0) { st->done = STOP_ZERO_PAP; return; }
-        const double alpha = st->gamma / pAp;
-        if (!(alpha == alpha) || isinf(alpha)) { st->done = STOP_NONFINITE; return; }
-        if (alpha <= 0.0) { st->done = STOP_NEGATIVE_ALPHA; return; }
-        if (alpha < DBL_MIN) { st->done = STOP_SUBNORMAL_ALPHA; return; }
-        st->alpha = alpha;
-        if (st->iter <= PCG_HIST) st->hist_alpha[st->iter - 1] = alpha;
-    }
+    put_sum(dot, gr, pap);
 }
 
-// x += alpha p; r -= alpha Ap; rr; convergence (GPUHybrid.cu:1482-1496)
 __device__ __forceinline__ double as_double(double v) { return v; }
 __device__ __forceinline__ double as_double(float2 v) { return (double)v.x + (double)v.y; }
 
-// AT: double, or float2 for the (hi, lo) product of the df32 SpMV.  r32
-// (optional): r rounded to FP32, the input of the mixed preconditioner's
-// FP32 residual -- converted here, where every lane of a warp converts one
-// entry (a partly predicated FP64 instruction costs the pipe a full warp).
+// alpha with the breakdown tests; x += alpha p; r -= alpha Ap; r.r
+// (GPUHybrid.cu:1463-1487).  Every CTA forms alpha from the parts of p.Ap, the
+// first one records the iteration's scalars.  AT: double, or float2 for the
+// (hi, lo) product of the df32 SpMV.  r32 (optional): r rounded to FP32, the
+// input of the mixed preconditioner's FP32 residual -- converted here, where
+// every lane of a warp converts one entry (a partly predicated FP64
+// instruction costs the pipe a full warp).
 template <typename AT>
 __global__ void __launch_bounds__(256) update_xr_kernel(int64_t n, double *__restrict__ x, double *__restrict__ r,
                                                         const double *__restrict__ p, const AT *__restrict__ Ap,
-                                                        PcgState *st, GridReduce gr, float *__restrict__ r32)
+                                                        PcgState *st, GridReduce gr, PcgSum pap, PcgSum rr,
+                                                        float *__restrict__ r32)
 {
+    pdl_enter();
     if (st->done) return;
-    const double alpha = st->alpha;
-    double s[1] = {0.0};
+    const double gamma = st->rz, pAp = get_sum(pap), alpha = gamma / pAp;
+    int stop = STOP_RUNNING;
+    if (pAp == 0.0) stop = STOP_ZERO_PAP;
+    else if (!(alpha == alpha) || isinf(alpha)) stop = STOP_NONFINITE;
+    else if (alpha <= 0.0) stop = STOP_NEGATIVE_ALPHA;
+    else if (alpha < DBL_MIN) stop = STOP_SUBNORMAL_ALPHA;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const int it = st->iter + 1;
+        st->iter = it;
+        st->pAp = pAp;
+        st->gamma = gamma;
+        if (stop) st->done = stop;
+        else {
+            st->alpha = alpha;
+            if (it <= PCG_HIST) st->hist_alpha[it - 1] = alpha;
+        }
+    }
+    if (stop) return;
+    double s = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         x[i] += alpha * p[i];
         const double ri = r[i] - alpha * as_double(Ap[i]);
         r[i] = ri;
         if (r32) r32[i] = (float)ri;
-        s[0] += ri * ri;
+        s += ri * ri;
     }
-    double tot[1];
-    if (grid_sum<1>(s, gr, tot)) {
-        const double rr = tot[0];
-        st->rr = rr;
-        if (!(rr == rr) || isinf(rr)) { st->done = STOP_NONFINITE; return; }
-        if (st->rel_eps > 0 && rr / st->bb < st->rel_eps) { st->done = STOP_CONVERGED_REL; return; }
-        if (st->abs_eps > 0 && rr < st->abs_eps) { st->done = STOP_CONVERGED_ABS; return; }
-        if (st->iter >= st->max_iter) { st->done = STOP_MAX_ITER; return; }
-    }
+    put_sum(s, gr, rr);
 }
 
-// p = z + beta p (GPUHybrid.cu:1506-1507); optionally also its df32 split
+// beta = r.z / gamma, p = z + beta p (GPUHybrid.cu:1501-1507), first: p = z;
+// optionally also the df32 split of p
 __global__ void __launch_bounds__(256) update_p_kernel(int64_t n, double *__restrict__ p, const double *__restrict__ z,
-                                                       const PcgState *st, float2 *__restrict__ p_df)
+                                                       PcgState *st, PcgSum rz, bool first, float2 *__restrict__ p_df)
 {
+    pdl_enter();
     if (st->done) return;
-    const double beta = st->beta;
+    const double g = get_sum(rz), beta = first ? 0.0 : g / st->gamma;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->rz = g;
+        if (!first) {
+            st->beta = beta;
+            if (st->iter >= 1 && st->iter <= PCG_HIST) st->hist_beta[st->iter - 1] = beta;
+        }
+    }
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = z[i] + beta * p[i];
+        const double v = first ? z[i] : z[i] + beta * p[i];
         p[i] = v;
         if (p_df) {
             const float h = (float)v;
@@ -237,8 +251,10 @@ __global__ void split_kernel(int64_t n, const double *__restrict__ src, float2 *
 // run them as partly predicated warps, each costing the FP64 pipe a full warp.
 template <int BD, int LANES>
 __global__ void __launch_bounds__(256) spmv_alpha_df_kernel(BsrDev A, const float2 *__restrict__ p_df,
-                                                            float2 *__restrict__ Ap, PcgState *st, GridReduce gr)
+                                                            float2 *__restrict__ Ap, const PcgState *st, GridReduce gr,
+                                                            PcgSum pap)
 {
+    pdl_enter();
     if (st->done) return;
     const int lane = threadIdx.x % LANES;
     constexpr int RPW = 32 / LANES;
@@ -260,20 +276,7 @@ __global__ void __launch_bounds__(256) spmv_alpha_df_kernel(BsrDev A, const floa
                 }
         }
     }
-    double dot[1] = {(double)dh + (double)dl};
-    double tot[1];
-    if (grid_sum<1>(dot, gr, tot)) {
-        st->iter += 1;
-        const double pAp = tot[0];
-        st->pAp = pAp;
-        if (pAp == 0.0) { st->done = STOP_ZERO_PAP; return; }
-        const double alpha = st->gamma / pAp;
-        if (!(alpha == alpha) || isinf(alpha)) { st->done = STOP_NONFINITE; return; }
-        if (alpha <= 0.0) { st->done = STOP_NEGATIVE_ALPHA; return; }
-        if (alpha < DBL_MIN) { st->done = STOP_SUBNORMAL_ALPHA; return; }
-        st->alpha = alpha;
-        if (st->iter <= PCG_HIST) st->hist_alpha[st->iter - 1] = alpha;
-    }
+    put_sum((double)dh + (double)dl, gr, pap);
 }
 
 __global__ void __launch_bounds__(256) dot_kernel(int64_t n, const double *__restrict__ a, const double *__restrict__ b,
@@ -284,13 +287,6 @@ __global__ void __launch_bounds__(256) dot_kernel(int64_t n, const double *__res
         s[0] += a[i] * b[i];
     double tot[1];
     if (grid_sum<1>(s, gr, tot)) *out = tot[0];
-}
-
-__global__ void copy_kernel(int64_t n, const double *__restrict__ src, double *__restrict__ dst, const int *done)
-{
-    if (done && *done) return;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = src[i];
 }
 
 __global__ void permute_kernel(int64_t nb, int bd, const int32_t *__restrict__ perm, const double *__restrict__ src,
@@ -319,22 +315,15 @@ __global__ void grad_pattern_kernel(int32_t n, const int32_t *__restrict__ outer
     }
 }
 
-// gamma bookkeeping from r.z: mode 1 initial gamma, mode 2 beta and new gamma
 __global__ void __launch_bounds__(256) rz_kernel(int64_t n, const double *__restrict__ r, const double *__restrict__ z,
-                                                 PcgState *st, int mode, GridReduce gr)
+                                                 const PcgState *st, GridReduce gr, PcgSum rz)
 {
+    pdl_enter();
     if (st->done) return;
-    double s[1] = {0.0};
+    double s = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        s[0] += r[i] * z[i];
-    double tot[1];
-    if (grid_sum<1>(s, gr, tot)) {
-        if (mode == 2) {
-            st->beta = tot[0] / st->gamma;
-            if (st->iter >= 1 && st->iter <= PCG_HIST) st->hist_beta[st->iter - 1] = st->beta;
-        }
-        st->gamma = tot[0];
-    }
+        s += r[i] * z[i];
+    put_sum(s, gr, rz);
 }
 
 __global__ void check_finite_kernel(int64_t n, const double *__restrict__ v, int *flag)
@@ -415,27 +404,38 @@ void residual_dispatch(const BsrDev &A, const VT *vals, const double *r, const X
     const int lanes = sizeof(VT) == 4 ? A.lanes32 : A.lanes;
     const int grid = grid_for((int64_t)A.nb * lanes, 256, sm_grid(16));
     switch (lanes) {
-    case 1: residual_kernel<BD, 1, VT, ACC, XT><<<grid, 256, 0, s>>>(A, vals, r, x, y, done); break;
-    case 2: residual_kernel<BD, 2, VT, ACC, XT><<<grid, 256, 0, s>>>(A, vals, r, x, y, done); break;
-    case 4: residual_kernel<BD, 4, VT, ACC, XT><<<grid, 256, 0, s>>>(A, vals, r, x, y, done); break;
-    case 8: residual_kernel<BD, 8, VT, ACC, XT><<<grid, 256, 0, s>>>(A, vals, r, x, y, done); break;
-    case 16: residual_kernel<BD, 16, VT, ACC, XT><<<grid, 256, 0, s>>>(A, vals, r, x, y, done); break;
-    default: residual_kernel<BD, 32, VT, ACC, XT><<<grid, 256, 0, s>>>(A, vals, r, x, y, done); break;
+    case 1: launch_pdl(residual_kernel<BD, 1, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
+    case 2: launch_pdl(residual_kernel<BD, 2, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
+    case 4: launch_pdl(residual_kernel<BD, 4, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
+    case 8: launch_pdl(residual_kernel<BD, 8, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
+    case 16: launch_pdl(residual_kernel<BD, 16, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
+    default: launch_pdl(residual_kernel<BD, 32, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
     }
 }
 
+// marks `sum` as produced by a launch of `grid` CTAs over n rows
+void produced(PcgSum &sum, int64_t n, int grid)
+{
+    sum.direct = n <= PCG_DIRECT_ROWS;
+    sum.count = sum.direct ? grid : 1;
+}
+
 template <int BD>
-void spmv_alpha_dispatch(const BsrDev &A, const double *p, double *Ap, PcgState *st, GridReduce gr, cudaStream_t s)
+void spmv_alpha_dispatch(const BsrDev &A, const double *p, double *Ap, const PcgState *st, GridReduce gr, PcgSum &pap,
+                         cudaStream_t s)
 {
     const int grid = grid_for((int64_t)A.nb * A.lanes, 256, sm_grid(16));
+    produced(pap, (int64_t)A.nb * BD, grid);
+#define LSS_SA(L_) launch_pdl(spmv_alpha_kernel<BD, L_>, grid, 256, 0, s, A, p, Ap, st, gr, pap)
     switch (A.lanes) {
-    case 1: spmv_alpha_kernel<BD, 1><<<grid, 256, 0, s>>>(A, p, Ap, st, gr); break;
-    case 2: spmv_alpha_kernel<BD, 2><<<grid, 256, 0, s>>>(A, p, Ap, st, gr); break;
-    case 4: spmv_alpha_kernel<BD, 4><<<grid, 256, 0, s>>>(A, p, Ap, st, gr); break;
-    case 8: spmv_alpha_kernel<BD, 8><<<grid, 256, 0, s>>>(A, p, Ap, st, gr); break;
-    case 16: spmv_alpha_kernel<BD, 16><<<grid, 256, 0, s>>>(A, p, Ap, st, gr); break;
-    default: spmv_alpha_kernel<BD, 32><<<grid, 256, 0, s>>>(A, p, Ap, st, gr); break;
+    case 1: LSS_SA(1); break;
+    case 2: LSS_SA(2); break;
+    case 4: LSS_SA(4); break;
+    case 8: LSS_SA(8); break;
+    case 16: LSS_SA(16); break;
+    default: LSS_SA(32); break;
     }
+#undef LSS_SA
 }
 
 }  // namespace
@@ -470,7 +470,7 @@ void residual32_dispatch(const BsrDev &A, const float *r32, const float *x32, fl
                          const double *r64, const float *x_lo, const int *done, cudaStream_t s)
 {
     const int grid = grid_for((int64_t)A.nb * A.lanes32, 256, sm_grid(16));
-#define LSS_R32(L_) residual32_kernel<BD, L_><<<grid, 256, 0, s>>>(A, r32, x32, y32, precise, r64, x_lo, done)
+#define LSS_R32(L_) launch_pdl(residual32_kernel<BD, L_>, grid, 256, 0, s, A, r32, x32, y32, precise, r64, x_lo, done)
     switch (A.lanes32) {
     case 1: LSS_R32(1); break;
     case 2: LSS_R32(2); break;
@@ -501,37 +501,41 @@ void launch_dot(int64_t n, const double *a, const double *b, double *out, GridRe
     LSS_LAUNCH_CHECK();
 }
 
-void launch_pcg_spmv_alpha(const BsrDev &A, const double *p, double *Ap, PcgState *st, GridReduce gr, cudaStream_t s)
+void launch_pcg_spmv_alpha(const BsrDev &A, const double *p, double *Ap, const PcgState *st, GridReduce gr,
+                           PcgSum &pap, cudaStream_t s)
 {
-    if (A.bd == 1) spmv_alpha_dispatch<1>(A, p, Ap, st, gr, s);
-    else if (A.bd == 2) spmv_alpha_dispatch<2>(A, p, Ap, st, gr, s);
-    else spmv_alpha_dispatch<3>(A, p, Ap, st, gr, s);
+    if (A.bd == 1) spmv_alpha_dispatch<1>(A, p, Ap, st, gr, pap, s);
+    else if (A.bd == 2) spmv_alpha_dispatch<2>(A, p, Ap, st, gr, pap, s);
+    else spmv_alpha_dispatch<3>(A, p, Ap, st, gr, pap, s);
     LSS_LAUNCH_CHECK();
 }
 
 template <int BD>
-void spmv_alpha_df_dispatch(const BsrDev &A, const float2 *pd, float2 *Ap, PcgState *st, GridReduce gr,
-                            cudaStream_t s)
+void spmv_alpha_df_dispatch(const BsrDev &A, const float2 *pd, float2 *Ap, const PcgState *st, GridReduce gr,
+                            PcgSum &pap, cudaStream_t s)
 {
     const int grid = grid_for((int64_t)A.nb * A.lanes, 256, sm_grid(16));
+    produced(pap, (int64_t)A.nb * BD, grid);
+#define LSS_SA(L_) launch_pdl(spmv_alpha_df_kernel<BD, L_>, grid, 256, 0, s, A, pd, Ap, st, gr, pap)
     switch (A.lanes) {
-    case 1: spmv_alpha_df_kernel<BD, 1><<<grid, 256, 0, s>>>(A, pd, Ap, st, gr); break;
-    case 2: spmv_alpha_df_kernel<BD, 2><<<grid, 256, 0, s>>>(A, pd, Ap, st, gr); break;
-    case 4: spmv_alpha_df_kernel<BD, 4><<<grid, 256, 0, s>>>(A, pd, Ap, st, gr); break;
-    case 8: spmv_alpha_df_kernel<BD, 8><<<grid, 256, 0, s>>>(A, pd, Ap, st, gr); break;
-    case 16: spmv_alpha_df_kernel<BD, 16><<<grid, 256, 0, s>>>(A, pd, Ap, st, gr); break;
-    default: spmv_alpha_df_kernel<BD, 32><<<grid, 256, 0, s>>>(A, pd, Ap, st, gr); break;
+    case 1: LSS_SA(1); break;
+    case 2: LSS_SA(2); break;
+    case 4: LSS_SA(4); break;
+    case 8: LSS_SA(8); break;
+    case 16: LSS_SA(16); break;
+    default: LSS_SA(32); break;
     }
+#undef LSS_SA
 }
 
-void launch_pcg_spmv_alpha_df(const BsrDev &A, const float2 *p_df, float2 *Ap_df, PcgState *st, GridReduce gr,
-                              cudaStream_t s)
+void launch_pcg_spmv_alpha_df(const BsrDev &A, const float2 *p_df, float2 *Ap_df, const PcgState *st, GridReduce gr,
+                              PcgSum &pap, cudaStream_t s)
 {
     if (A.nb > 0 && (!A.vals_df || !p_df || !Ap_df))
         fail(LSS_ERR_INTERNAL, "df32 SpMV launched without its operand arrays");
-    if (A.bd == 1) spmv_alpha_df_dispatch<1>(A, p_df, Ap_df, st, gr, s);
-    else if (A.bd == 2) spmv_alpha_df_dispatch<2>(A, p_df, Ap_df, st, gr, s);
-    else spmv_alpha_df_dispatch<3>(A, p_df, Ap_df, st, gr, s);
+    if (A.bd == 1) spmv_alpha_df_dispatch<1>(A, p_df, Ap_df, st, gr, pap, s);
+    else if (A.bd == 2) spmv_alpha_df_dispatch<2>(A, p_df, Ap_df, st, gr, pap, s);
+    else spmv_alpha_df_dispatch<3>(A, p_df, Ap_df, st, gr, pap, s);
     LSS_LAUNCH_CHECK();
 }
 
@@ -575,28 +579,27 @@ void launch_split(int64_t n, const double *src, float2 *dst, cudaStream_t s)
 }
 
 void launch_pcg_update_xr(int64_t n, double *x, double *r, const double *p, const double *Ap, PcgState *st,
-                          GridReduce gr, cudaStream_t s, float *r32)
+                          GridReduce gr, PcgSum pap, PcgSum &rr, cudaStream_t s, float *r32)
 {
-    update_xr_kernel<double><<<grid_for(n, 1024, sm_grid(16)), 256, 0, s>>>(n, x, r, p, Ap, st, gr, r32);
+    const int grid = grid_for(n, 1024, sm_grid(16));
+    produced(rr, n, grid);
+    launch_pdl(update_xr_kernel<double>, grid, 256, 0, s, n, x, r, p, Ap, st, gr, pap, rr, r32);
     LSS_LAUNCH_CHECK();
 }
 
 void launch_pcg_update_xr_df(int64_t n, double *x, double *r, const double *p, const float2 *Ap_df, PcgState *st,
-                             GridReduce gr, cudaStream_t s, float *r32)
+                             GridReduce gr, PcgSum pap, PcgSum &rr, cudaStream_t s, float *r32)
 {
-    update_xr_kernel<float2><<<grid_for(n, 1024, sm_grid(16)), 256, 0, s>>>(n, x, r, p, Ap_df, st, gr, r32);
+    const int grid = grid_for(n, 1024, sm_grid(16));
+    produced(rr, n, grid);
+    launch_pdl(update_xr_kernel<float2>, grid, 256, 0, s, n, x, r, p, Ap_df, st, gr, pap, rr, r32);
     LSS_LAUNCH_CHECK();
 }
 
-void launch_pcg_update_p(int64_t n, double *p, const double *z, const PcgState *st, cudaStream_t s, float2 *p_df)
+void launch_pcg_update_p(int64_t n, double *p, const double *z, PcgState *st, PcgSum rz, bool first, cudaStream_t s,
+                         float2 *p_df)
 {
-    update_p_kernel<<<grid_for(n, 1024, sm_grid(16)), 256, 0, s>>>(n, p, z, st, p_df);
-    LSS_LAUNCH_CHECK();
-}
-
-void launch_copy(int64_t n, const double *src, double *dst, const int *done, cudaStream_t s)
-{
-    copy_kernel<<<grid_for(n, 1024, sm_grid(16)), 256, 0, s>>>(n, src, dst, done);
+    launch_pdl(update_p_kernel, grid_for(n, 1024, sm_grid(16)), 256, 0, s, n, p, z, st, rz, first, p_df);
     LSS_LAUNCH_CHECK();
 }
 
@@ -607,10 +610,12 @@ void launch_permute(int64_t nb, int bd, const int32_t *perm, const double *src, 
     LSS_LAUNCH_CHECK();
 }
 
-void launch_pcg_rz(int64_t n, const double *r, const double *z, PcgState *st, int dot_mode, GridReduce gr,
+void launch_pcg_rz(int64_t n, const double *r, const double *z, const PcgState *st, GridReduce gr, PcgSum &rz,
                    cudaStream_t s)
 {
-    rz_kernel<<<grid_for(n, 1024, sm_grid(16)), 256, 0, s>>>(n, r, z, st, dot_mode, gr);
+    const int grid = grid_for(n, 1024, sm_grid(16));
+    produced(rz, n, grid);
+    launch_pdl(rz_kernel, grid, 256, 0, s, n, r, z, st, gr, rz);
     LSS_LAUNCH_CHECK();
 }
 

@@ -25,8 +25,6 @@
 
 namespace lss {
 
-void launch_pcg_rz(int64_t n, const double *r, const double *z, PcgState *st, int dot_mode, GridReduce gr,
-                   cudaStream_t s);
 void launch_check_finite(int64_t n, const double *v, int *flag, cudaStream_t s);
 
 namespace {
@@ -69,6 +67,10 @@ HybridSolver::HybridSolver(const Params &p) : p_(p)
     d_bad_.resize(1);
     gr_.partials = d_partials_.data();
     gr_.counter = d_counter_.data();
+    d_sums_.resize((size_t)3 * GRID_MAX);
+    pap_.part = d_sums_.data();
+    rr_.part = d_sums_.data() + GRID_MAX;
+    rz_.part = d_sums_.data() + 2 * GRID_MAX;
 }
 
 HybridSolver::~HybridSolver()
@@ -752,32 +754,28 @@ void HybridSolver::ensure_vectors()
 
 // ------------------------------------------------------------------ preconditioner
 
-void HybridSolver::mas_apply(const double *xin, double *z, bool acc, const double *rdot, int dot_mode, double scale,
+void HybridSolver::mas_apply(const double *xin, double *z, bool acc, const double *rdot, double scale, bool test,
                              float *z32, const float *xin32, float *z_lo)
 {
     launch_mas_apply(mas_, d_inv0_.data(), d_invc_.data(), d_v_.data(), d_u_.data(), mas_fp32_, xin, z, acc, scale,
-                     rdot, d_state_.data(), dot_mode, gr_, &d_state_.data()->done, stream_, z32, xin32, z_lo);
+                     rdot, d_state_.data(), test ? &rr_ : nullptr, rdot ? &rz_ : nullptr, gr_, stream_, z32, xin32,
+                     z_lo);
 }
 
-void HybridSolver::rz_dot(const double *r, const double *z, int dot_mode)
-{
-    launch_pcg_rz(n_vec(), r, z, d_state_.data(), dot_mode, gr_, stream_);
-}
-
-// z = M^-1 r.  dot_mode 0: nothing; 1: gamma = r.z; 2: beta, gamma update.
-void HybridSolver::precond(const double *r, double *z, int dot_mode, const float *r32)
+// z = M^-1 r
+void HybridSolver::precond(const double *r, double *z, bool dot, const float *r32, bool test)
 {
     const int *done = &d_state_.data()->done;
     const bool stiff = p_.do_hybrid && stiff_.ndof > 0 && !lanczos_mode_;
     if (!stiff) {  // GPUHybrid.cu:523-527
-        mas_apply(r, z, false, r, dot_mode, 1.0);
+        mas_apply(r, z, false, dot ? r : nullptr, 1.0, test);
         return;
     }
     if (!p_.multiplicative) {  // MASSolver.cu:583-615: z = M r + S^T A_SS^-1 S r
-        mas_apply(r, z, false, nullptr, 0, 1.0);
+        mas_apply(r, z, false, nullptr, 1.0, test);
         launch_stiff_gather(A_, stiff_, r, nullptr, false, done, stream_);
         stiff_correct(z, done);
-        if (dot_mode) rz_dot(r, z, dot_mode);
+        if (dot) launch_pcg_rz(n_vec(), r, z, d_state_.data(), gr_, rz_, stream_);
         return;
     }
     // GPUHybrid.cu:528-540 with omega-damped MAS in place of the V-cycle:
@@ -786,11 +784,11 @@ void HybridSolver::precond(const double *r, double *z, int dot_mode, const float
     // additive MAS has lambda_max(M A) of a few units, so w = omega_factor /
     // lambda_max(M A) is estimated at factorize time (estimate_omega).
     if (!p_.mixed) {
-        mas_apply(r, z, false, nullptr, 0, omega_);
+        mas_apply(r, z, false, nullptr, omega_, test);
         launch_stiff_gather(A_, stiff_, r, z, true, done, stream_);
         stiff_correct(z, done);
         launch_residual_spmv(A_, r, z, d_w_.data(), done, stream_);
-        mas_apply(d_w_.data(), z, true, r, dot_mode, omega_);
+        mas_apply(d_w_.data(), z, true, dot ? r : nullptr, omega_);
         return;
     }
     // mixed precision: z also goes out rounded to FP32 (the stiff correction
@@ -803,12 +801,12 @@ void HybridSolver::precond(const double *r, double *z, int dot_mode, const float
     }
     float *z32 = d_z32_.data();
     float *z_lo = precise_rows_ ? d_z_lo_.data() : nullptr;
-    mas_apply(r, z, false, nullptr, 0, omega_, z32, nullptr, z_lo);
+    mas_apply(r, z, false, nullptr, omega_, test, z32, nullptr, z_lo);
     launch_stiff_gather(A_, stiff_, r, z, true, done, stream_);
     stiff_correct(z, done, z32, z_lo);
     launch_residual32(A_, r32, z32, d_w32_.data(), done, stream_, precise_rows_ ? d_precise_.data() : nullptr, r,
                       z_lo);
-    mas_apply(nullptr, z, true, r, dot_mode, omega_, nullptr, d_w32_.data());
+    mas_apply(nullptr, z, true, dot ? r : nullptr, omega_, false, nullptr, d_w32_.data());
 }
 
 // ------------------------------------------------------------------ PCG
@@ -816,9 +814,9 @@ void HybridSolver::precond(const double *r, double *z, int dot_mode, const float
 void HybridSolver::outer_spmv_alpha()
 {
     if (outer_df())
-        launch_pcg_spmv_alpha_df(A_, d_p_df_.data(), d_ap_df_.data(), d_state_.data(), gr_, stream_);
+        launch_pcg_spmv_alpha_df(A_, d_p_df_.data(), d_ap_df_.data(), d_state_.data(), gr_, pap_, stream_);
     else
-        launch_pcg_spmv_alpha(A_, d_p_.data(), d_ap_.data(), d_state_.data(), gr_, stream_);
+        launch_pcg_spmv_alpha(A_, d_p_.data(), d_ap_.data(), d_state_.data(), gr_, pap_, stream_);
 }
 
 void HybridSolver::split_p()
@@ -832,12 +830,12 @@ void HybridSolver::iteration()
     float *r32 = p_.mixed ? d_r32_.data() : nullptr;
     if (outer_df())
         launch_pcg_update_xr_df(n_vec(), d_x_.data(), d_r_.data(), d_p_.data(), d_ap_df_.data(), d_state_.data(),
-                                gr_, stream_, r32);
+                                gr_, pap_, rr_, stream_, r32);
     else
         launch_pcg_update_xr(n_vec(), d_x_.data(), d_r_.data(), d_p_.data(), d_ap_.data(), d_state_.data(), gr_,
-                             stream_, r32);
-    precond(d_r_.data(), d_z_.data(), 2, r32);
-    launch_pcg_update_p(n_vec(), d_p_.data(), d_z_.data(), d_state_.data(), stream_,
+                             pap_, rr_, stream_, r32);
+    precond(d_r_.data(), d_z_.data(), true, r32, true);
+    launch_pcg_update_p(n_vec(), d_p_.data(), d_z_.data(), d_state_.data(), rz_, false, stream_,
                         outer_df() ? d_p_df_.data() : nullptr);
 }
 
@@ -918,9 +916,9 @@ void HybridSolver::run_pcg()
         // r = b - A x; z = M r; p = z; gamma = r.z   (GPUHybrid.cu:1441-1451)
         launch_residual_spmv(A_, d_b_.data(), d_x_.data(), d_r_.data(), nullptr, stream_);
         if (p_.max_iter > 0) {
-            precond(d_r_.data(), d_z_.data(), 1);
-            launch_copy(n, d_z_.data(), d_p_.data(), nullptr, stream_);
-            split_p();
+            precond(d_r_.data(), d_z_.data(), true);
+            launch_pcg_update_p(n, d_p_.data(), d_z_.data(), d_state_.data(), rz_, true, stream_,
+                                outer_df() ? d_p_df_.data() : nullptr);
         }
         while (launched < p_.max_iter) {
             const int chunk = std::min(p_.check_every, p_.max_iter - launched);
@@ -1051,7 +1049,7 @@ void HybridSolver::autotune_spmv()
             const float ms = pass == 0 ? time_it([&]() {
                                              if (df32())
                                                  launch_pcg_spmv_alpha_df(T, d_p_df_.data(), d_ap_df_.data(),
-                                                                          d_state_.data(), gr_, stream_);
+                                                                          d_state_.data(), gr_, pap_, stream_);
                                              else
                                                  launch_spmv(T, d_p_.data(), d_ap_.data(), nullptr, stream_);
                                          })
@@ -1128,9 +1126,9 @@ void HybridSolver::estimate_omega()
     d_x_.zero(stream_);
     lanczos_mode_ = true;
     try {
-        precond(d_r_.data(), d_z_.data(), 1);
-        launch_copy(n, d_z_.data(), d_p_.data(), nullptr, stream_);
-        split_p();
+        precond(d_r_.data(), d_z_.data(), true);
+        launch_pcg_update_p(n, d_p_.data(), d_z_.data(), d_state_.data(), rz_, true, stream_,
+                            outer_df() ? d_p_df_.data() : nullptr);
         for (int j = 0; j < k; ++j) iteration();
     } catch (...) {
         lanczos_mode_ = false;
@@ -1272,7 +1270,7 @@ void HybridSolver::op_mas(const double *r, double *z)
     LSS_CUDA(cudaMemcpyAsync(d_state_.data(), h_state_, sizeof(PcgState), cudaMemcpyHostToDevice, stream_));
     LSS_CUDA(cudaMemcpyAsync(d_tmp_.data(), r, n * sizeof(double), cudaMemcpyHostToDevice, stream_));
     launch_permute(pat_.nb, pat_.bd, d_perm_.data(), d_tmp_.data(), d_r_.data(), true, stream_);
-    mas_apply(d_r_.data(), d_z_.data(), false, nullptr, 0, 1.0);
+    mas_apply(d_r_.data(), d_z_.data(), false, nullptr, 1.0);
     launch_permute(pat_.nb, pat_.bd, d_perm_.data(), d_z_.data(), d_tmp_.data(), false, stream_);
     LSS_CUDA(cudaMemcpyAsync(z, d_tmp_.data(), n * sizeof(double), cudaMemcpyDeviceToHost, stream_));
     LSS_CUDA(cudaStreamSynchronize(stream_));
@@ -1287,7 +1285,7 @@ void HybridSolver::op_precond(const double *r, double *z)
     LSS_CUDA(cudaMemcpyAsync(d_state_.data(), h_state_, sizeof(PcgState), cudaMemcpyHostToDevice, stream_));
     LSS_CUDA(cudaMemcpyAsync(d_tmp_.data(), r, n * sizeof(double), cudaMemcpyHostToDevice, stream_));
     launch_permute(pat_.nb, pat_.bd, d_perm_.data(), d_tmp_.data(), d_r_.data(), true, stream_);
-    precond(d_r_.data(), d_z_.data(), 0);
+    precond(d_r_.data(), d_z_.data(), false);
     launch_permute(pat_.nb, pat_.bd, d_perm_.data(), d_z_.data(), d_tmp_.data(), false, stream_);
     LSS_CUDA(cudaMemcpyAsync(z, d_tmp_.data(), n * sizeof(double), cudaMemcpyDeviceToHost, stream_));
     LSS_CUDA(cudaStreamSynchronize(stream_));
@@ -1303,7 +1301,7 @@ void HybridSolver::op_time(int kind, int reps, double *ms, double *bytes)
     PcgState hs{};
     hs.bb = 1.0;
     hs.max_iter = 1 << 30;
-    hs.gamma = 1.0;
+    hs.gamma = hs.rz = 1.0;
     *h_state_ = hs;
     LSS_CUDA(cudaMemcpyAsync(d_state_.data(), h_state_, sizeof(PcgState), cudaMemcpyHostToDevice, stream_));
     // deterministic non-trivial operands
@@ -1321,8 +1319,8 @@ void HybridSolver::op_time(int kind, int reps, double *ms, double *bytes)
     auto body = [&]() {
         switch (kind) {
         case 0: launch_spmv(A_, d_p_.data(), d_ap_.data(), nullptr, stream_); break;
-        case 1: mas_apply(d_r_.data(), d_z_.data(), false, nullptr, 0, 1.0); break;
-        case 2: precond(d_r_.data(), d_z_.data(), 0); break;
+        case 1: mas_apply(d_r_.data(), d_z_.data(), false, nullptr, 1.0); break;
+        case 2: precond(d_r_.data(), d_z_.data(), false); break;
         case 4: launch_mas_level0(mas_, d_inv0_.data(), d_u_.data(), mas_fp32_, d_r_.data(), d_z_.data(), stream_);
             break;
         case 5:

@@ -82,15 +82,15 @@ private:
     void ensure_vectors();
     void run_pcg();
     // r32 (optional): r already rounded to FP32 (mixed precision); converted here otherwise
-    void precond(const double *r, double *z, int dot_mode, const float *r32 = nullptr);
-    void mas_apply(const double *xin, double *z, bool acc, const double *rdot, int dot_mode, double scale,
+    // dot: also form the parts of r.z (rz_); test: first test r.r (rr_) for convergence
+    void precond(const double *r, double *z, bool dot, const float *r32 = nullptr, bool test = false);
+    void mas_apply(const double *xin, double *z, bool acc, const double *rdot, double scale, bool test = false,
                    float *z32 = nullptr, const float *xin32 = nullptr, float *z_lo = nullptr);
     void estimate_omega();
     void autotune_spmv();
     void iteration();
     void launch_chunk(int iters);
     void invalidate_graph();
-    void rz_dot(const double *r, const double *z, int dot_mode);
     int64_t n_vec() const { return (int64_t)pat_.nb * pat_.bd; }
 
     Params p_;
@@ -159,14 +159,16 @@ private:
     bool df32() const { return p_.outer_spmv == 2 || (p_.outer_spmv == 0 && p_.mixed && p_.block_size > 1); }
     bool refine_fp64_ = false;  // refinement restarts of the current solve use the FP64 product
     bool outer_df() const { return df32() && !refine_fp64_; }
-    void outer_spmv_alpha();  // Ap, p.Ap, alpha with the configured outer SpMV
-    void split_p();           // refresh the df32 split of p (after p = z)
+    void outer_spmv_alpha();  // Ap and p.Ap (pap_) with the configured outer SpMV
+    void split_p();           // refresh the df32 split of p
     DBuf<PcgState> d_state_;
     PcgState *h_state_ = nullptr;
     DBuf<double> d_partials_, d_scalar_;
     DBuf<unsigned> d_counter_;
     DBuf<int> d_bad_;
     GridReduce gr_;
+    DBuf<double> d_sums_;
+    PcgSum pap_, rr_, rz_;  // the PCG's scalar sums, between the kernels that form and use them
     cudaGraphExec_t graph_exec_ = nullptr;
     int graph_iters_ = 0;
     size_t graph_nodes_ = 0;
