@@ -414,17 +414,17 @@ __device__ __forceinline__ void bank_segment_sums(const T *xs, uint8_t key, unsi
     }
 }
 
-// The restriction of r to every coarse level in one launch.
+// The restriction of r to level 1 and, in a large hierarchy, to level 2
+// (MasDev::base; the levels above are summed from there by the products that
+// need them, symv_coarse_kernel).
 //
-// A warp sums one partition's rows into its level-1 items and then reports to
-// the level-1 banks that hold them (arrive[g], at most two banks).  The warp
-// whose report is a bank's last queues it in its CTA, whose warps restrict the
-// queued banks to the next level the same way.  Nothing waits: whoever
-// completes a bank continues with it, and each sum has one fixed order whoever
-// runs it.  Level by level this took L - 1 launches of 5 to 11 us each, nearly
-// all latency.  (The products of the ready banks stay in a launch of their
-// own: run here, by the CTA that completes a bank, they pile up on the few
-// CTAs that hold a clamped face -- 235 us instead of 100 on 648k DOFs.)
+// A warp sums one partition's rows into its level-1 items.  For level 2 it then
+// reports to the level-1 banks that hold them (arrive[g], at most two banks);
+// the warp whose report is a bank's last queues it in its CTA, whose warps
+// restrict the queued banks.  Nothing waits: whoever completes a bank
+// continues with it, and each sum has one fixed order whoever runs it.  A
+// report costs 3 to 4 us of latency, so carrying it through every level took
+// 14 to 22 us a launch; one launch per level took more.
 template <int BD, typename T, typename XT>
 __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__restrict__ r, T *__restrict__ v,
                                                        PcgState *st, PcgSum rr)
@@ -447,31 +447,25 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
     constexpr int N = 32 * BD, W = 8;
     __shared__ T xs_all[W][N];
     __shared__ unsigned mask_all[W][32];
-    // ready banks, level << 28 | bank: at most 16 level-1 banks per round and
-    // twice the previous level's at each of up to five further levels
-    __shared__ unsigned queue[1024];
+    __shared__ int32_t queue[2 * W];  // ready level-1 banks: at most two per partition
     __shared__ int qn;
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     T *xs = xs_all[wl];
     unsigned *mask = mask_all[wl];
     if (threadIdx.x == 0) qn = 0;
     __syncthreads();
-    // reports items [i0, i0 + cnt) of level l as written; queues completed banks
-    auto report = [&](int l, int32_t i0, int cnt) {
+    // reports level-1 items [i0, i0 + cnt) as written; queues completed banks
+    auto report = [&](int32_t i0, int cnt) {
         __threadfence();
         __syncwarp();
         if (lane < 2 && cnt > 0) {
-            const int32_t b0 = i0 >> 5, b1 = (i0 + cnt - 1) >> 5, b = b0 + lane;
-            if (b <= b1) {
-                const int32_t g = m.boff[l] + b;
-                if (atomicAdd(m.arrive + g, 1u) + 1u == m.need[g]) {
-                    m.arrive[g] = 0u;
-                    __threadfence();
-                    queue[atomicAdd(&qn, 1)] = (unsigned)l << 28 | (unsigned)b;
-                }
+            const int32_t b = (i0 >> 5) + lane;
+            if (b <= (i0 + cnt - 1) >> 5 && atomicAdd(m.arrive + b, 1u) + 1u == m.need[b]) {
+                m.arrive[b] = 0u;
+                __threadfence();
+                queue[atomicAdd(&qn, 1)] = b;
             }
         }
-        __syncwarp();
     };
     for (int64_t p0 = (int64_t)blockIdx.x * W; p0 < m.nparts; p0 += (int64_t)gridDim.x * W) {
         const int64_t p = p0 + wl;
@@ -488,34 +482,89 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
             const int nc = m.ccnt0[p];
             __syncwarp();
             bank_segment_sums<BD, T>(xs, key, mask, nc, v + m.voff[1] + (int64_t)i0 * BD, lane);
-            report(1, i0, nc);
+            if (m.base > 1) report(i0, nc);
+            __syncwarp();
+        }
+        if (m.base == 1) continue;
+        __syncthreads();
+        for (int k = wl; k < qn; k += W) {
+            const int32_t b = queue[k], i0 = b * 32;
+            const int cnt = min(32, m.nitems[1] - i0);
+            const T *vl = v + m.voff[1] + (int64_t)i0 * BD;
+#pragma unroll
+            for (int q = 0; q < BD; ++q) {
+                const int e = q * 32 + lane;
+                xs[e] = e < cnt * BD ? __ldcg(vl + e) : T(0);
+            }
+            const uint8_t key = lane < cnt ? m.key[1][i0 + lane] : (uint8_t)0xff;
+            __syncwarp();
+            bank_segment_sums<BD, T>(xs, key, mask, m.ccnt[1][b], v + m.voff[2] + (int64_t)m.cbase[1][b] * BD, lane);
+            __syncwarp();
         }
         __syncthreads();
-        int head = 0, n = qn;
-        while (head < n) {
-            for (int k = head + wl; k < n; k += W) {
-                const int l = (int)(queue[k] >> 28);
-                if (l + 1 >= m.L) continue;
-                const int32_t b = (int32_t)(queue[k] & 0x0fffffffu), i0 = b * 32;
-                const int cnt = min(32, m.nitems[l] - i0);
-                const T *vl = v + m.voff[l] + (int64_t)i0 * BD;
-#pragma unroll
-                for (int q = 0; q < BD; ++q) {
-                    const int e = q * 32 + lane;
-                    xs[e] = e < cnt * BD ? __ldcg(vl + e) : T(0);
-                }
-                const uint8_t key = lane < cnt ? m.key[l][i0 + lane] : (uint8_t)0xff;
-                const int32_t j0 = m.cbase[l][b];
-                const int nc = m.ccnt[l][b];
-                __syncwarp();
-                bank_segment_sums<BD, T>(xs, key, mask, nc, v + m.voff[l + 1] + (int64_t)j0 * BD, lane);
-                report(l + 1, j0, nc);
-            }
-            __syncthreads();
-            head = n;
-            n = qn;
-        }
         if (threadIdx.x == 0) qn = 0;
+        __syncthreads();
+    }
+}
+
+// x of a coarse bank above the base level: every item's sum over the base-level
+// items below it (memb: base items grouped by their item at this level, in
+// order).  Items of up to 128 members take a warp, larger ones the whole CTA.
+template <int BD, typename T>
+__device__ __forceinline__ void gather_bank(const MasDev &m, int l, int32_t b, const T *__restrict__ v,
+                                            T *__restrict__ xs, T (*red)[32 * BD])
+{
+    constexpr int W = 8, BIG = 128;
+    const int tid = threadIdx.x, lane = tid & 31, wl = tid >> 5;
+    const int32_t *__restrict__ ptr = m.memb_ptr[l] + (int64_t)b * 32;
+    const int32_t *__restrict__ memb = m.memb[l];
+    const T *__restrict__ vb = v + m.voff[m.base];
+    const int cnt = min(32, m.nitems[l] - b * 32);
+    const int32_t lo = lane < cnt ? ptr[lane] : 0, hi = lane < cnt ? ptr[lane + 1] : 0;
+    const unsigned big = __ballot_sync(0xffffffffu, hi - lo > BIG);
+    for (int it = wl; it < 32; it += W) {
+        if (big >> it & 1u) continue;
+        const int32_t p0 = __shfl_sync(0xffffffffu, lo, it), p1 = __shfl_sync(0xffffffffu, hi, it);
+        T acc[BD];
+#pragma unroll
+        for (int c = 0; c < BD; ++c) acc[c] = T(0);
+#pragma unroll 4
+        for (int32_t j = p0 + lane; j < p1; j += 32) {
+            const T *e = vb + (int64_t)memb[j] * BD;
+#pragma unroll
+            for (int c = 0; c < BD; ++c) acc[c] += e[c];
+        }
+        if (p1 - p0 > 1)
+#pragma unroll
+            for (int c = 0; c < BD; ++c) acc[c] = warp_sum(acc[c]);
+        if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < BD; ++c) xs[c * 32 + it] = acc[c];
+    }
+    for (unsigned left = big; left; left &= left - 1) {
+        const int it = __ffs(left) - 1;
+        const int32_t p0 = __shfl_sync(0xffffffffu, lo, it), p1 = __shfl_sync(0xffffffffu, hi, it);
+        T acc[BD];
+#pragma unroll
+        for (int c = 0; c < BD; ++c) acc[c] = T(0);
+#pragma unroll 4
+        for (int32_t j = p0 + tid; j < p1; j += 32 * W) {
+            const T *e = vb + (int64_t)memb[j] * BD;
+#pragma unroll
+            for (int c = 0; c < BD; ++c) acc[c] += e[c];
+        }
+#pragma unroll
+        for (int c = 0; c < BD; ++c) acc[c] = warp_sum(acc[c]);
+        if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < BD; ++c) red[wl][c * 32] = acc[c];
+        __syncthreads();
+        if (tid < BD) {
+            T sum = red[0][tid * 32];
+#pragma unroll
+            for (int w = 1; w < W; ++w) sum += red[w][tid * 32];
+            xs[tid * 32 + it] = sum;
+        }
         __syncthreads();
     }
 }
@@ -525,8 +574,8 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
 // banks are few and L2-resident, so this is one latency, not a stream).  In a
 // bank without couplings between its items (uncoupled: Dirichlet rows, which
 // never merge and fill a third of the coarse banks of a clamped cube) every
-// entry off rotation 0 is an exact zero, and only that rotation is taken.
-// Level vectors are whole banks back to back: bank g starts at element g * N.
+// entry off rotation 0 is an exact zero, and only that rotation is taken.  Banks
+// above the base level first sum their items.  Level vectors are whole banks back to back: bank g starts at element g * N.
 template <int BD, typename T>
 __global__ void __launch_bounds__(256) symv_coarse_kernel(MasDev m, const T *__restrict__ invc,
                                                           const T *__restrict__ v, T *__restrict__ u,
@@ -541,7 +590,13 @@ __global__ void __launch_bounds__(256) symv_coarse_kernel(MasDev m, const T *__r
     const bool uncoupled = m.uncoupled[g];
     pdl_enter();
     if (done && *done) return;
-    if (tid < N) xs[o] = v[g * N + tid];
+    int l = 1;
+    while (l + 1 < m.L && g >= m.boff[l + 1]) ++l;
+    if (l <= m.base) {
+        if (tid < N) xs[o] = v[g * N + tid];
+    } else {
+        gather_bank<BD, T>(m, l, (int32_t)(g - m.boff[l]), v, xs, red);
+    }
     __syncthreads();
     T y[BD];
     const TileLd<T, false> ld{reinterpret_cast<const unsigned char *>(invc + g * m.tile_elems)};

@@ -123,7 +123,8 @@ private:
         d_chunk_r0_;
     CoarseMembers memb_;
     DBuf<uint8_t> d_key0_, d_ccnt0_, d_uncoupled_;
-    DBuf<unsigned> d_need_, d_arrive_;  // coarse banks: contributing banks below, arrivals of an apply
+    DBuf<unsigned> d_need_, d_arrive_;  // level-1 banks: contributing partitions, arrivals of an apply
+    DBuf<int32_t> d_membl_;             // base-level items by coarse item (MasDev::memb)
     std::vector<DBuf<uint8_t>> d_key_, d_ccnt_;
     std::vector<DBuf<int32_t>> d_cbase_;
     DBuf<char> d_inv0_, d_invc_, d_v_, d_u_;
