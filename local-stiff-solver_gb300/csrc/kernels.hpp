@@ -263,9 +263,9 @@ std::vector<StiffWarp> stiff_warps(const std::vector<int32_t> &off, const std::v
                                    int32_t ndense);
 
 void launch_stiff_extract(const BsrDev &A, const StiffDev &S, double *stage, cudaStream_t s);
-// dense inverses of the subdomains 0 .. nsub-1 (each at most STIFF_DENSE_MAX DOFs)
+// dense inverses of those of the subdomains 0 .. nsub-1 that have at most max_m DOFs
 constexpr int STIFF_DENSE_MAX = 160;
-void launch_stiff_invert(const StiffDev &S, const int32_t *h_off, int32_t nsub, double *inv, int *bad,
+void launch_stiff_invert(const StiffDev &S, const int32_t *h_off, int32_t nsub, int max_m, double *inv, int *bad,
                          cudaStream_t s);
 void launch_stiff_to_fp32(int64_t count, const double *src, float *dst, cudaStream_t s);
 // t = r_S - (A z)_S   (residual = true) or t = r_S

@@ -4,8 +4,10 @@
 //
 // Nested dissection: a connected node set above the leaf size is split by a
 // level set of a breadth-first search from a pseudo-peripheral node (the
-// smallest level near the median), thinned by moving separator nodes with no
-// neighbour on the far side back; disconnected sets become sibling subtrees.
+// smallest level that leaves 30% on either side), thinned by moving separator
+// nodes with no neighbour on the far side back, and so is each half; the three
+// separators make one front with four children.  Disconnected sets become
+// sibling subtrees.
 // Fronts are numbered in postorder (children first), and positions are
 // handed out front by front, so a subtree's variables are contiguous and a
 // front's own variables come last in it.  A front's boundary is the set of
@@ -22,9 +24,10 @@ namespace {
 // Node sets up to this many DOFs are eliminated as one front.  Every level of
 // the tree is two dependent launches of each solve and a chain of panel steps
 // of the factorization, while a front of this size is still a few microseconds
-// of FP64 work on the whole GPU: a 1,263-DOF ball in mixed precision took 145
-// us per iteration with leaves of 48 DOFs (six levels), 128 with 160 and 116
-// with 384 (three); 512 gains no more there and costs a fifth of the factorization.
+// of FP64 work on the whole GPU.  Mixed iterations with a 1.3k- and a 3.0k-DOF
+// ball: 88 and 129 us with leaves of 128 or 192 DOFs, 87 and 115 with 256, 76
+// and 115 with 384; 512 gains no more and costs a quarter of the factorization.
+// (Binary splits with leaves of 48 DOFs, six and more levels: 145 and 218 us.)
 constexpr int32_t LEAF_DOFS = 384;
 
 struct Nd {
@@ -34,14 +37,16 @@ struct Nd {
     int32_t cur = 0;
     std::vector<std::vector<int32_t>> own;       // fronts: own nodes
     std::vector<std::vector<int32_t>> children;  // fronts: child fronts (local ids)
+    std::vector<int32_t> bisections;             // fronts: dissection levels joined in it (a leaf: 1)
 
     Nd(const std::vector<int32_t> &o, const std::vector<int32_t> &a, int32_t nn, int32_t leaf)
         : aoff(o), adj(a), leaf_nodes(leaf), stamp(nn, 0), lvl(nn, -1)
     {
     }
 
-    int32_t make(std::vector<int32_t> nodes, std::vector<int32_t> kids)
+    int32_t make(std::vector<int32_t> nodes, std::vector<int32_t> kids, int32_t levels = 1)
     {
+        bisections.push_back(levels);
         std::sort(nodes.begin(), nodes.end());
         own.push_back(std::move(nodes));
         children.push_back(std::move(kids));
@@ -99,17 +104,53 @@ struct Nd {
             }
             return roots;
         }
+        std::vector<int32_t> A, B, own;
+        if (!split(order, st, A, B, own)) return {make(std::move(nodes), {})};
+        // the halves' separators join this one in a single front of four
+        // children (a half that is small, disconnected or unsplittable stays)
+        std::vector<std::vector<int32_t>> parts;
+        int32_t levels = 1;
+        for (std::vector<int32_t> *half : {&A, &B}) {
+            if ((int32_t)half->size() > leaf_nodes) {
+                const int32_t hs = ++cur;
+                mark(*half, hs);
+                const std::vector<int32_t> reach = bfs((*half)[0], hs);
+                std::vector<int32_t> a, b, sep;
+                if (reach.size() == half->size() && split(reach, hs, a, b, sep)) {
+                    levels = 2;
+                    own.insert(own.end(), sep.begin(), sep.end());
+                    parts.push_back(std::move(a));
+                    parts.push_back(std::move(b));
+                    continue;
+                }
+            }
+            parts.push_back(std::move(*half));
+        }
+        std::vector<int32_t> kids;
+        for (auto &part : parts) {
+            const std::vector<int32_t> k = dissect(std::move(part));
+            kids.insert(kids.end(), k.begin(), k.end());
+        }
+        return {make(std::move(own), std::move(kids), levels)};
+    }
+
+    // Splits the connected set stamped `st` (order: a breadth-first search of
+    // it) into A, B and the separator S between them; false if it has no
+    // separating level.
+    bool split(std::vector<int32_t> order, int32_t st, std::vector<int32_t> &A, std::vector<int32_t> &B,
+               std::vector<int32_t> &S2)
+    {
         // pseudo-peripheral start: the last node of a BFS, twice
         order = bfs(order.back(), st);
         order = bfs(order.back(), st);
         const int32_t depth = lvl[order.back()];
-        if (depth < 2) return {make(std::move(nodes), {})};
+        if (depth < 2) return false;
         std::vector<int32_t> count(depth + 1, 0);
         for (int32_t v : order) ++count[lvl[v]];
         // the separator level: the smallest level among those that leave at
         // least 30% of the nodes on either side (balanced subtrees keep the
         // tree shallow); the median level when no level does
-        const int64_t nn = (int64_t)nodes.size();
+        const int64_t nn = (int64_t)order.size();
         int32_t med = 0, acc = 0;
         while (med < depth && 2 * (acc + count[med]) < (int32_t)nn) acc += count[med++];
         int32_t best = std::clamp(med, 1, depth - 1);
@@ -124,21 +165,16 @@ struct Nd {
             }
             below += count[l];
         }
-        std::vector<int32_t> A, B, S;
+        std::vector<int32_t> S;
         for (int32_t v : order) (lvl[v] < best ? A : (lvl[v] > best ? B : S)).push_back(v);
         // thin: a separator node without a neighbour in B joins A
-        std::vector<int32_t> S2;
         for (int32_t v : S) {
             bool touches_b = false;
             for (int32_t k = aoff[v]; k < aoff[v + 1] && !touches_b; ++k)
                 touches_b = stamp[adj[k]] == st && lvl[adj[k]] > best;
             (touches_b ? S2 : A).push_back(v);
         }
-        if (A.empty() || B.empty() || S2.empty()) return {make(std::move(nodes), {})};
-        std::vector<int32_t> kids = dissect(std::move(A));
-        std::vector<int32_t> kb = dissect(std::move(B));
-        kids.insert(kids.end(), kb.begin(), kb.end());
-        return {make(std::move(S2), std::move(kids))};
+        return !(A.empty() || B.empty() || S2.empty());
     }
 };
 
@@ -158,7 +194,7 @@ MfSymbolic mf_symbolic(const std::vector<int32_t> &dofs, const std::vector<int32
     const int32_t nb = (int32_t)rows.size() - 1;
     std::vector<int32_t> node_local(nb, -1);
     std::vector<int32_t> pos_stamp(nj, -1);
-    std::vector<int32_t> parent;
+    std::vector<int32_t> parent, dissected;  // per front: its parent, dissection levels of its subtree
     int32_t pos = 0;
     M.bnd_off.push_back(0);
     M.child_off.push_back(0);
@@ -209,12 +245,15 @@ MfSymbolic mf_symbolic(const std::vector<int32_t> &dofs, const std::vector<int32
             std::vector<int32_t> kids;
             for (int32_t c : nd.children[f]) kids.push_back(fbase + c);
             std::sort(kids.begin(), kids.end());
-            int32_t h = 0;
+            int32_t h = 0, d = 0;
             for (int32_t c : kids) {
                 parent[c] = id;
                 h = std::max(h, M.height[c] + 1);
+                d = std::max(d, dissected[c]);
             }
             M.height.push_back(h);
+            dissected.push_back(d + nd.bisections[f]);
+            M.dissection_levels = std::max(M.dissection_levels, dissected.back());
             M.child.insert(M.child.end(), kids.begin(), kids.end());
             M.child_off.push_back((int32_t)M.child.size());
             M.bnd_off.push_back(0);  // set below, once every position of the subdomain is known

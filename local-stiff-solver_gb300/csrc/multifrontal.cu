@@ -30,13 +30,6 @@ namespace {
 
 constexpr int PW = 32;  // panel width / outputs per CTA
 
-struct MfView {
-    const int32_t *p0, *s, *u, *woff, *bnd_off, *bnd_pos, *child_off, *child, *ea_map, *front_of_pos, *pos2j,
-        *j2pos, *poff;
-    const int64_t *foff;
-    int32_t j_base, npos;
-};
-
 __device__ __forceinline__ int find_front(const MfWork &w, int64_t cta)
 {
     if (w.cta_item) return w.cta_item[cta];
@@ -360,7 +353,9 @@ __global__ void __launch_bounds__(256) mf_blk_write_kernel(MfView v, MfWork w, d
     }
 }
 
-// lower triangle of the swept columns: Fn[r][c] = Fn[c][r] for c < min(r, s)
+// lower triangle of the swept columns: Fn[r][c] = Fn[c][r] for c < min(r, s);
+// NEG (whole blocks, s = f): the inverse itself, both triangles negated
+template <bool NEG>
 __global__ void __launch_bounds__(256) mf_mirror_kernel(MfView v, MfWork w, double *__restrict__ F, int *bad)
 {
     const int i = find_front(w, blockIdx.x);
@@ -370,7 +365,13 @@ __global__ void __launch_bounds__(256) mf_mirror_kernel(MfView v, MfWork w, doub
     if (idx >= (int64_t)f * s) return;
     const int r = (int)(idx / s), c = (int)(idx % s);
     double *Fn = F + v.foff[N];
-    if (c < r) Fn[(int64_t)r * f + c] = Fn[(int64_t)c * f + r];
+    if (NEG) {
+        if (c < r) return;
+        const double val = -Fn[(int64_t)r * f + c];
+        if (!isfinite(val)) atomicOr(bad, 8);
+        Fn[(int64_t)r * f + c] = val;
+        Fn[(int64_t)c * f + r] = val;
+    } else if (c < r) Fn[(int64_t)r * f + c] = Fn[(int64_t)c * f + r];
     else if (!isfinite(Fn[(int64_t)r * f + c])) atomicOr(bad, 32);
 }
 
@@ -397,21 +398,34 @@ struct NrScratch1 {
     unsigned *cnt;  // per group: arrivals
 };
 
+// A GEMV CTA's part of its front in registers (warp = row slice, lane =
+// column): the fronts do not change within a solve, so these loads are issued
+// before anything the CTA has to wait for and overlap the gather of its vector
+// (8 loads at a time behind it added 3 us to a launch).
+struct FrontPart {
+    double a[NR_KROWS / 8];
+};
+__device__ __forceinline__ void load_part(FrontPart &p, const MfCta &c, const double *__restrict__ F)
+{
+    const int cl = threadIdx.x & 31, ks = threadIdx.x >> 5;
+    const double *Fc = F + c.foff + (int64_t)(c.q0 + ks) * c.f + c.col0 + cl;
+#pragma unroll
+    for (int j = 0; j < NR_KROWS / 8; ++j)
+        p.a[j] = cl < c.ncol && ks + 8 * j < c.nrow ? __ldg(Fc + (int64_t)(8 * j) * c.f) : 0.0;
+}
+
 // res[c] = sum over the CTA's rows of Fn[q][col0 + c] xs[q - q0]; slices in order
-__device__ __forceinline__ void gemv1(const double *__restrict__ Fn, int f, int col0, int ncol, int q0, int nrow,
-                                      const double *__restrict__ xs, double *__restrict__ red,
-                                      double *__restrict__ res)
+__device__ __forceinline__ void gemv1(const FrontPart &p, const MfCta &c, const double *__restrict__ xs,
+                                      double *__restrict__ red, double *__restrict__ res)
 {
     const int cl = threadIdx.x & 31, ks = threadIdx.x >> 5;
     double acc = 0.0;
-    if (cl < ncol) {
-        const double *Fc = Fn + (int64_t)q0 * f + col0 + cl;
-#pragma unroll 8
-        for (int q = ks; q < nrow; q += 8) acc += __ldg(Fc + (int64_t)q * f) * xs[q];
-    }
+#pragma unroll
+    for (int j = 0; j < NR_KROWS / 8; ++j)
+        if (ks + 8 * j < c.nrow) acc += p.a[j] * xs[ks + 8 * j];
     red[ks * 32 + cl] = acc;
     __syncthreads();
-    if (threadIdx.x < ncol) {
+    if (threadIdx.x < c.ncol) {
         double sum = 0.0;
 #pragma unroll
         for (int q = 0; q < 8; ++q) sum += red[q * 32 + threadIdx.x];
@@ -464,6 +478,8 @@ __global__ void __launch_bounds__(256) mf_forward_kernel(MfView v, const MfCta *
 {
     __shared__ double xs[NR_KROWS], red[256], res[NR_COLS1];
     const MfCta c = ctas[blockIdx.x];
+    FrontPart part;
+    load_part(part, c, F);
     pdl_enter();
     if (done && *done) return;
     const int t = threadIdx.x;
@@ -474,7 +490,7 @@ __global__ void __launch_bounds__(256) mf_forward_kernel(MfView v, const MfCta *
     }
     const double base = t < c.ncol ? mf_gather1(c, c.col0 + t, v, S, gptr, gsrc, W) : 0.0;
     __syncthreads();
-    gemv1(F + c.foff, c.f, c.col0, c.ncol, c.q0, c.nrow, xs, red, res);
+    gemv1(part, c, xs, red, res);
     if (!combine1(sc, c.kc, c.nkc, res, c.ncol)) return;
     if (t < c.ncol) W[(int64_t)c.woff + c.col0 + t] = base - res[t];
 }
@@ -491,6 +507,8 @@ __global__ void __launch_bounds__(256) mf_backward_kernel(MfView v, const MfCta 
 {
     __shared__ double vec[NR_KROWS], red[256], res[NR_COLS1];
     const MfCta c = ctas[blockIdx.x];
+    FrontPart part;
+    load_part(part, c, F);
     const int t = threadIdx.x, q = c.q0 + t;
     const int32_t bp = t < c.nrow && q >= c.s ? v.bnd_pos[c.bnd_off + q - c.s] : 0;
     const int32_t d = t < c.ncol ? S.dofs[v.pos2j[c.p0 + c.col0 + t]] : 0;
@@ -500,7 +518,7 @@ __global__ void __launch_bounds__(256) mf_backward_kernel(MfView v, const MfCta 
         vec[t] = q >= c.s ? X[bp] : (c.s == c.f ? mf_gather1(c, q, v, S, gptr, gsrc, W) : W[(int64_t)c.woff + q]);
     const double zd = t < c.ncol ? z[d] : 0.0;
     __syncthreads();
-    gemv1(F + c.foff, c.f, c.col0, c.ncol, c.q0, c.nrow, vec, red, res);
+    gemv1(part, c, vec, red, res);
     if (!combine1(sc, c.kc, c.nkc, res, c.ncol)) return;
     if (t < c.ncol) {
         X[c.p0 + c.col0 + t] = -res[t];
@@ -938,25 +956,20 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
     d_D_.resize(std::max<size_t>(dmax, 1) * PW * PW);
 }
 
-namespace {
-MfView make_view(const int32_t *p0, const int32_t *s, const int32_t *u, const int32_t *woff, const int32_t *bo,
-                 const int32_t *bp, const int32_t *co, const int32_t *ch, const int32_t *ea, const int32_t *fp,
-                 const int32_t *pj, const int32_t *jp, const int32_t *po, const int64_t *fo, int32_t j_base,
-                 int32_t npos)
+MfView MfFactor::view() const
 {
     MfView v;
-    v.p0 = p0; v.s = s; v.u = u; v.woff = woff; v.bnd_off = bo; v.bnd_pos = bp; v.child_off = co; v.child = ch;
-    v.ea_map = ea; v.front_of_pos = fp; v.pos2j = pj; v.j2pos = jp; v.poff = po; v.foff = fo;
-    v.j_base = j_base; v.npos = npos;
+    v.p0 = p0_; v.s = s_; v.u = u_; v.woff = woff_; v.bnd_off = bnd_off_; v.bnd_pos = bnd_pos_;
+    v.child_off = child_off_; v.child = child_; v.ea_map = ea_map_; v.front_of_pos = front_of_pos_; v.pos2j = pos2j_;
+    v.j2pos = j2pos_; v.poff = poff_; v.foff = foff_;
+    v.j_base = sym_.j_base; v.npos = sym_.npos;
     return v;
 }
-}  // namespace
 
 void MfFactor::factorize(const BsrDev &A, const StiffDev &S, int *bad, cudaStream_t st)
 {
     if (sym_.nfront == 0) return;
-    const MfView v = make_view(p0_, s_, u_, woff_, bnd_off_, bnd_pos_, child_off_, child_, ea_map_, front_of_pos_,
-                               pos2j_, j2pos_, poff_, foff_, sym_.j_base, sym_.npos);
+    const MfView v = view();
     double *F = d_F_.data();
     d_F_.zero(st);
     const unsigned ga = (unsigned)(((int64_t)sym_.npos * 32 + 255) / 256);
@@ -977,27 +990,61 @@ void MfFactor::factorize(const BsrDev &A, const StiffDev &S, int *bad, cudaStrea
             mf_sweep_small_kernel<<<L.small.count, 256, small_smem, st>>>(v, L.small, F, bad);
             LSS_LAUNCH_CHECK();
         }
-        if (L.diag.count) {
-            for (int k0 = 0; k0 < L.max_s_large; k0 += PW) {
-                mf_blk_diag_kernel<<<L.diag.count, 256, 0, st>>>(v, L.diag, F, k0, d_D_.data(), bad);
-                mf_blk_panel_kernel<<<(unsigned)L.panel.ctas, 256, 0, st>>>(v, L.panel, F, k0, d_D_.data(),
-                                                                            d_P_.data());
-                mf_blk_update_kernel<<<(unsigned)L.update.ctas, 256, 0, st>>>(v, L.update, F, k0, d_P_.data());
-                mf_blk_write_kernel<<<(unsigned)L.write.ctas, 256, 0, st>>>(v, L.write, F, k0, d_P_.data(),
-                                                                            d_D_.data());
-                LSS_LAUNCH_CHECK();
-            }
-            mf_mirror_kernel<<<(unsigned)L.mirror.ctas, 256, 0, st>>>(v, L.mirror, F, bad);
-            LSS_LAUNCH_CHECK();
-        }
+        if (L.diag.count) sweep_large(L, v, F, false, bad, st);
     }
+}
+
+// the blocked sweep of a level's large fronts; whole: as inverses of whole blocks
+void MfFactor::sweep_large(const Level &L, const MfView &v, double *F, bool whole, int *bad, cudaStream_t st)
+{
+    for (int k0 = 0; k0 < L.max_s_large; k0 += PW) {
+        mf_blk_diag_kernel<<<L.diag.count, 256, 0, st>>>(v, L.diag, F, k0, d_D_.data(), bad);
+        mf_blk_panel_kernel<<<(unsigned)L.panel.ctas, 256, 0, st>>>(v, L.panel, F, k0, d_D_.data(), d_P_.data());
+        mf_blk_update_kernel<<<(unsigned)L.update.ctas, 256, 0, st>>>(v, L.update, F, k0, d_P_.data());
+        mf_blk_write_kernel<<<(unsigned)L.write.ctas, 256, 0, st>>>(v, L.write, F, k0, d_P_.data(), d_D_.data());
+        LSS_LAUNCH_CHECK();
+    }
+    const unsigned grid = (unsigned)L.mirror.ctas;
+    if (whole) mf_mirror_kernel<true><<<grid, 256, 0, st>>>(v, L.mirror, F, bad);
+    else mf_mirror_kernel<false><<<grid, 256, 0, st>>>(v, L.mirror, F, bad);
+    LSS_LAUNCH_CHECK();
+}
+
+void MfFactor::setup_dense(const std::vector<int32_t> &off, const std::vector<int64_t> &inv_off, int32_t ndense,
+                           cudaStream_t s)
+{
+    MfSymbolic M;
+    M.bnd_off.push_back(0);
+    M.child_off.push_back(0);
+    for (int32_t k = 0; k < ndense; ++k) {
+        const int32_t m = off[k + 1] - off[k];
+        if (m <= MF_SMEM_F) continue;
+        M.p0.push_back(M.npos);
+        M.s.push_back(m);
+        M.u.push_back(0);
+        M.height.push_back(0);
+        M.foff.push_back(inv_off[k]);
+        M.woff.push_back(M.npos);
+        M.bnd_off.push_back(0);
+        M.child_off.push_back(0);
+        M.npos += m;
+        M.max_f = M.max_s = std::max(M.max_s, m);
+        ++M.nfront;
+    }
+    M.levels = M.nfront ? 1 : 0;
+    setup(M, s);  // no front storage of its own: the blocks are swept where they lie
+}
+
+void MfFactor::invert_dense(double *inv, int *bad, cudaStream_t s)
+{
+    if (empty()) return;
+    sweep_large(levels_[0], view(), inv, true, bad, s);
 }
 
 void MfFactor::solve(const StiffDev &S, double *z, float *z32, float *z_lo, const int *done, cudaStream_t st)
 {
     if (sym_.nfront == 0) return;
-    const MfView v = make_view(p0_, s_, u_, woff_, bnd_off_, bnd_pos_, child_off_, child_, ea_map_, front_of_pos_,
-                               pos2j_, j2pos_, poff_, foff_, sym_.j_base, sym_.npos);
+    const MfView v = view();
     const NrScratch1 sc{d_part1_.data(), d_nrcnt_.data()};
     const double *F = d_F_.data();
     for (const Level &L : levels_)
@@ -1033,8 +1080,7 @@ void MfFactor::solve_batch(const StiffDev &S, const double *t, float2 *z, const 
     if (sym_.nfront == 0) return;
     if (d_Fp_.size() < (size_t)sym_.elems) fail(LSS_ERR_INTERNAL, "batched multifrontal solve before make_pairs");
     constexpr int NR = 16;
-    const MfView v = make_view(p0_, s_, u_, woff_, bnd_off_, bnd_pos_, child_off_, child_, ea_map_, front_of_pos_,
-                               pos2j_, j2pos_, poff_, foff_, sym_.j_base, sym_.npos);
+    const MfView v = view();
     const size_t smem = NR_SMEM;
     raise_smem_limit((const void *)mf_forward_nr_kernel<NR>, smem);
     raise_smem_limit((const void *)mf_backward_nr_kernel<NR>, smem);

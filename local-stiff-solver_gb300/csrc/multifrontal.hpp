@@ -31,15 +31,19 @@
 
 namespace lss {
 
-// Fronts up to this size are swept by one CTA in shared memory.
-constexpr int MF_SMEM_F = 160;
+// Fronts up to this size are swept by one CTA in shared memory; beyond, the
+// blocked sweep spreads a front over the GPU (a sweep of 160 pivots on one SM
+// is bound by its FP64 pipe: 385 us, against about 45 us per 32 pivots blocked).
+constexpr int MF_SMEM_F = 64;
 
 // Host symbolic structure of all large subdomains together.  Positions
 // (elimination order) are global over the subdomains; the variables of a
 // subtree occupy a contiguous range of positions and a front's own variables
 // are the last of its subtree.
 struct MfSymbolic {
-    int32_t nfront = 0, npos = 0, levels = 0;
+    int32_t nfront = 0, npos = 0;
+    int32_t levels = 0;             // of the tree of fronts (launches of the solve and the factorization)
+    int32_t dissection_levels = 0;  // of the nested dissection: a front with four children joins two
     std::vector<int32_t> p0, s, u, height;     // per front
     std::vector<int64_t> foff;                 // per front: element offset of its f x f storage
     std::vector<int32_t> woff;                 // per front: offset of its solve vector (f entries)
@@ -79,6 +83,14 @@ struct MfCta {
     int32_t s, f, col0, ncol, q0, nrow, kc, nkc, woff, p0, bnd_off, pad;
 };
 
+// The symbolic arrays as kernels see them.
+struct MfView {
+    const int32_t *p0, *s, *u, *woff, *bnd_off, *bnd_pos, *child_off, *child, *ea_map, *front_of_pos, *pos2j,
+        *j2pos, *poff;
+    const int64_t *foff;
+    int32_t j_base, npos;
+};
+
 // The device side: symbolic arrays, front storage, solve vectors, and the
 // per-level work lists of every kernel.
 class MfFactor {
@@ -96,6 +108,12 @@ public:
                      cudaStream_t s);
     // the fronts as double-float pairs for solve_batch (after the fronts are final)
     void make_pairs(cudaStream_t s);
+    // The dense blocks above MF_SMEM_F as fronts without boundary, for the
+    // blocked sweep alone: invert_dense inverts them (given in the upper
+    // triangles) in place in the dense inverses' storage.
+    void setup_dense(const std::vector<int32_t> &off, const std::vector<int64_t> &inv_off, int32_t ndense,
+                     cudaStream_t s);
+    void invert_dense(double *inv, int *bad, cudaStream_t s);
     const MfSymbolic &symbolic() const { return sym_; }
     // device front storage (f x f per front, foff offsets), for merging factors
     const double *fronts() const { return d_F_.data(); }
@@ -109,6 +127,8 @@ private:
         int64_t fwd1 = 0, bwd1 = 0;  // descriptors of the single right-hand-side solve (into d_ctas_)
         int32_t nfwd1 = 0, nbwd1 = 0;
     };
+    MfView view() const;
+    void sweep_large(const Level &L, const MfView &v, double *F, bool whole, int *bad, cudaStream_t st);
     MfSymbolic sym_;
     std::vector<Level> levels_;
     DBuf<int32_t> d_i32_;  // symbolic arrays and work-list fronts

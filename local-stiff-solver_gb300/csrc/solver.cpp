@@ -609,6 +609,7 @@ void HybridSolver::setup_stiff()
         d_swarps_.release();
         d_st_.release();
         mf_ = std::make_unique<MfFactor>();
+        dense_ = std::make_unique<MfFactor>();
         h_sdofs_.clear();
         h_soff_.assign(1, 0);
         h_sinvoff_.clear();
@@ -634,12 +635,14 @@ void HybridSolver::setup_stiff()
         d_swarps_.upload(warps, stream_);
         stiff_.warps = d_swarps_.data();
         stiff_.nwarps = (int32_t)warps.size();
+        dense_->setup_dense(off, inv_off, ndense, stream_);
     }
     stats_["stiff_layout_reused"] = same ? 1.0 : 0.0;
     d_sinv_.zero(stream_);
     d_bad_.zero(stream_);
     launch_stiff_extract(A_, stiff_, d_sinv_.data(), stream_);
-    launch_stiff_invert(stiff_, off.data(), ndense, d_sinv_.data(), d_bad_.data(), stream_);
+    launch_stiff_invert(stiff_, off.data(), ndense, MF_SMEM_F, d_sinv_.data(), d_bad_.data(), stream_);
+    dense_->invert_dense(d_sinv_.data(), d_bad_.data(), stream_);
     if (ndense < stiff_.nsub) {
         if (!same) {
             auto t0 = clk::now();
@@ -652,7 +655,8 @@ void HybridSolver::setup_stiff()
         mf_->factorize(A_, stiff_, d_bad_.data(), stream_);
         const MfSymbolic &sym = mf_->symbolic();
         stats_["multifrontal_fronts"] = sym.nfront;
-        stats_["multifrontal_levels"] = sym.levels;
+        stats_["multifrontal_levels"] = sym.dissection_levels;
+        stats_["multifrontal_tree_levels"] = sym.levels;
         stats_["multifrontal_max_front"] = sym.max_f;
         stats_["multifrontal_fmas"] = sym.fmas;
         stats_["multifrontal_bytes"] = (double)mf_->bytes();

@@ -138,6 +138,7 @@ private:
     DBuf<float> d_sinv32_;
     DBuf<StiffWarp> d_swarps_;
     std::unique_ptr<MfFactor> mf_;  // subdomains above STIFF_DENSE_MAX DOFs
+    std::unique_ptr<MfFactor> dense_;  // sweeps of the dense blocks above MF_SMEM_F DOFs
     // host copies of the stiff layout (batched solves merge them)
     std::vector<int32_t> h_sdofs_, h_soff_;
     std::vector<int64_t> h_sinvoff_;

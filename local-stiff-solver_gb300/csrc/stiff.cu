@@ -5,8 +5,8 @@
 // (GPUHybrid.cu:993-1411), and applies next_z = z + S^T A_SS^-1 S (r - A z)
 // (dss_precond_iter, GPUHybrid.cu:544-675).  Here a subdomain of up to
 // STIFF_DENSE_MAX DOFs is gathered into a dense FP64 block, inverted in FP64
-// by the symmetric sweep (one CTA in shared memory) and applied as a GEMV
-// fused with the scatter; larger subdomains get the FP64
+// by the symmetric sweep (up to 64 DOFs one CTA in shared memory, beyond by the
+// blocked sweep of multifrontal.cu) and applied as a GEMV fused with the scatter; larger subdomains get the FP64
 // multifrontal factor (multifrontal.cu).  The residual rows r - A z are only
 // computed on the stiff rows (the reference forms the full product and
 // gathers it).
@@ -78,14 +78,16 @@ __device__ void sweep_invert_small(double *S, int ld, int N, double *col, double
     }
 }
 
-// one CTA per small subdomain (m <= 160), in place in global storage
+// one CTA per subdomain of at most max_m DOFs (the others are swept blocked),
+// in place in global storage
 __global__ void __launch_bounds__(256) invert_small_kernel(const int32_t *__restrict__ off,
                                                            const int64_t *__restrict__ inv_off,
-                                                           double *__restrict__ inv, int *bad)
+                                                           double *__restrict__ inv, int max_m, int *bad)
 {
     extern __shared__ double sm[];
     const int32_t s = blockIdx.x;  // the dense subdomains come first
     const int m = off[s + 1] - off[s], ld = m + 1;
+    if (m > max_m) return;
     double *S = sm, *col = sm + m * ld, *scol = col + m;
     double *g = inv + inv_off[s];
     for (int idx = threadIdx.x; idx < m * m; idx += blockDim.x) {
@@ -193,20 +195,16 @@ void launch_stiff_extract(const BsrDev &A, const StiffDev &S, double *stage, cud
     LSS_LAUNCH_CHECK();
 }
 
-void launch_stiff_invert(const StiffDev &S, const int32_t *h_off, int32_t nsub, double *inv, int *bad,
+void launch_stiff_invert(const StiffDev &S, const int32_t *h_off, int32_t nsub, int max_m, double *inv, int *bad,
                          cudaStream_t s)
 {
-    if (nsub == 0) return;
-    int maxm = 0;
-    for (int32_t q = 0; q < nsub; ++q) {
-        const int m = h_off[q + 1] - h_off[q];
-        if (m > STIFF_DENSE_MAX) fail(LSS_ERR_INTERNAL, "a dense stiff block above the shared-memory size");
-        maxm = std::max(maxm, m);
-    }
-    // (160 * 161 + 320) doubles = 204 KB of shared memory at most
-    const size_t smem = (size_t)(maxm * (maxm + 1) + 2 * maxm) * sizeof(double);
+    int m = 0;
+    for (int32_t q = 0; q < nsub; ++q)
+        if (h_off[q + 1] - h_off[q] <= max_m) m = std::max(m, h_off[q + 1] - h_off[q]);
+    if (m == 0) return;
+    const size_t smem = (size_t)(m * (m + 1) + 2 * m) * sizeof(double);
     raise_smem_limit((const void *)invert_small_kernel, smem);
-    invert_small_kernel<<<(unsigned)nsub, 256, smem, s>>>(S.off, S.inv_off, inv, bad);
+    invert_small_kernel<<<(unsigned)nsub, 256, smem, s>>>(S.off, S.inv_off, inv, max_m, bad);
     LSS_LAUNCH_CHECK();
 }
 
