@@ -190,9 +190,7 @@ struct MasDev {
     int base = 1;                       // levels up to this one are restricted level by level
     const int32_t *memb_ptr[MAS_MAXL] = {};  // l > base: per item, its range of memb
     const int32_t *memb[MAS_MAXL] = {};      // l > base: items of the base level grouped by their item at level l
-    const unsigned *need = nullptr;     // per level-1 bank: partitions that hold its items
     const uint8_t *uncoupled = nullptr; // per coarse bank: no couplings between its items
-    unsigned *arrive = nullptr;         // per level-1 bank: arrivals of the running apply (zero between applies)
     int64_t tile_elems = 0;             // inverse elements per bank
     int64_t bank_bytes0 = 0;            // > 0: level-0 banks hold FP32 diagonal and BF16 off-diagonal tiles, this stride
     int64_t level_elems = 0;            // elements of the level-vector buffers

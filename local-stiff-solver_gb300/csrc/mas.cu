@@ -414,97 +414,97 @@ __device__ __forceinline__ void bank_segment_sums(const T *xs, uint8_t key, unsi
     }
 }
 
-// The restriction of r to level 1 and, in a large hierarchy, to level 2
-// (MasDev::base; the levels above are summed from there by the products that
-// need them, symv_coarse_kernel).
-//
-// A warp sums one partition's rows into its level-1 items.  For level 2 it then
-// reports to the level-1 banks that hold them (arrive[g], at most two banks);
-// the warp whose report is a bank's last queues it in its CTA, whose warps
-// restrict the queued banks.  Nothing waits: whoever completes a bank
-// continues with it, and each sum has one fixed order whoever runs it.  A
-// report costs 3 to 4 us of latency, so carrying it through every level took
-// 14 to 22 us a launch; one launch per level took more.
+// The restriction of r to level 1: a warp sums one partition's rows into its
+// level-1 items.  In a large hierarchy a second launch sums the level-1 banks
+// into level 2 (MasDev::base); the levels above are summed from the base level
+// by the products that need them (symv_coarse_kernel).  Restricting completed
+// banks further inside this launch, found by arrival counters, saved launches
+// but paid a fence and an atomic per bank: 14 to 22 us with all levels, 41 us
+// with one on 33k partitions.
 template <int BD, typename T, typename XT>
 __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__restrict__ r, T *__restrict__ v,
                                                        PcgState *st, PcgSum rr)
 {
+    constexpr int N = 32 * BD, W = 8;
+    __shared__ T xs_all[W][N];
+    __shared__ unsigned mask_all[W][32];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    T *xs = xs_all[wl];
+    // a partition's bounds and items do not depend on the preceding kernel
+    int64_t p = (int64_t)blockIdx.x * W + wl;
+    const int64_t step = (int64_t)gridDim.x * W;
+    struct Part {
+        int32_t lo, cnt, i0;
+        int nc;
+        uint8_t key;
+    };
+    auto part = [&](int64_t q) {
+        Part t{0, 0, 0, 0, 0xff};
+        if (q < m.nparts) {
+            t.lo = m.part_off[q];
+            t.cnt = m.part_off[q + 1] - t.lo;
+            t.i0 = m.cbase0[q];
+            t.nc = m.ccnt0[q];
+            if (lane < t.cnt) t.key = m.key0[t.lo + lane];
+        }
+        return t;
+    };
+    Part t = part(p);
     pdl_enter();
     if (st && st->done) return;
     if (rr.part) {  // the updated residual's convergence tests (GPUHybrid.cu:1488-1496)
-        const double t = get_sum(rr);
+        const double s = get_sum(rr);
         int stop = STOP_RUNNING;
-        if (!(t == t) || isinf(t)) stop = STOP_NONFINITE;
-        else if (st->rel_eps > 0 && t / st->bb < st->rel_eps) stop = STOP_CONVERGED_REL;
-        else if (st->abs_eps > 0 && t < st->abs_eps) stop = STOP_CONVERGED_ABS;
+        if (!(s == s) || isinf(s)) stop = STOP_NONFINITE;
+        else if (st->rel_eps > 0 && s / st->bb < st->rel_eps) stop = STOP_CONVERGED_REL;
+        else if (st->abs_eps > 0 && s < st->abs_eps) stop = STOP_CONVERGED_ABS;
         else if (st->iter >= st->max_iter) stop = STOP_MAX_ITER;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
-            st->rr = t;
+            st->rr = s;
             if (stop) st->done = stop;
         }
         if (stop) return;
     }
+    for (; p < m.nparts; p += step) {
+        // the part's values are one contiguous run: coalesced loads
+#pragma unroll
+        for (int q = 0; q < BD; ++q) {
+            const int e = q * 32 + lane;
+            xs[e] = e < t.cnt * BD ? (T)r[(int64_t)t.lo * BD + e] : T(0);
+        }
+        const Part next = part(p + step);
+        __syncwarp();
+        bank_segment_sums<BD, T>(xs, t.key, mask_all[wl], t.nc, v + m.voff[1] + (int64_t)t.i0 * BD, lane);
+        __syncwarp();
+        t = next;
+    }
+}
+
+// level 1 -> level 2, a warp per level-1 bank
+template <int BD, typename T>
+__global__ void __launch_bounds__(256) restrict1_kernel(MasDev m, T *__restrict__ v, const int *done)
+{
     constexpr int N = 32 * BD, W = 8;
     __shared__ T xs_all[W][N];
     __shared__ unsigned mask_all[W][32];
-    __shared__ int32_t queue[2 * W];  // ready level-1 banks: at most two per partition
-    __shared__ int qn;
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const int32_t b = blockIdx.x * W + wl;
+    const bool valid = b < m.nbanks[1];
+    const int32_t i0 = b * 32;
+    const int cnt = valid ? min(32, m.nitems[1] - i0) : 0, nc = valid ? m.ccnt[1][b] : 0;
+    const int32_t j0 = valid ? m.cbase[1][b] : 0;
+    const uint8_t key = lane < cnt ? m.key[1][i0 + lane] : (uint8_t)0xff;
+    pdl_enter();
+    if (!valid || (done && *done)) return;
+    const T *vl = v + m.voff[1] + (int64_t)i0 * BD;
     T *xs = xs_all[wl];
-    unsigned *mask = mask_all[wl];
-    if (threadIdx.x == 0) qn = 0;
-    __syncthreads();
-    // reports level-1 items [i0, i0 + cnt) as written; queues completed banks
-    auto report = [&](int32_t i0, int cnt) {
-        __threadfence();
-        __syncwarp();
-        if (lane < 2 && cnt > 0) {
-            const int32_t b = (i0 >> 5) + lane;
-            if (b <= (i0 + cnt - 1) >> 5 && atomicAdd(m.arrive + b, 1u) + 1u == m.need[b]) {
-                m.arrive[b] = 0u;
-                __threadfence();
-                queue[atomicAdd(&qn, 1)] = b;
-            }
-        }
-    };
-    for (int64_t p0 = (int64_t)blockIdx.x * W; p0 < m.nparts; p0 += (int64_t)gridDim.x * W) {
-        const int64_t p = p0 + wl;
-        if (p < m.nparts) {
-            const int32_t lo = m.part_off[p], cnt = m.part_off[p + 1] - lo;
-            // the part's values are one contiguous run: coalesced loads
 #pragma unroll
-            for (int q = 0; q < BD; ++q) {
-                const int e = q * 32 + lane;
-                xs[e] = e < cnt * BD ? (T)r[(int64_t)lo * BD + e] : T(0);
-            }
-            const uint8_t key = lane < cnt ? m.key0[lo + lane] : (uint8_t)0xff;
-            const int32_t i0 = m.cbase0[p];
-            const int nc = m.ccnt0[p];
-            __syncwarp();
-            bank_segment_sums<BD, T>(xs, key, mask, nc, v + m.voff[1] + (int64_t)i0 * BD, lane);
-            if (m.base > 1) report(i0, nc);
-            __syncwarp();
-        }
-        if (m.base == 1) continue;
-        __syncthreads();
-        for (int k = wl; k < qn; k += W) {
-            const int32_t b = queue[k], i0 = b * 32;
-            const int cnt = min(32, m.nitems[1] - i0);
-            const T *vl = v + m.voff[1] + (int64_t)i0 * BD;
-#pragma unroll
-            for (int q = 0; q < BD; ++q) {
-                const int e = q * 32 + lane;
-                xs[e] = e < cnt * BD ? __ldcg(vl + e) : T(0);
-            }
-            const uint8_t key = lane < cnt ? m.key[1][i0 + lane] : (uint8_t)0xff;
-            __syncwarp();
-            bank_segment_sums<BD, T>(xs, key, mask, m.ccnt[1][b], v + m.voff[2] + (int64_t)m.cbase[1][b] * BD, lane);
-            __syncwarp();
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) qn = 0;
-        __syncthreads();
+    for (int q = 0; q < BD; ++q) {
+        const int e = q * 32 + lane;
+        xs[e] = e < cnt * BD ? vl[e] : T(0);
     }
+    __syncwarp();
+    bank_segment_sums<BD, T>(xs, key, mask_all[wl], nc, v + m.voff[2] + (int64_t)j0 * BD, lane);
 }
 
 // x of a coarse bank above the base level: every item's sum over the base-level
@@ -799,6 +799,8 @@ void mas_apply_dot_t(const MasDev &m, const T *inv0, const T *invc, T *v, T *u, 
     const int *done = &st->done;
     launch_pdl(restrict_kernel<BD, T, XT>, grid_for(m.nparts, 8, sm_grid(8)), 256, 0, s, m, xin, v, st,
                rr ? *rr : PcgSum{});
+    if (m.base > 1)
+        launch_pdl(restrict1_kernel<BD, T>, (unsigned)((m.nbanks[1] + 7) / 8), 256, 0, s, m, v, done);
     launch_pdl(symv_coarse_kernel<BD, T>, (unsigned)m.ncoarse, 256, 0, s, m, invc, (const T *)v, u, done);
 #define LSS_S0(A_, D_)                                                                                          \
     do {                                                                                                        \

@@ -39,51 +39,25 @@ template <int BD, int LANES>
 __global__ void __launch_bounds__(256) spmv_kernel(BsrDev A, const double *__restrict__ x, double *__restrict__ y,
                                                    const int *done)
 {
+    __shared__ double buf[rows_smem<BD, LANES>];
     if (done && *done) return;
-    const int lane = threadIdx.x % LANES;
-    constexpr int RPW = 32 / LANES;  // block rows per warp and sweep
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    // warp-uniform trip count: every lane reaches the group shuffles together
-    for (int64_t wr = w0 * RPW; wr < A.nb; wr += nw * RPW) {
-        const int64_t i = wr + (threadIdx.x & 31) / LANES;
-        const bool valid = i < A.nb;
-        double acc[BD];
-        bsr_block_row<BD, LANES, double, double, double>(A.rows, A.cols, A.vals, (int32_t)i, valid, x, lane, acc);
-        // lane l of the group stores the components k with k % LANES == l
-        // (all BD of them when LANES == 1)
-        if (valid) {
-#pragma unroll
-            for (int k = 0; k < BD; ++k)
-                if (k % LANES == lane) y[i * BD + k] = acc[k];
-        }
-    }
+    fp64_rows<BD, LANES>(A.rows, A.cols, A.vals, A.nb, x, buf,
+                         [&](int32_t i, int k, double v) { y[(int64_t)i * BD + k] = v; });
 }
 
-// y = r - A x, operator in VT precision, accumulation in ACC
-template <int BD, int LANES, typename VT, typename ACC, typename XT>
-__global__ void __launch_bounds__(256) residual_kernel(BsrDev A, const VT *__restrict__ vals,
-                                                       const double *__restrict__ r, const XT *__restrict__ x,
-                                                       double *__restrict__ y, const int *done)
+// y = r - A x
+template <int BD, int LANES>
+__global__ void __launch_bounds__(256) residual_kernel(BsrDev A, const double *__restrict__ r,
+                                                       const double *__restrict__ x, double *__restrict__ y,
+                                                       const int *done)
 {
+    __shared__ double buf[rows_smem<BD, LANES>];
     pdl_enter();
     if (done && *done) return;
-    const int lane = threadIdx.x % LANES;
-    constexpr int RPW = 32 / LANES;  // block rows per warp and sweep
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    // warp-uniform trip count: every lane reaches the group shuffles together
-    for (int64_t wr = w0 * RPW; wr < A.nb; wr += nw * RPW) {
-        const int64_t i = wr + (threadIdx.x & 31) / LANES;
-        const bool valid = i < A.nb;
-        ACC acc[BD];
-        bsr_block_row<BD, LANES, VT, XT, ACC>(A.rows, A.cols, vals, (int32_t)i, valid, x, lane, acc);
-        if (valid) {
-#pragma unroll
-            for (int k = 0; k < BD; ++k)
-                if (k % LANES == lane) y[i * BD + k] = r[i * BD + k] - (double)acc[k];
-        }
-    }
+    fp64_rows<BD, LANES>(A.rows, A.cols, A.vals, A.nb, x, buf, [&](int32_t i, int k, double v) {
+        const int64_t e = (int64_t)i * BD + k;
+        y[e] = r[e] - v;
+    });
 }
 
 // y32 = r - A x for the mixed preconditioner, rounded to FP32 (its result
@@ -139,28 +113,15 @@ __global__ void __launch_bounds__(256) spmv_alpha_kernel(BsrDev A, const double 
                                                          double *__restrict__ Ap, const PcgState *st, GridReduce gr,
                                                          PcgSum pap)
 {
+    __shared__ double buf[rows_smem<BD, LANES>];
     pdl_enter();
     if (st->done) return;
-    const int lane = threadIdx.x % LANES;
-    constexpr int RPW = 32 / LANES;  // block rows per warp and sweep
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     double dot = 0.0;
-    // warp-uniform trip count: every lane reaches the group shuffles together
-    for (int64_t wr = w0 * RPW; wr < A.nb; wr += nw * RPW) {
-        const int64_t i = wr + (threadIdx.x & 31) / LANES;
-        const bool valid = i < A.nb;
-        double acc[BD];
-        bsr_block_row<BD, LANES, double, double, double>(A.rows, A.cols, A.vals, (int32_t)i, valid, p, lane, acc);
-        if (valid) {
-#pragma unroll
-            for (int k = 0; k < BD; ++k)
-                if (k % LANES == lane) {
-                    Ap[i * BD + k] = acc[k];
-                    dot += p[i * BD + k] * acc[k];
-                }
-        }
-    }
+    fp64_rows<BD, LANES>(A.rows, A.cols, A.vals, A.nb, p, buf, [&](int32_t i, int k, double v) {
+        const int64_t e = (int64_t)i * BD + k;
+        Ap[e] = v;
+        dot += p[e] * v;
+    });
     put_sum(dot, gr, pap);
 }
 
@@ -397,20 +358,20 @@ void spmv_dispatch(const BsrDev &A, const double *x, double *y, const int *done,
     }
 }
 
-template <int BD, typename VT, typename ACC, typename XT>
-void residual_dispatch(const BsrDev &A, const VT *vals, const double *r, const XT *x, double *y,
-                       const int *done, cudaStream_t s)
+template <int BD>
+void residual_dispatch(const BsrDev &A, const double *r, const double *x, double *y, const int *done, cudaStream_t s)
 {
-    const int lanes = sizeof(VT) == 4 ? A.lanes32 : A.lanes;
-    const int grid = grid_for((int64_t)A.nb * lanes, 256, sm_grid(16));
-    switch (lanes) {
-    case 1: launch_pdl(residual_kernel<BD, 1, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
-    case 2: launch_pdl(residual_kernel<BD, 2, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
-    case 4: launch_pdl(residual_kernel<BD, 4, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
-    case 8: launch_pdl(residual_kernel<BD, 8, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
-    case 16: launch_pdl(residual_kernel<BD, 16, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
-    default: launch_pdl(residual_kernel<BD, 32, VT, ACC, XT>, grid, 256, 0, s, A, vals, r, x, y, done); break;
+    const int grid = grid_for((int64_t)A.nb * A.lanes, 256, sm_grid(16));
+#define LSS_RES(L_) launch_pdl(residual_kernel<BD, L_>, grid, 256, 0, s, A, r, x, y, done)
+    switch (A.lanes) {
+    case 1: LSS_RES(1); break;
+    case 2: LSS_RES(2); break;
+    case 4: LSS_RES(4); break;
+    case 8: LSS_RES(8); break;
+    case 16: LSS_RES(16); break;
+    default: LSS_RES(32); break;
     }
+#undef LSS_RES
 }
 
 // marks `sum` as produced by a launch of `grid` CTAs over n rows
@@ -459,9 +420,9 @@ void launch_spmv(const BsrDev &A, const double *x, double *y, const int *done, c
 void launch_residual_spmv(const BsrDev &A, const double *r, const double *x, double *y, const int *done,
                           cudaStream_t s)
 {
-    if (A.bd == 1) residual_dispatch<1, double, double, double>(A, A.vals, r, x, y, done, s);
-    else if (A.bd == 2) residual_dispatch<2, double, double, double>(A, A.vals, r, x, y, done, s);
-    else residual_dispatch<3, double, double, double>(A, A.vals, r, x, y, done, s);
+    if (A.bd == 1) residual_dispatch<1>(A, r, x, y, done, s);
+    else if (A.bd == 2) residual_dispatch<2>(A, r, x, y, done, s);
+    else residual_dispatch<3>(A, r, x, y, done, s);
     LSS_LAUNCH_CHECK();
 }
 

@@ -258,22 +258,10 @@ void HybridSolver::analyze(int32_t n, int64_t nnz, const int32_t *outer, const i
     mas_.ncoarse = boff;
     mas_.level_elems = voff;
     mas_.cmap = d_cmap_.data();
-    // how many partitions report to every level-1 bank (a partition's items are
-    // consecutive, so they lie in at most two banks)
-    std::vector<unsigned> need(std::max(cs_.nbanks[1], 1), 0u);
-    for (size_t b = 0; b < cs_.cbase0.size(); ++b)
-        if (cs_.ccnt0[b])
-            for (int32_t q = cs_.cbase0[b] >> 5; q <= (cs_.cbase0[b] + cs_.ccnt0[b] - 1) >> 5; ++q) ++need[q];
-    d_need_.upload(need, stream_);
-    d_arrive_.resize(need.size());
-    d_arrive_.zero(stream_);
-    mas_.need = d_need_.data();
-    mas_.arrive = d_arrive_.data();
-    // The levels above the base level sum their items from it.  Level 2 costs the
-    // restriction a report and a second step (2 us of an apply), level 1 as base
-    // makes one CTA add up to all of its items: with 1k level-1 items base 1 is
-    // 2 us faster, with 4k even in FP32 and 8 us slower in FP64, with 11k 18
-    // (FP32) and 40 us (FP64) slower.
+    // The levels above the base level sum their items from it.  Level 2 costs a
+    // second restriction launch (2 us), level 1 as base makes one CTA add up to
+    // all of its items: with 1k level-1 items base 1 is 2 us faster, with 4k even
+    // in FP32 and 8 us slower in FP64, with 11k 18 (FP32) and 40 us (FP64) slower.
     mas_.base = cs_.L > 2 && cs_.nitems[1] > 2048 ? 2 : 1;
     std::vector<int32_t> memb;
     std::vector<std::pair<size_t, size_t>> at(cs_.L);

@@ -123,7 +123,6 @@ private:
         d_chunk_r0_;
     CoarseMembers memb_;
     DBuf<uint8_t> d_key0_, d_ccnt0_, d_uncoupled_;
-    DBuf<unsigned> d_need_, d_arrive_;  // level-1 banks: contributing partitions, arrivals of an apply
     DBuf<int32_t> d_membl_;             // base-level items by coarse item (MasDev::memb)
     std::vector<DBuf<uint8_t>> d_key_, d_ccnt_;
     std::vector<DBuf<int32_t>> d_cbase_;

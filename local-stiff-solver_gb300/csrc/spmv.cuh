@@ -24,12 +24,11 @@ __device__ __forceinline__ T group_sum(T v)
     return v;
 }
 
-// y[0..BD) = (A x)[block row i], reduced over the LANES-wide group (valid in
-// every lane of the group).  VT: stored value type; XT: x type; ACC: accumulator.
-// Every lane of the warp must call it (the group reduction is a full-warp
-// shuffle); a group without a row passes valid = false and gets zeros.
+// y[0..BD) = this lane's part of (A x)[block row i]: the blocks l = lane,
+// lane + LANES, ...  VT: stored value type; XT: x type; ACC: accumulator.  A
+// group without a row passes valid = false and gets zeros.
 template <int BD, int LANES, typename VT, typename XT, typename ACC>
-__device__ __forceinline__ void bsr_block_row(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols,
+__device__ __forceinline__ void bsr_block_row_part(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols,
                                               const VT *__restrict__ vals, int32_t i, bool valid,
                                               const XT *__restrict__ x, int lane, ACC (&y)[BD])
 {
@@ -48,25 +47,62 @@ __device__ __forceinline__ void bsr_block_row(const int32_t *__restrict__ rows, 
 #pragma unroll
             for (int k = 0; k < BD; ++k) y[r] += (ACC)__ldcs(v + (int64_t)(r * BD + k) * len + l) * xv[k];
     }
+}
+
+// y[0..BD) = (A x)[block row i], reduced over the LANES-wide group (valid in
+// every lane of the group).  Every lane of the warp must call it (the group
+// reduction is a full-warp shuffle).
+template <int BD, int LANES, typename VT, typename XT, typename ACC>
+__device__ __forceinline__ void bsr_block_row(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols,
+                                              const VT *__restrict__ vals, int32_t i, bool valid,
+                                              const XT *__restrict__ x, int lane, ACC (&y)[BD])
+{
+    bsr_block_row_part<BD, LANES, VT, XT, ACC>(rows, cols, vals, i, valid, x, lane, y);
 #pragma unroll
     for (int r = 0; r < BD; ++r) y[r] = group_sum<LANES>(y[r]);
 }
 
-// One scalar row (component comp of block row i) of A x, warp-wide (valid in all lanes).
-template <int BD, typename VT, typename XT>
-__device__ __forceinline__ double bsr_scalar_row(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols,
-                                                 const VT *__restrict__ vals, int32_t i, int comp,
-                                                 const XT *__restrict__ x, int lane)
+// A x in FP64 over the block rows, 256 threads per CTA, out(i, k, value) once
+// per scalar row.  The lanes' parts meet in shared memory, one thread adding
+// the LANES parts of one scalar row: an FP64 add costs the pipe a whole warp
+// however it is predicated, and the group's shuffle reduction ran log2(LANES)
+// of them per component in every warp (a third of the instructions of a 3 x 3
+// product at eight lanes; here a sixth) and left the epilogue to one lane in
+// eight.  `buf`: rows_smem<BD, LANES> doubles.
+template <int BD, int LANES>
+constexpr int rows_smem = LANES == 1 ? 1 : 256 / LANES * BD * (LANES + 1);
+
+template <int BD, int LANES, typename Out>
+__device__ __forceinline__ void fp64_rows(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols,
+                                          const double *__restrict__ vals, int32_t nb, const double *__restrict__ x,
+                                          double *__restrict__ buf, Out out)
 {
-    const int32_t b = rows[i], e = rows[i + 1], len = e - b;
-    const VT *__restrict__ v = vals + (int64_t)b * (BD * BD);
-    double acc = 0.0;
-    for (int32_t l = lane; l < len; l += 32) {
-        const int32_t c = cols[b + l];
+    constexpr int RP = 256 / LANES;  // block rows per CTA and sweep
+    const int lane = threadIdx.x % LANES, row = threadIdx.x / LANES;
+    for (int64_t r0 = (int64_t)blockIdx.x * RP; r0 < nb; r0 += (int64_t)gridDim.x * RP) {
+        const bool valid = r0 + row < nb;
+        double acc[BD];
+        bsr_block_row_part<BD, LANES, double, double, double>(rows, cols, vals, (int32_t)(r0 + row), valid, x, lane,
+                                                              acc);
+        if (LANES == 1) {
+            if (valid)
 #pragma unroll
-        for (int k = 0; k < BD; ++k) acc += (double)v[(int64_t)(comp * BD + k) * len + l] * (double)x[(int64_t)c * BD + k];
+                for (int k = 0; k < BD; ++k) out((int32_t)(r0 + row), k, acc[k]);
+            continue;
+        }
+#pragma unroll
+        for (int k = 0; k < BD; ++k) buf[(row * BD + k) * (LANES + 1) + lane] = acc[k];
+        __syncthreads();
+        for (int o = threadIdx.x; o < RP * BD; o += 256) {
+            const int32_t i = (int32_t)(r0 + o / BD);
+            if (i >= nb) break;
+            double sum = buf[o * (LANES + 1)];
+#pragma unroll
+            for (int q = 1; q < LANES; ++q) sum += buf[o * (LANES + 1) + q];
+            out(i, o % BD, sum);
+        }
+        __syncthreads();
     }
-    return group_sum<32>(acc);
 }
 
 // ---- double-float (an FP32 pair hi + lo) arithmetic on the FP32 pipe.  The
