@@ -24,6 +24,28 @@ __device__ __forceinline__ T group_sum(T v)
     return v;
 }
 
+// The blocks l = lane, lane + LANES, ... of a row, block(l, column) each.  Up to
+// eight lanes the steps are paired by hand: unrolled by the compiler, the lanes
+// with an odd count ran the loop's remainder apart, three rounds of products
+// for a row of 15 blocks on eight lanes instead of two (648k DOFs in FP64: 93
+// against 70 us, 3.0M in double-float 225 against 208).  From 16 lanes on a row
+// is mostly one step, where the plain loop is shorter (207k: 23 against 26 us).
+template <int LANES, typename Block>
+__device__ __forceinline__ void row_steps(const int32_t *__restrict__ cols, int32_t len, int lane, Block block)
+{
+    if constexpr (LANES >= 16) {
+#pragma unroll 2
+        for (int32_t l = lane; l < len; l += LANES) block(l, __ldcs(cols + l));
+    } else {
+        for (int32_t l = lane; l < len; l += 2 * LANES) {
+            const bool two = l + LANES < len;
+            const int32_t c = __ldcs(cols + l), c2 = two ? __ldcs(cols + l + LANES) : c;
+            block(l, c);
+            if (two) block(l + LANES, c2);
+        }
+    }
+}
+
 // y[0..BD) = this lane's part of (A x)[block row i]: the blocks l = lane,
 // lane + LANES, ...  VT: stored value type; XT: x type; ACC: accumulator.  A
 // group without a row passes valid = false and gets zeros.
@@ -36,9 +58,7 @@ __device__ __forceinline__ void bsr_block_row_part(const int32_t *__restrict__ r
     const VT *__restrict__ v = vals + (int64_t)b * (BD * BD);
 #pragma unroll
     for (int r = 0; r < BD; ++r) y[r] = ACC(0);
-#pragma unroll 2
-    for (int32_t l = lane; l < len; l += LANES) {
-        const int32_t c = __ldcs(cols + b + l);
+    row_steps<LANES>(cols + b, len, lane, [&](int32_t l, int32_t c) {
         ACC xv[BD];
 #pragma unroll
         for (int k = 0; k < BD; ++k) xv[k] = (ACC)x[(int64_t)c * BD + k];
@@ -46,7 +66,7 @@ __device__ __forceinline__ void bsr_block_row_part(const int32_t *__restrict__ r
         for (int r = 0; r < BD; ++r)
 #pragma unroll
             for (int k = 0; k < BD; ++k) y[r] += (ACC)__ldcs(v + (int64_t)(r * BD + k) * len + l) * xv[k];
-    }
+    });
 }
 
 // y[0..BD) = (A x)[block row i], reduced over the LANES-wide group (valid in
@@ -145,9 +165,7 @@ __device__ __forceinline__ void bsr_block_row_df(const int32_t *__restrict__ row
     const float2 *__restrict__ v = vals + (int64_t)b * (BD * BD);
 #pragma unroll
     for (int r = 0; r < BD; ++r) sh[r] = sl[r] = 0.f;
-#pragma unroll 2
-    for (int32_t l = lane; l < len; l += LANES) {
-        const int32_t c = __ldcs(cols + b + l);
+    row_steps<LANES>(cols + b, len, lane, [&](int32_t l, int32_t c) {
         float2 xv[BD];
 #pragma unroll
         for (int k = 0; k < BD; ++k) xv[k] = x[(int64_t)c * BD + k];
@@ -158,7 +176,7 @@ __device__ __forceinline__ void bsr_block_row_df(const int32_t *__restrict__ row
                 const float2 a = __ldcs(v + (int64_t)(r * BD + k) * len + l);
                 df_fma(sh[r], sl[r], a.x, a.y, xv[k].x, xv[k].y);
             }
-    }
+    });
 #pragma unroll
     for (int r = 0; r < BD; ++r)
 #pragma unroll
