@@ -125,6 +125,10 @@ __global__ void __launch_bounds__(256) spmv_alpha_kernel(BsrDev A, const double 
     put_sum(dot, gr, pap);
 }
 
+// The vector updates take VEC rows per thread, all loaded before any is stored
+// (their stores keep the compiler from hoisting the next row's loads).
+constexpr int VEC = 4, VEC_ROWS = 256 * VEC;
+
 __device__ __forceinline__ double as_double(double v) { return v; }
 __device__ __forceinline__ double as_double(float2 v) { return (double)v.x + (double)v.y; }
 
@@ -162,12 +166,28 @@ __global__ void __launch_bounds__(256) update_xr_kernel(int64_t n, double *__res
     }
     if (stop) return;
     double s = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        x[i] += alpha * p[i];
-        const double ri = r[i] - alpha * as_double(Ap[i]);
-        r[i] = ri;
-        if (r32) r32[i] = (float)ri;
-        s += ri * ri;
+    for (int64_t i0 = (int64_t)blockIdx.x * VEC_ROWS + threadIdx.x; i0 < n; i0 += (int64_t)gridDim.x * VEC_ROWS) {
+        double xv[VEC], pv[VEC], rv[VEC];
+        AT av[VEC];
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            const int64_t i = i0 + j * 256;
+            if (i >= n) break;
+            xv[j] = x[i];
+            pv[j] = p[i];
+            rv[j] = r[i];
+            av[j] = Ap[i];
+        }
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            const int64_t i = i0 + j * 256;
+            if (i >= n) break;
+            x[i] = xv[j] + alpha * pv[j];
+            const double ri = rv[j] - alpha * as_double(av[j]);
+            r[i] = ri;
+            if (r32) r32[i] = (float)ri;
+            s += ri * ri;
+        }
     }
     put_sum(s, gr, rr);
 }
@@ -187,12 +207,25 @@ __global__ void __launch_bounds__(256) update_p_kernel(int64_t n, double *__rest
             if (st->iter >= 1 && st->iter <= PCG_HIST) st->hist_beta[st->iter - 1] = beta;
         }
     }
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = first ? z[i] : z[i] + beta * p[i];
-        p[i] = v;
-        if (p_df) {
-            const float h = (float)v;
-            p_df[i] = make_float2(h, (float)(v - (double)h));
+    for (int64_t i0 = (int64_t)blockIdx.x * VEC_ROWS + threadIdx.x; i0 < n; i0 += (int64_t)gridDim.x * VEC_ROWS) {
+        double zv[VEC], pv[VEC];
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            const int64_t i = i0 + j * 256;
+            if (i >= n) break;
+            zv[j] = z[i];
+            pv[j] = first ? 0.0 : p[i];
+        }
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            const int64_t i = i0 + j * 256;
+            if (i >= n) break;
+            const double v = first ? zv[j] : zv[j] + beta * pv[j];
+            p[i] = v;
+            if (p_df) {
+                const float h = (float)v;
+                p_df[i] = make_float2(h, (float)(v - (double)h));
+            }
         }
     }
 }
