@@ -113,6 +113,43 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], GridReduce gr, double 
     return false;
 }
 
+// Conversions between FP64 and FP32 on the integer pipe, to the same bits as the
+// casts: a cast costs the FP64 pipe (two lanes per clock and SM) as much as a
+// multiply-add.  Values outside the ranges below (zeros, denormals, infinities,
+// NaN, extreme exponents) take the cast.
+__device__ __forceinline__ double to_double(float f)
+{
+    const uint32_t u = __float_as_uint(f), e = (u >> 23) & 0xffu;
+    if (e == 0u || e == 255u) return (double)f;
+    return __hiloint2double((int)((u & 0x80000000u) | ((e + 896u) << 20) | ((u >> 3) & 0xfffffu)), (int)(u << 29));
+}
+
+// v rounded to FP32 (round to nearest even)
+__device__ __forceinline__ float to_float(double v)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v), e = (hi >> 20) & 0x7ffu;
+    if (e - 897u > 252u) return (float)v;
+    const uint32_t m = ((hi & 0xfffffu) << 3) | (lo >> 29), rem = lo & 0x1fffffffu;
+    const uint32_t up = rem > 0x10000000u || (rem == 0x10000000u && (m & 1u)) ? 1u : 0u;
+    return __uint_as_float((hi & 0x80000000u) | ((((e - 896u) << 23) | m) + up));
+}
+
+// (fl32(v), fl32(v - fl32(v)))
+__device__ __forceinline__ float2 split_double(double v)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v), e = (hi >> 20) & 0x7ffu;
+    if (e - 949u > 200u) {
+        const float h = (float)v;
+        return make_float2(h, (float)(v - (double)h));
+    }
+    const uint32_t m = ((hi & 0xfffffu) << 3) | (lo >> 29), rem = lo & 0x1fffffffu;
+    const uint32_t up = rem > 0x10000000u || (rem == 0x10000000u && (m & 1u)) ? 1u : 0u;
+    // v - fl32(v) = +-(rem or rem - 2^29) * 2^(e - 1075), an integer of 29 bits scaled exactly
+    const int d = (int)rem - (int)(up << 29);
+    const float l = __fmul_rn((float)((hi & 0x80000000u) ? -d : d), __uint_as_float((e - 948u) << 23));
+    return make_float2(__uint_as_float((hi & 0x80000000u) | ((((e - 896u) << 23) | m) + up)), l);
+}
+
 // The PCG's scalar sums.  The kernel that forms the addends leaves the sum's
 // parts with put_sum; the next kernel that needs the scalar adds them in every
 // CTA with get_sum.  PcgSum::direct: one part per CTA, nothing else -- the

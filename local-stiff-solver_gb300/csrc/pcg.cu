@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(256) spmv_alpha_kernel(BsrDev A, const double 
 constexpr int VEC = 4, VEC_ROWS = 256 * VEC;
 
 __device__ __forceinline__ double as_double(double v) { return v; }
-__device__ __forceinline__ double as_double(float2 v) { return (double)v.x + (double)v.y; }
+__device__ __forceinline__ double as_double(float2 v) { return to_double(v.x) + to_double(v.y); }
 
 // alpha with the breakdown tests; x += alpha p; r -= alpha Ap; r.r
 // (GPUHybrid.cu:1463-1487).  Every CTA forms alpha from the parts of p.Ap, the
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) update_xr_kernel(int64_t n, double *__res
             x[i] = xv[j] + alpha * pv[j];
             const double ri = rv[j] - alpha * as_double(av[j]);
             r[i] = ri;
-            if (r32) r32[i] = (float)ri;
+            if (r32) r32[i] = to_float(ri);
             s += ri * ri;
         }
     }
@@ -222,10 +222,7 @@ __global__ void __launch_bounds__(256) update_p_kernel(int64_t n, double *__rest
             if (i >= n) break;
             const double v = first ? zv[j] : zv[j] + beta * pv[j];
             p[i] = v;
-            if (p_df) {
-                const float h = (float)v;
-                p_df[i] = make_float2(h, (float)(v - (double)h));
-            }
+            if (p_df) p_df[i] = split_double(v);
         }
     }
 }
@@ -233,9 +230,7 @@ __global__ void __launch_bounds__(256) update_p_kernel(int64_t n, double *__rest
 __global__ void split_kernel(int64_t n, const double *__restrict__ src, float2 *__restrict__ dst)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = src[i];
-        const float h = (float)v;
-        dst[i] = make_float2(h, (float)(v - (double)h));
+        dst[i] = split_double(src[i]);
     }
 }
 

@@ -84,3 +84,22 @@ def test_stiff_apply_edge_sizes(bs, m, built):
     rest[dofs] = False
     assert np.all(d[rest] == 0.0)
     s.close()
+
+
+@pytest.mark.parametrize("n", [3, 96, 3000])
+def test_double_float_split_matches_casts(n, built):
+    """The FP64 <-> FP32 conversions on the integer pipe equal the casts bit for
+    bit: through A = I the double-float product returns fl32(x) + fl32(x -
+    fl32(x)) exactly, for every sign, zeros, ties, denormal and extreme exponents."""
+    s = make_solver(3, "mixed", do_hybrid_precond=False)
+    s.factorize(sp.identity(n, format="csc"))
+    rng = np.random.default_rng(n)
+    for scale in (0, 30, 60, 126, 160):
+        x = rng.standard_normal(n) * 2.0 ** rng.uniform(-scale, min(scale, 100), size=n)
+        x[::7] = 0.0
+        x[1::11] = np.float64(np.float32(x[1::11])) * (1.0 + 2.0 ** -24)  # a tie of the high word
+        x[2::13] = np.float32(x[2::13])                                    # no low word
+        hi = x.astype(np.float32)
+        lo = (x - hi.astype(np.float64)).astype(np.float32)
+        np.testing.assert_array_equal(s.spmv_outer(x), hi.astype(np.float64) + lo.astype(np.float64))
+    s.close()
