@@ -234,16 +234,21 @@ __global__ void __launch_bounds__(256) assemble_coarse_sum_kernel(MasDev m, Coar
         }
 }
 
-// Symmetric sweep inversion of S (N x N, leading dimension ld, in shared
-// memory): the Gauss-Jordan variant of MASPreconditioner.cu:799-900, which
-// leaves -A^-1 in S.  Only the upper triangle (t <= c) is read and kept:
-// the sweep preserves symmetry, so half the FP64 updates suffice.  The
-// triangle's entries are dealt to the CTA's threads in linear order, so
-// every update instruction runs on full warps (a partly predicated FP64
-// instruction costs the pipe a whole warp).  Flags zero / non-finite pivots.
-// Needs blockDim.x == 256.
+// place of entry (t, c), t <= c, in the packed upper triangle
 template <int N>
-__device__ void sweep_invert(double *S, int ld, double *col, double *scol, int *bad)
+__device__ __forceinline__ int tri(int t, int c) { return t * N - t * (t - 1) / 2 + c - t; }
+
+// Symmetric sweep inversion of S (the upper triangle of an N x N matrix, packed
+// by rows, in shared memory): the Gauss-Jordan variant of
+// MASPreconditioner.cu:799-900, which leaves -A^-1 in S.  The sweep preserves
+// symmetry, so half the FP64 updates suffice.  The triangle's entries are dealt
+// to the CTA's threads in packed order: every update instruction runs on full
+// warps (a partly predicated FP64 instruction costs the pipe a whole warp) and
+// every access to S is consecutive, and 37 KB for a 96 x 96 bank leave room for
+// four CTAs per SM to cover each other's barriers (square storage: two).
+// Flags zero / non-finite pivots.  Needs blockDim.x == 256.
+template <int N>
+__device__ void sweep_invert(double *S, double *col, double *scol, int *bad)
 {
     constexpr int NE = N * (N + 1) / 2;
     constexpr int PER = (NE + 255) / 256;
@@ -262,28 +267,38 @@ __device__ void sweep_invert(double *S, int ld, double *col, double *scol, int *
             tc[k] = ((uint32_t)t << 16) | (uint32_t)(t + (e - off));
         }
     }
+    // the division of a pivot is left to one warp, while the others write the
+    // previous pivot's column back: run by all eight it cost the pipe as much as
+    // two thirds of the updates
+    __shared__ double rp;
+    auto reciprocal = [&](int p) {
+        const double piv = S[tri<N>(p, p)];
+        if (!isfinite(piv) || piv == 0.0) atomicOr(bad, 1);
+        rp = 1.0 / piv;
+    };
+    if (tid == 255) reciprocal(0);
+    __syncthreads();
     for (int p = 0; p < N; ++p) {
-        const double piv = S[p * ld + p];
-        const double rpiv = 1.0 / piv;  // one division per pivot; the column is scaled by multiplication
+        const double rpiv = rp;  // the column is scaled by multiplication
         for (int t = tid; t < N; t += 256) {
-            const double cv = (t == p) ? 0.0 : (t < p ? S[t * ld + p] : S[p * ld + t]);
+            const double cv = (t == p) ? 0.0 : S[t < p ? tri<N>(t, p) : tri<N>(p, t)];
             col[t] = cv;
             scol[t] = cv * rpiv;
         }
-        if (tid == 0 && (!isfinite(piv) || piv == 0.0)) atomicOr(bad, 1);
         __syncthreads();
+        // the pivot's own row and column (zeros in col and scol) keep their
+        // values here and are replaced below
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             if (tc[k] == ~0u) continue;
-            const int t = (int)(tc[k] >> 16), c = (int)(tc[k] & 0xffffu);
-            if (t != p && c != p) S[t * ld + c] -= scol[t] * col[c];
+            S[tid + k * 256] -= scol[tc[k] >> 16] * col[tc[k] & 0xffffu];
         }
         __syncthreads();
         for (int t = tid; t < N; t += 256) {
-            if (t == p) S[p * ld + p] = -rpiv;
-            else if (t < p) S[t * ld + p] = scol[t];
-            else S[p * ld + t] = scol[t];
+            if (t == p) S[tri<N>(p, p)] = -rpiv;
+            else S[t < p ? tri<N>(t, p) : tri<N>(p, t)] = scol[t];
         }
+        if (tid == 255 && p + 1 < N) reciprocal(p + 1);
         __syncthreads();
     }
 }
@@ -294,18 +309,18 @@ __device__ void sweep_invert(double *S, int ld, double *col, double *scol, int *
 // is gathered straight from the operator's rows; a coarse bank from its dense
 // Galerkin staging (upper triangle).
 template <int BD, typename T, bool BF0>
-__global__ void __launch_bounds__(256, 2) mas_invert_kernel(BsrDev A, const int32_t *__restrict__ part_off,
+__global__ void __launch_bounds__(256, 4) mas_invert_kernel(BsrDev A, const int32_t *__restrict__ part_off,
                                                             int64_t nparts, void *__restrict__ out0,
                                                             const double *__restrict__ stagec, T *__restrict__ outc,
                                                             int *bad, uint8_t *__restrict__ uncoupled)
 {
-    constexpr int N = 32 * BD, LD = N + 1;
+    constexpr int N = 32 * BD, NE = N * (N + 1) / 2;
     extern __shared__ double sm[];
-    double *S = sm, *col = sm + N * LD, *scol = col + N;
+    double *S = sm, *col = sm + NE, *scol = col + N;
     const bool fine = (int64_t)blockIdx.x < nparts;
     const int64_t bank = fine ? blockIdx.x : (int64_t)blockIdx.x - nparts;
     if (fine) {
-        for (int idx = threadIdx.x; idx < N * LD; idx += blockDim.x) S[idx] = 0.0;
+        for (int idx = threadIdx.x; idx < NE; idx += blockDim.x) S[idx] = 0.0;
         __syncthreads();
         const int32_t lo = part_off[bank], hi = part_off[bank + 1];
         const int g = threadIdx.x & 7;  // eight threads per block row
@@ -320,13 +335,13 @@ __global__ void __launch_bounds__(256, 2) mas_invert_kernel(BsrDev A, const int3
 #pragma unroll
                     for (int bj = 0; bj < BD; ++bj) {
                         const int r = bi * 32 + (i - lo), c = bj * 32 + (j - lo);
-                        if (r <= c) S[r * LD + c] = v[(int64_t)(bi * BD + bj) * len + l];
+                        if (r <= c) S[tri<N>(r, c)] = v[(int64_t)(bi * BD + bj) * len + l];
                     }
             }
         }
         __syncthreads();
         for (int t = threadIdx.x; t < N; t += blockDim.x)
-            if (S[t * LD + t] == 0.0) S[t * LD + t] = 1.0;  // padding (MASPreconditioner.cu:779-796)
+            if (S[tri<N>(t, t)] == 0.0) S[tri<N>(t, t)] = 1.0;  // padding (MASPreconditioner.cu:779-796)
     } else {
         const double *src = stagec + bank * N * N;
         bool coupled = false;  // an entry between two different items of the bank
@@ -336,15 +351,15 @@ __global__ void __launch_bounds__(256, 2) mas_invert_kernel(BsrDev A, const int3
             double v = src[(int64_t)r * N + c];
             coupled |= ((r ^ c) & 31) != 0 && v != 0.0;
             if (r == c && v == 0.0) v = 1.0;
-            S[r * LD + c] = v;
+            S[tri<N>(r, c)] = v;
         }
         coupled = __syncthreads_or(coupled);
         if (threadIdx.x == 0) uncoupled[bank] = coupled ? 0 : 1;
     }
     __syncthreads();
-    sweep_invert<N>(S, LD, col, scol, bad);
+    sweep_invert<N>(S, col, scol, bad);
     // the swept entry (i, j), i <= j
-    auto entry = [&](int i, int j) -> double { return S[i * LD + j]; };
+    auto entry = [&](int i, int j) -> double { return S[tri<N>(i, j)]; };
     // tiles
     if (BF0 && fine) {  // FP32 diagonal tiles, BF16 off-diagonal tiles (round to nearest even)
         unsigned char *dst = reinterpret_cast<unsigned char *>(out0) + bank * (int64_t)(BD * 17 * 32 * 4 + BD * (BD - 1) / 2 * 2048);
@@ -848,7 +863,7 @@ static void invert_t(const BsrDev &A, const MasDev &m, const double *stagec, voi
                      uint8_t *uncoupled, cudaStream_t s)
 {
     constexpr int N = 32 * BD;
-    const size_t smem = (size_t)(N * (N + 1) + 2 * N) * sizeof(double);
+    const size_t smem = (size_t)(N * (N + 1) / 2 + 2 * N) * sizeof(double);
     raise_smem_limit((const void *)mas_invert_kernel<BD, T, BF0>, smem);
     mas_invert_kernel<BD, T, BF0><<<(unsigned)((int64_t)m.nparts + m.ncoarse), 256, smem, s>>>(
         A, m.part_off, m.nparts, out0, stagec, (T *)outc, bad, uncoupled);
