@@ -401,17 +401,22 @@ void HybridSolver::select_stiff(const CscView &A)
     auto tsel0 = clk::now();
     if (p_.select_l1) {
         const int32_t n = A.n;
-        DBuf<double> rn(n);
-        DBuf<GmmState> st(1);
+        DBuf<double> &rn = d_rn_, &bmargin = d_bmargin_;
+        DBuf<GmmState> &st = d_gmm_;
+        DBuf<double2> &resp = d_resp_;
+        DBuf<uint32_t> &bits = d_bits_;
+        DBuf<int32_t> &bcount = d_bcount_, &boffs = d_boffs_;
+        const int nblk = (n + 255) / 256;
+        rn.resize(n);
+        st.resize(1);
+        resp.resize(n);
+        bits.resize(((size_t)n + 31) / 32);
+        bcount.resize(nblk);
+        bmargin.resize(nblk);
         st.zero(stream_);
         if (d_outer_.size() != (size_t)n + 1) d_outer_.upload(h_outer_, stream_);
         launch_row_l1_norms(n, A.nnz, d_outer_.data(), d_csc_.data(), rn.data(), stream_);
-        DBuf<double2> resp(n);
-        DBuf<uint32_t> bits(((size_t)n + 31) / 32);
         launch_gmm(n, rn.data(), st.data(), p_.max_gmm_iterations, p_.gmm_tol, gr_, stream_, resp.data());
-        const int nblk = (n + 255) / 256;
-        DBuf<int32_t> bcount(nblk), boffs(nblk);
-        DBuf<double> bmargin(nblk);
         launch_gmm_mark(n, rn.data(), st.data(), p_.jump_threshold, bcount.data(), bmargin.data(), stream_,
                         bits.data());
         std::vector<int32_t> hc = bcount.download(stream_);
@@ -456,7 +461,8 @@ void HybridSolver::select_stiff(const CscView &A)
         if (m > 0) {
             DBuf<int32_t> dsel;
             dsel.upload(sel, stream_);
-            DBuf<uint8_t> mask((size_t)pat_.n);
+            DBuf<uint8_t> &mask = d_mask_;
+            mask.resize((size_t)pat_.n);
             mask.zero(stream_);
             DBuf<double> ddiag(m), doff(m);
             launch_gershgorin(pat_.nb, pat_.bd, d_rows_.data(), d_cols_.data(), d_vals_.data(), d_perm_.data(),

@@ -168,6 +168,13 @@ private:
     DBuf<unsigned> d_counter_;
     DBuf<int> d_bad_;
     GridReduce gr_;
+    // selection workspaces, kept per pattern
+    DBuf<double> d_rn_, d_bmargin_;
+    DBuf<double2> d_resp_;
+    DBuf<uint32_t> d_bits_;
+    DBuf<GmmState> d_gmm_;
+    DBuf<int32_t> d_bcount_, d_boffs_;
+    DBuf<uint8_t> d_mask_;
     DBuf<double> d_sums_;
     PcgSum pap_, rr_, rz_;  // the PCG's scalar sums, between the kernels that form and use them
     cudaGraphExec_t graph_exec_ = nullptr;

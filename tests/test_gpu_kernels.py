@@ -103,3 +103,51 @@ def test_double_float_split_matches_casts(n, built):
         lo = (x - hi.astype(np.float64)).astype(np.float32)
         np.testing.assert_array_equal(s.spmv_outer(x), hi.astype(np.float64) + lo.astype(np.float64))
     s.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("hybrid", [True, False])
+def test_refactorized_solves_match_fresh_ones(precision, hybrid, built):
+    """The iterations captured for one factorization serve later ones of the
+    pattern: solves after a change of values, of the stiff set (other sizes,
+    none) and back equal those of a new solver bit for bit."""
+    from lss import gen
+    rng = np.random.default_rng(4)
+    n = (11, 10, 9)
+    E, _ = gen.sphere_inclusion_E(*n, np.random.Generator(np.random.PCG64(5)), radius=0.2, E_in=1e4)
+    F, _ = gen.sphere_inclusion_E(*n, np.random.Generator(np.random.PCG64(6)), radius=0.3, E_in=1e5)
+    mats = [gen.elasticity_cube(*n, e) for e in (E, F, np.ones_like(E), 1.7 * E, E)]
+    b = rng.standard_normal(mats[0].shape[0])
+    params = {"gmm_jump_threshold": 10.0, "min_subdomain_size": 4, "do_hybrid_precond": hybrid}
+    kept = make_solver(3, precision, **params)
+    first = None
+    for k, A in enumerate(mats):
+        kept.factorize(A)
+        x = kept.solve(b)
+        fresh = make_solver(3, precision, **params)
+        fresh.factorize(A)
+        np.testing.assert_array_equal(x, fresh.solve(b), err_msg=str(k))
+        np.testing.assert_array_equal(kept.solve(b), x)
+        if first is None:
+            first = x
+        fresh.close()
+    np.testing.assert_array_equal(x, first)
+    kept.close()
+
+
+@pytest.mark.parametrize("max_iter", [0, 1, 3, 4, 5, 9])
+def test_iteration_limit(max_iter, built):
+    """The limit holds whatever its place in a chunk of iterations, and a solve
+    from the point it left continues to convergence."""
+    A = block_system(700, 3, seed=1)
+    b = np.random.default_rng(2).standard_normal(A.shape[0])
+    s = make_solver(3, do_hybrid_precond=False, max_iter=max_iter)
+    s.factorize(A)
+    x = s.solve(b)
+    info = s.get_info()
+    assert info["num_iterations"] == max_iter and info["status"] == "max_iterations"
+    s.set_parameters({"GPUHybrid": {"max_iter": 1000}})
+    y = s.solve(b, x.copy())
+    assert s.get_info()["status"] == "converged_rel"
+    assert np.linalg.norm(b - A.T @ y) <= 1e-10 * np.linalg.norm(b)
+    s.close()
