@@ -164,6 +164,9 @@ void BatchSolver::merge()
     int32_t nb = 0, np = 0;
     int64_t nnzb = 0;
     bool any_precise = false;
+    int64_t all_parts = 0;
+    for (const HybridSolver *H : sys_) all_parts += (int64_t)H->pat_.part.part_offsets.size() - 1;
+    const int32_t per_chunk = (int32_t)std::clamp<int64_t>(all_parts / sm_grid(5), 1, BATCH_CHUNK);
     for (int32_t s = 0; s < ns; ++s) {
         const HybridSolver &H = *sys_[s];
         const Pattern &P = H.pat_;
@@ -175,7 +178,7 @@ void BatchSolver::merge()
         const auto &po = P.part.part_offsets;
         const int32_t nps = (int32_t)po.size() - 1;
         for (int32_t q = 1; q <= nps; ++q) part_off.push_back(nb + po[q]);
-        for (int32_t q = 0; q < nps; q += BATCH_CHUNK) {
+        for (int32_t q = 0; q < nps; q += per_chunk) {
             chunk_sys.push_back(s);
             chunk_p0.push_back(np + q);
         }

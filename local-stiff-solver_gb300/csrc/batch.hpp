@@ -33,7 +33,10 @@
 namespace lss {
 
 constexpr int BK = 16;           // right-hand sides per system in a batch
-constexpr int BATCH_CHUNK = 8;   // MAS partitions (<= 32 block rows each) per chunk
+// MAS partitions (<= 32 block rows each) per chunk at most; fewer while that
+// leaves less than five CTAs per SM: 146k DOFs in chunks of eight are 190 CTAs,
+// eight warps per SM for kernels that wait on memory
+constexpr int BATCH_CHUNK = 8;
 
 class HybridSolver;
 
