@@ -13,7 +13,7 @@
 // front's vector is gathered by the GEMV CTAs, in the batched solve by a
 // launch before), then one backward GEMV launch per level (root first; in the
 // batched solve a scatter ends it).  GEMV CTAs take 32 output columns and at
-// most 256 of a front's rows; larger fronts split their rows over several CTAs
+// most 64 (batched: 128) of a front's rows; larger fronts split their rows over several CTAs
 // whose partial sums the last CTA of the group adds in a fixed order.  The
 // per-level launches use programmatic dependent launch.  The solve with one
 // right-hand side is FP64; the batched solve with 16 reads the fronts as
@@ -378,12 +378,12 @@ __global__ void __launch_bounds__(256) mf_mirror_kernel(MfView v, MfWork w, doub
 // ---- solve
 
 constexpr int NR_COLS = 32;    // output columns per GEMV CTA of the solves
-constexpr int NR_KROWS = 256;  // front rows per GEMV CTA of the solves
+constexpr int NR_KROWS = 128;  // front rows per GEMV CTA of the batched solve (256: 128 ms on six systems, 121)
 
 __host__ __device__ __forceinline__ int nr_kchunks(int rows) { return (rows + NR_KROWS - 1) / NR_KROWS; }
 
 // ---- solve with one right-hand side (FP64): one launch per level and
-// direction.  GEMV CTAs of 32 columns x at most 256 front rows (8 warps = 8
+// direction.  GEMV CTAs of 32 columns x at most 64 front rows (8 warps = 8
 // row slices, lane = column) gather their part of the front's vector
 // themselves (right-hand side + the children's contributions, children in
 // order); fronts with more rows are split over several CTAs whose partial
@@ -391,7 +391,11 @@ __host__ __device__ __forceinline__ int nr_kchunks(int rows) { return (rows + NR
 // sizes and offsets are one descriptor (the work-list search and the symbolic
 // arrays behind it were six dependent loads), and the backward pass updates z.
 
-constexpr int NR_COLS1 = 32;
+// rows per CTA: an SM takes 2 us over 256 x 32 FP64 multiply-adds and a level
+// has few CTAs, so shorter chunks gain more than their combination costs (1.3k-
+// and 3.0k-DOF balls, mixed: 72 and 108 us per iteration at 256 rows, 68 and 105
+// at 128, 66 and 102 at 64)
+constexpr int NR_COLS1 = 32, NR_KROWS1 = 64;
 
 struct NrScratch1 {
     double *part;   // per CTA of a launch: NR_COLS1 partial sums
@@ -403,14 +407,14 @@ struct NrScratch1 {
 // before anything the CTA has to wait for and overlap the gather of its vector
 // (8 loads at a time behind it added 3 us to a launch).
 struct FrontPart {
-    double a[NR_KROWS / 8];
+    double a[NR_KROWS1 / 8];
 };
 __device__ __forceinline__ void load_part(FrontPart &p, const MfCta &c, const double *__restrict__ F)
 {
     const int cl = threadIdx.x & 31, ks = threadIdx.x >> 5;
     const double *Fc = F + c.foff + (int64_t)(c.q0 + ks) * c.f + c.col0 + cl;
 #pragma unroll
-    for (int j = 0; j < NR_KROWS / 8; ++j)
+    for (int j = 0; j < NR_KROWS1 / 8; ++j)
         p.a[j] = cl < c.ncol && ks + 8 * j < c.nrow ? __ldg(Fc + (int64_t)(8 * j) * c.f) : 0.0;
 }
 
@@ -421,7 +425,7 @@ __device__ __forceinline__ void gemv1(const FrontPart &p, const MfCta &c, const 
     const int cl = threadIdx.x & 31, ks = threadIdx.x >> 5;
     double acc = 0.0;
 #pragma unroll
-    for (int j = 0; j < NR_KROWS / 8; ++j)
+    for (int j = 0; j < NR_KROWS1 / 8; ++j)
         if (ks + 8 * j < c.nrow) acc += p.a[j] * xs[ks + 8 * j];
     red[ks * 32 + cl] = acc;
     __syncthreads();
@@ -448,6 +452,7 @@ __device__ __forceinline__ bool combine1(NrScratch1 sc, int kc, int nkc, double 
     __threadfence();
     if (threadIdx.x < ncol) {
         double sum = 0.0;
+#pragma unroll 8
         for (int j = 0; j < nkc; ++j) sum += __ldcg(sc.part + (g + j) * NR_COLS1 + threadIdx.x);
         res[threadIdx.x] = sum;
     }
@@ -476,7 +481,7 @@ __global__ void __launch_bounds__(256) mf_forward_kernel(MfView v, const MfCta *
                                                          const double *__restrict__ F, double *__restrict__ W,
                                                          NrScratch1 sc, const int *done)
 {
-    __shared__ double xs[NR_KROWS], red[256], res[NR_COLS1];
+    __shared__ double xs[NR_KROWS1], red[256], res[NR_COLS1];
     const MfCta c = ctas[blockIdx.x];
     FrontPart part;
     load_part(part, c, F);
@@ -505,7 +510,7 @@ __global__ void __launch_bounds__(256) mf_backward_kernel(MfView v, const MfCta 
                                                           double *__restrict__ z, float *__restrict__ z32,
                                                           float *__restrict__ z_lo, const int *done)
 {
-    __shared__ double vec[NR_KROWS], red[256], res[NR_COLS1];
+    __shared__ double vec[NR_KROWS1], red[256], res[NR_COLS1];
     const MfCta c = ctas[blockIdx.x];
     FrontPart part;
     load_part(part, c, F);
@@ -544,7 +549,7 @@ __global__ void __launch_bounds__(256) mf_backward_kernel(MfView v, const MfCta 
 // children's contributions into each front's vector (extend-add as a gather,
 // children in order), then GEMV CTAs apply c = w_bnd - P w_own.  Backward,
 // per level: GEMV CTAs apply x_own = F11^-1 (w_own - F12 x_bnd).  A GEMV CTA
-// takes 32 output columns and at most 256 of the front's rows: its 256
+// takes 32 output columns and at most 128 of the front's rows: its 256
 // threads are 32 columns x 8 row slices (thread t: column t % 32, rows
 // t / 32 + 8 j), each keeping all NR sums of its column; the slices meet in
 // shared memory in slice order.  A front with more rows splits them over
@@ -866,7 +871,7 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
     // GEMV CTAs of the single right-hand-side solve
     std::vector<MfCta> ctas;
     auto add_ctas = [&](int32_t id, int32_t first, int32_t cols, int32_t rows) {
-        const int32_t nkc = nr_kchunks(rows);
+        const int32_t nkc = (rows + NR_KROWS1 - 1) / NR_KROWS1;
         for (int32_t c0 = 0; c0 < cols; c0 += NR_COLS1)
             for (int32_t kc = 0; kc < nkc; ++kc) {
                 MfCta c;
@@ -875,8 +880,8 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
                 c.f = M.s[id] + M.u[id];
                 c.col0 = first + c0;
                 c.ncol = std::min(NR_COLS1, cols - c0);
-                c.q0 = kc * NR_KROWS;
-                c.nrow = std::min(NR_KROWS, rows - c.q0);
+                c.q0 = kc * NR_KROWS1;
+                c.nrow = std::min(NR_KROWS1, rows - c.q0);
                 c.kc = kc;
                 c.nkc = nkc;
                 c.woff = M.woff[id];
