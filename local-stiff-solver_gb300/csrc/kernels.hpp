@@ -52,6 +52,7 @@ struct GmmState {
     double m0, m1, v0, v1, w0, w1;        // current parameters
     double em0, em1, ev0, ev1, ew0, ew1;  // parameters of the last E-step
     double s0, s1;                        // responsibilities' sums of the last E-step
+    double lg[4], elg[4];                 // log w0, log w1, -log(2 pi v0) / 2, -log(2 pi v1) / 2 of both sets
     int esteps, converged, pad0, pad1;
 };
 

@@ -99,6 +99,45 @@ __global__ void __launch_bounds__(256) stats_kernel(int32_t n, const double *__r
     }
 }
 
+// E-step of one row (GPUHybrid.cu:800-818), evaluated without contraction so
+// that it rounds like the reference expression tree.
+struct Resp {
+    double g0, g1, lg0, lg1;
+};
+// The logarithms that every row shares, five of a row's nine transcendentals:
+// formed once per parameter set, by the thread that finishes the set (formed by
+// every thread, which holds a row or two, they cost as much as the rows).
+__device__ __forceinline__ void shared_logs(double w0, double w1, double v0, double v1, double (&lg)[4])
+{
+    const double two_pi = 2.0 * 3.14159265358979323846;
+    lg[0] = log(w0);
+    lg[1] = log(w1);
+    lg[2] = __dmul_rn(-0.5, log(__dmul_rn(two_pi, v0)));
+    lg[3] = __dmul_rn(-0.5, log(__dmul_rn(two_pi, v1)));
+}
+struct Mixture {
+    double m0, m1, v0, v1, log_w0, log_w1, half_log0, half_log1;
+    __device__ __forceinline__ Mixture(double m0_, double m1_, double v0_, double v1_, const double (&lg)[4])
+        : m0(m0_), m1(m1_), v0(v0_), v1(v1_), log_w0(lg[0]), log_w1(lg[1]), half_log0(lg[2]), half_log1(lg[3])
+    {
+    }
+};
+__device__ __forceinline__ Resp estep(double x, const Mixture &q)
+{
+    const double d0 = __dsub_rn(x, q.m0), d1 = __dsub_rn(x, q.m1);
+    const double logN0 = __dsub_rn(q.half_log0, __ddiv_rn(__dmul_rn(__dmul_rn(0.5, d0), d0), q.v0));
+    const double logN1 = __dsub_rn(q.half_log1, __ddiv_rn(__dmul_rn(__dmul_rn(0.5, d1), d1), q.v1));
+    const double lg0 = __dadd_rn(q.log_w0, logN0), lg1 = __dadd_rn(q.log_w1, logN1);
+    const double mx = fmax(lg0, lg1);
+    const double lt = __dadd_rn(mx, log(__dadd_rn(exp(__dsub_rn(lg0, mx)), exp(__dsub_rn(lg1, mx)))));
+    Resp r;
+    r.g0 = exp(__dsub_rn(lg0, lt));
+    r.g1 = exp(__dsub_rn(lg1, lt));
+    r.lg0 = lg0;
+    r.lg1 = lg1;
+    return r;
+}
+
 __global__ void __launch_bounds__(256) var_kernel(int32_t n, const double *__restrict__ rn, GmmState *st,
                                                   GridReduce gr)
 {
@@ -119,44 +158,10 @@ __global__ void __launch_bounds__(256) var_kernel(int32_t n, const double *__res
         st->v1 = st->var;
         st->w0 = 0.5;
         st->w1 = 0.5;
+        shared_logs(0.5, 0.5, st->var, st->var, st->lg);
         st->esteps = 0;
         st->converged = 0;
     }
-}
-
-// E-step of one row (GPUHybrid.cu:800-818), evaluated without contraction so
-// that it rounds like the reference expression tree.
-struct Resp {
-    double g0, g1, lg0, lg1;
-};
-// the parameters and the logarithms that every row shares (five of a row's
-// nine transcendentals, and FP64 arithmetic is what the E-step costs)
-struct Mixture {
-    double m0, m1, v0, v1, log_w0, log_w1, half_log0, half_log1;
-    __device__ __forceinline__ Mixture(double w0, double w1, double m0_, double m1_, double v0_, double v1_)
-        : m0(m0_), m1(m1_), v0(v0_), v1(v1_)
-    {
-        const double two_pi = 2.0 * 3.14159265358979323846;
-        log_w0 = log(w0);
-        log_w1 = log(w1);
-        half_log0 = __dmul_rn(-0.5, log(__dmul_rn(two_pi, v0)));
-        half_log1 = __dmul_rn(-0.5, log(__dmul_rn(two_pi, v1)));
-    }
-};
-__device__ __forceinline__ Resp estep(double x, const Mixture &q)
-{
-    const double d0 = __dsub_rn(x, q.m0), d1 = __dsub_rn(x, q.m1);
-    const double logN0 = __dsub_rn(q.half_log0, __ddiv_rn(__dmul_rn(__dmul_rn(0.5, d0), d0), q.v0));
-    const double logN1 = __dsub_rn(q.half_log1, __ddiv_rn(__dmul_rn(__dmul_rn(0.5, d1), d1), q.v1));
-    const double lg0 = __dadd_rn(q.log_w0, logN0), lg1 = __dadd_rn(q.log_w1, logN1);
-    const double mx = fmax(lg0, lg1);
-    const double lt = __dadd_rn(mx, log(__dadd_rn(exp(__dsub_rn(lg0, mx)), exp(__dsub_rn(lg1, mx)))));
-    Resp r;
-    r.g0 = exp(__dsub_rn(lg0, lt));
-    r.g1 = exp(__dsub_rn(lg1, lt));
-    r.lg0 = lg0;
-    r.lg1 = lg1;
-    return r;
 }
 
 // pass A: responsibilities with the current parameters; sums of g and g*x;
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(256) em_pass_a(int32_t n, const double *__rest
 {
     if (st->converged) return;
     const double w0 = st->w0, w1 = st->w1, m0 = st->m0, m1 = st->m1, v0 = st->v0, v1 = st->v1;
-    const Mixture mix(w0, w1, m0, m1, v0, v1);
+    const Mixture mix(m0, m1, v0, v1, st->lg);
     double s[4] = {0.0, 0.0, 0.0, 0.0};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -181,6 +186,7 @@ __global__ void __launch_bounds__(256) em_pass_a(int32_t n, const double *__rest
     double t[4];
     if (grid_sum<4>(s, gr, t)) {
         st->ew0 = w0; st->ew1 = w1; st->em0 = m0; st->em1 = m1; st->ev0 = v0; st->ev1 = v1;
+        for (int q = 0; q < 4; ++q) st->elg[q] = st->lg[q];
         st->s0 = t[0];
         st->s1 = t[1];
         st->w0 = t[0] / n;
@@ -198,9 +204,9 @@ __global__ void __launch_bounds__(256) em_pass_b(int32_t n, const double *__rest
                                                  GridReduce gr, double tol, const double2 *__restrict__ resp)
 {
     if (st->converged) return;
-    const double w0 = st->ew0, w1 = st->ew1, m0 = st->em0, m1 = st->em1, v0 = st->ev0, v1 = st->ev1;
+    const double m0 = st->em0, m1 = st->em1, v0 = st->ev0, v1 = st->ev1;
     const double nm0 = st->m0, nm1 = st->m1;
-    const Mixture mix(w0, w1, m0, m1, v0, v1);
+    const Mixture mix(m0, m1, v0, v1, st->elg);
     double s[2] = {0.0, 0.0};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -222,6 +228,7 @@ __global__ void __launch_bounds__(256) em_pass_b(int32_t n, const double *__rest
         const double nv0 = t[0] / st->s0 + var_reg, nv1 = t[1] / st->s1 + var_reg;
         st->v0 = nv0;
         st->v1 = nv1;
+        shared_logs(st->w0, st->w1, nv0, nv1, st->lg);
         if (fabs(nm0 - m0) / fabs(m0) < tol && fabs(nm1 - m1) / fabs(m1) < tol &&
             fabs(nv0 - v0) / fabs(v0) < tol && fabs(nv1 - v1) / fabs(v1) < tol)
             st->converged = 1;
@@ -242,7 +249,7 @@ __global__ void __launch_bounds__(256) mark_kernel(int32_t n, const double *__re
     bool flag = false;
     double margin = INFINITY;
     if (i < n && st->esteps > 0) {
-        const Resp r = estep(rn[i], Mixture(st->ew0, st->ew1, st->em0, st->em1, st->ev0, st->ev1));
+        const Resp r = estep(rn[i], Mixture(st->em0, st->em1, st->ev0, st->ev1, st->elg));
         flag = jump && (r.g0 < r.g1);
         margin = fabs(r.lg0 - r.lg1);
     }
@@ -276,7 +283,7 @@ __global__ void __launch_bounds__(256) scatter_kernel(int32_t n, const double *_
     if (bits) {
         flag = i < n && (bits[i >> 5] >> (i & 31) & 1u);
     } else if (i < n && jump) {
-        const Resp r = estep(rn[i], Mixture(st->ew0, st->ew1, st->em0, st->em1, st->ev0, st->ev1));
+        const Resp r = estep(rn[i], Mixture(st->em0, st->em1, st->ev0, st->ev1, st->elg));
         flag = r.g0 < r.g1;
     }
     const unsigned b = __ballot_sync(0xffffffffu, flag);
