@@ -466,9 +466,14 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
     };
     Part t = part(p);
     pdl_enter();
-    if (st && st->done) return;
-    if (rr.part) {  // the updated residual's convergence tests (GPUHybrid.cu:1488-1496)
+    const bool over = st && st->done;
+    if (!rr.part) {
+        if (over) return;
+    } else {  // the updated residual's convergence tests (GPUHybrid.cu:1488-1496)
+        // the first CTA may set done while another reads it: no thread leaves ahead
+        // of the sum's barriers, and all that stay come to the same verdict
         const double s = get_sum(rr);
+        if (over) return;
         int stop = STOP_RUNNING;
         if (!(s == s) || isinf(s)) stop = STOP_NONFINITE;
         else if (st->rel_eps > 0 && s / st->bb < st->rel_eps) stop = STOP_CONVERGED_REL;

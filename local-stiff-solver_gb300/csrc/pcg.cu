@@ -146,8 +146,11 @@ __global__ void __launch_bounds__(256) update_xr_kernel(int64_t n, double *__res
                                                         float *__restrict__ r32)
 {
     pdl_enter();
-    if (st->done) return;
+    // the first CTA may set done while another reads it: no thread leaves ahead of
+    // the sum's barriers, and all that stay come to the same verdict
+    const bool over = st->done != 0;
     const double gamma = st->rz, pAp = get_sum(pap), alpha = gamma / pAp;
+    if (over) return;
     int stop = STOP_RUNNING;
     if (pAp == 0.0) stop = STOP_ZERO_PAP;
     else if (!(alpha == alpha) || isinf(alpha)) stop = STOP_NONFINITE;
