@@ -131,12 +131,13 @@ void launch_dot(int64_t n, const double *a, const double *b, double *out, GridRe
 void launch_pcg_spmv_alpha(const BsrDev &A, const double *p, double *Ap, const PcgState *st, GridReduce gr,
                            PcgSum &pap, cudaStream_t s);
 // alpha = r.z / p.Ap with the reference's breakdown tests; x += alpha p;
-// r -= alpha Ap; the parts of r.r.  r32 (optional): also r rounded to FP32
-void launch_pcg_update_xr(int64_t n, double *x, double *r, const double *p, const double *Ap, PcgState *st,
-                          GridReduce gr, PcgSum pap, PcgSum &rr, cudaStream_t s, float *r32 = nullptr);
-// the same with A p as df32 (hi, lo) pairs
-void launch_pcg_update_xr_df(int64_t n, double *x, double *r, const double *p, const float2 *Ap_df, PcgState *st,
-                             GridReduce gr, PcgSum pap, PcgSum &rr, cudaStream_t s, float *r32 = nullptr);
+// r -= alpha Ap (Ap_df, Ap: one of them); the parts of r.r; r restricted to the
+// level-1 items of m (v: level vectors, FP32 or FP64).  r32 (optional): also r
+// rounded to FP32
+struct MasDev;
+void launch_pcg_update_xr(const MasDev &m, double *x, double *r, const double *p, const double *Ap,
+                          const float2 *Ap_df, PcgState *st, GridReduce gr, PcgSum pap, PcgSum &rr, void *v, bool fp32,
+                          cudaStream_t s, float *r32 = nullptr);
 void launch_df_to_double(int64_t n, const float2 *src, double *dst, cudaStream_t s);
 // the damping estimate's probe, v_i = ((i * 2654435761) mod 2^32) / 2^32 - 0.5 over
 // original indices i, written in the permuted order
@@ -223,14 +224,15 @@ void launch_mas_invert(const BsrDev &A, const MasDev &m, const double *stagec, v
 int64_t mas_bank_bytes_bf16(int bd);
 // z = scale * MAS^-1 xin, or z += scale * MAS^-1 xin with acc; rz (optional):
 // the parts of rdot.z.  rr (optional): the sum of the residual just updated,
-// against which the first launch tests for convergence (GPUHybrid.cu:1488-1496).
+// which the first launch but the restriction tests for convergence
+// (GPUHybrid.cu:1488-1496).  restricted: v already holds xin restricted to level 1.
 // z32 (optional): also store z rounded to FP32 (the input of the FP32 residual)
 // and, with z_lo, the remainder z - z32 rounded to FP32.
 // xin32 (optional, FP32 MAS only): an FP32 input used in place of xin.
 void launch_mas_apply(const MasDev &m, const void *inv0, const void *invc, void *v, void *u, bool fp32,
                       const double *xin, double *z, bool acc, double scale, const double *rdot, PcgState *st,
                       const PcgSum *rr, PcgSum *rz, GridReduce gr, cudaStream_t s, float *z32 = nullptr,
-                      const float *xin32 = nullptr, float *z_lo = nullptr);
+                      const float *xin32 = nullptr, float *z_lo = nullptr, bool restricted = false);
 
 // level-0 bank SYMV alone (z = Inv_0 xin + coarse correction already in u), for timing
 void launch_mas_level0(const MasDev &m, const void *inv0, const void *u, bool fp32, const double *xin, double *z,

@@ -22,6 +22,7 @@
 
 #include "device_common.cuh"
 #include "kernels.hpp"
+#include "mas.cuh"
 
 namespace lss {
 
@@ -397,38 +398,6 @@ __global__ void __launch_bounds__(256, 4) mas_invert_kernel(BsrDev A, const int3
 
 // ------------------------------------------------------------------ apply
 
-// Segmented sums of one bank: 32 items (values staged item-major in xs; lane j
-// passes the target aggregate of item j, 0xff for none) into ncc aggregates.
-// Output slot s = k * BD + c (aggregate k, component c) belongs to a group of P
-// lanes, P the largest power of two with ncc * BD * P <= 32 (1 beyond): lane q
-// of the group adds the items j = q, q + P, ... of aggregate k in order, found
-// by its mask, and the group's sums meet by shuffles.  An FP64 add costs the
-// pipe a whole warp however few lanes take part: one aggregate (a connected
-// partition) takes 4 + 3 adds and 32 aggregates (uncoupled items) one add per
-// pass, where testing every item against every slot took 32 per pass.
-template <int BD, typename T>
-__device__ __forceinline__ void bank_segment_sums(const T *xs, uint8_t key, unsigned *mask, int ncc,
-                                                  T *__restrict__ out, int lane)
-{
-    const unsigned same = __match_any_sync(0xffffffffu, (unsigned)key);
-    if (key < 32 && __ffs(same) - 1 == lane) mask[key] = same;
-    __syncwarp();
-    const int slots = ncc * BD;
-    int lg = 0;
-    while (lg < 5 && (slots << (lg + 1)) <= 32) ++lg;
-    const int sub = lane & ((1 << lg) - 1);
-    // every 2^lg-th item, starting at sub
-    const unsigned every = (lg == 0 ? ~0u : lg == 1 ? 0x55555555u : lg == 2 ? 0x11111111u : lg == 3 ? 0x01010101u
-                            : lg == 4 ? 0x00010001u : 1u) << sub;
-    for (int s0 = 0; s0 < slots; s0 += 32 >> lg) {
-        const int sl = s0 + (lane >> lg), k = sl / BD, c = sl - k * BD;
-        T acc = T(0);
-        for (unsigned m = sl < slots ? mask[k] & every : 0u; m; m &= m - 1) acc += xs[(__ffs(m) - 1) * BD + c];
-        for (int o = (1 << lg) >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (sl < slots && sub == 0) out[sl] = acc;
-    }
-}
-
 // The restriction of r to level 1: a warp sums one partition's rows into its
 // level-1 items.  In a large hierarchy a second launch sums the level-1 banks
 // into level 2 (MasDev::base); the levels above are summed from the base level
@@ -438,7 +407,7 @@ __device__ __forceinline__ void bank_segment_sums(const T *xs, uint8_t key, unsi
 // with one on 33k partitions.
 template <int BD, typename T, typename XT>
 __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__restrict__ r, T *__restrict__ v,
-                                                       PcgState *st, PcgSum rr)
+                                                       const int *done)
 {
     constexpr int N = 32 * BD, W = 8;
     __shared__ T xs_all[W][N];
@@ -448,43 +417,9 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
     // a partition's bounds and items do not depend on the preceding kernel
     int64_t p = (int64_t)blockIdx.x * W + wl;
     const int64_t step = (int64_t)gridDim.x * W;
-    struct Part {
-        int32_t lo, cnt, i0;
-        int nc;
-        uint8_t key;
-    };
-    auto part = [&](int64_t q) {
-        Part t{0, 0, 0, 0, 0xff};
-        if (q < m.nparts) {
-            t.lo = m.part_off[q];
-            t.cnt = m.part_off[q + 1] - t.lo;
-            t.i0 = m.cbase0[q];
-            t.nc = m.ccnt0[q];
-            if (lane < t.cnt) t.key = m.key0[t.lo + lane];
-        }
-        return t;
-    };
-    Part t = part(p);
+    MasPart t = mas_part(m, p, lane);
     pdl_enter();
-    const bool over = st && st->done;
-    if (!rr.part) {
-        if (over) return;
-    } else {  // the updated residual's convergence tests (GPUHybrid.cu:1488-1496)
-        // the first CTA may set done while another reads it: no thread leaves ahead
-        // of the sum's barriers, and all that stay come to the same verdict
-        const double s = get_sum(rr);
-        if (over) return;
-        int stop = STOP_RUNNING;
-        if (!(s == s) || isinf(s)) stop = STOP_NONFINITE;
-        else if (st->rel_eps > 0 && s / st->bb < st->rel_eps) stop = STOP_CONVERGED_REL;
-        else if (st->abs_eps > 0 && s < st->abs_eps) stop = STOP_CONVERGED_ABS;
-        else if (st->iter >= st->max_iter) stop = STOP_MAX_ITER;
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            st->rr = s;
-            if (stop) st->done = stop;
-        }
-        if (stop) return;
-    }
+    if (done && *done) return;
     for (; p < m.nparts; p += step) {
         // the part's values are one contiguous run: coalesced loads
 #pragma unroll
@@ -492,7 +427,7 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
             const int e = q * 32 + lane;
             xs[e] = e < t.cnt * BD ? (T)r[(int64_t)t.lo * BD + e] : T(0);
         }
-        const Part next = part(p + step);
+        const MasPart next = mas_part(m, p + step, lane);
         __syncwarp();
         bank_segment_sums<BD, T>(xs, t.key, mask_all[wl], t.nc, v + m.voff[1] + (int64_t)t.i0 * BD, lane);
         __syncwarp();
@@ -502,7 +437,7 @@ __global__ void __launch_bounds__(256) restrict_kernel(MasDev m, const XT *__res
 
 // level 1 -> level 2, a warp per level-1 bank
 template <int BD, typename T>
-__global__ void __launch_bounds__(256) restrict1_kernel(MasDev m, T *__restrict__ v, const int *done)
+__global__ void __launch_bounds__(256) restrict1_kernel(MasDev m, T *__restrict__ v, PcgState *st, PcgSum rr)
 {
     constexpr int N = 32 * BD, W = 8;
     __shared__ T xs_all[W][N];
@@ -515,7 +450,7 @@ __global__ void __launch_bounds__(256) restrict1_kernel(MasDev m, T *__restrict_
     const int32_t j0 = valid ? m.cbase[1][b] : 0;
     const uint8_t key = lane < cnt ? m.key[1][i0 + lane] : (uint8_t)0xff;
     pdl_enter();
-    if (!valid || (done && *done)) return;
+    if (pcg_stops(st, rr) || !valid) return;
     const T *vl = v + m.voff[1] + (int64_t)i0 * BD;
     T *xs = xs_all[wl];
 #pragma unroll
@@ -599,7 +534,7 @@ __device__ __forceinline__ void gather_bank(const MasDev &m, int l, int32_t b, c
 template <int BD, typename T>
 __global__ void __launch_bounds__(256) symv_coarse_kernel(MasDev m, const T *__restrict__ invc,
                                                           const T *__restrict__ v, T *__restrict__ u,
-                                                          const int *done)
+                                                          PcgState *st, PcgSum rr)
 {
     constexpr int N = 32 * BD, W = 8;
     __shared__ T xs[N];
@@ -609,7 +544,7 @@ __global__ void __launch_bounds__(256) symv_coarse_kernel(MasDev m, const T *__r
     const int o = (tid % BD) * 32 + tid / BD;  // component-major place of element tid
     const bool uncoupled = m.uncoupled[g];
     pdl_enter();
-    if (done && *done) return;
+    if (pcg_stops(st, rr)) return;
     int l = 1;
     while (l + 1 < m.L && g >= m.boff[l + 1]) ++l;
     if (l <= m.base) {
@@ -813,15 +748,19 @@ void symv0_launch(const MasDev &m, const T *inv0, const T *u, const XT *xin, dou
 template <int BD, typename T, typename XT>
 void mas_apply_dot_t(const MasDev &m, const T *inv0, const T *invc, T *v, T *u, const XT *xin, double *z,
                      bool acc, double scale, const double *rdot, PcgState *st, const PcgSum *rr, PcgSum *rz,
-                     GridReduce gr, cudaStream_t s, float *z32, float *z_lo)
+                     GridReduce gr, cudaStream_t s, float *z32, float *z_lo, bool restricted)
 {
     if (m.L < 2) fail(LSS_ERR_INTERNAL, "a MAS hierarchy has at least one coarse level");
     const int *done = &st->done;
-    launch_pdl(restrict_kernel<BD, T, XT>, grid_for(m.nparts, 8, sm_grid(8)), 256, 0, s, m, xin, v, st,
-               rr ? *rr : PcgSum{});
-    if (m.base > 1)
-        launch_pdl(restrict1_kernel<BD, T>, (unsigned)((m.nbanks[1] + 7) / 8), 256, 0, s, m, v, done);
-    launch_pdl(symv_coarse_kernel<BD, T>, (unsigned)m.ncoarse, 256, 0, s, m, invc, (const T *)v, u, done);
+    // the first launch after the residual's update tests it for convergence
+    PcgSum test = rr ? *rr : PcgSum{};
+    if (!restricted)
+        launch_pdl(restrict_kernel<BD, T, XT>, grid_for(m.nparts, 8, sm_grid(8)), 256, 0, s, m, xin, v, done);
+    if (m.base > 1) {
+        launch_pdl(restrict1_kernel<BD, T>, (unsigned)((m.nbanks[1] + 7) / 8), 256, 0, s, m, v, st, test);
+        test = PcgSum{};
+    }
+    launch_pdl(symv_coarse_kernel<BD, T>, (unsigned)m.ncoarse, 256, 0, s, m, invc, (const T *)v, u, st, test);
 #define LSS_S0(A_, D_)                                                                                          \
     do {                                                                                                        \
         if (std::is_same<T, float>::value && m.bank_bytes0 > 0)                                                 \
@@ -930,14 +869,14 @@ void launch_mas_level0(const MasDev &m, const void *inv0, const void *u, bool fp
 void launch_mas_apply(const MasDev &m, const void *inv0, const void *invc, void *v, void *u, bool fp32,
                       const double *xin, double *z, bool acc, double scale, const double *rdot, PcgState *st,
                       const PcgSum *rr, PcgSum *rz, GridReduce gr, cudaStream_t s, float *z32, const float *xin32,
-                      float *z_lo)
+                      float *z_lo, bool restricted)
 {
 #define LSS_MAS(BD_, T_)                                                                                          \
     mas_apply_dot_t<BD_, T_, double>(m, (const T_ *)inv0, (const T_ *)invc, (T_ *)v, (T_ *)u, xin, z, acc, scale, \
-                                     rdot, st, rr, rz, gr, s, z32, z_lo)
+                                     rdot, st, rr, rz, gr, s, z32, z_lo, restricted)
 #define LSS_MAS32(BD_)                                                                                            \
     mas_apply_dot_t<BD_, float, float>(m, (const float *)inv0, (const float *)invc, (float *)v, (float *)u, xin32, \
-                                       z, acc, scale, rdot, st, rr, rz, gr, s, z32, z_lo)
+                                       z, acc, scale, rdot, st, rr, rz, gr, s, z32, z_lo, restricted)
     if (xin32) {
         if (!fp32) fail(LSS_ERR_INTERNAL, "an FP32 input needs the FP32 MAS");
         if (m.bd == 1) LSS_MAS32(1);

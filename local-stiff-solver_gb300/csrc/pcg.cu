@@ -12,6 +12,7 @@
 
 #include "device_common.cuh"
 #include "kernels.hpp"
+#include "mas.cuh"
 #include "spmv.cuh"
 
 namespace lss {
@@ -132,19 +133,35 @@ constexpr int VEC = 4, VEC_ROWS = 256 * VEC;
 __device__ __forceinline__ double as_double(double v) { return v; }
 __device__ __forceinline__ double as_double(float2 v) { return to_double(v.x) + to_double(v.y); }
 
+// partitions a warp takes at a time: one of block size 1 alone leaves too few
+// loads in flight and too many CTAs that sum p.Ap
+__host__ __device__ constexpr int XR_PARTS(int bd) { return bd == 1 ? 2 : 1; }
+
 // alpha with the breakdown tests; x += alpha p; r -= alpha Ap; r.r
-// (GPUHybrid.cu:1463-1487).  Every CTA forms alpha from the parts of p.Ap, the
-// first one records the iteration's scalars.  AT: double, or float2 for the
-// (hi, lo) product of the df32 SpMV.  r32 (optional): r rounded to FP32, the
-// input of the mixed preconditioner's FP32 residual -- converted here, where
-// every lane of a warp converts one entry (a partly predicated FP64
-// instruction costs the pipe a full warp).
-template <typename AT>
-__global__ void __launch_bounds__(256) update_xr_kernel(int64_t n, double *__restrict__ x, double *__restrict__ r,
+// (GPUHybrid.cu:1463-1487), and the restriction of the new r to the MAS's level-1
+// items: a warp takes whole partitions, whose rows it holds anyway.  As a launch
+// of its own behind this one the restriction read r again; an iteration took
+// 54.9 us instead of 52.6 at 2k DOF (FP64), 67.4 / 65.2 at 24k, 114 / 108 at 207k,
+// 831 / 804 at 3M (mixed), 145.8 / 142.7 on a 150k Laplacian (FP64).
+// Every CTA forms alpha from the parts of p.Ap, the first one
+// records the iteration's scalars.  AT: double, or float2 for the (hi, lo) product
+// of the df32 SpMV; T: the MAS's type.  r32 (optional): r rounded to FP32, the
+// input of the mixed preconditioner's FP32 residual.
+template <int BD, typename AT, typename T>
+__global__ void __launch_bounds__(256) update_xr_kernel(MasDev m, double *__restrict__ x, double *__restrict__ r,
                                                         const double *__restrict__ p, const AT *__restrict__ Ap,
                                                         PcgState *st, GridReduce gr, PcgSum pap, PcgSum rr,
-                                                        float *__restrict__ r32)
+                                                        T *__restrict__ v, float *__restrict__ r32)
 {
+    constexpr int W = 8, K = XR_PARTS(BD);
+    __shared__ T xs_all[W][K][32 * BD];
+    __shared__ unsigned mask_all[W][32];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    int64_t q = ((int64_t)blockIdx.x * W + wl) * K;
+    const int64_t step = (int64_t)gridDim.x * W * K;
+    MasPart t[K];  // constant: read ahead of the preceding kernel's end
+#pragma unroll
+    for (int k = 0; k < K; ++k) t[k] = mas_part(m, q + k, lane);
     pdl_enter();
     // the first CTA may set done while another reads it: no thread leaves ahead of
     // the sum's barriers, and all that stay come to the same verdict
@@ -169,27 +186,52 @@ __global__ void __launch_bounds__(256) update_xr_kernel(int64_t n, double *__res
     }
     if (stop) return;
     double s = 0.0;
-    for (int64_t i0 = (int64_t)blockIdx.x * VEC_ROWS + threadIdx.x; i0 < n; i0 += (int64_t)gridDim.x * VEC_ROWS) {
-        double xv[VEC], pv[VEC], rv[VEC];
-        AT av[VEC];
+    for (; q < m.nparts; q += step) {
+        double xv[K][BD], pv[K][BD], rv[K][BD];
+        AT av[K][BD];
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) {
-            const int64_t i = i0 + j * 256;
-            if (i >= n) break;
-            xv[j] = x[i];
-            pv[j] = p[i];
-            rv[j] = r[i];
-            av[j] = Ap[i];
+        for (int k = 0; k < K; ++k) {
+#pragma unroll
+            for (int j = 0; j < BD; ++j) {
+                const int e = j * 32 + lane;
+                if (e >= t[k].cnt * BD) break;
+                const int64_t i = (int64_t)t[k].lo * BD + e;
+                xv[k][j] = x[i];
+                pv[k][j] = p[i];
+                rv[k][j] = r[i];
+                av[k][j] = Ap[i];
+            }
         }
+        MasPart next[K];
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) {
-            const int64_t i = i0 + j * 256;
-            if (i >= n) break;
-            x[i] = xv[j] + alpha * pv[j];
-            const double ri = rv[j] - alpha * as_double(av[j]);
-            r[i] = ri;
-            if (r32) r32[i] = to_float(ri);
-            s += ri * ri;
+        for (int k = 0; k < K; ++k) next[k] = mas_part(m, q + step + k, lane);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            T *xs = xs_all[wl][k];
+#pragma unroll
+            for (int j = 0; j < BD; ++j) {
+                const int e = j * 32 + lane;
+                if (e >= t[k].cnt * BD) break;
+                const int64_t i = (int64_t)t[k].lo * BD + e;
+                x[i] = xv[k][j] + alpha * pv[k][j];
+                const double ri = rv[k][j] - alpha * as_double(av[k][j]);
+                r[i] = ri;
+                if (sizeof(T) == 4 || r32) {
+                    const float f = to_float(ri);
+                    if (r32) r32[i] = f;
+                    if (sizeof(T) == 4) xs[e] = (T)f;
+                }
+                if (sizeof(T) == 8) xs[e] = (T)ri;
+                s += ri * ri;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            bank_segment_sums<BD, T>(xs_all[wl][k], t[k].key, mask_all[wl], t[k].nc,
+                                     v + m.voff[1] + (int64_t)t[k].i0 * BD, lane);
+            __syncwarp();
+            t[k] = next[k];
         }
     }
     put_sum(s, gr, rr);
@@ -570,21 +612,26 @@ void launch_split(int64_t n, const double *src, float2 *dst, cudaStream_t s)
     LSS_LAUNCH_CHECK();
 }
 
-void launch_pcg_update_xr(int64_t n, double *x, double *r, const double *p, const double *Ap, PcgState *st,
-                          GridReduce gr, PcgSum pap, PcgSum &rr, cudaStream_t s, float *r32)
+void launch_pcg_update_xr(const MasDev &m, double *x, double *r, const double *p, const double *Ap,
+                          const float2 *Ap_df, PcgState *st, GridReduce gr, PcgSum pap, PcgSum &rr, void *v, bool fp32,
+                          cudaStream_t s, float *r32)
 {
-    const int grid = grid_for(n, 1024, sm_grid(16));
-    produced(rr, n, grid);
-    launch_pdl(update_xr_kernel<double>, grid, 256, 0, s, n, x, r, p, Ap, st, gr, pap, rr, r32);
-    LSS_LAUNCH_CHECK();
-}
-
-void launch_pcg_update_xr_df(int64_t n, double *x, double *r, const double *p, const float2 *Ap_df, PcgState *st,
-                             GridReduce gr, PcgSum pap, PcgSum &rr, cudaStream_t s, float *r32)
-{
-    const int grid = grid_for(n, 1024, sm_grid(16));
-    produced(rr, n, grid);
-    launch_pdl(update_xr_kernel<float2>, grid, 256, 0, s, n, x, r, p, Ap_df, st, gr, pap, rr, r32);
+    const int grid = grid_for(m.nparts, 8 * XR_PARTS(m.bd), sm_grid(8));
+    produced(rr, (int64_t)m.nb * m.bd, grid);
+#define LSS_XR(BD_, AT_, T_, A_) \
+    launch_pdl(update_xr_kernel<BD_, AT_, T_>, grid, 256, 0, s, m, x, r, p, A_, st, gr, pap, rr, (T_ *)v, r32)
+#define LSS_XR_BD(BD_)                                 \
+    do {                                               \
+        if (Ap_df && fp32) LSS_XR(BD_, float2, float, Ap_df); \
+        else if (Ap_df) LSS_XR(BD_, float2, double, Ap_df);   \
+        else if (fp32) LSS_XR(BD_, double, float, Ap);        \
+        else LSS_XR(BD_, double, double, Ap);                 \
+    } while (0)
+    if (m.bd == 1) LSS_XR_BD(1);
+    else if (m.bd == 2) LSS_XR_BD(2);
+    else LSS_XR_BD(3);
+#undef LSS_XR_BD
+#undef LSS_XR
     LSS_LAUNCH_CHECK();
 }
 

@@ -779,7 +779,7 @@ void HybridSolver::mas_apply(const double *xin, double *z, bool acc, const doubl
 {
     launch_mas_apply(mas_, d_inv0_.data(), d_invc_.data(), d_v_.data(), d_u_.data(), mas_fp32_, xin, z, acc, scale,
                      rdot, d_state_.data(), test ? &rr_ : nullptr, rdot ? &rz_ : nullptr, gr_, stream_, z32, xin32,
-                     z_lo);
+                     z_lo, test);
 }
 
 // z = M^-1 r
@@ -848,12 +848,9 @@ void HybridSolver::iteration()
 {
     outer_spmv_alpha();
     float *r32 = p_.mixed ? d_r32_.data() : nullptr;
-    if (outer_df())
-        launch_pcg_update_xr_df(n_vec(), d_x_.data(), d_r_.data(), d_p_.data(), d_ap_df_.data(), d_state_.data(),
-                                gr_, pap_, rr_, stream_, r32);
-    else
-        launch_pcg_update_xr(n_vec(), d_x_.data(), d_r_.data(), d_p_.data(), d_ap_.data(), d_state_.data(), gr_,
-                             pap_, rr_, stream_, r32);
+    launch_pcg_update_xr(mas_, d_x_.data(), d_r_.data(), d_p_.data(), d_ap_.data(),
+                         outer_df() ? d_ap_df_.data() : nullptr, d_state_.data(), gr_, pap_, rr_, d_v_.data(),
+                         mas_fp32_, stream_, r32);
     precond(d_r_.data(), d_z_.data(), true, r32, true);
     launch_pcg_update_p(n_vec(), d_p_.data(), d_z_.data(), d_state_.data(), rz_, false, stream_,
                         outer_df() ? d_p_df_.data() : nullptr);

@@ -82,7 +82,8 @@ private:
     void ensure_vectors();
     void run_pcg();
     // r32 (optional): r already rounded to FP32 (mixed precision); converted here otherwise
-    // dot: also form the parts of r.z (rz_); test: first test r.r (rr_) for convergence
+    // dot: also form the parts of r.z (rz_); test: r comes from the PCG's update,
+    // restricted to level 1 already and with r.r (rr_) to be tested for convergence
     void precond(const double *r, double *z, bool dot, const float *r32 = nullptr, bool test = false);
     void mas_apply(const double *xin, double *z, bool acc, const double *rdot, double scale, bool test = false,
                    float *z32 = nullptr, const float *xin32 = nullptr, float *z_lo = nullptr);

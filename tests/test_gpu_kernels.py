@@ -151,3 +151,32 @@ def test_iteration_limit(max_iter, built):
     assert s.get_info()["status"] == "converged_rel"
     assert np.linalg.norm(b - A.T @ y) <= 1e-10 * np.linalg.norm(b)
     s.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("bs", [1, 2, 3])
+@pytest.mark.parametrize("nb,isolated", [(1, 0), (2, 1), (31, 0), (33, 0), (70, 64), (1100, 200), (5000, 1500), (80000, 0)])
+def test_iterations_follow_the_preconditioner(bs, nb, isolated, precision, built):
+    """Four iterations (the update restricts the residual for the next MAS apply)
+    against PCG on the host with the same preconditioner applied by itself.  A
+    stopped system is within 1e-10 |b| of its residual, 1e-8 of x (eigenvalues
+    of 0.5 to about 30); a residual's last bit may round to another FP32 value
+    in the mixed preconditioner: 1e-5."""
+    A = block_system(nb, bs, seed=3 * nb + bs, isolated=isolated)
+    b = np.random.default_rng(nb).standard_normal(A.shape[0])
+    s = make_solver(bs, precision, do_hybrid_precond=False, max_iter=4)
+    s.factorize(A)
+    x = s.solve(b)
+    its = s.get_info()["num_iterations"]
+    assert 1 <= its <= 4 and (its == 4 or nb < 100)
+    y, r, p, rz = np.zeros_like(b), b.copy(), 0.0, 1.0
+    for _ in range(its):
+        if np.linalg.norm(r) <= 1e-14 * np.linalg.norm(b):
+            break
+        z = s.precond(r)
+        p, rz = z + (r @ z / rz) * p, r @ z
+        q = A.T @ p
+        alpha = rz / (p @ q)
+        y, r = y + alpha * p, r - alpha * q
+    assert np.linalg.norm(x - y) <= (1e-8 if precision == "fp64" else 1e-5) * np.linalg.norm(y)
+    s.close()
