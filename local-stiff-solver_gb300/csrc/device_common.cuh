@@ -152,7 +152,7 @@ __device__ __forceinline__ float2 split_double(double v)
 
 // The PCG's scalar sums.  The kernel that forms the addends leaves the sum's
 // parts with put_sum; the next kernel that needs the scalar adds them in every
-// CTA with get_sum.  PcgSum::direct: one part per CTA, nothing else -- the
+// CTA with from_sum.  PcgSum::direct: one part per CTA, nothing else -- the
 // fence, counter and last-CTA tail of grid_sum cost 3 to 4 us at the end of a
 // kernel, the consumer's sum 0.6 us at its start.  Otherwise grid_sum leaves
 // one part: with many CTAs per SM summing, the parts' FP64 adds would cost the
@@ -170,38 +170,47 @@ __device__ __forceinline__ void put_sum(double v, GridReduce gr, PcgSum out)
     if (grid_sum<1>(a, gr, tot)) out.part[0] = tot[0];
 }
 
-// The sum, in every thread of the CTA (all of them must call it).  A warp takes
-// 128 parts, four a lane: every warp that takes part costs the FP64 pipe five
-// shuffled adds of 16 clocks whatever it holds, and several CTAs of an SM sum at
-// once (304 parts over 8 warps: 61 warp-wide adds, over 3: 27).
-__device__ __forceinline__ double get_sum(PcgSum in)
+// f(sum), formed by thread 0, in every thread of the CTA (all of them must call
+// it).  What a scalar costs the FP64 pipe is warps: 16 clocks an instruction
+// whatever the lanes.  A warp takes 128 parts, four a lane, since every warp that
+// takes part adds five shuffled sums of its own (304 parts over 8 warps: 61
+// warp-wide adds, over 3: 27), and the quotients and tests that follow run in one
+// warp, not in all eight of every CTA (a division in each: 5 to 10 us of an
+// SM's pipe under the 8 to 16 CTAs of a long vector update).  An iteration went
+// from 107 to 103 us at 207k DOF, 805 to 798 at 3M (mixed), 147.1 to 145.2 on a
+// 150k Laplacian, 82.5 to 81.3 at 24k (FP64).
+template <typename F>
+__device__ __forceinline__ auto from_sum(PcgSum in, F f)
 {
-    if (in.count == 1) return __ldcg(in.part);
-    __shared__ double smem[33];
-    const int warps = min((int)blockDim.x / 32, (in.count + 127) / 128), w = threadIdx.x >> 5, t = threadIdx.x;
-    if (w < warps) {
-        double a = 0.0;
-        for (int i0 = t; i0 < in.count; i0 += 128 * warps) {
-            double b[4];
+    __shared__ double smem[32];
+    __shared__ decltype(f(0.0)) res;
+    const int t = threadIdx.x, w = t >> 5, warps = min((int)blockDim.x / 32, (in.count + 127) / 128);
+    double a = 0.0;
+    if (in.count == 1) {
+        if (t == 0) a = __ldcg(in.part);
+    } else {
+        if (w < warps) {
+            for (int i0 = t; i0 < in.count; i0 += 128 * warps) {
+                double b[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int i = i0 + j * 32 * warps;
-                b[j] = i < in.count ? __ldcg(in.part + i) : 0.0;
+                for (int j = 0; j < 4; ++j) {
+                    const int i = i0 + j * 32 * warps;
+                    b[j] = i < in.count ? __ldcg(in.part + i) : 0.0;
+                }
+                a += (b[0] + b[1]) + (b[2] + b[3]);
             }
-            a += (b[0] + b[1]) + (b[2] + b[3]);
+            a = warp_sum(a);
+            if ((t & 31) == 0) smem[w] = a;
         }
-        a = warp_sum(a);
-        if ((t & 31) == 0) smem[w] = a;
+        if (warps > 1) {
+            __syncthreads();
+            if (t == 0)
+                for (int k = 1; k < warps; ++k) a += smem[k];
+        }
     }
+    if (t == 0) res = f(a);
     __syncthreads();
-    if (warps == 1) return smem[0];
-    if (t == 0) {
-        double a = smem[0];
-        for (int k = 1; k < warps; ++k) a += smem[k];
-        smem[32] = a;
-    }
-    __syncthreads();
-    return smem[32];
+    return res;
 }
 
 // Grid-wide min/max (deterministic, order independent).

@@ -69,18 +69,19 @@ __device__ __forceinline__ bool pcg_stops(PcgState *st, PcgSum rr)
 {
     const bool over = st->done != 0;
     if (!rr.part) return over;
-    const double s = get_sum(rr);
-    if (over) return true;
-    int stop = STOP_RUNNING;
-    if (!(s == s) || isinf(s)) stop = STOP_NONFINITE;
-    else if (st->rel_eps > 0 && s / st->bb < st->rel_eps) stop = STOP_CONVERGED_REL;
-    else if (st->abs_eps > 0 && s < st->abs_eps) stop = STOP_CONVERGED_ABS;
-    else if (st->iter >= st->max_iter) stop = STOP_MAX_ITER;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        st->rr = s;
-        if (stop) st->done = stop;
-    }
-    return stop != STOP_RUNNING;
+    const int stop = from_sum(rr, [&](double s) {
+        int c = STOP_RUNNING;
+        if (!(s == s) || isinf(s)) c = STOP_NONFINITE;
+        else if (st->rel_eps > 0 && s / st->bb < st->rel_eps) c = STOP_CONVERGED_REL;
+        else if (st->abs_eps > 0 && s < st->abs_eps) c = STOP_CONVERGED_ABS;
+        else if (st->iter >= st->max_iter) c = STOP_MAX_ITER;
+        if (blockIdx.x == 0 && !over) {
+            st->rr = s;
+            if (c) st->done = c;
+        }
+        return c;
+    });
+    return over || stop != STOP_RUNNING;
 }
 
 }  // namespace lss

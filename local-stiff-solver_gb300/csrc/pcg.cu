@@ -166,25 +166,32 @@ __global__ void __launch_bounds__(256) update_xr_kernel(MasDev m, double *__rest
     // the first CTA may set done while another reads it: no thread leaves ahead of
     // the sum's barriers, and all that stay come to the same verdict
     const bool over = st->done != 0;
-    const double gamma = st->rz, pAp = get_sum(pap), alpha = gamma / pAp;
-    if (over) return;
-    int stop = STOP_RUNNING;
-    if (pAp == 0.0) stop = STOP_ZERO_PAP;
-    else if (!(alpha == alpha) || isinf(alpha)) stop = STOP_NONFINITE;
-    else if (alpha <= 0.0) stop = STOP_NEGATIVE_ALPHA;
-    else if (alpha < DBL_MIN) stop = STOP_SUBNORMAL_ALPHA;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const int it = st->iter + 1;
-        st->iter = it;
-        st->pAp = pAp;
-        st->gamma = gamma;
-        if (stop) st->done = stop;
-        else {
-            st->alpha = alpha;
-            if (it <= PCG_HIST) st->hist_alpha[it - 1] = alpha;
+    struct Step {
+        double alpha;
+        int stop;
+    };
+    const Step ab = from_sum(pap, [&](double pAp) {
+        const double gamma = st->rz, a = gamma / pAp;
+        int c = STOP_RUNNING;
+        if (pAp == 0.0) c = STOP_ZERO_PAP;
+        else if (!(a == a) || isinf(a)) c = STOP_NONFINITE;
+        else if (a <= 0.0) c = STOP_NEGATIVE_ALPHA;
+        else if (a < DBL_MIN) c = STOP_SUBNORMAL_ALPHA;
+        if (blockIdx.x == 0 && !over) {
+            const int it = st->iter + 1;
+            st->iter = it;
+            st->pAp = pAp;
+            st->gamma = gamma;
+            if (c) st->done = c;
+            else {
+                st->alpha = a;
+                if (it <= PCG_HIST) st->hist_alpha[it - 1] = a;
+            }
         }
-    }
-    if (stop) return;
+        return Step{a, c};
+    });
+    if (over || ab.stop) return;
+    const double alpha = ab.alpha;
     double s = 0.0;
     for (; q < m.nparts; q += step) {
         double xv[K][BD], pv[K][BD], rv[K][BD];
@@ -244,14 +251,17 @@ __global__ void __launch_bounds__(256) update_p_kernel(int64_t n, double *__rest
 {
     pdl_enter();
     if (st->done) return;
-    const double g = get_sum(rz), beta = first ? 0.0 : g / st->gamma;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        st->rz = g;
-        if (!first) {
-            st->beta = beta;
-            if (st->iter >= 1 && st->iter <= PCG_HIST) st->hist_beta[st->iter - 1] = beta;
+    const double beta = from_sum(rz, [&](double g) {
+        const double b = first ? 0.0 : g / st->gamma;
+        if (blockIdx.x == 0) {
+            st->rz = g;
+            if (!first) {
+                st->beta = b;
+                if (st->iter >= 1 && st->iter <= PCG_HIST) st->hist_beta[st->iter - 1] = b;
+            }
         }
-    }
+        return b;
+    });
     for (int64_t i0 = (int64_t)blockIdx.x * VEC_ROWS + threadIdx.x; i0 < n; i0 += (int64_t)gridDim.x * VEC_ROWS) {
         double zv[VEC], pv[VEC];
 #pragma unroll
@@ -454,11 +464,20 @@ void produced(PcgSum &sum, int64_t n, int grid)
     sum.count = sum.direct ? grid : 1;
 }
 
+// CTAs of the outer product.  Eight per SM are resident at most; where its
+// consumers add a part per CTA there are no more than those (207k DOF: 2432 parts
+// cost the update 1 us more than 1216).
+template <int BD>
+int product_grid(const BsrDev &A)
+{
+    return grid_for((int64_t)A.nb * A.lanes, 256, sm_grid((int64_t)A.nb * BD <= PCG_DIRECT_ROWS ? 8 : 16));
+}
+
 template <int BD>
 void spmv_alpha_dispatch(const BsrDev &A, const double *p, double *Ap, const PcgState *st, GridReduce gr, PcgSum &pap,
                          cudaStream_t s)
 {
-    const int grid = grid_for((int64_t)A.nb * A.lanes, 256, sm_grid(16));
+    const int grid = product_grid<BD>(A);
     produced(pap, (int64_t)A.nb * BD, grid);
 #define LSS_SA(L_) launch_pdl(spmv_alpha_kernel<BD, L_>, grid, 256, 0, s, A, p, Ap, st, gr, pap)
     switch (A.lanes) {
@@ -548,7 +567,7 @@ template <int BD>
 void spmv_alpha_df_dispatch(const BsrDev &A, const float2 *pd, float2 *Ap, const PcgState *st, GridReduce gr,
                             PcgSum &pap, cudaStream_t s)
 {
-    const int grid = grid_for((int64_t)A.nb * A.lanes, 256, sm_grid(16));
+    const int grid = product_grid<BD>(A);
     produced(pap, (int64_t)A.nb * BD, grid);
 #define LSS_SA(L_) launch_pdl(spmv_alpha_df_kernel<BD, L_>, grid, 256, 0, s, A, pd, Ap, st, gr, pap)
     switch (A.lanes) {
