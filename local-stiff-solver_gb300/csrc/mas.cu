@@ -399,7 +399,8 @@ __global__ void __launch_bounds__(256, 4) mas_invert_kernel(BsrDev A, const int3
 // ------------------------------------------------------------------ apply
 
 // The restriction of r to level 1: a warp sums one partition's rows into its
-// level-1 items.  In a large hierarchy a second launch sums the level-1 banks
+// level-1 items (the PCG's update does the same for the residual it leaves,
+// update_xr_kernel).  In a large hierarchy a second launch sums the level-1 banks
 // into level 2 (MasDev::base); the levels above are summed from the base level
 // by the products that need them (symv_coarse_kernel).  Restricting completed
 // banks further inside this launch, found by arrival counters, saved launches
