@@ -98,6 +98,8 @@ void launch_spmv(const BsrDev &A, const double *x, double *y, const int *done, c
 // y = r - A x in FP64
 void launch_residual_spmv(const BsrDev &A, const double *r, const double *x, double *y, const int *done,
                           cudaStream_t s);
+// the same to twice the precision, rounded once
+void launch_residual_twice(const BsrDev &A, const double *r, const double *x, double *y, cudaStream_t s);
 // y32 = r32 - A x32 in FP32 with the FP32 operator copy (the mixed
 // preconditioner's residual); block rows flagged in `precise` (optional) are
 // evaluated in double-float from r64, the df32 values and x32 + x_lo.

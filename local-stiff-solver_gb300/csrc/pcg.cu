@@ -61,6 +61,52 @@ __global__ void __launch_bounds__(256) residual_kernel(BsrDev A, const double *_
     });
 }
 
+// y = r - A x with every product and sum carried in two doubles (TwoProd,
+// TwoSum: Ogita, Rump and Oishi's Dot2) and rounded once; LANES threads per
+// block row.  It starts the PCG's restarts (run_pcg): at most one launch each.
+template <int BD, int LANES>
+__global__ void __launch_bounds__(256) residual_twice_kernel(BsrDev A, const double *__restrict__ r,
+                                                             const double *__restrict__ x, double *__restrict__ y)
+{
+    const int lane = threadIdx.x % LANES;
+    const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) / LANES;
+    const bool valid = i < A.nb;
+    const int32_t b = valid ? A.rows[i] : 0, len = valid ? A.rows[i + 1] - b : 0;
+    const double *__restrict__ v = A.vals + (int64_t)b * (BD * BD);
+    auto add = [](double &h, double &l, double p, double e) {  // (h, l) += p + e
+        const double t = __dadd_rn(h, p), z = __dsub_rn(t, h);
+        l = __dadd_rn(l, __dadd_rn(e, __dadd_rn(__dsub_rn(h, __dsub_rn(t, z)), __dsub_rn(p, z))));
+        h = t;
+    };
+    double sh[BD], sl[BD];
+#pragma unroll
+    for (int k = 0; k < BD; ++k) {  // the first lane starts from -r
+        sh[k] = valid && lane == 0 ? -r[i * BD + k] : 0.0;
+        sl[k] = 0.0;
+    }
+    for (int32_t q = lane; q < len; q += LANES) {
+        const int64_t c = A.cols[b + q];
+#pragma unroll
+        for (int j = 0; j < BD; ++j) {
+            const double xv = x[c * BD + j];
+#pragma unroll
+            for (int k = 0; k < BD; ++k) {
+                const double a = v[(int64_t)(k * BD + j) * len + q], p = __dmul_rn(a, xv);
+                add(sh[k], sl[k], p, __fma_rn(a, xv, -p));
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < BD; ++k) {
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) {
+            const double h = __shfl_xor_sync(0xffffffffu, sh[k], o), l = __shfl_xor_sync(0xffffffffu, sl[k], o);
+            add(sh[k], sl[k], h, l);
+        }
+        if (valid && lane == 0) y[i * BD + k] = -__dadd_rn(sh[k], sl[k]);
+    }
+}
+
 // y32 = r - A x for the mixed preconditioner, rounded to FP32 (its result
 // feeds the FP32 MAS).  Rows flagged in `precise` (the stiff rows: there r - A
 // z cancels terms many orders larger than the result -- entries of 1e7 times a
@@ -515,6 +561,18 @@ void launch_residual_spmv(const BsrDev &A, const double *r, const double *x, dou
     if (A.bd == 1) residual_dispatch<1>(A, r, x, y, done, s);
     else if (A.bd == 2) residual_dispatch<2>(A, r, x, y, done, s);
     else residual_dispatch<3>(A, r, x, y, done, s);
+    LSS_LAUNCH_CHECK();
+}
+
+void launch_residual_twice(const BsrDev &A, const double *r, const double *x, double *y, cudaStream_t s)
+{
+    if (A.nb == 0) return;
+    if (A.bd == 1) residual_twice_kernel<1, 4><<<(unsigned)(((int64_t)A.nb * 4 + 255) / 256), 256, 0, s>>>(A, r, x, y);
+    else {
+        const unsigned grid = (unsigned)(((int64_t)A.nb * 8 + 255) / 256);
+        if (A.bd == 2) residual_twice_kernel<2, 8><<<grid, 256, 0, s>>>(A, r, x, y);
+        else residual_twice_kernel<3, 8><<<grid, 256, 0, s>>>(A, r, x, y);
+    }
     LSS_LAUNCH_CHECK();
 }
 

@@ -931,7 +931,12 @@ void HybridSolver::run_pcg()
     double res2 = 0.0, prev_res2 = INFINITY;
     for (int attempt = 0;; ++attempt) {
         // r = b - A x; z = M r; p = z; gamma = r.z   (GPUHybrid.cu:1441-1451)
-        launch_residual_spmv(A_, d_b_.data(), d_x_.data(), d_r_.data(), nullptr, stream_);
+        // A restart's r carries its own rounding into x, amplified by A^-1 (1e-9 |x|
+        // where the moduli span 1e6, another error for every order of the sums), so
+        // it is formed to twice the precision: 14 hard seeds of a 150k Laplacian and
+        // 8 of a 24k ball at contrast 1e6 went from 3.5e-10 |x| off to 6e-13.
+        if (attempt > 0) launch_residual_twice(A_, d_b_.data(), d_x_.data(), d_r_.data(), stream_);
+        else launch_residual_spmv(A_, d_b_.data(), d_x_.data(), d_r_.data(), nullptr, stream_);
         if (p_.max_iter > 0) {
             precond(d_r_.data(), d_z_.data(), true);
             launch_pcg_update_p(n, d_p_.data(), d_z_.data(), d_state_.data(), rz_, true, stream_,

@@ -180,3 +180,37 @@ def test_iterations_follow_the_preconditioner(bs, nb, isolated, precision, built
         y, r = y + alpha * p, r - alpha * q
     assert np.linalg.norm(x - y) <= (1e-8 if precision == "fp64" else 1e-5) * np.linalg.norm(y)
     s.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("seed", [2, 4])
+def test_restart_leaves_no_residual_rounding(seed, precision, built):
+    """A restarted solve is not off by what the rounding of an FP64 residual does
+    to x, |A^-1 (fl(b - A x) - (b - A x))|: that is the error of any restart from
+    such a residual, another one for every order of its sums.  Moduli of 1e6
+    leave a residual of 5e-10 or more at a tolerance of 1e-10, so a restart cuts
+    the first pass's error, of that size, by 2 (5e-10 / 1e-10)^2 = 50: a tenth of
+    it is allowed."""
+    import scipy.sparse.linalg as spla
+    from lss import gen
+    rng = np.random.Generator(np.random.PCG64(seed))
+    E, _ = gen.sphere_inclusion_E(16, 16, 16, rng, E_in=1e6)
+    A = gen.elasticity_cube(16, 16, 16, E)
+    b = rng.standard_normal(A.shape[0])
+    s = make_solver(3, precision, gmm_jump_threshold=10.0, min_subdomain_size=4)
+    s.factorize(A)
+    x = s.solve(b)
+    assert s.get_info()["refinements"] >= 1
+    s.close()
+    lu = spla.splu(A.tocsc())
+    wide = A.data.astype(np.longdouble)
+
+    def residual(v):
+        return b.astype(np.longdouble) - np.add.reduceat(wide * v[A.indices], A.indptr[:-1])
+
+    y = np.zeros(len(b), np.longdouble)
+    for _ in range(4):
+        y = y + lu.solve(residual(y).astype(np.float64))
+    z = y.astype(np.float64)
+    rounding = lu.solve(((b - A @ z) - residual(z.astype(np.longdouble))).astype(np.float64))
+    assert np.linalg.norm(x - z) <= 0.1 * np.linalg.norm(rounding)
