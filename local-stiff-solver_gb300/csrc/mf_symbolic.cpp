@@ -5,9 +5,9 @@
 // Nested dissection: a connected node set above the leaf size is split by a
 // level set of a breadth-first search from a pseudo-peripheral node (the
 // smallest level that leaves 30% on either side), thinned by moving separator
-// nodes with no neighbour on the far side back, and so is each half; the three
-// separators make one front with four children.  Disconnected sets become
-// sibling subtrees.
+// nodes with no neighbour on the far side back, and in a set of up to JOIN_DOFS so
+// is each half; the three separators then make one front with four children.
+// Disconnected sets become sibling subtrees.
 // Fronts are numbered in postorder (children first), and positions are
 // handed out front by front, so a subtree's variables are contiguous and a
 // front's own variables come last in it.  A front's boundary is the set of
@@ -30,17 +30,26 @@ namespace {
 // (Binary splits with leaves of 48 DOFs, six and more levels: 145 and 218 us.)
 constexpr int32_t LEAF_DOFS = 384;
 
+// Node sets above this many DOFs are split in two only: a joined front's pivots
+// cost three separators' cube where two levels cost one's and two smaller ones',
+// which the saved level pays for in small fronts alone.  Joined at every size,
+// balls of 25k, 85k and 179k DOFs took 43, 439 and 1821 ms to factorize, with
+// this limit 31, 250 and 958 (leaves of 48 DOFs in binary splits: 54, 383 and
+// 1359).  Between 3k and 14k DOFs the level costs an iteration 10 to 20 us and
+// saves the factorization 0.1 to 3 ms.
+constexpr int32_t JOIN_DOFS = 3072;
+
 struct Nd {
     const std::vector<int32_t> &aoff, &adj;  // local node graph (no self loops)
-    int32_t leaf_nodes;
+    int32_t leaf_nodes, join_nodes;
     std::vector<int32_t> stamp, lvl;
     int32_t cur = 0;
     std::vector<std::vector<int32_t>> own;       // fronts: own nodes
     std::vector<std::vector<int32_t>> children;  // fronts: child fronts (local ids)
     std::vector<int32_t> bisections;             // fronts: dissection levels joined in it (a leaf: 1)
 
-    Nd(const std::vector<int32_t> &o, const std::vector<int32_t> &a, int32_t nn, int32_t leaf)
-        : aoff(o), adj(a), leaf_nodes(leaf), stamp(nn, 0), lvl(nn, -1)
+    Nd(const std::vector<int32_t> &o, const std::vector<int32_t> &a, int32_t nn, int32_t leaf, int32_t join)
+        : aoff(o), adj(a), leaf_nodes(leaf), join_nodes(join), stamp(nn, 0), lvl(nn, -1)
     {
     }
 
@@ -106,12 +115,13 @@ struct Nd {
         }
         std::vector<int32_t> A, B, own;
         if (!split(order, st, A, B, own)) return {make(std::move(nodes), {})};
-        // the halves' separators join this one in a single front of four
-        // children (a half that is small, disconnected or unsplittable stays)
+        // the halves' separators join this one in a single front of four children
+        // (a half that is small, disconnected or unsplittable stays)
         std::vector<std::vector<int32_t>> parts;
         int32_t levels = 1;
+        const bool join = (int32_t)order.size() <= join_nodes;
         for (std::vector<int32_t> *half : {&A, &B}) {
-            if ((int32_t)half->size() > leaf_nodes) {
+            if (join && (int32_t)half->size() > leaf_nodes) {
                 const int32_t hs = ++cur;
                 mark(*half, hs);
                 const std::vector<int32_t> reach = bfs((*half)[0], hs);
@@ -221,7 +231,7 @@ MfSymbolic mf_symbolic(const std::vector<int32_t> &dofs, const std::vector<int32
             }
             aoff.push_back((int32_t)adj.size());
         }
-        Nd nd(aoff, adj, nn, std::max(1, LEAF_DOFS / bd));
+        Nd nd(aoff, adj, nn, std::max(1, LEAF_DOFS / bd), JOIN_DOFS / bd);
         std::vector<int32_t> all(nn);
         std::iota(all.begin(), all.end(), 0);
         nd.dissect(std::move(all));

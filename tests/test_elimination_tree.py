@@ -40,6 +40,17 @@ def test_tree_is_shallow(nodes, radius, built):
     assert t["fmas"] > 0
 
 
+@pytest.mark.parametrize("nodes,radius", [(26, 0.43), (31, 0.42), (37, 0.43)])
+def test_factorization_work(nodes, radius, built):
+    """Nested dissection of a ball of n DOFs by halves down to 48 takes about
+    16 n^2 multiply-adds (8.1 G at 25k DOFs, 30.5 G at 46.5k).  Half as many
+    again are allowed for larger leaves and joined levels: joined up to the
+    root, they take 30 n^2."""
+    A, dofs = _ball(nodes, radius)
+    t = lss.stiff_elimination_tree(A, 3, dofs)
+    assert t["fmas"] <= 24.0 * len(dofs) ** 2, (len(dofs), t)
+
+
 def test_tree_is_deterministic(built):
     A, dofs = _ball(16, 0.45)
     assert lss.stiff_elimination_tree(A, 3, dofs) == lss.stiff_elimination_tree(A, 3, dofs)
