@@ -46,16 +46,14 @@ struct Nd {
     int32_t cur = 0;
     std::vector<std::vector<int32_t>> own;       // fronts: own nodes
     std::vector<std::vector<int32_t>> children;  // fronts: child fronts (local ids)
-    std::vector<int32_t> bisections;             // fronts: dissection levels joined in it (a leaf: 1)
 
     Nd(const std::vector<int32_t> &o, const std::vector<int32_t> &a, int32_t nn, int32_t leaf, int32_t join)
         : aoff(o), adj(a), leaf_nodes(leaf), join_nodes(join), stamp(nn, 0), lvl(nn, -1)
     {
     }
 
-    int32_t make(std::vector<int32_t> nodes, std::vector<int32_t> kids, int32_t levels = 1)
+    int32_t make(std::vector<int32_t> nodes, std::vector<int32_t> kids)
     {
-        bisections.push_back(levels);
         std::sort(nodes.begin(), nodes.end());
         own.push_back(std::move(nodes));
         children.push_back(std::move(kids));
@@ -118,7 +116,6 @@ struct Nd {
         // the halves' separators join this one in a single front of four children
         // (a half that is small, disconnected or unsplittable stays)
         std::vector<std::vector<int32_t>> parts;
-        int32_t levels = 1;
         const bool join = (int32_t)order.size() <= join_nodes;
         for (std::vector<int32_t> *half : {&A, &B}) {
             if (join && (int32_t)half->size() > leaf_nodes) {
@@ -127,7 +124,6 @@ struct Nd {
                 const std::vector<int32_t> reach = bfs((*half)[0], hs);
                 std::vector<int32_t> a, b, sep;
                 if (reach.size() == half->size() && split(reach, hs, a, b, sep)) {
-                    levels = 2;
                     own.insert(own.end(), sep.begin(), sep.end());
                     parts.push_back(std::move(a));
                     parts.push_back(std::move(b));
@@ -141,7 +137,7 @@ struct Nd {
             const std::vector<int32_t> k = dissect(std::move(part));
             kids.insert(kids.end(), k.begin(), k.end());
         }
-        return {make(std::move(own), std::move(kids), levels)};
+        return {make(std::move(own), std::move(kids))};
     }
 
     // Splits the connected set stamped `st` (order: a breadth-first search of
@@ -204,7 +200,7 @@ MfSymbolic mf_symbolic(const std::vector<int32_t> &dofs, const std::vector<int32
     const int32_t nb = (int32_t)rows.size() - 1;
     std::vector<int32_t> node_local(nb, -1);
     std::vector<int32_t> pos_stamp(nj, -1);
-    std::vector<int32_t> parent, dissected;  // per front: its parent, dissection levels of its subtree
+    std::vector<int32_t> parent;
     int32_t pos = 0;
     M.bnd_off.push_back(0);
     M.child_off.push_back(0);
@@ -255,15 +251,12 @@ MfSymbolic mf_symbolic(const std::vector<int32_t> &dofs, const std::vector<int32
             std::vector<int32_t> kids;
             for (int32_t c : nd.children[f]) kids.push_back(fbase + c);
             std::sort(kids.begin(), kids.end());
-            int32_t h = 0, d = 0;
+            int32_t h = 0;
             for (int32_t c : kids) {
                 parent[c] = id;
                 h = std::max(h, M.height[c] + 1);
-                d = std::max(d, dissected[c]);
             }
             M.height.push_back(h);
-            dissected.push_back(d + nd.bisections[f]);
-            M.dissection_levels = std::max(M.dissection_levels, dissected.back());
             M.child.insert(M.child.end(), kids.begin(), kids.end());
             M.child_off.push_back((int32_t)M.child.size());
             M.bnd_off.push_back(0);  // set below, once every position of the subdomain is known

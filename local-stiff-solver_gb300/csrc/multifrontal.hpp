@@ -41,9 +41,7 @@ constexpr int MF_SMEM_F = 64;
 // subtree occupy a contiguous range of positions and a front's own variables
 // are the last of its subtree.
 struct MfSymbolic {
-    int32_t nfront = 0, npos = 0;
-    int32_t levels = 0;             // of the tree of fronts (launches of the solve and the factorization)
-    int32_t dissection_levels = 0;  // of the nested dissection: a front with four children joins two
+    int32_t nfront = 0, npos = 0, levels = 0;  // levels of the tree of fronts
     std::vector<int32_t> p0, s, u, height;     // per front
     std::vector<int64_t> foff;                 // per front: element offset of its f x f storage
     std::vector<int32_t> woff;                 // per front: offset of its solve vector (f entries)

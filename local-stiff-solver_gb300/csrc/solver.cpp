@@ -649,8 +649,8 @@ void HybridSolver::setup_stiff()
         mf_->factorize(A_, stiff_, d_bad_.data(), stream_);
         const MfSymbolic &sym = mf_->symbolic();
         stats_["multifrontal_fronts"] = sym.nfront;
-        stats_["multifrontal_levels"] = sym.dissection_levels;
-        stats_["multifrontal_tree_levels"] = sym.levels;
+        stats_["multifrontal_levels"] = sym.levels;
+        stats_["multifrontal_tree_levels"] = sym.levels;  // the same under a second name
         stats_["multifrontal_max_front"] = sym.max_f;
         stats_["multifrontal_fmas"] = sym.fmas;
         stats_["multifrontal_bytes"] = (double)mf_->bytes();

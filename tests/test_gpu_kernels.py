@@ -86,6 +86,24 @@ def test_stiff_apply_edge_sizes(bs, m, built):
     s.close()
 
 
+@pytest.mark.parametrize("nodes", [100, 300, 2000])
+def test_info_reports_the_tree_of_fronts(nodes, built):
+    """get_info's multifrontal counts are those of the host plan: one front, a
+    joined front, a tree with splits in two.  The subdomain is a chain of nodes,
+    whose tree has the same levels and fronts in the solver's order."""
+    import lss
+    chain = sp.diags([1.0, 4.0, 1.0], [-1, 0, 1], shape=(2100, 2100))
+    A = sp.kron(chain, np.ones((3, 3)) + sp.identity(3), format="csc")
+    A.sort_indices()
+    dofs = np.arange(30, 30 + 3 * nodes)
+    s = make_solver(3, select_bad_dofs_from_l1_norm=False, decompose_subdomains=False, expand_subdomains=False)
+    s.set_problematic_dofs(dofs)
+    s.factorize(A)
+    info, plan = s.get_info(), lss.stiff_elimination_tree(A, 3, dofs)
+    s.close()
+    assert (info["multifrontal_levels"], info["multifrontal_fronts"]) == (plan["levels"], plan["fronts"])
+
+
 @pytest.mark.parametrize("n", [3, 96, 3000])
 def test_double_float_split_matches_casts(n, built):
     """The FP64 <-> FP32 conversions on the integer pipe equal the casts bit for
