@@ -13,7 +13,8 @@
 // front's vector is gathered by the GEMV CTAs, in the batched solve by a
 // launch before), then one backward GEMV launch per level (root first; in the
 // batched solve a scatter ends it).  GEMV CTAs take 32 output columns and at
-// most 64 (batched: 128) of a front's rows; larger fronts split their rows over several CTAs
+// most 64 to 512 (by the level's size; batched: 128) of a front's rows; larger
+// fronts split their rows over several CTAs
 // whose partial sums the last CTA of the group adds in a fixed order.  The
 // per-level launches use programmatic dependent launch.  The solve with one
 // right-hand side is FP64; the batched solve with 16 reads the fronts as
@@ -383,8 +384,8 @@ constexpr int NR_KROWS = 128;  // front rows per GEMV CTA of the batched solve (
 __host__ __device__ __forceinline__ int nr_kchunks(int rows) { return (rows + NR_KROWS - 1) / NR_KROWS; }
 
 // ---- solve with one right-hand side (FP64): one launch per level and
-// direction.  GEMV CTAs of 32 columns x at most 64 front rows (8 warps = 8
-// row slices, lane = column) gather their part of the front's vector
+// direction.  GEMV CTAs of 32 columns x a chunk of front rows (8 warps = 8
+// row slices, lane = column; 64 rows at a time) gather their part of the front's vector
 // themselves (right-hand side + the children's contributions, children in
 // order); fronts with more rows are split over several CTAs whose partial
 // sums the last CTA of the group adds in row-chunk order.  All of a CTA's
@@ -394,8 +395,13 @@ __host__ __device__ __forceinline__ int nr_kchunks(int rows) { return (rows + NR
 // rows per CTA: an SM takes 2 us over 256 x 32 FP64 multiply-adds and a level
 // has few CTAs, so shorter chunks gain more than their combination costs (1.3k-
 // and 3.0k-DOF balls, mixed: 72 and 108 us per iteration at 256 rows, 68 and 105
-// at 128, 66 and 102 at 64)
-constexpr int NR_COLS1 = 32, NR_KROWS1 = 64;
+// at 128, 66 and 102 at 64).  A level of more CTAs than the GPU holds takes
+// longer chunks, up to 512 rows, as long as that leaves it full: a CTA's gather,
+// sums and arrival are latencies, 1 us of an SM per CTA for 0.5 us of products.
+// 64 rows at every size took 330 and 1087 us per iteration with stiff blocks of
+// 25k and 85k DOFs, this rule 302 and 796 (256 rows behind a launch that
+// assembles, with smaller fronts: 598 and 962).
+constexpr int NR_COLS1 = 32, NR_KROWS1 = 64, NR_KMAX1 = 512;
 
 struct NrScratch1 {
     double *part;   // per CTA of a launch: NR_COLS1 partial sums
@@ -405,13 +411,15 @@ struct NrScratch1 {
 // A GEMV CTA's part of its front in registers (warp = row slice, lane =
 // column): the fronts do not change within a solve, so these loads are issued
 // before anything the CTA has to wait for and overlap the gather of its vector
-// (8 loads at a time behind it added 3 us to a launch).
+// (8 loads at a time behind it added 3 us to a launch).  Of a longer chunk these
+// are the first 64 rows; the others are loaded as the products reach them (loaded
+// 64 rows ahead: 64 registers, four CTAs per SM, 814 against 808 us at 85k DOFs).
 struct FrontPart {
     double a[NR_KROWS1 / 8];
 };
-__device__ __forceinline__ void load_part(FrontPart &p, const MfCta &c, const double *__restrict__ F)
+__device__ __forceinline__ void load_part(FrontPart &p, const MfCta &c, int r0, const double *__restrict__ F)
 {
-    const int cl = threadIdx.x & 31, ks = threadIdx.x >> 5;
+    const int cl = threadIdx.x & 31, ks = r0 + (threadIdx.x >> 5);
     const double *Fc = F + c.foff + (int64_t)(c.q0 + ks) * c.f + c.col0 + cl;
 #pragma unroll
     for (int j = 0; j < NR_KROWS1 / 8; ++j)
@@ -419,14 +427,20 @@ __device__ __forceinline__ void load_part(FrontPart &p, const MfCta &c, const do
 }
 
 // res[c] = sum over the CTA's rows of Fn[q][col0 + c] xs[q - q0]; slices in order
-__device__ __forceinline__ void gemv1(const FrontPart &p, const MfCta &c, const double *__restrict__ xs,
-                                      double *__restrict__ red, double *__restrict__ res)
+__device__ __forceinline__ void gemv1(FrontPart &p, const MfCta &c, const double *__restrict__ F,
+                                      const double *__restrict__ xs, double *__restrict__ red,
+                                      double *__restrict__ res)
 {
     const int cl = threadIdx.x & 31, ks = threadIdx.x >> 5;
     double acc = 0.0;
+    for (int r0 = 0;;) {
 #pragma unroll
-    for (int j = 0; j < NR_KROWS1 / 8; ++j)
-        if (ks + 8 * j < c.nrow) acc += p.a[j] * xs[ks + 8 * j];
+        for (int j = 0; j < NR_KROWS1 / 8; ++j)
+            if (r0 + ks + 8 * j < c.nrow) acc += p.a[j] * xs[r0 + ks + 8 * j];
+        r0 += NR_KROWS1;
+        if (r0 >= c.nrow) break;
+        load_part(p, c, r0, F);
+    }
     red[ks * 32 + cl] = acc;
     __syncthreads();
     if (threadIdx.x < c.ncol) {
@@ -481,21 +495,21 @@ __global__ void __launch_bounds__(256) mf_forward_kernel(MfView v, const MfCta *
                                                          const double *__restrict__ F, double *__restrict__ W,
                                                          NrScratch1 sc, const int *done)
 {
-    __shared__ double xs[NR_KROWS1], red[256], res[NR_COLS1];
+    __shared__ double xs[NR_KMAX1], red[256], res[NR_COLS1];
     const MfCta c = ctas[blockIdx.x];
     FrontPart part;
-    load_part(part, c, F);
+    load_part(part, c, 0, F);
     pdl_enter();
     if (done && *done) return;
     const int t = threadIdx.x;
-    if (t < c.nrow) {
-        const double a = mf_gather1(c, c.q0 + t, v, S, gptr, gsrc, W);
-        xs[t] = a;
-        if (c.col0 == c.s) W[(int64_t)c.woff + c.q0 + t] = a;
+    for (int r = t; r < c.nrow; r += 256) {
+        const double a = mf_gather1(c, c.q0 + r, v, S, gptr, gsrc, W);
+        xs[r] = a;
+        if (c.col0 == c.s) W[(int64_t)c.woff + c.q0 + r] = a;
     }
     const double base = t < c.ncol ? mf_gather1(c, c.col0 + t, v, S, gptr, gsrc, W) : 0.0;
     __syncthreads();
-    gemv1(part, c, xs, red, res);
+    gemv1(part, c, F, xs, red, res);
     if (!combine1(sc, c.kc, c.nkc, res, c.ncol)) return;
     if (t < c.ncol) W[(int64_t)c.woff + c.col0 + t] = base - res[t];
 }
@@ -510,20 +524,30 @@ __global__ void __launch_bounds__(256) mf_backward_kernel(MfView v, const MfCta 
                                                           double *__restrict__ z, float *__restrict__ z32,
                                                           float *__restrict__ z_lo, const int *done)
 {
-    __shared__ double vec[NR_KROWS1], red[256], res[NR_COLS1];
+    __shared__ double vec[NR_KMAX1], red[256], res[NR_COLS1];
     const MfCta c = ctas[blockIdx.x];
     FrontPart part;
-    load_part(part, c, F);
-    const int t = threadIdx.x, q = c.q0 + t;
-    const int32_t bp = t < c.nrow && q >= c.s ? v.bnd_pos[c.bnd_off + q - c.s] : 0;
+    load_part(part, c, 0, F);
+    const int t = threadIdx.x;
+    // boundary positions of the rows t and t + 256
+    int32_t bp[NR_KMAX1 / 256];
+#pragma unroll
+    for (int k = 0; k < NR_KMAX1 / 256; ++k) {
+        const int r = t + 256 * k, q = c.q0 + r;
+        bp[k] = r < c.nrow && q >= c.s ? v.bnd_pos[c.bnd_off + q - c.s] : 0;
+    }
     const int32_t d = t < c.ncol ? S.dofs[v.pos2j[c.p0 + c.col0 + t]] : 0;
     pdl_enter();
     if (done && *done) return;
-    if (t < c.nrow)
-        vec[t] = q >= c.s ? X[bp] : (c.s == c.f ? mf_gather1(c, q, v, S, gptr, gsrc, W) : W[(int64_t)c.woff + q]);
+#pragma unroll
+    for (int k = 0; k < NR_KMAX1 / 256; ++k) {
+        const int r = t + 256 * k, q = c.q0 + r;
+        if (r >= c.nrow) break;
+        vec[r] = q >= c.s ? X[bp[k]] : (c.s == c.f ? mf_gather1(c, q, v, S, gptr, gsrc, W) : W[(int64_t)c.woff + q]);
+    }
     const double zd = t < c.ncol ? z[d] : 0.0;
     __syncthreads();
-    gemv1(part, c, vec, red, res);
+    gemv1(part, c, F, vec, red, res);
     if (!combine1(sc, c.kc, c.nkc, res, c.ncol)) return;
     if (t < c.ncol) {
         X[c.p0 + c.col0 + t] = -res[t];
@@ -868,37 +892,54 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
         }, true);
         for (int32_t id : lv_large[h]) L.max_s_large = std::max(L.max_s_large, M.s[id]);
     }
-    // GEMV CTAs of the single right-hand-side solve
+    // GEMV CTAs of the single right-hand-side solve: cols columns from first on of
+    // rows rows of every front of a level
     std::vector<MfCta> ctas;
-    auto add_ctas = [&](int32_t id, int32_t first, int32_t cols, int32_t rows) {
-        const int32_t nkc = (rows + NR_KROWS1 - 1) / NR_KROWS1;
-        for (int32_t c0 = 0; c0 < cols; c0 += NR_COLS1)
-            for (int32_t kc = 0; kc < nkc; ++kc) {
-                MfCta c;
-                c.foff = M.foff[id];
-                c.s = M.s[id];
-                c.f = M.s[id] + M.u[id];
-                c.col0 = first + c0;
-                c.ncol = std::min(NR_COLS1, cols - c0);
-                c.q0 = kc * NR_KROWS1;
-                c.nrow = std::min(NR_KROWS1, rows - c.q0);
-                c.kc = kc;
-                c.nkc = nkc;
-                c.woff = M.woff[id];
-                c.p0 = M.p0[id];
-                c.bnd_off = M.bnd_off[id];
-                c.pad = 0;
-                ctas.push_back(c);
+    struct Part {
+        int32_t first, cols, rows;
+    };
+    const int64_t resident = sm_grid(5);
+    auto add_ctas = [&](const std::vector<int32_t> &fronts, auto part_of) {
+        int32_t chunk = NR_KROWS1;
+        for (; chunk < NR_KMAX1; chunk *= 2) {
+            int64_t n = 0;
+            for (int32_t id : fronts) {
+                const Part p = part_of(id);
+                n += (int64_t)((p.cols + NR_COLS1 - 1) / NR_COLS1) * ((p.rows + chunk - 1) / chunk);
             }
+            if (n <= resident) break;
+        }
+        for (int32_t id : fronts) {
+            const Part p = part_of(id);
+            const int32_t nkc = (p.rows + chunk - 1) / chunk;
+            for (int32_t c0 = 0; c0 < p.cols; c0 += NR_COLS1)
+                for (int32_t kc = 0; kc < nkc; ++kc) {
+                    MfCta c;
+                    c.foff = M.foff[id];
+                    c.s = M.s[id];
+                    c.f = M.s[id] + M.u[id];
+                    c.col0 = p.first + c0;
+                    c.ncol = std::min(NR_COLS1, p.cols - c0);
+                    c.q0 = kc * chunk;
+                    c.nrow = std::min(chunk, p.rows - c.q0);
+                    c.kc = kc;
+                    c.nkc = nkc;
+                    c.woff = M.woff[id];
+                    c.p0 = M.p0[id];
+                    c.bnd_off = M.bnd_off[id];
+                    c.pad = 0;
+                    ctas.push_back(c);
+                }
+        }
     };
     int64_t max1 = 1;
     for (int h = 0; h < M.levels; ++h) {
         Level &L = levels_[h];
         L.fwd1 = (int64_t)ctas.size();
-        for (int32_t id : lv_all[h]) add_ctas(id, M.s[id], M.u[id], M.s[id]);
+        add_ctas(lv_all[h], [&](int32_t id) { return Part{M.s[id], M.u[id], M.s[id]}; });
         L.nfwd1 = (int32_t)((int64_t)ctas.size() - L.fwd1);
         L.bwd1 = (int64_t)ctas.size();
-        for (int32_t id : lv_all[h]) add_ctas(id, 0, M.s[id], M.s[id] + M.u[id]);
+        add_ctas(lv_all[h], [&](int32_t id) { return Part{0, M.s[id], M.s[id] + M.u[id]}; });
         L.nbwd1 = (int32_t)((int64_t)ctas.size() - L.bwd1);
         max1 = std::max<int64_t>({max1, L.nfwd1, L.nbwd1});
     }

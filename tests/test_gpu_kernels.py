@@ -86,6 +86,27 @@ def test_stiff_apply_edge_sizes(bs, m, built):
     s.close()
 
 
+@pytest.mark.parametrize("m", [8001, 16002, 30000])
+def test_stiff_apply_long_row_chunks(m, built):
+    """A_SS^-1 r where a level of the tree has more CTAs than the GPU holds at 64
+    rows each (1.4k, 2.8k and 5.3k): chunks of 128 to 512 rows, with
+    remainders.  Diagonally dominant as above: 1e-12 of a sparse LU."""
+    import scipy.sparse.linalg as spla
+    A = block_system(11000, 3, seed=m)
+    dofs = np.arange(5, 5 + m)
+    s = make_solver(3, extra={"composition": "additive"}, select_bad_dofs_from_l1_norm=False,
+                    decompose_subdomains=False, expand_subdomains=False)
+    s.set_problematic_dofs(dofs)
+    s.factorize(A)
+    r = np.random.default_rng(m).standard_normal(A.shape[0])
+    z = s.mas_apply(r)
+    d = s.precond(r) - z
+    np.testing.assert_array_equal(s.precond(r) - z, d)  # fixed order of every sum
+    s.close()
+    x = spla.splu(A[dofs][:, dofs].tocsc()).solve(r[dofs], trans="T")
+    assert np.linalg.norm(d[dofs] - x) <= 1e-12 * (np.linalg.norm(x) + np.linalg.norm(z[dofs]))
+
+
 @pytest.mark.parametrize("nodes", [100, 300, 2000])
 def test_info_reports_the_tree_of_fronts(nodes, built):
     """get_info's multifrontal counts are those of the host plan: one front, a
