@@ -35,7 +35,7 @@ struct BatchSolver::Impl {
     BatchStiff St;
     MfFactor mf;
     // operator and chunks
-    DBuf<int32_t> rows, cols, chunk_sys, chunk_p0, sys_chunk0, part_off;
+    DBuf<int32_t> rows, cols, chunk_sys, chunk_p0, chunk_row0, sys_chunk0, part_off;
     DBuf<double> vals, omega, partials;
     DBuf<float> vals32;
     DBuf<float2> vals_df;
@@ -155,7 +155,7 @@ void BatchSolver::merge()
     const int32_t ns = (int32_t)sys_.size();
     constexpr int BDIM = 3;
     // ---- operator, parts, chunks
-    std::vector<int32_t> rows{0}, cols, part_off{0}, chunk_sys, chunk_p0, sys_chunk0{0};
+    std::vector<int32_t> rows{0}, cols, part_off{0}, chunk_sys, chunk_p0, chunk_row0, sys_chunk0{0};
     std::vector<uint8_t> precise;
     std::vector<double> omega;
     D.row0.assign(ns, 0);
@@ -181,6 +181,7 @@ void BatchSolver::merge()
         for (int32_t q = 0; q < nps; q += per_chunk) {
             chunk_sys.push_back(s);
             chunk_p0.push_back(np + q);
+            chunk_row0.push_back(nb);
         }
         sys_chunk0.push_back((int32_t)chunk_sys.size());
         if (H.h_precise_.size() == (size_t)P.nb) {
@@ -202,6 +203,7 @@ void BatchSolver::merge()
     D.part_off.upload(part_off, st);
     D.chunk_sys.upload(chunk_sys, st);
     D.chunk_p0.upload(chunk_p0, st);
+    D.chunk_row0.upload(chunk_row0, st);
     D.sys_chunk0.upload(sys_chunk0, st);
     D.omega.upload(omega, st);
     if (any_precise) D.precise.upload(precise, st);
@@ -221,7 +223,7 @@ void BatchSolver::merge()
         }
     }
     const int32_t nchunk = (int32_t)chunk_sys.size();
-    D.partials.resize((size_t)std::max(nchunk, 1) * BK * 2);
+    D.partials.resize((size_t)std::max(np, 1) * BK);
     D.counters.resize(ns);
     D.counters.zero(st);
     D.lane.resize((size_t)ns * BK);
@@ -478,6 +480,7 @@ void BatchSolver::merge()
     B.precise = any_precise ? D.precise.data() : nullptr;
     B.chunk_sys = D.chunk_sys.data();
     B.chunk_p0 = D.chunk_p0.data();
+    B.chunk_row0 = D.chunk_row0.data();
     B.sys_chunk0 = D.sys_chunk0.data();
     B.part_off = D.part_off.data();
     B.omega = D.omega.data();

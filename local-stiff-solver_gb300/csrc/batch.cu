@@ -14,8 +14,10 @@
 // Work decomposition.  A chunk is up to BATCH_CHUNK (batch.hpp) consecutive MAS
 // partitions of one system (<= 32 block rows each); row kernels run one CTA
 // per chunk, and a system whose lanes have all stopped skips its chunks.
-// Per-lane sums are reduced per CTA, written to a partials slot of the chunk,
-// and summed in chunk order by the last CTA of the system to arrive.
+// Per-lane sums are formed per partition (the threads' rows follow from their
+// place in the system), written to the partition's slot, and summed by the last
+// CTA of the system to arrive, in an order of the system's own: a system's results
+// depend neither on the chunks nor on the other systems of the batch.
 #include <cfloat>
 
 #include "batch.hpp"
@@ -58,6 +60,7 @@ struct Chunk {
     int sys;
     int32_t r0, r1;  // block rows
     int32_t p0, p1;  // MAS partitions
+    int32_t row0;    // the system's first block row
 };
 
 __device__ __forceinline__ Chunk chunk_of(const BatchDev &B, int c)
@@ -68,54 +71,89 @@ __device__ __forceinline__ Chunk chunk_of(const BatchDev &B, int c)
     k.p1 = B.chunk_p0[c + 1];
     k.r0 = B.part_off[k.p0];
     k.r1 = B.part_off[k.p1];
+    k.row0 = B.chunk_row0[c];
     return k;
 }
 
-// Per-lane totals of NV values over the chunks of one system.  part[v] holds
-// the CTA's sum of value v for right-hand side threadIdx.x (threads < BK).
-// Returns true in the threads < BK of the last CTA of the system to arrive,
-// where tot[v] is the system's sum in a fixed order; the counter is reset.
+// the first row i >= lo with (i - row0) % N == t: N threads (warps) share a
+// system's rows by their place in it
+template <int N>
+__device__ __forceinline__ int32_t first_row(int32_t lo, int32_t row0, int t)
+{
+    return lo + ((t - (lo - row0)) & (N - 1));
+}
+
+// A thread's way through the chunk's partitions along ascending rows (block rows,
+// or scalar rows with rows = BD): reach(i) puts the sums of the partitions that
+// end before row i (zeros for those without a row of the thread), end() the rest.
+struct PartCursor {
+    int32_t q = 0, n, p0, hi, rows;
+    __device__ __forceinline__ PartCursor(const BatchDev &B, const Chunk &ch, int rows_ = 1)
+        : n(ch.p1 - ch.p0), p0(ch.p0), hi(B.part_off[ch.p0 + 1] * rows_), rows(rows_)
+    {
+    }
+    template <typename Put>
+    __device__ __forceinline__ void reach(const BatchDev &B, int32_t i, Put put)
+    {
+        while (i >= hi) {
+            put(q++);
+            hi = B.part_off[p0 + q + 1] * rows;
+        }
+    }
+    template <typename Put>
+    __device__ __forceinline__ void end(Put put)
+    {
+        while (q < n) put(q++);
+    }
+};
+
+__device__ __forceinline__ double lane_value(double v) { return v; }
+__device__ __forceinline__ double lane_value(float2 v) { return df_val(v); }
+
+// The sums of the chunk's partitions, added up from red[partition][row group][rhs].
+template <int R, typename T>
+__device__ __forceinline__ void put_parts(const BatchDev &B, const Chunk &ch, const T (&red)[BATCH_CHUNK][R][BK])
+{
+    __syncthreads();
+    const int q = threadIdx.x >> 4, k = threadIdx.x & (BK - 1);
+    if (q >= ch.p1 - ch.p0) return;
+    double s = 0.0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) s += lane_value(red[q][r][k]);
+    B.partials[(int64_t)(ch.p0 + q) * BK + k] = s;
+}
+
+// Per-lane totals over the partitions of one system, whose sums are in
+// B.partials.  Returns true in the threads < BK of the last CTA of the system to
+// arrive, where tot is the system's sum in a fixed order; the counter is reset.
 // Needs 256 threads.
-template <int NV>
-__device__ bool sys_finish(const BatchDev &B, int c, int sys, const double (&part)[NV], double (&tot)[NV])
+__device__ bool sys_finish(const BatchDev &B, int sys, double &tot)
 {
     __shared__ bool last;
     const int t = threadIdx.x;
-    if (t < BK)
-#pragma unroll
-        for (int v = 0; v < NV; ++v) B.partials[((int64_t)c * BK + t) * NV + v] = part[v];
     __threadfence();
     __syncthreads();
-    if (t == 0) {
-        const unsigned arrived = atomicAdd(B.counters + sys, 1u);
-        last = arrived == (unsigned)(B.sys_chunk0[sys + 1] - B.sys_chunk0[sys] - 1);
-    }
+    const int32_t c0 = B.sys_chunk0[sys], c1 = B.sys_chunk0[sys + 1];
+    if (t == 0) last = atomicAdd(B.counters + sys, 1u) == (unsigned)(c1 - c0 - 1);
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    // thread (g, k): right-hand side k over the chunks g, g + 16, ...; the sixteen
-    // sums meet in order (one thread per right-hand side took 12 us over 80 chunks)
-    __shared__ double fin[NV][16][BK];
+    // thread (g, k): right-hand side k over the partitions g, g + 16, ...; the
+    // sixteen sums meet in order (one thread per right-hand side took 12 us over 80)
+    __shared__ double fin[16][BK];
     static_assert(BK == 16, "256 threads = 16 groups x 16 right-hand sides");
     {
         const int g = t >> 4, k = t & (BK - 1);
-        double acc[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) acc[v] = 0.0;
-#pragma unroll 4
-        for (int q = B.sys_chunk0[sys] + g; q < B.sys_chunk0[sys + 1]; q += 16)
-#pragma unroll
-            for (int v = 0; v < NV; ++v) acc[v] += __ldcg(B.partials + ((int64_t)q * BK + k) * NV + v);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) fin[v][g][k] = acc[v];
+        double acc = 0.0;
+        const int32_t p1 = B.chunk_p0[c1];
+#pragma unroll 8
+        for (int32_t q = B.chunk_p0[c0] + g; q < p1; q += 16) acc += __ldcg(B.partials + (int64_t)q * BK + k);
+        fin[g][k] = acc;
     }
     __syncthreads();
     if (t < BK) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            tot[v] = fin[v][0][t];
-            for (int g = 1; g < 16; ++g) tot[v] += fin[v][g][t];
-        }
+        tot = fin[0][t];
+        for (int g = 1; g < 16; ++g) tot += fin[g][t];
     }
     if (t == 0) B.counters[sys] = 0u;
     return t < BK;
@@ -161,15 +199,22 @@ __device__ __forceinline__ void row_blocks(const BatchDev &B, int32_t b, int32_t
     }
 }
 
-__global__ void __launch_bounds__(256) spmm_alpha_kernel(BatchDev B, const float2 *__restrict__ p,
+__global__ void __launch_bounds__(256, 4) spmm_alpha_kernel(BatchDev B, const float2 *__restrict__ p,
                                                          float2 *__restrict__ ap)
 {
     constexpr int U = 2;
     const Chunk ch = chunk_of(B, blockIdx.x);
     if (B.sys_done[ch.sys]) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, h = lane >> 4, k = lane & 15;
+    __shared__ float2 red[BATCH_CHUNK][8][BK];
     float dh = 0.f, dl = 0.f;
-    for (int32_t I = ch.r0 + w; I < ch.r1; I += 8) {
+    PartCursor at(B, ch);
+    auto put = [&](int q) {
+        if (h == 0) red[q][w][k] = make_float2(dh, dl);
+        dh = dl = 0.f;
+    };
+    for (int32_t I = first_row<8>(ch.r0, ch.row0, w); I < ch.r1; I += 8) {
+        at.reach(B, I, put);
         const int32_t b = B.rows[I], len = B.rows[I + 1] - b;
         const float2 *__restrict__ v = B.vals_df + (int64_t)b * 9;
         // one double-float accumulator per (block slot u, row r): 3 U independent chains
@@ -221,18 +266,15 @@ __global__ void __launch_bounds__(256) spmm_alpha_kernel(BatchDev B, const float
             }
         }
     }
-    __shared__ double red[8][BK];
-    if (h == 0) red[w][k] = (double)dh + (double)dl;
-    __syncthreads();
-    double part[1] = {0.0}, tot[1];
-    if (threadIdx.x < BK)
-        for (int q = 0; q < 8; ++q) part[0] += red[q][threadIdx.x];
-    if (sys_finish<1>(B, blockIdx.x, ch.sys, part, tot)) {
+    at.end(put);
+    put_parts(B, ch, red);
+    double tot;
+    if (sys_finish(B, ch.sys, tot)) {
         BatchLane &L = B.lane[ch.sys * BK + threadIdx.x];
         if (!L.done) {
             // GPUHybrid.cu:1458-1480 per lane
             L.iter += 1;
-            const double pAp = tot[0];
+            const double pAp = tot;
             L.pAp = pAp;
             const double alpha = L.gamma / pAp;
             if (pAp == 0.0) L.done = STOP_ZERO_PAP;
@@ -256,29 +298,34 @@ __global__ void __launch_bounds__(256) update_xr_kernel(BatchDev B, float2 *__re
     const bool live = !L.done;
     const double alpha = L.alpha;
     const float ah = (float)alpha, al = (float)(alpha - (double)ah);
+    __shared__ float2 red[BATCH_CHUNK][16][BK];
+    const int g = threadIdx.x >> 4;
     float rh = 0.f, rl = 0.f;
-    const int64_t e1 = (int64_t)ch.r1 * BD * BK;
+    PartCursor at(B, ch, BD);
+    auto put = [&](int q) {
+        red[q][g][k] = make_float2(rh, rl);
+        rh = rl = 0.f;
+    };
 #pragma unroll 4
-    for (int64_t e = (int64_t)ch.r0 * BD * BK + threadIdx.x; e < e1; e += blockDim.x) {
+    for (int32_t i = first_row<16>(ch.r0 * BD, ch.row0 * BD, g); i < ch.r1 * BD; i += 16) {
         if (!live) continue;
+        at.reach(B, i, put);
+        const int64_t e = (int64_t)i * BK + k;
         x[e] = df_sum(x[e], df_mul(p[e], ah, al));
         const float2 d = df_mul(ap[e], ah, al);
         const float2 ri = df_sum(r[e], make_float2(-d.x, -d.y));
         r[e] = ri;
         df_fma(rh, rl, ri.x, ri.y, ri.x, ri.y);
     }
-    __shared__ double red[16][BK];
-    red[threadIdx.x >> 4][k] = (double)rh + (double)rl;
-    __syncthreads();
-    double part[1] = {0.0}, tot[1];
-    if (threadIdx.x < BK)
-        for (int q = 0; q < 16; ++q) part[0] += red[q][threadIdx.x];
-    const bool fin = sys_finish<1>(B, blockIdx.x, ch.sys, part, tot);
+    at.end(put);
+    put_parts(B, ch, red);
+    double tot;
+    const bool fin = sys_finish(B, ch.sys, tot);
     if (fin) {
         BatchLane &M = B.lane[ch.sys * BK + threadIdx.x];
         if (!M.done) {
             // GPUHybrid.cu:1482-1496 per lane
-            const double rr = tot[0];
+            const double rr = tot;
             M.rr = rr;
             if (!(rr == rr) || isinf(rr)) M.done = STOP_NONFINITE;
             else if (M.rel_eps > 0 && rr / M.bb < M.rel_eps) M.done = STOP_CONVERGED_REL;
@@ -331,8 +378,15 @@ __global__ void __launch_bounds__(256) residual64_kernel(BatchDev B, const doubl
 {
     const Chunk ch = chunk_of(B, blockIdx.x);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, h = lane >> 4, k = lane & 15;
+    __shared__ double red[BATCH_CHUNK][8][BK];
     double acc_rr = 0.0;
-    for (int32_t I = ch.r0 + w; I < ch.r1; I += 8) {
+    PartCursor at(B, ch);
+    auto put = [&](int q) {
+        if (h == 0) red[q][w][k] = acc_rr;
+        acc_rr = 0.0;
+    };
+    for (int32_t I = first_row<8>(ch.r0, ch.row0, w); I < ch.r1; I += 8) {
+        at.reach(B, I, put);
         const int32_t b = B.rows[I], len = B.rows[I + 1] - b;
         const double *__restrict__ v = B.vals + (int64_t)b * 9;
         double y[BD] = {0.0, 0.0, 0.0};
@@ -364,13 +418,10 @@ __global__ void __launch_bounds__(256) residual64_kernel(BatchDev B, const doubl
             }
         }
     }
-    __shared__ double red[8][BK];
-    if (h == 0) red[w][k] = acc_rr;
-    __syncthreads();
-    double part[1] = {0.0}, tot[1];
-    if (threadIdx.x < BK)
-        for (int q = 0; q < 8; ++q) part[0] += red[q][threadIdx.x];
-    if (sys_finish<1>(B, blockIdx.x, ch.sys, part, tot)) out_rr[ch.sys * BK + threadIdx.x] = tot[0];
+    at.end(put);
+    put_parts(B, ch, red);
+    double tot;
+    if (sys_finish(B, ch.sys, tot)) out_rr[ch.sys * BK + threadIdx.x] = tot;
 }
 
 // ---------------------------------------------------------------- MAS (FP32), BK right-hand sides
@@ -723,7 +774,7 @@ __global__ void __launch_bounds__(BANK_THREADS) symv0_kernel(BatchDev B, MasDev 
     const float oh = (float)om, ol = (float)(om - (double)oh);
     const float *u1 = u + m.voff[1] * BK;
     const int k = threadIdx.x & (BK - 1);
-    float dh = 0.f, dl = 0.f;
+    float2 dot[BATCH_CHUNK];  // the thread's part of r.z per partition, in registers
     auto job = [&](int i, const float *&tile, const XT *&x, int &cnt) {
         const int32_t p = ch.p0 + i, lo = m.part_off[p];
         tile = inv0 + (int64_t)p * NB * NB;  // pre-expanded
@@ -736,6 +787,7 @@ __global__ void __launch_bounds__(BANK_THREADS) symv0_kernel(BatchDev B, MasDev 
         const bool coarse = m.L > 1 && m.ccnt0[p] > 0;
         const int32_t cb = coarse ? m.cbase0[p] : 0;
         const int r0 = threadIdx.x >> 4, nrow = 3 * cnt;
+        float dh = 0.f, dl = 0.f;
         // every gather of the thread's rows first, then the arithmetic
         float cu[RPT];
         float2 zo[RPT], rv[RPT];
@@ -761,20 +813,25 @@ __global__ void __launch_bounds__(BANK_THREADS) symv0_kernel(BatchDev B, MasDev 
             z[e] = val;
             if (DOT) df_fma(dh, dl, rv[j].x, rv[j].y, val.x, val.y);
         }
+        if (DOT)
+#pragma unroll
+            for (int q = 0; q < BATCH_CHUNK; ++q)
+                if (q == i) dot[q] = make_float2(dh, dl);
     };
     if (!bank_pipeline<XT, true>(smem_raw, ch.p1 - ch.p0, job, epi, B.err)) return;
     if (DOT) {
-        __shared__ double red[BANK_THREADS / BK][BK];
-        red[threadIdx.x >> 4][k] = (double)dh + (double)dl;
-        __syncthreads();
-        double part[1] = {0.0}, tot[1];
-        if (threadIdx.x < BK)
-            for (int q = 0; q < BANK_THREADS / BK; ++q) part[0] += red[q][threadIdx.x];
-        if (sys_finish<1>(B, blockIdx.x, ch.sys, part, tot)) {
+        // the stages are free again
+        float2(&red)[BATCH_CHUNK][16][BK] = *reinterpret_cast<float2(*)[BATCH_CHUNK][16][BK]>(smem_raw);
+#pragma unroll
+        for (int q = 0; q < BATCH_CHUNK; ++q)
+            if (q < ch.p1 - ch.p0) red[q][threadIdx.x >> 4][k] = dot[q];
+        put_parts(B, ch, red);
+        double tot;
+        if (sys_finish(B, ch.sys, tot)) {
             BatchLane &L = B.lane[ch.sys * BK + threadIdx.x];
             if (!L.done) {
-                if (DOT == 2) L.beta = tot[0] / L.gamma;  // GPUHybrid.cu:1501-1504
-                L.gamma = tot[0];
+                if (DOT == 2) L.beta = tot / L.gamma;  // GPUHybrid.cu:1501-1504
+                L.gamma = tot;
             }
         }
     }
@@ -959,16 +1016,23 @@ __global__ void __launch_bounds__(256) lane_norms_kernel(BatchDev B, const doubl
 {
     const Chunk ch = chunk_of(B, blockIdx.x);
     const int k = threadIdx.x & (BK - 1);
+    __shared__ double red[BATCH_CHUNK][16][BK];
+    const int g = threadIdx.x >> 4;
     double s2 = 0.0;
-    const int64_t e1 = (int64_t)ch.r1 * BD * BK;
-    for (int64_t e = (int64_t)ch.r0 * BD * BK + threadIdx.x; e < e1; e += blockDim.x) s2 += b[e] * b[e];
-    __shared__ double red[16][BK];
-    red[threadIdx.x >> 4][k] = s2;
-    __syncthreads();
-    double part[1] = {0.0}, tot[1];
-    if (threadIdx.x < BK)
-        for (int q = 0; q < 16; ++q) part[0] += red[q][threadIdx.x];
-    if (sys_finish<1>(B, blockIdx.x, ch.sys, part, tot)) out[ch.sys * BK + threadIdx.x] = tot[0];
+    PartCursor at(B, ch, BD);
+    auto put = [&](int q) {
+        red[q][g][k] = s2;
+        s2 = 0.0;
+    };
+    for (int32_t i = first_row<16>(ch.r0 * BD, ch.row0 * BD, g); i < ch.r1 * BD; i += 16) {
+        at.reach(B, i, put);
+        const double v = b[(int64_t)i * BK + k];
+        s2 += v * v;
+    }
+    at.end(put);
+    put_parts(B, ch, red);
+    double tot;
+    if (sys_finish(B, ch.sys, tot)) out[ch.sys * BK + threadIdx.x] = tot;
 }
 
 __global__ void __launch_bounds__(256) zero_done_lanes_kernel(BatchDev B, double *__restrict__ x)

@@ -35,7 +35,10 @@ namespace lss {
 constexpr int BK = 16;           // right-hand sides per system in a batch
 // MAS partitions (<= 32 block rows each) per chunk at most; fewer while that
 // leaves less than five CTAs per SM: 146k DOFs in chunks of eight are 190 CTAs,
-// eight warps per SM for kernels that wait on memory
+// eight warps per SM for kernels that wait on memory (an iteration of six systems
+// of 5k to 60k DOFs: 658 us in chunks of eight, 502 of four, 478 of two, 490 of
+// one; of 64 systems of 8k to 192k DOFs: 5511, 5605, 6034, 6946).  No result
+// depends on it: sums are formed per partition.
 constexpr int BATCH_CHUNK = 8;
 
 class HybridSolver;
@@ -58,13 +61,14 @@ struct BatchDev {
     const uint8_t *precise = nullptr;   // block rows whose preconditioner residual runs in double-float
     // chunks: chunk c = parts [chunk_p0[c], chunk_p0[c+1]) of system chunk_sys[c]
     const int32_t *chunk_sys = nullptr, *chunk_p0 = nullptr;
+    const int32_t *chunk_row0 = nullptr;  // per chunk: its system's first block row
     const int32_t *sys_chunk0 = nullptr;  // nsys + 1
     const int32_t *part_off = nullptr;    // merged MAS parts (nparts + 1), block-row offsets
     const double *omega = nullptr;        // per system: damping of MAS in the multiplicative form
     BatchLane *lane = nullptr;            // nsys * BK
     const int *sys_done = nullptr;        // per system: every lane stopped
     int *err = nullptr;                   // != 0: a bulk copy did not arrive (sys_done[nsys])
-    double *partials = nullptr;           // nchunk * BK * 2
+    double *partials = nullptr;           // nparts * BK
     unsigned *counters = nullptr;         // nsys
 };
 

@@ -107,3 +107,43 @@ def test_batch_pcg_rejects_other_forms(built):
     with pytest.raises(lss.LssError) as e:
         lss.Batch([s])
     assert "mixed precision" in str(e.value)
+
+
+def test_batch_companions_do_not_change_a_system(built):
+    """A system's results are the same bits whatever it is solved with: small
+    companions (chunks of one partition), or larger ones before it (chunks of two
+    or more, other merged offsets)."""
+    import torch
+    import lss
+    from lss import gen
+    dev = torch.device("cuda", 0)
+    rng = np.random.Generator(np.random.PCG64(3))
+    solvers, vals, bs, parts = [], [], [], []
+    for nodes in (12, 9, 40, 11):
+        E, _ = gen.sphere_inclusion_E(nodes, nodes, nodes, rng, radius=0.25, E_in=1e4)
+        A = gen.elasticity_cube(nodes, nodes, nodes, E).tocsc()
+        A.sum_duplicates()
+        s = lss.Solver.create({"solver": "GPUHybrid", "GPUHybrid": PARAMS, "gb300": {"precision": "mixed"}})
+        s.analyze_pattern(A)
+        solvers.append(s)
+        parts.append(len(lss.partition_pattern(A, 3)[1]) - 1)
+        vals.append(torch.tensor(A.data, dtype=torch.float64, device=dev))
+        bs.append(torch.tensor(rng.standard_normal((lss.BATCH_RHS, A.shape[0])), dtype=torch.float64, device=dev))
+    wave = 5 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert sum(parts[:2]) < 2 * wave <= sum(parts)
+
+    def solve(members):
+        batch = lss.Batch([solvers[i] for i in members])
+        batch.factorize_device([vals[i].data_ptr() for i in members])
+        xs = [torch.zeros_like(bs[i]) for i in members]
+        torch.cuda.synchronize()
+        its = batch.solve_device([bs[i].data_ptr() for i in members], [x.data_ptr() for x in xs])
+        torch.cuda.synchronize()
+        k = members.index(0)
+        return its[k].copy(), xs[k].cpu().numpy()
+
+    its, x = solve([0, 1])
+    for members in ([1, 0], [2, 0], [3, 2, 1, 0]):
+        other_its, other = solve(members)
+        np.testing.assert_array_equal(other_its, its, err_msg=str(members))
+        np.testing.assert_array_equal(other, x, err_msg=str(members))
