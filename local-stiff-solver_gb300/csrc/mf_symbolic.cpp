@@ -21,15 +21,6 @@
 namespace lss {
 namespace {
 
-// Node sets up to this many DOFs are eliminated as one front.  Every level of
-// the tree is two dependent launches of each solve and a chain of panel steps
-// of the factorization, while a front of this size is still a few microseconds
-// of FP64 work on the whole GPU.  Mixed iterations with a 1.3k- and a 3.0k-DOF
-// ball: 88 and 129 us with leaves of 128 or 192 DOFs, 87 and 115 with 256, 76
-// and 115 with 384; 512 gains no more and costs a quarter of the factorization.
-// (Binary splits with leaves of 48 DOFs, six and more levels: 145 and 218 us.)
-constexpr int32_t LEAF_DOFS = 384;
-
 // Node sets above this many DOFs are split in two only: a joined front's pivots
 // cost three separators' cube where two levels cost one's and two smaller ones',
 // which the saved level pays for in small fronts alone.  Joined at every size,
@@ -38,6 +29,23 @@ constexpr int32_t LEAF_DOFS = 384;
 // 1359).  Between 3k and 14k DOFs the level costs an iteration 10 to 20 us and
 // saves the factorization 0.1 to 3 ms.
 constexpr int32_t JOIN_DOFS = 3072;
+
+// Node sets up to this many DOFs are eliminated as one front, in a subdomain of m
+// DOFs.  Every level of the tree is two dependent launches of each solve and a
+// chain of panel steps of the factorization, while a front of 384 is still a few
+// microseconds of FP64 work on the whole GPU.  Mixed iterations with a 1.3k- and a
+// 3.0k-DOF ball: 88 and 129 us with leaves of 128 or 192 DOFs, 87 and 115 with 256,
+// 76 and 115 with 384; 512 gains no more and costs a quarter of the factorization.
+// (Binary splits with leaves of 48 DOFs, six and more levels: 145 and 218 us.)
+// Between 3.2k and 7k DOFs 256 saves up to a fifth of the factorization and loses
+// no level; 64 loses one, 5 to 18 us an iteration.
+// A large subdomain has leaves enough to fill the GPU at 64 DOFs, which are swept
+// in shared memory; of 384, their n (384 + u)^2 multiply-adds and entries outgrow
+// the levels they save, above all where separators are small: chains of 13.5k and
+// 108k DOFs factorized in 2.1 and 12.9 ms (64: 0.7 and 3.1), a disk of 322k DOFs in
+// 51.7 (20.4) with twice the storage, balls of 14k and 47k in 15.2 and 85 (13.0 and
+// 78), and no iteration of these was faster by more than 7%.
+int32_t leaf_dofs(int32_t m) { return m <= JOIN_DOFS ? 384 : (m <= 8192 ? 256 : 64); }
 
 struct Nd {
     const std::vector<int32_t> &aoff, &adj;  // local node graph (no self loops)
@@ -227,7 +235,7 @@ MfSymbolic mf_symbolic(const std::vector<int32_t> &dofs, const std::vector<int32
             }
             aoff.push_back((int32_t)adj.size());
         }
-        Nd nd(aoff, adj, nn, std::max(1, LEAF_DOFS / bd), JOIN_DOFS / bd);
+        Nd nd(aoff, adj, nn, std::max(1, leaf_dofs(m) / bd), JOIN_DOFS / bd);
         std::vector<int32_t> all(nn);
         std::iota(all.begin(), all.end(), 0);
         nd.dissect(std::move(all));

@@ -8,6 +8,7 @@ log2(n / 48) (the leaf size), not the near-linear chains of a separator choice
 that ignores balance.  Also: deterministic, and every variable in one front."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 import lss
 from lss import gen
@@ -49,6 +50,29 @@ def test_factorization_work(nodes, radius, built):
     A, dofs = _ball(nodes, radius)
     t = lss.stiff_elimination_tree(A, 3, dofs)
     assert t["fmas"] <= 24.0 * len(dofs) ** 2, (len(dofs), t)
+
+
+def _disk(nodes):
+    T, I = sp.diags([-1.0, 2.0, -1.0], [-1, 0, 1], shape=(nodes, nodes)), sp.identity(nodes)
+    i, c = np.arange(nodes * nodes), (nodes - 1) / 2.0
+    inside = i[(i % nodes - c) ** 2 + (i // nodes - c) ** 2 <= (0.4 * nodes) ** 2]
+    return sp.csc_matrix(sp.kron(T, I) + sp.kron(I, T)), 1, inside
+
+
+def _chain(nodes):
+    T = sp.diags([-1.0, 4.0, -1.0], [-1, 0, 1], shape=(nodes, nodes))
+    return sp.csc_matrix(sp.kron(T, np.ones((3, 3)))), 3, np.arange(30, 3 * nodes - 30)
+
+
+@pytest.mark.parametrize("make,nodes", [(_disk, 130), (_disk, 200), (_chain, 3000), (_chain, 8000)])
+def test_factorization_work_of_thin_subdomains(make, nodes, built):
+    """Where separators are small the leaves are the work: 0.5 (64 + 48)^2 = 6272
+    multiply-adds per DOF for leaves of 64 DOFs and a boundary of 48 (leaves of 384
+    DOFs: over 70000), and a fifth of that again for the tree above them."""
+    A, bs, dofs = make(nodes)
+    A.sort_indices()
+    t = lss.stiff_elimination_tree(A, bs, dofs)
+    assert len(dofs) > 8192 and t["fmas"] <= 8000.0 * len(dofs), (len(dofs), t)
 
 
 def test_tree_is_deterministic(built):
