@@ -805,7 +805,7 @@ int64_t MfFactor::bytes() const
                      d_i64_.bytes());
 }
 
-void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
+void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st, bool solve)
 {
     sym_ = sym;
     levels_.clear();
@@ -820,7 +820,7 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
     std::vector<std::vector<int32_t>> lv_all(M.levels), lv_small(M.levels), lv_large(M.levels), lv_ea(M.levels);
     for (int32_t id = 0; id < nf; ++id) {
         const int h = M.height[id];
-        lv_all[h].push_back(id);
+        if (solve) lv_all[h].push_back(id);
         if (M.child_off[id + 1] > M.child_off[id]) lv_ea[h].push_back(id);
         (M.s[id] + M.u[id] <= MF_SMEM_F ? lv_small : lv_large)[h].push_back(id);
     }
@@ -988,7 +988,6 @@ void MfFactor::setup(const MfSymbolic &sym, cudaStream_t st)
     j2pos_ = b32 + a_jp;
     poff_ = b32 + a_po;
     foff_ = b64 + a_fo;
-    // shared memory of the solve kernels, set here: solve() runs inside graph captures
     d_F_.resize(M.elems);
     d_w_.resize(std::max<int64_t>(M.welems, 1));
     // scratch of the split fronts' partial sums (both solves), zeroed counters
@@ -1078,7 +1077,7 @@ void MfFactor::setup_dense(const std::vector<int32_t> &off, const std::vector<in
         ++M.nfront;
     }
     M.levels = M.nfront ? 1 : 0;
-    setup(M, s);  // no front storage of its own: the blocks are swept where they lie
+    setup(M, s, false);  // no front storage of its own: the blocks are swept where they lie
 }
 
 void MfFactor::invert_dense(double *inv, int *bad, cudaStream_t s)

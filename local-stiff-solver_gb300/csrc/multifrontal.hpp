@@ -93,7 +93,8 @@ struct MfView {
 // per-level work lists of every kernel.
 class MfFactor {
 public:
-    void setup(const MfSymbolic &sym, cudaStream_t s);  // uploads the plan
+    // uploads the plan; solve: with the solves' work lists
+    void setup(const MfSymbolic &sym, cudaStream_t s, bool solve = true);
     bool empty() const { return sym_.nfront == 0; }
     // numeric factorization (values of A in the permuted operator)
     void factorize(const BsrDev &A, const StiffDev &S, int *bad, cudaStream_t s);

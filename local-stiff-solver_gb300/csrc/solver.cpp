@@ -220,12 +220,6 @@ void HybridSolver::analyze(int32_t n, int64_t nnz, const int32_t *outer, const i
     memb_.nitem = (int64_t)cs_.item_seg.size() - 1;
     memb_.nchunk = (int64_t)cs_.chunk_item.size();
     memb_.nseg = (int64_t)cs_.seg_c0.size() - 1;
-    d_key_.clear();
-    d_ccnt_.clear();
-    d_cbase_.clear();
-    d_key_.resize(cs_.L);
-    d_ccnt_.resize(cs_.L);
-    d_cbase_.resize(cs_.L);
     mas_ = MasDev();
     mas_.L = cs_.L;
     mas_.bd = pat_.bd;
@@ -246,14 +240,14 @@ void HybridSolver::analyze(int32_t n, int64_t nnz, const int32_t *outer, const i
         voff += (int64_t)cs_.nbanks[l] * 32 * pat_.bd;
         mas_.boff[l] = boff;
         boff += cs_.nbanks[l];
-        if (l + 1 < cs_.L) {
-            d_key_[l].upload(cs_.key[l], stream_);
-            d_ccnt_[l].upload(cs_.ccnt[l], stream_);
-            d_cbase_[l].upload(cs_.cbase[l], stream_);
-            mas_.key[l] = d_key_[l].data();
-            mas_.ccnt[l] = d_ccnt_[l].data();
-            mas_.cbase[l] = d_cbase_[l].data();
-        }
+    }
+    if (cs_.L > 2) {  // level 1 -> 2, the only restriction by a launch of its own
+        d_key1_.upload(cs_.key[1], stream_);
+        d_ccnt1_.upload(cs_.ccnt[1], stream_);
+        d_cbase1_.upload(cs_.cbase[1], stream_);
+        mas_.key[1] = d_key1_.data();
+        mas_.ccnt[1] = d_ccnt1_.data();
+        mas_.cbase[1] = d_cbase1_.data();
     }
     mas_.ncoarse = boff;
     mas_.level_elems = voff;

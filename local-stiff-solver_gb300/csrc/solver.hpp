@@ -125,8 +125,8 @@ private:
     CoarseMembers memb_;
     DBuf<uint8_t> d_key0_, d_ccnt0_, d_uncoupled_;
     DBuf<int32_t> d_membl_;             // base-level items by coarse item (MasDev::memb)
-    std::vector<DBuf<uint8_t>> d_key_, d_ccnt_;
-    std::vector<DBuf<int32_t>> d_cbase_;
+    DBuf<uint8_t> d_key1_, d_ccnt1_;
+    DBuf<int32_t> d_cbase1_;
     DBuf<char> d_inv0_, d_invc_, d_v_, d_u_;
     DBuf<double> d_stagec_, d_cpartial_;  // coarse Galerkin staging, kept per pattern
     bool mas_fp32_ = false;
