@@ -35,8 +35,12 @@ struct PcgSum {
     int count = 1;
     int direct = 0;          // one part per CTA of the producing kernel
 };
-// consumers of at most two CTAs per SM add the parts themselves
-constexpr int64_t PCG_DIRECT_ROWS = 2 * 152 * 1024;
+// Up to this many rows the consumers add the parts themselves, above them the last
+// CTA of the producer does.  Measured, last CTA / consumers, us per iteration in FP64
+// and mixed: 81k DOFs 68 / 62 and 45 / 38, 207k 125 / 117 and 72 / 58, 311k 166 / 159
+// and 87 / 74, 648k 283 / 285 and 140 / 134.  The consumers' adds grow with their
+// CTAs; between 311k and 648k rows the line could lie higher, in FP64 not above.
+constexpr int64_t PCG_DIRECT_ROWS = 311296;
 
 inline int grid_for(long long work_items, int items_per_cta, int max_ctas)
 {

@@ -595,10 +595,11 @@ template <int BD>
 struct BankGroup {
     static constexpr int WB = BD == 3 ? 4 : BD, GB = 4 / WB;
 };
-// Stages of shared memory per CTA: with four of up to 20 KB, three CTAs per SM
-// keep nine groups in flight (two stages on six CTAs kept six: 147 us against
-// 122 us at 33k FP32 banks); the larger FP64 stages are bound by the FP64
-// pipe, where five one-stage CTAs cover each other's loads.
+// Stages of shared memory per CTA: two of up to 20 KB, a group's product beside
+// the next one's copy, in five CTAs per SM.  More stages leave fewer CTAs (FP32
+// level 0 of 3.0M / 648k DOFs with two, three, four stages: 100.5 / 24.7, 113 /
+// 28.2, 143 / 34.6 us).  The larger FP64 stages are bound by the FP64 pipe, where
+// five one-stage CTAs cover each other's loads.
 template <int BD, typename T, bool BF>
 constexpr int bank_stages()
 {

@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(256) spmv_alpha_kernel(BsrDev A, const double 
     put_sum(dot, gr, pap);
 }
 
-// The vector updates take VEC rows per thread, all loaded before any is stored
-// (their stores keep the compiler from hoisting the next row's loads).
+// update_p_kernel takes VEC rows per thread, all loaded before any is stored (its
+// stores keep the compiler from hoisting the next row's loads).
 constexpr int VEC = 4, VEC_ROWS = 256 * VEC;
 
 __device__ __forceinline__ double as_double(double v) { return v; }
