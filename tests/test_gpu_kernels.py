@@ -253,3 +253,73 @@ def test_restart_leaves_no_residual_rounding(seed, precision, built):
     z = y.astype(np.float64)
     rounding = lu.solve(((b - A @ z) - residual(z.astype(np.longdouble))).astype(np.float64))
     assert np.linalg.norm(x - z) <= 0.1 * np.linalg.norm(rounding)
+
+
+@pytest.mark.parametrize("bs", [1, 2, 3])
+def test_mas_apply_two_restriction_launches(bs, built):
+    """MAS with more than 2048 level-1 items, whose levels above 2 are summed from
+    level 2, against the CPU restatement as above (the same kind of system, the
+    same bounds)."""
+    import lss
+    from oracle import oracle as O
+    nb = 9000
+    A = block_system(nb, bs, seed=nb + bs, isolated=3000)
+    items = lss.coarse_space(A, bs)[0]
+    assert items[1] > 2048 and len(items) > 3
+    r = np.random.default_rng(nb).standard_normal(A.shape[0])
+    zo = None
+    for precision, tol in (("fp64", 1e-12), ("mixed", 1e-4)):
+        s = make_solver(bs, precision, do_hybrid_precond=False)
+        s.factorize(A)
+        if zo is None:
+            perm, offs = s.partition()
+            zo = O.CpuSolver(A, {"block_size": bs, "do_hybrid_precond": False}, perm=perm, part_offsets=offs).precond(r)
+        z = s.mas_apply(r)
+        s.close()
+        assert np.linalg.norm(z - zo) <= tol * np.linalg.norm(zo), precision
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("bs,nb", [(1, 600_000), (3, 295_000)])
+def test_iterations_of_large_systems(bs, nb, precision, built):
+    """Four iterations as above where the scalars' sums are finished by the last
+    CTA (more than 311,296 rows) and the CTAs of the update and of the restriction
+    take several partitions in turn (more than 19,456 and 9,728)."""
+    A = block_system(nb, bs, seed=bs)
+    b = np.random.default_rng(nb).standard_normal(A.shape[0])
+    s = make_solver(bs, precision, do_hybrid_precond=False, max_iter=4)
+    s.factorize(A)
+    assert len(s.partition()[1]) - 1 > (19_456 if bs == 1 else 9_728)
+    x = s.solve(b)
+    assert s.get_info()["num_iterations"] == 4
+    y, r, p, rz = np.zeros_like(b), b.copy(), 0.0, 1.0
+    for _ in range(4):
+        z = s.precond(r)
+        p, rz = z + (r @ z / rz) * p, r @ z
+        q = A.T @ p
+        alpha = rz / (p @ q)
+        y, r = y + alpha * p, r - alpha * q
+    s.close()
+    assert np.linalg.norm(x - y) <= (1e-8 if precision == "fp64" else 1e-5) * np.linalg.norm(y)
+
+
+def test_stiff_apply_of_many_subdomains(built):
+    """A_SS^-1 r on 40 stiff pieces of 1,200 DOFs with fronts of up to 440 rows:
+    levels of thousands of CTAs at 64 rows, taken in chunks of 512 with more rows
+    than a CTA has threads.  Bounds as above."""
+    import scipy.sparse.linalg as spla
+    A = block_system(20000, 3, seed=9, reach=12)
+    nodes = np.concatenate([np.arange(500 * k, 500 * k + 400) for k in range(40)])
+    dofs = (3 * nodes[:, None] + np.arange(3)).ravel()
+    s = make_solver(3, extra={"composition": "additive"}, select_bad_dofs_from_l1_norm=False,
+                    decompose_subdomains=False, expand_subdomains=False)
+    s.set_problematic_dofs(dofs)
+    s.factorize(A)
+    info = s.get_info()
+    assert info["multifrontal_subdomains"] == 40 and info["multifrontal_max_front"] > 256, info
+    r = np.random.default_rng(9).standard_normal(A.shape[0])
+    z = s.mas_apply(r)
+    d = s.precond(r) - z
+    s.close()
+    x = spla.splu(A[dofs][:, dofs].tocsc()).solve(r[dofs], trans="T")
+    assert np.linalg.norm(d[dofs] - x) <= 1e-12 * (np.linalg.norm(x) + np.linalg.norm(z[dofs]))
